@@ -345,9 +345,12 @@ int obs_points_affect_points(obs_context* ctx, int core, int result, int accum, 
   if (!e) e = h2d(dsy, sy, S);
   if (!e && sr) e = h2d(dsr, sr, S);
   if (!e) e = h2d(dss, ss, S);
-  if (!e) e = h2d(dtx, tx, T);
-  if (!e) e = h2d(dty, ty, T);
-  if (!e && tr) e = h2d(dtr, tr, T);
+  // one set on itself (the same arrays): one device copy, which the pair-symmetric sum asks for
+  const bool self = ns == nt && tx == sx && ty == sy && tr == sr;
+  if (self) { dtx = dsx; dty = dsy; dtr = dsr; }
+  if (!e && !self) e = h2d(dtx, tx, T);
+  if (!e && !self) e = h2d(dty, ty, T);
+  if (!e && !self && tr) e = h2d(dtr, tr, T);
   if (!e && vel) e = h2d(dtu, tu, T);
   if (!e && vel) e = h2d(dtv, tv, T);
   for (int k = 0; k < nextra && !e; ++k) e = h2d(dex[k], extra[k], T);

@@ -128,6 +128,10 @@ int run_p2p(obs_context* ctx, const P2PRequest& rq) {
   const bool thick = rq.tr != nullptr;
   const bool comp = rq.accum == OBS_COMPENSATED;
   if (rq.ns == 0 || rq.nt == 0) return OBS_OK;
+  if (p2p_sym_applies(ctx, rq)) {
+    const int s = run_p2p_sym(ctx, rq);
+    if (s != OBS_ERR_ALLOC) return s;             // no room for its partials: the one-sided sum below
+  }
   const int res = rq.result;
   const int kcore = (res == RES_PSI) ? CORE_RM : rq.core;
   cudaStream_t st = ctx->stream;

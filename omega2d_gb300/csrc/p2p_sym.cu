@@ -1,0 +1,224 @@
+// p2p_sym.cu -- launch planning of the self-interaction sums that evaluate each unordered pair
+// once (p2p_sym.cuh), their packing and the reduction of their partials.
+#include <algorithm>
+#include <cstring>
+
+#include "obs_context.h"
+#include "p2p_sym.cuh"
+
+namespace obs {
+
+namespace {
+
+// Particles in groups of 32 in processing order, padded to whole row blocks with far particles of
+// zero strength, and the radius extrema (meta[0] = ~min, meta[1] = max bits).
+__global__ void sym_pack_kernel(const float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ r,
+                                const float* __restrict__ g, const int* __restrict__ perm, int n, int npad, int core,
+                                SymGroup* __restrict__ out, unsigned* __restrict__ meta) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  int j = (i < n && perm) ? perm[i] : i;
+  if ((unsigned)j >= (unsigned)n) j = 0;          // never taken for i < n: perm is a permutation
+  const float rr = (i < n && r) ? r[j] : 0.0f;
+  if (i < npad) {
+    const bool real = i < n;
+    const float X = real ? x[j] : SYM_FAR, Y = real ? y[j] : SYM_FAR;
+    const float G = real ? g[j] : 0.0f, z = real ? radius_term(core, rr) : 1.0f;
+    SymGroup& o = out[i / SYM_GRP];
+    o.xy[i % SYM_GRP] = make_float4(X, X, Y, Y);
+    o.g[i % SYM_GRP] = make_float2(G, G);
+    o.z[i % SYM_GRP] = make_float2(z, z);
+  }
+  unsigned rmin = (i < n) ? __float_as_uint(rr) : ~0u;
+  unsigned rmax = (i < n) ? __float_as_uint(rr) : 0u;
+  int any = (i < n) ? 1 : 0;
+  for (int o = 16; o > 0; o >>= 1) {
+    rmin = min(rmin, __shfl_xor_sync(0xffffffffu, rmin, o));
+    rmax = max(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
+    any |= __shfl_xor_sync(0xffffffffu, any, o);
+  }
+  if ((threadIdx.x & 31) == 0 && any) {
+    atomicMax(&meta[0], ~rmin);
+    atomicMax(&meta[1], rmax);
+  }
+}
+
+__device__ __forceinline__ void df_add(float& hi, float& lo, float bh, float bl) {
+  two_sum_acc(hi, lo, bh);
+  lo += bl;
+}
+
+// Adds a particle's partials of this pass (its row block's pieces, then the row blocks before its
+// own, each in order) to its running sum; the last pass stores the result.  A block takes 64
+// particles; four threads share one, each every fourth partial, added up in thread order.
+constexpr int SYM_RED_T = 64, SYM_RED_SUB = 4;
+__global__ void __launch_bounds__(SYM_RED_T * SYM_RED_SUB) sym_reduce_kernel(const SymArgs a, const P2PArgs o) {
+  __shared__ float4 red[SYM_RED_SUB][SYM_RED_T];
+  const int l = threadIdx.x % SYM_RED_T, sub = threadIdx.x / SYM_RED_T;
+  const int j = blockIdx.x * SYM_RED_T + l;
+  const int jb = j / SYM_ROWS;                     // the particle's row block (the same for all of a block)
+  float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  if (j < a.n) {
+    const int k = jb - a.blk0;
+    if (k >= 0 && k < a.nblk) {
+      // the pieces of row block k: ranges r0 .. r1 hold its units
+      const int p0 = sym_prefix(a, k), p1 = sym_prefix(a, k + 1) - 1;
+      int r0 = (int)((long long)p0 * a.nrange / a.total), r1 = (int)((long long)p1 * a.nrange / a.total);
+      while (sym_range_begin(a, r0 + 1) <= p0) ++r0;
+      while (sym_range_begin(a, r0) > p0) --r0;
+      while (sym_range_begin(a, r1 + 1) <= p1) ++r1;
+      while (sym_range_begin(a, r1) > p1) --r1;
+      const float2* rp = a.rowpart + (size_t)k * 2 * SYM_ROWS + (j - jb * SYM_ROWS);
+#pragma unroll 4
+      for (int r = r0 + sub; r <= r1; r += SYM_RED_SUB) {
+        const float2 u = __ldcg(rp + (size_t)r * 2 * SYM_ROWS), v = __ldcg(rp + (size_t)r * 2 * SYM_ROWS + SYM_ROWS);
+        df_add(s.x, s.y, u.x, u.y);
+        df_add(s.z, s.w, -v.x, -v.y);
+      }
+    }
+    const int kc = min(a.nblk, jb - a.blk0);       // row blocks of this pass before the particle's own
+    const float2* cp = a.colpart + j;
+#pragma unroll 8
+    for (int m = sub; m < kc; m += SYM_RED_SUB) {
+      const float2 c = __ldcg(cp + (size_t)m * a.npad);
+      two_sum_acc(s.x, s.y, -c.x);
+      two_sum_acc(s.z, s.w, c.y);
+    }
+  }
+  red[sub][l] = s;
+  __syncthreads();
+  if (sub != 0 || j >= a.n) return;
+  for (int q = 1; q < SYM_RED_SUB; ++q) {
+    const float4 t = red[q][l];
+    df_add(s.x, s.y, t.x, t.y);
+    df_add(s.z, s.w, t.z, t.w);
+  }
+  if (!a.first) {
+    const float4 t = a.run[j];
+    df_add(s.x, s.y, t.x, t.y);
+    df_add(s.z, s.w, t.z, t.w);
+  }
+  if (!a.last) {
+    a.run[j] = s;
+    return;
+  }
+  const double c[2] = {(double)s.x + (double)s.y, (double)s.z + (double)s.w};
+  store_target<RES_VEL>(o, j, c);
+}
+
+template <int CORE>
+cudaError_t sym_launch(bool comp, const SymArgs& a, int grid, cudaStream_t st) {
+  if (comp) p2p_sym_kernel<CORE, true><<<grid, SYM_THREADS, 0, st>>>(a);
+  else p2p_sym_kernel<CORE, false><<<grid, SYM_THREADS, 0, st>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t sym_dispatch(int core, bool comp, const SymArgs& a, int grid, cudaStream_t st) {
+  switch (core) {
+    case CORE_RM: return sym_launch<CORE_RM>(comp, a, grid, st);
+    case CORE_GAUSS: return sym_launch<CORE_GAUSS>(comp, a, grid, st);
+    case CORE_V2: return sym_launch<CORE_V2>(comp, a, grid, st);
+    case CORE_WL: return sym_launch<CORE_WL>(comp, a, grid, st);
+    case CORE_V3: return sym_launch<CORE_V3>(comp, a, grid, st);
+    case CORE_SING: return sym_launch<CORE_SING>(comp, a, grid, st);
+    case CORE_CEXP: return sym_launch<CORE_CEXP>(comp, a, grid, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+constexpr int SYM_OCC = 4;                            // CTAs per SM (__launch_bounds__: 128 registers)
+constexpr size_t SYM_COL_BYTES = (size_t)1 << 30;     // column partials held at once
+
+}  // namespace
+
+// One set as sources and targets (the same arrays) with two-radius cores: every size.  Measured
+// against the one-sided kernels (compensated, uniform clouds, calls back to back): 300 particles
+// 31 vs 48 us (both at the host's rate of issue), 1,200 31 vs 63, 7,000 52 vs 55 (its least
+// gain: hardly more units than CTA slots), 20,000 Rosenhead-Moore 114 vs 163, 65,536 Vatistas-2
+// 962 vs 1216, with varying radii 987 vs 1475; the 1M Gaussian patch 195 vs 249 ms.  An order or
+// kernel variant asked for by name keeps the one-sided kernels.
+bool p2p_sym_applies(const obs_context* ctx, const P2PRequest& rq) {
+  if (rq.result != RES_VEL || ctx->kernel_variant != OBS_VARIANT_AUTO || ctx->target_order != OBS_ORDER_AUTO) return false;
+  if (rq.ns != rq.nt || rq.sx != rq.tx || rq.sy != rq.ty) return false;
+  if (rq.core != CORE_SING && (!rq.tr || rq.tr != rq.sr)) return false;
+  return true;
+}
+
+int run_p2p_sym(obs_context* ctx, const P2PRequest& rq) {
+  const int n = rq.nt;
+  const bool comp = rq.accum == OBS_COMPENSATED;
+  cudaStream_t st = ctx->stream;
+  const int nblk = (n + SYM_ROWS - 1) / SYM_ROWS;
+  const int npad = nblk * SYM_ROWS;
+  const int ngrp = (n + SYM_GRP - 1) / SYM_GRP;
+  const int slots = SYM_OCC * ctx->num_sms;
+  const bool binned = (rq.core == CORE_GAUSS || rq.core == CORE_CEXP) && (double)n * n >= 3e8;
+  const int pass_blk = std::min(nblk, std::max(1, (int)(SYM_COL_BYTES / ((size_t)npad * sizeof(float2)))));
+  const int max_range = 8 * slots;
+
+  auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
+  const size_t hdr = 256;
+  const size_t o_pts = hdr;
+  const size_t o_run = o_pts + (size_t)(npad / SYM_GRP) * sizeof(SymGroup);
+  const size_t o_col = o_run + (pass_blk < nblk ? al((size_t)npad * sizeof(float4)) : 0);
+  const size_t o_row = o_col + al((size_t)pass_blk * npad * sizeof(float2));
+  const size_t o_perm = o_row + (size_t)(max_range + pass_blk) * 2 * SYM_ROWS * sizeof(float2);
+  const size_t o_sort = o_perm + (binned ? al((size_t)n * sizeof(int)) : 0);
+  const size_t bytes = o_sort + (binned ? bin_scratch_bytes(n) : 0);
+  int s = ctx->work.ensure(bytes, st);
+  if (s) return s;
+  WorkHeader* h = ctx->work.as<WorkHeader>(0);
+  int* perm = binned ? ctx->work.as<int>(o_perm) : nullptr;
+
+  timing_begin(ctx);
+  cudaError_t e = cudaMemsetAsync(h, 0, sizeof(WorkHeader), st);
+  int nl = 0;
+  if (e == cudaSuccess && binned) e = bin_order(rq.sx, rq.sy, n, ctx->work.as<char>(o_sort), perm, st, &nl);
+  if (e != cudaSuccess) return cuda_status(e);
+  sym_pack_kernel<<<(npad + 255) / 256, 256, 0, st>>>(rq.sx, rq.sy, rq.sr, rq.ss, perm, n, npad, rq.core,
+                                                      ctx->work.as<SymGroup>(o_pts), h->meta);
+  ctx->launches += nl + 1;
+  if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e);
+
+  SymArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.grp = ctx->work.as<SymGroup>(o_pts);
+  a.n = n; a.npad = npad; a.ngrp = ngrp;
+  a.counter = &h->counter;
+  a.meta = h->meta;
+  a.status = ctx->d_status;
+  a.colpart = ctx->work.as<float2>(o_col);
+  a.rowpart = ctx->work.as<float2>(o_row);
+  a.run = ctx->work.as<float4>(o_run);
+  P2PArgs o;
+  std::memset(&o, 0, sizeof(o));
+  o.nt = n;
+  o.perm = perm;
+  o.out[0] = rq.tu; o.out[1] = rq.tv;
+  o.finalize = (rq.flags & OBS_FLAG_FINALIZE) ? 1 : 0;
+  o.fsx = rq.fsx; o.fsy = rq.fsy;
+
+  timing_main_begin(ctx);
+  for (int b = 0; b < nblk; b += pass_blk) {
+    a.blk0 = b;
+    a.nblk = std::min(pass_blk, nblk - b);
+    a.first = b == 0;
+    a.last = b + a.nblk == nblk;
+    const int K = a.nblk;
+    a.total = K * (ngrp - SYM_GPB * b) - (SYM_GPB / 2) * K * (K - 1);
+    // one range per resident CTA for small sets; up to eight (32 units or more each) for large
+    // ones, whose units differ in cost (near and far column groups)
+    const int per = a.total / slots;
+    a.nrange = std::min(a.total, slots * std::min(8, std::max(1, per / 32)));
+    if (!a.first && (e = cudaMemsetAsync(&h->counter, 0, sizeof(int), st)) != cudaSuccess) return cuda_status(e);
+    if ((e = sym_dispatch(rq.core, comp, a, std::min(a.nrange, slots), st)) != cudaSuccess) return cuda_status(e);
+    if (a.last) timing_main_end(ctx);
+    // particles before this pass's first row block take nothing from it
+    sym_reduce_kernel<<<(n + SYM_RED_T - 1) / SYM_RED_T, SYM_RED_T * SYM_RED_SUB, 0, st>>>(a, o);
+    ctx->launches += 2;
+    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e);
+  }
+  timing_end(ctx);
+  return OBS_OK;
+}
+
+}  // namespace obs

@@ -1,0 +1,336 @@
+// p2p_sym.cuh -- velocity of a particle set on itself, each unordered pair evaluated once.
+//
+// points_affect_points with one set as sources and targets (src/Influence.h:56-416): the core
+// K(d^2) of a pair is the same for both particles, so one evaluation serves the two interactions
+//   row a <- column b:  u_a += G_b K (y_b - y_a),  v_a -= G_b K (x_b - x_a)
+//   column b <- row a:  u_b -= G_a K (y_b - y_a),  v_b += G_a K (x_b - x_a)
+// which is 10 f32x2 operations and one reciprocal (or square root) per two interactions, where
+// the one-sided kernel (p2p_packed.cuh) spends 14 and two.  Bound: the registers' read ports.  An
+// f32x2 operation takes 2.1 SM clocks per scheduler with one or two distinct register operands
+// and 3.1 with three (measured; two scalar FMAs in its place take as long), so the four
+// accumulations of a pair of pairs cost half of its 24 clocks; MUFU is at 50 %, the FMA pipe at
+// 67 %.  Other orders and groupings of the same operations, the accumulations as scalars, and 16
+// to 48 rows per thread pair all came within 5 % of one another.  Measured (compensated, one-sided
+// -> here): 1M Gaussian patch 249 -> 196 ms (5.1e12 interactions/s), 131,072 Vatistas-2 plain 4.29
+// -> 3.43 ms, 33,001 Vatistas-2 with varying radii 415 -> 298 us, ten Euler steps of 20,000
+// Rosenhead-Moore 1.65 -> 1.19 ms.
+//
+// Layout: a row block is 1024 particles, eight per thread of a 128-thread CTA in f32x2 register
+// pairs (a warp owns 256 consecutive ones); columns are taken 32 at a time, one per lane: in
+// step s of 32 lane l meets column l ^ s (a conflict-free shared-memory read) with its eight
+// rows, and the column's running sum (the eight terms added first) moves to the lane that meets it next by shuffle, so after 32
+// steps every lane holds its own column's sum over the warp's 256 rows.  The four warps' sums are
+// added in shared memory and leave as one FP32 pair per (row block, column); a row's own sums
+// stay in registers over a whole run of columns (folded into two-sum pairs every 32 columns when
+// compensated).  Rows against their own block are one-sided.
+//
+// Work: row block k meets every 32-column group from its own first one on; these (block, group)
+// units in order form a line of `total` units cut into equal ranges that the CTAs take from a
+// counter.  A range may cross blocks; each (range, block) piece writes one row partial at slot
+// range + block (strictly increasing along the line, so unique).  sym_reduce_kernel adds a
+// particle's row partials and column partials in a fixed order: results do not depend on timing.
+// Column partials take 8 bytes per (row block, particle); large sets run in passes over the row
+// blocks that keep them within a fixed scratch size.
+#pragma once
+
+#include "p2p_kernel.cuh"
+
+namespace obs {
+
+constexpr int SYM_THREADS = 128;
+constexpr int SYM_NP = 4;                          // f32x2 row pairs per thread
+constexpr int SYM_ROWS = SYM_THREADS * 2 * SYM_NP; // 1024 rows per block
+constexpr int SYM_WROWS = 64 * SYM_NP;             // rows per warp
+constexpr int SYM_GRP = 32;                        // columns per group
+constexpr int SYM_TG = 8;                          // groups per staged tile
+constexpr int SYM_TILE = SYM_GRP * SYM_TG;
+constexpr int SYM_GPB = SYM_ROWS / SYM_GRP;        // groups per row block
+constexpr float SYM_FAR = 1.0e18f;                 // padding coordinate: K there is finite and tiny
+
+// A group's 32 columns as staged, every value twice for the packed operands: a warp's reads of
+// column (lane ^ s) touch each bank once.
+struct __align__(128) SymGroup {
+  float4 xy[SYM_GRP];      // (x, x, y, y)
+  float2 g[SYM_GRP];       // strength
+  float2 z[SYM_GRP];       // radius term
+};
+static_assert(sizeof(SymGroup) == 1024, "group record");
+
+struct SymArgs {
+  const SymGroup* grp;     // the particles in groups of 32, padded to whole row blocks
+  int n;                 // particles
+  int npad;              // nblk * SYM_ROWS
+  int ngrp;              // 32-column groups holding a particle
+  int blk0, nblk;        // row blocks of this pass
+  int total;             // (block, group) units of this pass
+  int nrange;
+  int* counter;
+  const unsigned* meta;  // radius extrema (~min, max bits)
+  int* status;
+  float2* colpart;       // [nblk][npad] (sum G K dy, sum G K dx)
+  float2* rowpart;       // [nrange + nblk][2][SYM_ROWS] (hi, lo)
+  float4* run;           // [npad] running sums (u hi, u lo, v hi, v lo) over the passes
+  int first, last;       // first / last pass
+};
+
+// units of the pass before row block k (of the pass)
+__device__ __forceinline__ int sym_prefix(const SymArgs& a, int k) {
+  return k * (a.ngrp - SYM_GPB * a.blk0) - (SYM_GPB / 2) * k * (k - 1);
+}
+__device__ __forceinline__ int sym_range_begin(const SymArgs& a, int r) {
+  return (int)((long long)a.total * r / a.nrange);
+}
+
+struct SymUni {
+  float us2, ucf, cfl, lim;
+};
+
+// K of two pairs from d^2 (Rosenhead-Moore: from d^2 + s^2); zz: the pairs' radius terms summed (uniform radii: one constant).  FORM 0: the
+// far form 1/d^2 of the Gaussian and compact exponential cores; 1: the core with one radius for
+// all; 2: the core with every particle's own radius.
+template <int CORE, int FORM>
+__device__ __forceinline__ float2 sym_core(float2 d2, float2 zz, const SymUni& q) {
+  const float2 one = f2(1.0f, 1.0f), m1 = f2(-1.0f, -1.0f);
+  if constexpr (FORM == 0) {
+    return f2(rcp_a(d2.x), rcp_a(d2.y));
+  } else if constexpr (CORE == CORE_RM) {
+    return f2(rcp_a(d2.x), rcp_a(d2.y));
+  } else if constexpr (CORE == CORE_V2) {
+    const float2 w = __ffma2_rn(d2, d2, zz);
+    return f2(rsqrt_a(w.x), rsqrt_a(w.y));
+  } else if constexpr (CORE == CORE_WL) {
+    const float2 dd = __fadd2_rn(d2, zz);
+    const float2 w = __fmul2_rn(dd, dd);
+    return __fmul2_rn(__fadd2_rn(dd, zz), f2(rcp_a(w.x), rcp_a(w.y)));
+  } else if constexpr (CORE == CORE_V3) {
+    const float2 w = __ffma2_rn(__fmul2_rn(d2, d2), d2, zz);
+    return f2(ex2_a(lg2_a(w.x) * (-1.0f / 3.0f)), ex2_a(lg2_a(w.y) * (-1.0f / 3.0f)));
+  } else if constexpr (CORE == CORE_SING) {
+    return f2(d2.x > 0.0f ? rcp_a(d2.x) : 0.0f, d2.y > 0.0f ? rcp_a(d2.y) : 0.0f);
+  } else {
+    const float2 cf = (FORM == 1) ? f2(q.ucf, q.ucf) : f2(rcp_a(zz.x), rcp_a(zz.y));
+    const float2 ood2 = f2(rcp_a(d2.x), rcp_a(d2.y));
+    if constexpr (CORE == CORE_GAUSS) {
+      // x = d^2/s^2 > 16: 1/d^2; x < 0.001: 1/s^2; else (1 - e^-x)/d^2, on t = -x log2(e)
+      const float2 t = (FORM == 1) ? __fmul2_rn(d2, f2(q.cfl, q.cfl)) : __fmul2_rn(__fmul2_rn(d2, cf), f2(-kLog2e, -kLog2e));
+      const float2 e = f2(ex2_a(t.x), ex2_a(t.y));
+      float2 k = __fmul2_rn(ood2, __ffma2_rn(e, m1, one));
+      k.x = (t.x < -16.0f * kLog2e) ? ood2.x : ((t.x > -0.001f * kLog2e) ? cf.x : k.x);
+      k.y = (t.y < -16.0f * kLog2e) ? ood2.y : ((t.y > -0.001f * kLog2e) ? cf.y : k.y);
+      return k;
+    } else {
+      // compact exponential, y = (d/s)^3 > 16: 1/d^2; y < 0.001: (d/s^3)(1 - y/2); else (1 - e^-y)/d^2
+      const float2 x = __fmul2_rn(d2, cf);
+      const float2 sq = f2(sqrt_a(x.x), sqrt_a(x.y));
+      const float2 y = __fmul2_rn(x, sq);
+      const float2 t = __fmul2_rn(y, f2(-kLog2e, -kLog2e));
+      const float2 e = f2(ex2_a(t.x), ex2_a(t.y));
+      float2 k = __fmul2_rn(ood2, __ffma2_rn(e, m1, one));
+      k.x = (y.x > 16.0f) ? ood2.x : k.x;
+      k.y = (y.y > 16.0f) ? ood2.y : k.y;
+      k.x = (y.x < 0.001f) ? sq.x * cf.x * fmaf(-0.5f, y.x, 1.0f) : k.x;
+      k.y = (y.y < 0.001f) ? sq.y * cf.y * fmaf(-0.5f, y.y, 1.0f) : k.y;
+      return k;
+    }
+  }
+}
+
+// one 32-column group against the warp's rows; cu, cv: the column sums, back at their own lane
+// at the end.  zrow: this thread's rows' radius terms in shared memory (FORM 2).
+template <int CORE, int FORM>
+__device__ __forceinline__ void sym_group(const SymGroup& grp, int lane, const SymUni& q,
+                                          const float2 (&nx)[SYM_NP], const float2 (&ny)[SYM_NP],
+                                          const float2 (&g)[SYM_NP], const float* __restrict__ zrow,
+                                          float2 (&u)[SYM_NP], float2 (&vn)[SYM_NP], float& cu, float& cv) {
+  cu = cv = 0.0f;
+#pragma unroll 4
+  for (int s = 0; s < SYM_GRP; ++s) {
+    float2 su = f2(0.0f, 0.0f), sv = f2(0.0f, 0.0f);   // this step's eight rows
+    const int col = lane ^ s;
+    const float4 c = grp.xy[col];
+    const float2 cx = f2(c.x, c.y), cy = f2(c.z, c.w), cg = grp.g[col];
+    float2 cz = f2(0.0f, 0.0f);
+    if constexpr (FORM == 2) cz = grp.z[col];
+#pragma unroll
+    for (int p = 0; p < SYM_NP; ++p) {
+      const float2 dx = __fadd2_rn(cx, nx[p]);
+      const float2 dy = __fadd2_rn(cy, ny[p]);
+      float2 zz = f2(q.us2, q.us2);
+      if constexpr (FORM == 2)
+        zz = __fadd2_rn(cz, f2(zrow[(2 * p) * SYM_THREADS], zrow[(2 * p + 1) * SYM_THREADS]));
+      // Rosenhead-Moore takes d^2 + s^2 in the same two operations
+      const float2 d2 = __ffma2_rn(dx, dx, CORE == CORE_RM ? __ffma2_rn(dy, dy, zz) : __fmul2_rn(dy, dy));
+      const float2 k = sym_core<CORE, FORM>(d2, zz, q);
+      const float2 rr = __fmul2_rn(cg, k), rc = __fmul2_rn(g[p], k);
+      u[p] = __ffma2_rn(rr, dy, u[p]);
+      vn[p] = __ffma2_rn(rr, dx, vn[p]);
+      su = (p == 0) ? __fmul2_rn(rc, dy) : __ffma2_rn(rc, dy, su);
+      sv = (p == 0) ? __fmul2_rn(rc, dx) : __ffma2_rn(rc, dx, sv);
+    }
+    // hand the column's sums to the lane that meets it next (after the last step: to its own)
+    const int m = (s ^ (s + 1)) & 31;
+    cu = __shfl_xor_sync(0xffffffffu, cu + (su.x + su.y), m);
+    cv = __shfl_xor_sync(0xffffffffu, cv + (sv.x + sv.y), m);
+  }
+}
+
+template <int CORE, bool COMP>
+__global__ void __launch_bounds__(SYM_THREADS, 4) p2p_sym_kernel(const SymArgs a) {
+  constexpr bool MASKED = CORE == CORE_GAUSS || CORE == CORE_CEXP;
+  __shared__ SymGroup tile[NSTAGE][SYM_TG];
+  __shared__ float2 csum[SYM_THREADS / 32][SYM_TILE];   // per-warp column sums of the tile
+  __shared__ float zrow[2 * SYM_NP * SYM_THREADS];
+  __shared__ __align__(8) uint64_t bar[NSTAGE];
+  __shared__ int s_range;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) {
+    for (int s = 0; s < NSTAGE; ++s) mbar_init(&bar[s], 1);
+    fence_mbar_init();
+  }
+  __syncthreads();
+  const bool unif = CORE == CORE_SING || ~a.meta[0] == a.meta[1];
+  SymUni q;
+  q.us2 = unif ? 2.0f * radius_term(CORE, __uint_as_float(a.meta[1])) : 0.0f;
+  q.ucf = __frcp_rn(q.us2);
+  q.cfl = -q.ucf * kLog2e;
+  // far when every pair has d^2/s^2 > 16 (Gaussian) or (d/s)^3 > 16 (compact exponential), 1 % margin
+  q.lim = (CORE == CORE_CEXP ? 6.4131f : 16.16f) * q.us2;
+
+  uint32_t kt = 0;                                 // tiles consumed: barrier phase
+  for (;;) {
+    if (tid == 0) s_range = atomicAdd(a.counter, 1);
+    __syncthreads();
+    const int range = *static_cast<volatile int*>(&s_range);
+    if (range >= a.nrange) break;
+    int pos = sym_range_begin(a, range);
+    const int end = sym_range_begin(a, range + 1);
+    int k = 0;
+    {
+      int hi = a.nblk - 1;                         // the block whose units hold pos
+      while (k < hi) {
+        const int m = (k + hi + 1) >> 1;
+        if (sym_prefix(a, m) <= pos) k = m;
+        else hi = m - 1;
+      }
+    }
+    for (; pos < end; ++k) {
+      const int kbeg = sym_prefix(a, k), kend = min(end, sym_prefix(a, k + 1));
+      const int blk = a.blk0 + k;
+      const int g0 = SYM_GPB * blk + (pos - kbeg);          // first column group of this piece
+      const int ng = kend - pos;
+      const int gdiag = SYM_GPB * (blk + 1);                // groups below this are the block's own
+      const int ntile = (ng + SYM_TG - 1) / SYM_TG;
+      pos = kend;
+      auto fetch = [&](int t, int st) {                     // thread 0
+        const int cnt = min(SYM_TG, ng - t * SYM_TG);
+        const uint32_t bytes = (uint32_t)(cnt * sizeof(SymGroup));
+        mbar_arrive_expect_tx(&bar[st], bytes);
+        bulk_g2s(&tile[st][0], a.grp + (g0 + t * SYM_TG), bytes, &bar[st]);
+      };
+      if (tid == 0) {
+        fence_proxy_async_smem();
+        for (int s = 0; s < NSTAGE && s < ntile; ++s) fetch(s, (kt + s) % NSTAGE);
+      }
+      float2 nx[SYM_NP], ny[SYM_NP], g[SYM_NP], u[SYM_NP], vn[SYM_NP], hu[SYM_NP], lu[SYM_NP], hv[SYM_NP], lv[SYM_NP];
+      float bx0 = 3.0e38f, bx1 = -3.0e38f, by0 = 3.0e38f, by1 = -3.0e38f;
+      const int row0 = blk * SYM_ROWS + warp * SYM_WROWS + lane;
+#pragma unroll
+      for (int p = 0; p < SYM_NP; ++p) {
+        float4 w[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          // the 32 rows of (p, h) are one group
+          const SymGroup& r = a.grp[blk * SYM_GPB + warp * (SYM_WROWS / 32) + 2 * p + h];
+          const float4 xy = r.xy[lane];
+          w[h] = make_float4(xy.x, xy.z, r.g[lane].x, r.z[lane].x);
+          if (row0 + (2 * p + h) * 32 < a.n) {
+            bx0 = fminf(bx0, w[h].x); bx1 = fmaxf(bx1, w[h].x);
+            by0 = fminf(by0, w[h].y); by1 = fmaxf(by1, w[h].y);
+          }
+          if (!unif) zrow[(2 * p + h) * SYM_THREADS + tid] = w[h].w;   // read by this thread alone
+        }
+        nx[p] = f2(-w[0].x, -w[1].x);
+        ny[p] = f2(-w[0].y, -w[1].y);
+        g[p] = f2(w[0].z, w[1].z);
+        u[p] = vn[p] = hu[p] = lu[p] = hv[p] = lv[p] = f2(0.0f, 0.0f);
+      }
+      if (MASKED) {
+        for (int o = 16; o > 0; o >>= 1) {
+          bx0 = fminf(bx0, __shfl_xor_sync(0xffffffffu, bx0, o));
+          bx1 = fmaxf(bx1, __shfl_xor_sync(0xffffffffu, bx1, o));
+          by0 = fminf(by0, __shfl_xor_sync(0xffffffffu, by0, o));
+          by1 = fmaxf(by1, __shfl_xor_sync(0xffffffffu, by1, o));
+        }
+      }
+      for (int t = 0; t < ntile; ++t, ++kt) {
+        const int st = kt % NSTAGE;
+        const bool ok = mbar_wait_bounded(&bar[st], (kt / NSTAGE) & 1u, WAIT_TRIES);
+        if (__syncthreads_or(!ok)) {
+          if (tid == 0) {
+            record_failure(a.status, DEV_ERR_TIMEOUT, 240 + st, (int)kt, range);
+            for (int s = 0; s < NSTAGE; ++s) (void)mbar_wait_bounded(&bar[(kt + s) % NSTAGE], ((kt + s) / NSTAGE) & 1u, WAIT_TRIES);
+          }
+          return;
+        }
+        const int cnt = min(SYM_TG, ng - t * SYM_TG);
+        for (int b = 0; b < cnt; ++b) {
+          const SymGroup& grp = tile[st][b];
+          float cu, cv;
+          if (!unif) {
+            sym_group<CORE, 2>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, cu, cv);
+          } else if constexpr (MASKED) {
+            const float4 c = grp.xy[lane];
+            const float ex = fmaxf(0.0f, fmaxf(bx0 - c.x, c.x - bx1));
+            const float ey = fmaxf(0.0f, fmaxf(by0 - c.z, c.z - by1));
+            // negated, so that a NaN coordinate takes the near form
+            if (__any_sync(0xffffffffu, !(fmaf(ex, ex, ey * ey) > q.lim)))
+              sym_group<CORE, 1>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, cu, cv);
+            else
+              sym_group<CORE, 0>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, cu, cv);
+          } else {
+            sym_group<CORE, 1>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, cu, cv);
+          }
+          csum[warp][b * SYM_GRP + lane] = make_float2(cu, cv);
+          if constexpr (COMP) {
+#pragma unroll
+            for (int p = 0; p < SYM_NP; ++p) {
+              two_sum2(hu[p], lu[p], u[p]);
+              two_sum2(hv[p], lv[p], vn[p]);
+              u[p] = vn[p] = f2(0.0f, 0.0f);
+            }
+          }
+        }
+        __syncthreads();                           // the tile is consumed, its column sums are complete
+        if (tid == 0 && t + NSTAGE < ntile) {
+          fence_proxy_async_smem();
+          fetch(t + NSTAGE, st);
+        }
+        // the next tile's sums are written after the barrier that opens it
+        const int c0 = (g0 + t * SYM_TG) * SYM_GRP;
+        for (int c = tid; c < cnt * SYM_GRP; c += SYM_THREADS) {
+          if (c0 + c < gdiag * SYM_GRP || c0 + c >= a.n) continue;
+          const float2 s0 = csum[0][c], s1 = csum[1][c], s2 = csum[2][c], s3 = csum[3][c];
+          a.colpart[(size_t)k * a.npad + c0 + c] = make_float2((s0.x + s1.x) + (s2.x + s3.x), (s0.y + s1.y) + (s2.y + s3.y));
+        }
+      }
+      float2* rp = a.rowpart + (size_t)(range + k) * 2 * SYM_ROWS;
+#pragma unroll
+      for (int p = 0; p < SYM_NP; ++p) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int i = warp * SYM_WROWS + (2 * p + h) * 32 + lane;
+          if (COMP) {
+            rp[i] = h ? make_float2(hu[p].y, lu[p].y) : make_float2(hu[p].x, lu[p].x);
+            rp[SYM_ROWS + i] = h ? make_float2(hv[p].y, lv[p].y) : make_float2(hv[p].x, lv[p].x);
+          } else {
+            rp[i] = make_float2(h ? u[p].y : u[p].x, 0.0f);
+            rp[SYM_ROWS + i] = make_float2(h ? vn[p].y : vn[p].x, 0.0f);
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+}
+
+}  // namespace obs

@@ -1,0 +1,55 @@
+"""GPU tests of the self-interaction sum that evaluates each unordered pair once (csrc/p2p_sym.cuh), at the edges of
+its 32-column groups and 1024-row blocks and over several passes, against the FP64 oracle and the one-sided kernels."""
+import numpy as np
+import pytest
+
+import omega2d_gb300 as og
+from conftest import rel_err
+
+pytestmark = pytest.mark.gpu
+
+CORES = [og.CORE_RM, og.CORE_GAUSSIAN, og.CORE_V2, og.CORE_WL, og.CORE_V3, og.CORE_SINGULAR, og.CORE_COMPACT_EXP]
+
+
+def cloud(n, seed, spread, rad=0.02):
+    rng = np.random.default_rng(seed)
+    x, y = rng.uniform(-1, 1, (2, n)).astype(np.float32)
+    r = (rad * rng.uniform(1 - spread, 1 + spread, n)).astype(np.float32)
+    return x, y, r, rng.normal(0, 1 / np.sqrt(n), n).astype(np.float32)
+
+
+def self_velocity(ctx, core, accum, x, y, r, s):
+    p = og.Points(x, y, r, s, u=np.full(x.size, 0.5, np.float32))
+    og.points_affect_points(p, p, og.VELONLY, og.ExecEnv(core, accum, ctx), finalize=True, fs=(1.0, -0.25))
+    return p.u, p.v
+
+
+# the tolerances of the packed kernels' tests: FP32 pairs with compensated or plain sums
+@pytest.mark.parametrize("core", CORES)
+@pytest.mark.parametrize("accum,tol", [(og.COMPENSATED, 2e-6), (og.PLAIN_F32, 2e-5)])
+@pytest.mark.parametrize("n,spread", [(1, 0.0), (2, 0.5), (33, 0.0), (1023, 0.5), (1025, 0.0), (2081, 0.5), (5121, 0.0)])
+def test_self_sum_matches_fp64(ctx, restatement, core, accum, tol, n, spread):
+    x, y, r, s = cloud(n, 7 * n + core, spread)
+    if n > 1024:                       # coincident particles, in one block and in two
+        x[5], y[5] = x[0], y[0]
+        x[n - 1], y[n - 1] = x[1], y[1]
+    u, v = self_velocity(ctx, core, accum, x, y, r, s)
+    u64, v64, _ = restatement.points_affect_points(core, 1, x, y, r, s, x, y, r, fp64=True, tu=np.full(n, 0.5),
+                                                   tv=np.zeros(n))
+    assert rel_err(1.0 + u64 / (2 * np.pi), u) < tol
+    assert rel_err(-0.25 + v64 / (2 * np.pi), v) < tol
+
+
+@pytest.mark.parametrize("core,n,spread", [(og.CORE_GAUSSIAN, 400_003, 0.0), (og.CORE_V2, 390_001, 0.5)])
+def test_several_passes_match_one_sided(ctx, core, n, spread):
+    """More row blocks than one pass holds: the running sums carry over, and a repeat gives the same bits."""
+    x, y, r, s = cloud(n, n, spread, 0.004)
+    u, v = self_velocity(ctx, core, og.COMPENSATED, x, y, r, s)
+    u2, v2 = self_velocity(ctx, core, og.COMPENSATED, x, y, r, s)
+    assert np.array_equal(u, u2) and np.array_equal(v, v2)
+    try:
+        ctx.set_kernel_variant(og.VARIANT_PACKED4)
+        uo, vo = self_velocity(ctx, core, og.COMPENSATED, x, y, r, s)
+    finally:
+        ctx.set_kernel_variant(og.VARIANT_AUTO)
+    assert rel_err(uo, u) < 2e-6 and rel_err(vo, v) < 2e-6
