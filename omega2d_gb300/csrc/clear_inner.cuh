@@ -144,15 +144,16 @@ OBS_HD void cut_entry(const Geo& g, float p, float& smult, float& dshift) {
 }
 
 // A lower bound, in FP32, on the squared distance seg_closest computes for one panel (its
-// exact float/double arithmetic).  The differences ax, ay, bx, by, the cross product c and the
-// dot product are formed exactly as seg_closest forms them, so they are the same floats; only
-// t = dot/blensq is taken as dot * ibl (ibl = 1/blensq in FP32, within a few ulps).  Where t is
-// at least 2^-20 inside (0, 1), seg_closest takes the panel case, c^2/blensq; where it is at
-// least 2^-20 outside, the node case, min(ax^2 + ay^2, ex^2 + ey^2) -- either way the FP32 value
-// is within a few ulps of seg_closest's double-then-float one, and (1 - 2^-20) times it bounds
-// that from below.  In the 2^-20 band around 0 and 1 the bound is the smaller of the two cases
-// (seg_closest's value is one of them).  Non-finite inputs give NaN or inf, which never reject.
-OBS_HD float seg_lower_bound(float x0, float y0, float x1, float y1, float ibl, float tx, float ty) {
+// exact float/double arithmetic), and an upper bound ub on it.  The differences ax, ay, bx, by,
+// the cross product c and the dot product are formed exactly as seg_closest forms them, so they
+// are the same floats; only t = dot/blensq is taken as dot * ibl (ibl = 1/blensq in FP32, within
+// a few ulps).  Where t is at least 2^-20 inside (0, 1), seg_closest takes the panel case,
+// c^2/blensq; where it is at least 2^-20 outside, the node case, min(ax^2 + ay^2, ex^2 + ey^2) --
+// either way the FP32 value is within a few ulps of seg_closest's double-then-float one, and
+// (1 -+ 2^-20) times it bounds that from below and above.  In the 2^-20 band around 0 and 1 the
+// bounds are the smaller and the larger of the two cases (seg_closest's value is one of them).
+// Non-finite inputs give NaN or inf, which never reject.
+OBS_HD float seg_bounds(float x0, float y0, float x1, float y1, float ibl, float tx, float ty, float& ub) {
   const float bx = x1 - x0, by = y1 - y0;
   const float ax = tx - x0, ay = ty - y0;
   const float t = (ax * bx + ay * by) * ibl;
@@ -164,7 +165,33 @@ OBS_HD float seg_lower_bound(float x0, float y0, float x1, float y1, float ibl, 
   const bool inside = t > eps && t < 1.0f - eps;
   const bool outside = t < -eps || t > 1.0f + eps;
   const float d = inside ? dp : (outside ? dn : fminf(dp, dn));
+  ub = (inside ? dp : (outside ? dn : fmaxf(dp, dn))) * 1.00000095367431640625f;
   return d * 0.99999904632568359375f;
+}
+
+// Panels are taken in groups of 32 consecutive ones; box = (xmin, ymin, xmax, ymax) of a group's
+// nodes.  The squared distance of a point to the box:
+constexpr int GROUP = 32;
+struct Box {
+  float x0, y0, x1, y1;
+};
+OBS_HD float box_dist2(const Box& b, float tx, float ty) {
+  const float dx = fmaxf(0.0f, fmaxf(b.x0 - tx, tx - b.x1));
+  const float dy = fmaxf(0.0f, fmaxf(b.y0 - ty, ty - b.y1));
+  return dx * dx + dy * dy;
+}
+
+// No panel of the box can be the closest or tie it when T bounds the squared minimum (root =
+// sqrt(T)).  For a panel of length |b| at true distance d, seg_closest's distance is at least
+// d - 2^-21 (d + |b|): the cross product is off by at most 2^-23 |a| |b|, |a| <= d + |b| where the
+// foot lies on the panel, and a foot misplaced past an end by the rounding of t moves it by at
+// most 2^-22 |a|.  The box is no farther than d and its sides together no shorter than |b|, so the
+// margins (2e-5 = 2^-15.6 of the distance, 5e-6 = 2^-17.6 of the sides) cover that and the rounding
+// here.  NaN or infinite operands reject nothing.
+OBS_HD bool box_beyond(const Box& b, float tx, float ty, float root) {
+  const float s = root * 1.00002f + ((b.x1 - b.x0) + (b.y1 - b.y0)) * 5.0e-6f;
+  const float d2 = box_dist2(b, tx, ty);
+  return d2 > (s * s) * 1.00002f && d2 <= 3.0e38f;
 }
 
 // bound > T (1 + 2^-16): the panel cannot be the closest or tie it when T bounds the minimum
@@ -241,39 +268,59 @@ OBS_HD int clear_apply(const Geo& g, const Closest& c, int method, float cutoff_
 // One point, tested until it passes (at most max_sweeps times), against all panels of g read
 // from its arrays.  rad = the point's core radius (ips for field points).  Returns the number
 // of modifications, or -1 when max_sweeps ran out; lost receives the circulation removed
-// (method 0).  Each sweep takes two passes: the panel with the smallest lower bound gives, by
-// its exact distance, a bound T on the minimum; then only panels whose lower bound does not
-// exceed T are evaluated exactly, in panel order.  The reference's hits are the panels at the
-// exact minimum (ties included, in panel order), which this reproduces bit for bit.  The CUDA
-// kernel runs the same passes over panel records staged in shared memory.
+// (method 0).  Each sweep bounds the squared minimum by T, the smallest upper bound in the group
+// whose box is nearest; then, in panel order, the groups whose box T does not reject are
+// entered (tightening T), and their panels whose lower bound T does not reject are evaluated
+// exactly.  The reference's hits are the panels at the exact minimum (ties included, in panel
+// order), which this reproduces bit for bit.  The CUDA kernel takes the same steps, a warp at a
+// time.
 OBS_HD int clear_point(const Geo& g, int method, float cutoff_mult, float ips, float rad, float& x, float& y,
                        float& s, double& lost, int max_sweeps) {
+  const int ng = (g.npan + GROUP - 1) / GROUP;
+  auto box_of = [&](int k) {
+    Box b{INFINITY, INFINITY, -INFINITY, -INFINITY};
+    const int j1 = (k + 1) * GROUP < g.npan ? (k + 1) * GROUP : g.npan;
+    for (int q = 2 * k * GROUP; q < 2 * j1; ++q) {
+      const float nx = g.nx[g.idx[q]], ny = g.ny[g.idx[q]];
+      b.x0 = fminf(b.x0, nx); b.x1 = fmaxf(b.x1, nx);
+      b.y0 = fminf(b.y0, ny); b.y1 = fmaxf(b.y1, ny);
+    }
+    return b;
+  };
+  auto bounds = [&](int j, float& ub) {
+    const unsigned a = g.idx[2 * j], b = g.idx[2 * j + 1];
+    const float bx = g.nx[b] - g.nx[a], by = g.ny[b] - g.ny[a];
+    return seg_bounds(g.nx[a], g.ny[a], g.nx[b], g.ny[b], 1.0f / (bx * bx + by * by), x, y, ub);
+  };
+  auto tighten = [&](int k, float T) {
+    for (int j = k * GROUP; j < (k + 1) * GROUP && j < g.npan; ++j) {
+      float ub;
+      (void)bounds(j, ub);
+      if (ub < T) T = ub;
+    }
+    return T;
+  };
   int crops = 0;
   lost = 0.0;
   for (int sweep = 0; sweep < max_sweeps; ++sweep) {
-    float lbmin = 3.4028234663852886e38f;
-    int jstar = -1;
-    for (int j = 0; j < g.npan; ++j) {
-      const unsigned a = g.idx[2 * j], b = g.idx[2 * j + 1];
-      const float bx = g.nx[b] - g.nx[a], by = g.ny[b] - g.ny[a];
-      const float lb = seg_lower_bound(g.nx[a], g.ny[a], g.nx[b], g.ny[b], 1.0f / (bx * bx + by * by), x, y);
-      if (lb < lbmin) { lbmin = lb; jstar = j; }
+    int k0 = 0;
+    float best = INFINITY;
+    for (int k = 0; k < ng; ++k) {
+      const float d = box_dist2(box_of(k), x, y);
+      if (d < best) { best = d; k0 = k; }
     }
-    float T = INFINITY;                           // no candidate: no rejection
-    if (jstar >= 0) {
-      const unsigned a = g.idx[2 * jstar], b = g.idx[2 * jstar + 1];
-      float cx, cy;
-      int kind, which;
-      seg_closest(g.nx[a], g.ny[a], g.nx[b], g.ny[b], x, y, T, cx, cy, kind, which);
-    }
+    float T = ng ? tighten(k0, INFINITY) : INFINITY;
     Closest c;
     closest_init(c);
-    for (int j = 0; j < g.npan; ++j) {
-      const unsigned a = g.idx[2 * j], b = g.idx[2 * j + 1];
-      const float x0 = g.nx[a], y0 = g.ny[a], x1 = g.nx[b], y1 = g.ny[b];
-      const float bx = x1 - x0, by = y1 - y0;
-      if (beyond(seg_lower_bound(x0, y0, x1, y1, 1.0f / (bx * bx + by * by), x, y), T)) continue;
-      closest_add(g, c, a, b, x0, y0, x1, y1, g.pnx[j], g.pny[j], x, y);
+    for (int k = 0; k < ng; ++k) {
+      if (box_beyond(box_of(k), x, y, sqrtf(T))) continue;
+      T = tighten(k, T);
+      for (int j = k * GROUP; j < (k + 1) * GROUP && j < g.npan; ++j) {
+        float ub;
+        if (beyond(bounds(j, ub), T)) continue;
+        const unsigned a = g.idx[2 * j], b = g.idx[2 * j + 1];
+        closest_add(g, c, a, b, g.nx[a], g.ny[a], g.nx[b], g.ny[b], g.pnx[j], g.pny[j], x, y);
+      }
     }
     const int r = clear_apply(g, c, method, cutoff_mult, ips, rad, x, y, s, lost);
     if (r != 1) return crops;
