@@ -56,22 +56,6 @@ struct AdjArgs {
   int direct;
 };
 
-// fold radius extrema as in p2p_host.cu
-__device__ __forceinline__ void fold_extrema2(bool active, float r, unsigned* meta) {
-  unsigned rmin = active ? __float_as_uint(r) : ~0u;
-  unsigned rmax = active ? __float_as_uint(r) : 0u;
-  int any = active ? 1 : 0;
-  for (int o = 16; o > 0; o >>= 1) {
-    rmin = min(rmin, __shfl_xor_sync(0xffffffffu, rmin, o));
-    rmax = max(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
-    any |= __shfl_xor_sync(0xffffffffu, any, o);
-  }
-  if ((threadIdx.x & 31) == 0 && any) {
-    atomicMax(&meta[0], ~rmin);
-    atomicMax(&meta[1], rmax);
-  }
-}
-
 // elements: (x, y, radius term, G) | (lam_u, lam_v, 0, 0); padded with zero cotangent and zero
 // strength at the origin with radius term 1 (finite for every core)
 __global__ void pack_adj_kernel(const float* __restrict__ x, const float* __restrict__ y,
@@ -87,12 +71,14 @@ __global__ void pack_adj_kernel(const float* __restrict__ x, const float* __rest
     out[2 * i] = make_float4(0.0f, 0.0f, 1.0f, 0.0f);
     out[2 * i + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   }
-  fold_extrema2(i < n && r != nullptr, rr, meta);
+  const bool real = i < n && r != nullptr;
+  fold_extrema_block(real ? __float_as_uint(rr) : ~0u, real ? __float_as_uint(rr) : 0u, meta);
 }
 
 __global__ void owner_meta_kernel(const float* __restrict__ r, int n, unsigned* __restrict__ meta) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  fold_extrema2(i < n, i < n ? r[i] : 0.0f, meta + 2);
+  const unsigned b = i < n ? __float_as_uint(r[i]) : 0u;
+  fold_extrema_block(i < n ? b : ~0u, b, meta + 2);
 }
 
 template <int CORE, int MODE, bool THICK, bool UNIF>

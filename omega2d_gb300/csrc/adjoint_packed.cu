@@ -60,21 +60,6 @@ struct PAArgs {
   int direct;
 };
 
-__device__ __forceinline__ void fold_radius(bool active, float r, unsigned* meta) {
-  unsigned rmin = active ? __float_as_uint(r) : ~0u;
-  unsigned rmax = active ? __float_as_uint(r) : 0u;
-  int any = active ? 1 : 0;
-  for (int o = 16; o > 0; o >>= 1) {
-    rmin = min(rmin, __shfl_xor_sync(0xffffffffu, rmin, o));
-    rmax = max(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
-    any |= __shfl_xor_sync(0xffffffffu, any, o);
-  }
-  if ((threadIdx.x & 31) == 0 && any) {
-    atomicMax(&meta[0], ~rmin);
-    atomicMax(&meta[1], rmax);
-  }
-}
-
 // elements in the (optionally permuted) order; padding: zero cotangent and strength at the
 // origin with radius term 1
 template <int MODE>
@@ -106,12 +91,14 @@ __global__ void pa_pack_kernel(const float* __restrict__ x, const float* __restr
     o[0] = o[1] = o[2] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     o[3] = make_float4(1.0f, 1.0f, 0.0f, 0.0f);
   }
-  fold_radius(i < n && r != nullptr, rr, meta);
+  const bool real = i < n && r != nullptr;
+  fold_extrema_block(real ? __float_as_uint(rr) : ~0u, real ? __float_as_uint(rr) : 0u, meta);
 }
 
 __global__ void pa_owner_meta_kernel(const float* __restrict__ r, int n, unsigned* __restrict__ meta) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  fold_radius(i < n, i < n ? r[i] : 0.0f, meta + 2);
+  const unsigned b = i < n ? __float_as_uint(r[i]) : 0u;
+  fold_extrema_block(i < n ? b : ~0u, b, meta + 2);
 }
 
 // owner constants of one register pair

@@ -5,8 +5,11 @@
 // apart than 4 core radii and take the reference's far-field form G/d^2 without an
 // exponential.  This file produces that order:
 //   1. bounding box of the points (order-preserving float keys, atomic max);
-//   2. 16-bit Morton key of each point's cell in a 256 x 256 grid over the box;
-//   3. stable LSD radix sort of (key, index) in two 8-bit passes: per-tile digit counts (and
+//   2. Morton key of each point's cell in a 256 x 256 grid over the box (16 bits), or its place
+//      along the Hilbert curve through 256 x 256 or 4096 x 4096 cells (16 or 24 bits), whose
+//      consecutive cells always touch, so that no run of points spans one of the Morton order's
+//      jumps;
+//   3. stable LSD radix sort of (key, index) in two or three 8-bit passes: per-tile digit counts (and
 //      digit totals), per-digit offsets over the tiles (one warp per digit), and a stable
 //      scatter whose in-tile ranks
 //      come from warp match + per-warp digit counts, so the order is a function of the input
@@ -20,12 +23,12 @@ namespace obs {
 
 namespace {
 
-constexpr int BIN_BITS = 8;                       // cells per axis: 256
+constexpr int RS_BITS = 8;                        // digit of a radix pass
 constexpr int RS_THREADS = 256;                   // = number of digits per pass
 constexpr int RS_CHUNKS = 4;
 constexpr int RS_TILE = RS_THREADS * RS_CHUNKS;   // points per radix tile
 constexpr int RS_WARPS = RS_THREADS / 32;
-constexpr int HDR_BYTES = 4096;                   // bb | digit totals of pass 1 | of pass 2
+constexpr int HDR_BYTES = 4096;                   // bb | digit totals of passes 1, 2, 3
 
 // order-preserving map of a float to an unsigned key (and back)
 __device__ __forceinline__ unsigned ord_key(float f) {
@@ -68,21 +71,44 @@ __device__ __forceinline__ unsigned spread8(unsigned v) {
   return v;
 }
 
-__device__ __forceinline__ unsigned cell_of(float v, float lo, float scale) {
-  const float c = fminf(fmaxf((v - lo) * scale, 0.0f), (float)((1 << BIN_BITS) - 1));   // NaN -> 0
+// place of cell (x, y) along the Hilbert curve of 2^bits x 2^bits cells: from the top bit down, the
+// quadrant's rank, then the quadrant turned into the curve's base orientation
+__device__ __forceinline__ unsigned hilbert_key(unsigned x, unsigned y, int bits) {
+  const unsigned top = (1u << bits) - 1u;
+  unsigned d = 0;
+  for (int b = bits - 1; b >= 0; --b) {
+    const unsigned rx = (x >> b) & 1u, ry = (y >> b) & 1u;
+    d = (d << 2) | ((3u * rx) ^ ry);
+    if (ry == 0u) {
+      if (rx) {
+        x = top - x;
+        y = top - y;
+      }
+      const unsigned t = x;
+      x = y;
+      y = t;
+    }
+  }
+  return d;
+}
+
+__device__ __forceinline__ unsigned cell_of(float v, float lo, float scale, float top) {
+  const float c = fminf(fmaxf((v - lo) * scale, 0.0f), top);   // NaN -> 0
   return (unsigned)c;
 }
 
 __global__ void bin_key_kernel(const float* __restrict__ x, const float* __restrict__ y, int n,
-                               const unsigned* __restrict__ bb, unsigned* __restrict__ keys) {
+                               const unsigned* __restrict__ bb, int bits, bool hilbert, unsigned* __restrict__ keys) {
+  const float cells = (float)(1 << bits);
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float x0 = ord_val(~bb[0]), x1 = ord_val(bb[1]);
   const float y0 = ord_val(~bb[2]), y1 = ord_val(bb[3]);
   const float wx = x1 - x0, wy = y1 - y0;
-  const float sx = (wx > 0.0f) ? (float)(1 << BIN_BITS) / wx : 0.0f;
-  const float sy = (wy > 0.0f) ? (float)(1 << BIN_BITS) / wy : 0.0f;
-  keys[i] = spread8(cell_of(x[i], x0, sx)) | (spread8(cell_of(y[i], y0, sy)) << 1);
+  const float sx = (wx > 0.0f) ? cells / wx : 0.0f;
+  const float sy = (wy > 0.0f) ? cells / wy : 0.0f;
+  const unsigned cx = cell_of(x[i], x0, sx, cells - 1.0f), cy = cell_of(y[i], y0, sy, cells - 1.0f);
+  keys[i] = hilbert ? hilbert_key(cx, cy, bits) : (spread8(cx) | (spread8(cy) << 1));
 }
 
 // digit counts of one tile: table[digit * ntiles + tile]; digit totals into tot[256] (zeroed)
@@ -196,13 +222,14 @@ size_t bin_scratch_bytes(int n) {
 }
 
 cudaError_t bin_order(const float* x, const float* y, int n, void* scratch, int* perm, cudaStream_t st,
-                      int* launches) {
+                      int* launches, BinCurve curve) {
   if (n <= 0) return cudaSuccess;
+  const int bits = curve == BIN_HILBERT12 ? 12 : 8;
   const int ntiles = (n + RS_TILE - 1) / RS_TILE;
+  const int passes = bits > RS_BITS ? 3 : 2;      // 2 * bits key bits
   char* p = static_cast<char*>(scratch);
   unsigned* bb = reinterpret_cast<unsigned*>(p);
-  unsigned* tot0 = reinterpret_cast<unsigned*>(p + 256);
-  unsigned* tot1 = tot0 + RS_THREADS;
+  unsigned* tot = reinterpret_cast<unsigned*>(p + 256);
   unsigned* table = reinterpret_cast<unsigned*>(p + HDR_BYTES);
   unsigned* ka = reinterpret_cast<unsigned*>(p + HDR_BYTES + al256(RS_THREADS * (size_t)ntiles * sizeof(unsigned)));
   unsigned* kb = ka + al256((size_t)n * sizeof(unsigned)) / sizeof(unsigned);
@@ -212,16 +239,20 @@ cudaError_t bin_order(const float* x, const float* y, int n, void* scratch, int*
   const int threads = 256;
   const int blocks = (n + threads - 1) / threads;
   bin_bbox_kernel<<<blocks < 512 ? blocks : 512, threads, 0, st>>>(x, y, n, bb);
-  bin_key_kernel<<<blocks, threads, 0, st>>>(x, y, n, bb, ka);
-  // pass 1: low digit, identity payload, (ka) -> (kb, vb)
-  rs_count_kernel<<<ntiles, RS_THREADS, 0, st>>>(ka, n, 0, table, ntiles, tot0);
-  rs_offsets_kernel<<<RS_THREADS / 8, 256, 0, st>>>(table, ntiles, tot0);
-  rs_scatter_kernel<<<ntiles, RS_THREADS, 0, st>>>(ka, nullptr, n, 0, table, ntiles, kb, vb);
-  // pass 2: high digit, (kb, vb) -> (ka, perm)
-  rs_count_kernel<<<ntiles, RS_THREADS, 0, st>>>(kb, n, BIN_BITS, table, ntiles, tot1);
-  rs_offsets_kernel<<<RS_THREADS / 8, 256, 0, st>>>(table, ntiles, tot1);
-  rs_scatter_kernel<<<ntiles, RS_THREADS, 0, st>>>(kb, vb, n, BIN_BITS, table, ntiles, ka, perm);
-  if (launches) *launches += 8;
+  bin_key_kernel<<<blocks, threads, 0, st>>>(x, y, n, bb, bits, curve != BIN_MORTON8, ka);
+  // low digit first; the first pass has the identity payload, the last one writes perm
+  const int* vin = nullptr;
+  for (int q = 0; q < passes; ++q) {
+    int* vout = ((passes - 1 - q) & 1) ? vb : perm;
+    rs_count_kernel<<<ntiles, RS_THREADS, 0, st>>>(ka, n, q * RS_BITS, table, ntiles, tot + q * RS_THREADS);
+    rs_offsets_kernel<<<RS_THREADS / 8, 256, 0, st>>>(table, ntiles, tot + q * RS_THREADS);
+    rs_scatter_kernel<<<ntiles, RS_THREADS, 0, st>>>(ka, vin, n, q * RS_BITS, table, ntiles, kb, vout);
+    unsigned* t = ka;
+    ka = kb;
+    kb = t;
+    vin = vout;
+  }
+  if (launches) *launches += 2 + 3 * passes;
   return cudaGetLastError();
 }
 

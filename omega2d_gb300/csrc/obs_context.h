@@ -127,12 +127,15 @@ cudaError_t packed_res_dispatch(int res, bool thick, bool comp, const P2PArgs* a
                                 int* occ);
 cudaError_t packed_launch_pack(const float* sx, const float* sy, const float* sr, const float* ss, const int* perm,
                                int ns, int ns_pad, int core, float4* out, unsigned* meta, cudaStream_t st);
-// Spatial (Morton) order of n points (bin_order.cu).  `scratch` holds bin_scratch_bytes(n)
-// bytes, 256-aligned.  On return perm[k] is the caller's index of the k-th point in the order;
-// the order is stable, so it depends on the input alone.  bin_gather writes x, y (and r, g when
-// given) in that order.
+// Spatial order of n points (bin_order.cu): along the Morton curve of 256 x 256 cells or the
+// Hilbert curve of 256 x 256 or 4096 x 4096.  `scratch` holds bin_scratch_bytes(n) bytes,
+// 256-aligned.  On return perm[k] is the caller's index of the k-th point in the order; the order
+// is stable, so it depends on the input alone.  bin_gather writes x, y (and r, g when given) in
+// that order.
+enum BinCurve { BIN_MORTON8, BIN_HILBERT8, BIN_HILBERT12 };
 size_t bin_scratch_bytes(int n);
-cudaError_t bin_order(const float* x, const float* y, int n, void* scratch, int* perm, cudaStream_t st, int* launches);
+cudaError_t bin_order(const float* x, const float* y, int n, void* scratch, int* perm, cudaStream_t st, int* launches,
+                      BinCurve curve = BIN_MORTON8);
 cudaError_t bin_gather(const int* perm, const float* x, const float* y, const float* r, const float* g, int n,
                        float* bx, float* by, float* br, float* bg, cudaStream_t st, int* launches);
 

@@ -183,6 +183,28 @@ __device__ __forceinline__ void core_eval(float d2, float zs, float zt, float us
   }
 }
 
+// Radius extrema of a block of up to 256 threads (bit patterns: radii are non-negative; ~0 and 0 for
+// a thread without one), folded into meta[0] = ~min, meta[1] = max with one pair of atomics.
+__device__ __forceinline__ void fold_extrema_block(unsigned rmin, unsigned rmax, unsigned* meta) {
+  __shared__ unsigned red[2][8];
+  rmin = __reduce_min_sync(0xffffffffu, rmin);
+  rmax = __reduce_max_sync(0xffffffffu, rmax);
+  if ((threadIdx.x & 31) == 0) {
+    red[0][threadIdx.x >> 5] = rmin;
+    red[1][threadIdx.x >> 5] = rmax;
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (unsigned w = 1; w < blockDim.x >> 5; ++w) {
+    rmin = min(rmin, red[0][w]);
+    rmax = max(rmax, red[1][w]);
+  }
+  if (rmin <= rmax) {
+    atomicMax(&meta[0], ~rmin);
+    atomicMax(&meta[1], rmax);
+  }
+}
+
 // ---------------------------------------------------------------- compensated accumulation
 // Knuth two-sum: hi + lo accumulates b exactly up to the rounding of lo itself.
 __device__ __forceinline__ void two_sum_acc(float& hi, float& lo, float b) {

@@ -27,19 +27,7 @@ __global__ void pack_sources_dup_kernel(const float* __restrict__ sx, const floa
     out[PK_ELEM * i + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     out[PK_ELEM * i + 2] = make_float4(1.0f, 1.0f, 0.0f, 0.0f);
   }
-  // radius extrema, as pack_sources_kernel does
-  unsigned rmin = (i < ns) ? __float_as_uint(r) : ~0u;
-  unsigned rmax = (i < ns) ? __float_as_uint(r) : 0u;
-  int any = (i < ns) ? 1 : 0;
-  for (int o = 16; o > 0; o >>= 1) {
-    rmin = min(rmin, __shfl_xor_sync(0xffffffffu, rmin, o));
-    rmax = max(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
-    any |= __shfl_xor_sync(0xffffffffu, any, o);
-  }
-  if ((threadIdx.x & 31) == 0 && any) {
-    atomicMax(&meta[0], ~rmin);
-    atomicMax(&meta[1], rmax);
-  }
+  fold_extrema_block(i < ns ? __float_as_uint(r) : ~0u, i < ns ? __float_as_uint(r) : 0u, meta);
 }
 
 template <int CORE, int NP>

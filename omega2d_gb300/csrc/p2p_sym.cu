@@ -28,18 +28,7 @@ __global__ void sym_pack_kernel(const float* __restrict__ x, const float* __rest
     o.g[i % SYM_GRP] = make_float2(G, G);
     o.z[i % SYM_GRP] = make_float2(z, z);
   }
-  unsigned rmin = (i < n) ? __float_as_uint(rr) : ~0u;
-  unsigned rmax = (i < n) ? __float_as_uint(rr) : 0u;
-  int any = (i < n) ? 1 : 0;
-  for (int o = 16; o > 0; o >>= 1) {
-    rmin = min(rmin, __shfl_xor_sync(0xffffffffu, rmin, o));
-    rmax = max(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
-    any |= __shfl_xor_sync(0xffffffffu, any, o);
-  }
-  if ((threadIdx.x & 31) == 0 && any) {
-    atomicMax(&meta[0], ~rmin);
-    atomicMax(&meta[1], rmax);
-  }
+  fold_extrema_block(i < n ? __float_as_uint(rr) : ~0u, i < n ? __float_as_uint(rr) : 0u, meta);
 }
 
 __device__ __forceinline__ void df_add(float& hi, float& lo, float bh, float bl) {

@@ -1,23 +1,25 @@
-// tree.cu -- O(N log N) velocity of vortex particles: a treecode over Morton-ordered sources.
+// tree.cu -- O(N log N) velocity of vortex particles: a treecode over Hilbert-ordered sources.
 //
 // The reference's execution environment names a Barnes-Hut summation (summation_t barneshut,
 // src/ExecEnv.h:26-31) that it never runs internally; an external build reaches onbody's
 // treecode through external_vel_solver_* (src/Influence.h:31-38, 74-98).  This is that
 // summation on the GPU, for the velocity (results_t velonly) of every core:
 //
-//   * sources are put in Morton order (bin_order.cu); a leaf is a run of 32 consecutive sources
+//   * sources are put in Hilbert order (bin_order.cu); a leaf is a run of 32 consecutive sources
 //     (one warp), a node at level L+1 groups 4 consecutive nodes of level L, up to one root;
 //   * each node keeps its bounding box, a centre c (the box centre), a radius rho bounding
 //     |z_j - c| over its sources, the largest radius term of its sources, and P multipole
 //     coefficients b_k = sum_j G_j ((z_j - c)/rho)^k (complex; normalised by rho so that every
 //     power lies in the unit disc) -- formed by warp reductions at the leaves and shifted up the
 //     levels with the binomial theorem ((z - c')/rho' = s (z - c)/rho + t, |s| + |t| <= 1);
-//   * one warp takes 32 Morton-consecutive targets and walks the tree with a warp-uniform stack:
-//     a node is evaluated through its expansion,
+//   * one warp takes 64 Hilbert-consecutive targets, two per lane in f32x2 register pairs, and
+//     walks the tree with a stack, up to 32 nodes (one per lane) at a time: a node is evaluated
+//     through its expansion,
 //        sum_j G_j / (z - z_j) = (1/(z - c)) sum_k b_k w^k,   w = rho/(z - c),
 //     when rho <= theta (|z - c| - r) for the warp's target box (r its half diagonal), so |w|
 //     <= theta and the truncation after P terms is below theta^P/(1 - theta) of the node's
-//     sum |G_j|/|z - z_j|; and only when every (target, source) pair of the node lies in the
+//     sum |G_j|/|z - z_j| (a node farther away stops at the first term count whose |w|^p is below
+//     theta^P / 4: about half of 24 terms on average); and only when every (target, source) pair of the node lies in the
 //     core's far regime, where the core is 1/d^2: for the Gaussian and the compact exponential
 //     that is the reference's own cut-off (d^2/s^2 > 16, (d/s)^3 > 16: the far branch IS 1/d^2,
 //     src/CoreFunc.h:119-131), for the singular core always, and for Rosenhead-Moore,
@@ -27,7 +29,17 @@
 //
 // With u + i v = i conj(F), F = sum_j G_j / (z - z_j): u = Im F, v = Re F (unscaled, as the
 // direct sums; finalize_vels semantics optional).  Per-node contributions are accumulated with
-// two-sums.  Results are deterministic: the traversal order is a function of the inputs.
+// two-sums.  Small target sets split a group's nodes over two or four warps, every one of them
+// walking the same tree and taking its share in turn.  Results are deterministic: the traversal
+// order is a function of the inputs.
+//
+// 1M Gaussian patch, self interaction: 4.4 ms (44 ms in Morton order with 32 targets per warp and
+// every node at full order).  Most of the 44 ms was a tail: a run of targets or sources across one
+// of the Morton curve's jumps has a box the size of the domain, and its warp opened nearly every
+// leaf (twenty times the mean cost in a sample of such groups, more at worst); along the Hilbert
+// curve the worst group costs 1.7 times the mean and the mean group accepts half as many nodes.
+// What is left is the near leaves (about 170 per group, three quarters of the instructions): issue
+// active 62 %, FMA pipe 43 %, MUFU 34 %.  Sorting, tree and extrema take 0.35 ms.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -45,22 +57,37 @@ constexpr int TREE_FAN = 4;          // children per node
 constexpr int TREE_PMAX = 32;        // coefficient stride per node (largest order)
 constexpr int TREE_MAXLEV = 16;      // 32 * 4^15 sources
 constexpr int TREE_WARPS = 4;        // warps per block (leaf, up and evaluation kernels)
-constexpr int TREE_STACK = 96;       // > 1 + 3 * TREE_MAXLEV: the depth-first stack never overflows
+constexpr int TREE_STACK = 576;      // traversal stack entries per warp
+constexpr int TREE_RESERVE = 64;     // of these, kept for taking nodes one at a time: > 1 + 3 * TREE_MAXLEV
+constexpr int TREE_FINE = 32768;     // more points than this are sorted on the 4096 x 4096 grid
 constexpr int TREE_LEVBITS = 26;     // stack entry: level << 26 | index within the level
 constexpr double kTreeInv2Pi = 0.15915494309189535;   // 0.5/pi, finalize_vels (src/ElementBase.h:216)
 
-__constant__ float c_binom[TREE_PMAX][TREE_PMAX];
+// binomial coefficients for the upward shifts (exact in double, rounded once)
+struct Binomials {
+  float v[TREE_PMAX][TREE_PMAX];
+  constexpr Binomials() : v() {
+    for (int k = 0; k < TREE_PMAX; ++k) {
+      double c = 1.0;
+      for (int m = 0; m < TREE_PMAX; ++m) {
+        v[k][m] = m <= k ? (float)c : 0.0f;
+        c = c * (double)(k - m) / (double)(m + 1);
+      }
+    }
+  }
+};
+__constant__ constexpr Binomials c_binom;
 
 struct TreeNodes {
   float4* geo;       // (cx, cy, rho, zmax)
   float4* box;       // (xmin, ymin, xmax, ymax)
-  float2* coef;      // [node][TREE_PMAX]
+  float4* coef;      // [node][TREE_PMAX] (re, re, im, im): twice for the packed evaluation
 };
 
 struct TreeArgs {
-  const float4* sp4; // sources in Morton order: (x, y, radius term, strength)
+  const float4* sp4; // sources in Hilbert order: (x, y, radius term, strength)
   int ns;
-  const float* tx;   // targets in Morton order (tr: radius, null for field points)
+  const float* tx;   // targets in Hilbert order (tr: radius, null for field points)
   const float* ty;
   const float* tr;
   const int* tperm;  // caller's index of the k-th sorted target
@@ -73,6 +100,8 @@ struct TreeArgs {
   int lev_cnt[TREE_MAXLEV];
   int P;
   float theta;
+  float lterm;       // log2(theta^P / 4): a node stops at the first p with p log2|w| below it
+  int split;         // warps per target group (1, 2 or 4)
   int finalize;
   double fsx, fsy;
   int* status;
@@ -118,10 +147,10 @@ __global__ void __launch_bounds__(TREE_WARPS * 32) tree_leaf_kernel(const float*
   const float rn = rho > 0.0f ? rho : 1.0f;
   const float wr = v ? dx / rn : 0.0f, wi = v ? dy / rn : 0.0f;
   float pr = g, pi = 0.0f;                          // G w^k
-  float2* cf = nd.coef + (size_t)leaf * TREE_PMAX;
+  float4* cf = nd.coef + (size_t)leaf * TREE_PMAX;
   for (int k = 0; k < P; ++k) {
     const float sr_ = warp_add(pr), si_ = warp_add(pi);
-    if (lane == 0) cf[k] = make_float2(sr_, si_);
+    if (lane == 0) cf[k] = make_float4(sr_, sr_, si_, si_);
     const float t = pr * wr - pi * wi;
     pi = pr * wi + pi * wr;
     pr = t;
@@ -132,59 +161,83 @@ __global__ void __launch_bounds__(TREE_WARPS * 32) tree_leaf_kernel(const float*
   }
 }
 
-// one level up: one warp per parent (children 4q .. 4q+3 of the level below)
-__global__ void __launch_bounds__(TREE_WARPS * 32) tree_up_kernel(TreeNodes nd, int off_c, int cnt_c, int off_p,
-                                                                  int cnt_p, int P) {
+// One level up: a block per parent, a warp per child (children 4q .. 4q+3 of the level below); the
+// children's shifted coefficients are added in child order.  The levels above the leaves are small
+// and wait on latency: with one warp per parent going through its children in turn, and the powers
+// by repeated multiplication, a level took 25 us (eight of them 240 us of the 1M patch).
+static_assert(TREE_WARPS == TREE_FAN, "a warp per child");
+__global__ void __launch_bounds__(TREE_WARPS * 32) tree_up_kernel(TreeNodes nd, int off_c, int cnt_c, int off_p, int P) {
   __shared__ float sp[TREE_WARPS][TREE_PMAX];
   __shared__ float2 tp[TREE_WARPS][TREE_PMAX];
+  __shared__ float2 cc[TREE_WARPS][TREE_PMAX];
+  __shared__ float2 sum[TREE_WARPS][TREE_PMAX];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int q = blockIdx.x * TREE_WARPS + w;
-  if (q >= cnt_p) return;                           // warp-uniform
-  const int c0 = q * TREE_FAN, c1 = min(c0 + TREE_FAN, cnt_c);
+  const int q = blockIdx.x;
+  const int c0 = q * TREE_FAN, nc = min(TREE_FAN, cnt_c - c0);
+  const bool have = w < nc;                         // warp-uniform
+  if (have && lane < P) {
+    const float4 b = nd.coef[(size_t)(off_c + c0 + w) * TREE_PMAX + lane];
+    cc[w][lane] = make_float2(b.x, b.z);
+  }
   float x0 = __int_as_float(0x7f800000), y0 = x0, x1 = -x0, y1 = -x0, zmax = 0.0f;
-  for (int c = c0; c < c1; ++c) {
-    const float4 b = nd.box[off_c + c];
+  for (int c = 0; c < nc; ++c) {
+    const float4 b = nd.box[off_c + c0 + c];
     x0 = fminf(x0, b.x); y0 = fminf(y0, b.y); x1 = fmaxf(x1, b.z); y1 = fmaxf(y1, b.w);
-    zmax = fmaxf(zmax, nd.geo[off_c + c].w);
+    zmax = fmaxf(zmax, nd.geo[off_c + c0 + c].w);
   }
   const float cx = 0.5f * (x0 + x1), cy = 0.5f * (y0 + y1);
   float rho = 0.0f;
-  for (int c = c0; c < c1; ++c) {
-    const float4 gc = nd.geo[off_c + c];
+  for (int c = 0; c < nc; ++c) {
+    const float4 gc = nd.geo[off_c + c0 + c];
     const float ex = gc.x - cx, ey = gc.y - cy;
     rho = fmaxf(rho, sqrtf(ex * ex + ey * ey) + gc.z);
   }
   const float rn = rho > 0.0f ? rho : 1.0f;
   float ar = 0.0f, ai = 0.0f;
-  for (int c = c0; c < c1; ++c) {
-    const float4 gc = nd.geo[off_c + c];
+  if (have) {
+    const float4 gc = nd.geo[off_c + c0 + w];
     const float rnc = gc.z > 0.0f ? gc.z : 1.0f;
-    // (z - c)/rn = s (z - c_child)/rnc + t
-    const float s = rnc / rn, tr = (gc.x - cx) / rn, ti = (gc.y - cy) / rn;
+    // (z - c)/rn = s (z - c_child)/rnc + t; lane m: s^m and t^m by squaring
+    float s = rnc / rn, tr = (gc.x - cx) / rn, ti = (gc.y - cy) / rn;
     float pws = 1.0f, pwr = 1.0f, pwi = 0.0f;
-    for (int m = 0; m < lane; ++m) {                // lane m: s^m and t^m
-      pws *= s;
-      const float t = pwr * tr - pwi * ti;
-      pwi = pwr * ti + pwi * tr;
-      pwr = t;
+#pragma unroll
+    for (int b = 0; b < 5; ++b) {
+      if ((lane >> b) & 1) {
+        pws *= s;
+        const float t = pwr * tr - pwi * ti;
+        pwi = pwr * ti + pwi * tr;
+        pwr = t;
+      }
+      s *= s;
+      const float t = tr * tr - ti * ti;
+      ti = 2.0f * tr * ti;
+      tr = t;
     }
     sp[w][lane] = pws;
     tp[w][lane] = make_float2(pwr, pwi);
-    __syncwarp();
-    if (lane < P) {
-      const float2* cf = nd.coef + (size_t)(off_c + c) * TREE_PMAX;
-      for (int m = 0; m <= lane; ++m) {
-        const float2 b = cf[m];
-        const float2 t = tp[w][lane - m];
-        const float f = c_binom[lane][m] * sp[w][m];
-        ar += f * (b.x * t.x - b.y * t.y);
-        ai += f * (b.x * t.y + b.y * t.x);
-      }
-    }
-    __syncwarp();
   }
+  __syncwarp();
+  if (have && lane < P) {
+#pragma unroll 4
+    for (int m = 0; m <= lane; ++m) {
+      const float2 b = cc[w][m];
+      const float2 t = tp[w][lane - m];
+      const float f = c_binom.v[lane][m] * sp[w][m];
+      ar += f * (b.x * t.x - b.y * t.y);
+      ai += f * (b.x * t.y + b.y * t.x);
+    }
+  }
+  sum[w][lane] = make_float2(ar, ai);
+  __syncthreads();
+  if (w != 0) return;
   const int node = off_p + q;
-  if (lane < P) nd.coef[(size_t)node * TREE_PMAX + lane] = make_float2(ar, ai);
+  if (lane < P) {
+    for (int c = 1; c < nc; ++c) {
+      ar += sum[c][lane].x;
+      ai += sum[c][lane].y;
+    }
+    nd.coef[(size_t)node * TREE_PMAX + lane] = make_float4(ar, ar, ai, ai);
+  }
   if (lane == 0) {
     nd.geo[node] = make_float4(cx, cy, rho, zmax);
     nd.box[node] = make_float4(x0, y0, x1, y1);
@@ -205,20 +258,78 @@ __device__ __forceinline__ bool tree_far(float d2, float zsum) {
   else return d2 > 0.0f && d2 * d2 * d2 > 8388608.0f * zsum;                              // s^6/(3 d^6) < 2^-24
 }
 
+// a leaf's sources in shared memory, every value twice for the packed operands
+struct TreeLeaf {
+  float4 xy[TREE_LEAF];    // (-x, -x, -y, -y)
+  float4 gz[TREE_LEAF];    // (-G, -G, z, z)
+};
+
+// sums of -G K dy (= u) and -G K dx (= -v) of a leaf's cnt sources at the lane's two targets
+template <int CORE, bool THICK, bool FAR>
+__device__ __forceinline__ void tree_leaf_sum(const TreeLeaf& lf, int cnt, float2 tx, float2 ty, float2 tz, bool unif,
+                                              float cf, float cfl, float2& au, float2& av) {
+  if (!FAR && CORE == CORE_GAUSS && unif) {
+    // (1 - e^-x)/d^2; x < 0.001 -> 1/s^2 (src/CoreFunc.h:111-181).  The reference's 1/d^2 for
+    // x > 16 is within 1.2e-7 of this form, one ulp, so it needs no select here
+    const float thr_small = -0.001f * kLog2e;
+    const float2 cfl2 = f2(cfl, cfl), m1 = f2(-1.0f, -1.0f), one = f2(1.0f, 1.0f);
+#pragma unroll 4
+    for (int k = 0; k < cnt; ++k) {
+      const float4 P = lf.xy[k], Q = lf.gz[k];
+      const float2 dx = __fadd2_rn(tx, f2(P.x, P.y)), dy = __fadd2_rn(ty, f2(P.z, P.w));
+      const float2 d2 = __ffma2_rn(dx, dx, __fmul2_rn(dy, dy));
+      const float2 t = __fmul2_rn(d2, cfl2);
+      const float2 ood2 = f2(rcp_a(d2.x), rcp_a(d2.y));
+      const float2 ome = __ffma2_rn(f2(ex2_a(t.x), ex2_a(t.y)), m1, one);
+      float2 K = __fmul2_rn(ood2, ome);
+      K.x = (t.x > thr_small) ? cf : K.x;
+      K.y = (t.y > thr_small) ? cf : K.y;
+      const float2 fn = __fmul2_rn(f2(Q.x, Q.y), K);
+      au = __ffma2_rn(fn, dy, au);
+      av = __ffma2_rn(fn, dx, av);
+    }
+  } else {
+#pragma unroll 4
+    for (int k = 0; k < cnt; ++k) {
+      const float4 P = lf.xy[k], Q = lf.gz[k];
+      const float2 dx = __fadd2_rn(tx, f2(P.x, P.y)), dy = __fadd2_rn(ty, f2(P.z, P.w));
+      const float2 d2 = __ffma2_rn(dx, dx, __fmul2_rn(dy, dy));
+      float K0, K1, B;
+      if constexpr (FAR) {
+        K0 = rcp_a(d2.x);
+        K1 = rcp_a(d2.y);
+      } else {
+        core_eval<CORE, THICK, false, false>(d2.x, Q.z, tz.x, 0.0f, 0.0f, K0, B);
+        core_eval<CORE, THICK, false, false>(d2.y, Q.z, tz.y, 0.0f, 0.0f, K1, B);
+      }
+      const float2 fn = __fmul2_rn(f2(Q.x, Q.y), f2(K0, K1));
+      au = __ffma2_rn(fn, dy, au);
+      av = __ffma2_rn(fn, dx, av);
+    }
+  }
+}
+
 template <int CORE, bool THICK>
-__global__ void __launch_bounds__(TREE_WARPS * 32) tree_eval_kernel(const TreeArgs a) {
-  __shared__ int stk[TREE_WARPS][TREE_STACK];
-  __shared__ float4 leafs[TREE_WARPS][TREE_LEAF];
+__global__ void __launch_bounds__(TREE_WARPS * 32, 6) tree_eval_kernel(const TreeArgs a) {
+  constexpr unsigned FULL = 0xffffffffu;
+  __shared__ int stk_all[TREE_WARPS][TREE_STACK];
+  __shared__ TreeLeaf leafs[TREE_WARPS];
+  __shared__ float4 red[TREE_WARPS][64];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int wg = blockIdx.x * TREE_WARPS + w;
-  if (wg * 32 >= a.nt) return;                      // warp-uniform
-  const int i = wg * 32 + lane;
-  const bool v = i < a.nt;
+  int* stk = stk_all[w];
+  TreeLeaf& lf = leafs[w];
+  const int part = w % a.split;
+  const int grp = blockIdx.x * (TREE_WARPS / a.split) + w / a.split;
+  const bool live = grp * 64 < a.nt;                // warp-uniform
+  const int i0 = grp * 64 + lane, i1 = i0 + 32;
+  const bool v0 = live && i0 < a.nt, v1 = live && i1 < a.nt;
   const float inf = __int_as_float(0x7f800000);
-  const float tx = v ? a.tx[i] : 0.0f, ty = v ? a.ty[i] : 0.0f;
-  const float tz = (THICK && v) ? radius_term(CORE, a.tr[i]) : 0.0f;
-  // Gaussian with one radius for every source (and every target): the near leaf sums take the
-  // packed form below, with the core's cut-offs on t = -x log2(e), x = d^2 / s^2
+  // a lane without a second (or first) target repeats a real one
+  const int j0 = v0 ? i0 : a.nt - 1, j1 = v1 ? i1 : j0;
+  const float2 tx = f2(a.tx[j0], a.tx[j1]), ty = f2(a.ty[j0], a.ty[j1]);
+  const float2 tz = THICK ? f2(radius_term(CORE, a.tr[j0]), radius_term(CORE, a.tr[j1])) : f2(0.0f, 0.0f);
+  // Gaussian with one radius for every source (and every target): the packed near leaf sums, with
+  // the core's cut-offs on t = -x log2(e), x = d^2 / s^2
   bool gunif = false;
   float gcf = 0.0f, gcfl = 0.0f;
   if constexpr (CORE == CORE_GAUSS) {
@@ -230,20 +341,23 @@ __global__ void __launch_bounds__(TREE_WARPS * 32) tree_eval_kernel(const TreeAr
       gcfl = -gcf * kLog2e;
     }
   }
-  const float bx0 = warp_min(v ? tx : inf), bx1 = warp_max(v ? tx : -inf);
-  const float by0 = warp_min(v ? ty : inf), by1 = warp_max(v ? ty : -inf);
-  const float ztmax = warp_max(tz);
+  const float bx0 = warp_min(v0 ? fminf(tx.x, tx.y) : inf), bx1 = warp_max(v0 ? fmaxf(tx.x, tx.y) : -inf);
+  const float by0 = warp_min(v0 ? fminf(ty.x, ty.y) : inf), by1 = warp_max(v0 ? fmaxf(ty.x, ty.y) : -inf);
+  const float ztmax = warp_max(fmaxf(tz.x, tz.y));
   const float ctx_ = 0.5f * (bx0 + bx1), cty = 0.5f * (by0 + by1);
   const float rt = 0.5f * sqrtf((bx1 - bx0) * (bx1 - bx0) + (by1 - by0) * (by1 - by0));
-  float hu = 0.0f, lu = 0.0f, hv = 0.0f, lv = 0.0f;
+  float2 hu = f2(0.0f, 0.0f), lu = hu, hv = hu, lv = hu;
   const int top = a.nlev - 1;
-  if (lane == 0)
-    for (int q = 0; q < a.lev_cnt[top]; ++q) stk[w][q] = (top << TREE_LEVBITS) | q;
-  int sp = a.lev_cnt[top];                          // 1 by construction
+  if (lane == 0) stk[0] = top << TREE_LEVBITS;      // the root: one node by construction
+  int sp = live ? 1 : 0;
+  int turn = 0;                                     // nodes and leaves met so far, shared out in turn
   __syncwarp();
   while (sp > 0) {
-    const int e = stk[w][--sp];
-    __syncwarp();
+    // up to 32 nodes off the stack, fewer when their children might not fit above the reserve
+    const int take = max(1, min(min(sp, 32), (TREE_STACK - TREE_RESERVE - sp) / 3));
+    const bool have = lane < take;
+    const int e = have ? stk[sp - 1 - lane] : 0;
+    sp -= take;
     const int lev = e >> TREE_LEVBITS, q = e & ((1 << TREE_LEVBITS) - 1);
     const int node = a.lev_off[lev] + q;
     const float4 gn = a.nodes.geo[node];
@@ -253,114 +367,107 @@ __global__ void __launch_bounds__(TREE_WARPS * 32) tree_eval_kernel(const TreeAr
     const float dmin2 = gx * gx + gy * gy;
     const float ex = gn.x - ctx_, ey = gn.y - cty;
     const float sep = sqrtf(ex * ex + ey * ey) - rt;
-    const bool accept = sep > 0.0f && gn.z <= a.theta * sep && tree_far<CORE>(dmin2, gn.w + ztmax);
-    if (accept) {
+    const bool far = tree_far<CORE>(dmin2, gn.w + ztmax);
+    const bool accept = have && sep > 0.0f && gn.z <= a.theta * sep && far;
+    const bool leaf = have && !accept && lev == 0;
+    const bool open = have && !accept && lev > 0;
+    // terms: |w| <= gn.z / sep for every target of the warp
+    const float lw = lg2_a(gn.z * rcp_a(sep));      // <= log2(theta) where accepted; -inf for a point node
+    const int terms = max(1, min(a.P, (int)ceilf(a.lterm * rcp_a(fminf(lw, -1.0e-3f)))));
+    // children onto the stack, first child of the first node on top
+    const int c0 = q * TREE_FAN;
+    const int nc = open ? min(c0 + TREE_FAN, a.lev_cnt[lev - 1]) - c0 : 0;
+    int incl = nc;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(FULL, incl, o);
+      if (lane >= o) incl += t;
+    }
+    const int total = __shfl_sync(FULL, incl, 31);
+    if (sp + total > TREE_STACK) {                  // cannot happen (take); recorded, not taken
+      if (lane == 0) record_failure(a.status, DEV_ERR_BOUNDS, 1100, grp, sp);
+      break;
+    }
+    __syncwarp();                                   // every lane has read its entry
+    for (int c = 0; c < nc; ++c) stk[sp + total - (incl - nc) - 1 - c] = ((lev - 1) << TREE_LEVBITS) | (c0 + c);
+    sp += total;
+    __syncwarp();
+    for (unsigned m = __ballot_sync(FULL, accept); m; m &= m - 1) {
+      if (turn++ % a.split != part) continue;
       // F = (1/(z - c)) sum_k b_k w^k, w = rn/(z - c); u += Im F, v += Re F
-      const float2* cf = a.nodes.coef + (size_t)node * TREE_PMAX;
-      const float rn = gn.z > 0.0f ? gn.z : 1.0f;
-      const float dx = tx - gn.x, dy = ty - gn.y;
-      const float inv = rcp_a(dx * dx + dy * dy);
-      const float wr = rn * dx * inv, wi = -rn * dy * inv;
-      float2 h = cf[a.P - 1];
-      for (int k = a.P - 2; k >= 0; --k) {
-        const float2 b = cf[k];
-        const float t = fmaf(h.x, wr, fmaf(-h.y, wi, b.x));
-        h.y = fmaf(h.x, wi, fmaf(h.y, wr, b.y));
-        h.x = t;
-      }
-      const float fr = (dx * h.x + dy * h.y) * inv, fi = (dx * h.y - dy * h.x) * inv;
-      if (v) {
-        two_sum_acc(hu, lu, fi);
-        two_sum_acc(hv, lv, fr);
-      }
-    } else if (lev == 0) {
-      // direct sum over the leaf's sources (warp-broadcast loads): with the core, or -- when every
-      // pair lies in the core's far regime, the leaf being too close for its expansion -- with
-      // the far form 1/d^2 the core takes there.  Two sources per f32x2 operation: the leaf is
-      // staged as pairs, ps[2 kp] = (-x, -x', -y, -y'), ps[2 kp + 1] = (z, z', -G, -G') for
-      // sources 2 kp and 2 kp + 1 (one load per lane; padding past the leaf's end has G = 0)
-      const int cnt = min(TREE_LEAF, a.ns - q * TREE_LEAF);
-      __syncwarp();
-      {
-        const float4 p = a.sp4[q * TREE_LEAF + min(lane, cnt - 1)];
-        float* st = reinterpret_cast<float*>(&leafs[w][0]) + (lane >> 1) * 8 + (lane & 1);
-        st[0] = -p.x;
-        st[2] = -p.y;
-        st[4] = p.z;
-        st[6] = (lane < cnt) ? -p.w : 0.0f;
-      }
-      __syncwarp();
-      const float4* ps = leafs[w];
-      const int np2 = (cnt + 1) >> 1;
-      const float2 tx2 = f2(tx, tx), ty2 = f2(ty, ty);
-      float2 au = f2(0.0f, 0.0f), av = f2(0.0f, 0.0f);   // sum -G K dy (= u), sum -G K dx (= -v)
-      if (tree_far<CORE>(dmin2, gn.w + ztmax)) {
+      const int b = __ffs(m) - 1;
+      const float4* cf = a.nodes.coef + (size_t)__shfl_sync(FULL, node, b) * TREE_PMAX;
+      const float rho = __shfl_sync(FULL, gn.z, b);
+      const float rn = rho > 0.0f ? rho : 1.0f;
+      const float cx = -__shfl_sync(FULL, gn.x, b), cy = -__shfl_sync(FULL, gn.y, b);
+      const int p = __shfl_sync(FULL, terms, b);
+      const float2 dx = __fadd2_rn(tx, f2(cx, cx)), dy = __fadd2_rn(ty, f2(cy, cy));
+      const float2 d2 = __ffma2_rn(dx, dx, __fmul2_rn(dy, dy));
+      const float2 inv = f2(rcp_a(d2.x), rcp_a(d2.y));
+      const float2 ri = __fmul2_rn(f2(rn, rn), inv);
+      const float2 wr = __fmul2_rn(ri, dx), nwi = __fmul2_rn(ri, dy);
+      const float2 wi = f2(-nwi.x, -nwi.y);
+      float2 hr = f2(0.0f, 0.0f), hi = hr;
 #pragma unroll 4
-        for (int kp = 0; kp < np2; ++kp) {
-          const float4 P = ps[2 * kp], Q = ps[2 * kp + 1];
-          const float2 dx = __fadd2_rn(tx2, f2(P.x, P.y)), dy = __fadd2_rn(ty2, f2(P.z, P.w));
-          const float2 d2 = __ffma2_rn(dx, dx, __fmul2_rn(dy, dy));
-          const float2 fn = __fmul2_rn(f2(Q.z, Q.w), f2(rcp_a(d2.x), rcp_a(d2.y)));
-          au = __ffma2_rn(fn, dy, au);
-          av = __ffma2_rn(fn, dx, av);
-        }
-      } else if (CORE == CORE_GAUSS && gunif) {
-        // (1 - e^-x)/d^2; x > 16 -> 1/d^2; x < 0.001 -> 1/s^2 (src/CoreFunc.h:111-181)
-        const float thr_far = -16.0f * kLog2e, thr_small = -0.001f * kLog2e;
-        const float2 cfl2 = f2(gcfl, gcfl), m1 = f2(-1.0f, -1.0f), one = f2(1.0f, 1.0f);
-#pragma unroll 2
-        for (int kp = 0; kp < np2; ++kp) {
-          const float4 P = ps[2 * kp], Q = ps[2 * kp + 1];
-          const float2 dx = __fadd2_rn(tx2, f2(P.x, P.y)), dy = __fadd2_rn(ty2, f2(P.z, P.w));
-          const float2 d2 = __ffma2_rn(dx, dx, __fmul2_rn(dy, dy));
-          const float2 t = __fmul2_rn(d2, cfl2);
-          const float2 ood2 = f2(rcp_a(d2.x), rcp_a(d2.y));
-          const float2 ome = __ffma2_rn(f2(ex2_a(t.x), ex2_a(t.y)), m1, one);
-          float2 k = __fmul2_rn(ood2, ome);
-          k.x = (t.x < thr_far) ? ood2.x : ((t.x > thr_small) ? gcf : k.x);
-          k.y = (t.y < thr_far) ? ood2.y : ((t.y > thr_small) ? gcf : k.y);
-          const float2 fn = __fmul2_rn(f2(Q.z, Q.w), k);
-          au = __ffma2_rn(fn, dy, au);
-          av = __ffma2_rn(fn, dx, av);
-        }
-      } else {
-#pragma unroll 2
-        for (int kp = 0; kp < np2; ++kp) {
-          const float4 P = ps[2 * kp], Q = ps[2 * kp + 1];
-          const float2 dx = __fadd2_rn(tx2, f2(P.x, P.y)), dy = __fadd2_rn(ty2, f2(P.z, P.w));
-          const float2 d2 = __ffma2_rn(dx, dx, __fmul2_rn(dy, dy));
-          float K0, K1, B;
-          core_eval<CORE, THICK, false, false>(d2.x, Q.x, tz, 0.0f, 0.0f, K0, B);
-          core_eval<CORE, THICK, false, false>(d2.y, Q.y, tz, 0.0f, 0.0f, K1, B);
-          const float2 fn = __fmul2_rn(f2(Q.z, Q.w), f2(K0, K1));
-          au = __ffma2_rn(fn, dy, au);
-          av = __ffma2_rn(fn, dx, av);
-        }
+      for (int k = p - 1; k >= 0; --k) {
+        const float4 c = cf[k];
+        const float2 t = __ffma2_rn(hr, wr, __ffma2_rn(hi, nwi, f2(c.x, c.y)));
+        hi = __ffma2_rn(hr, wi, __ffma2_rn(hi, wr, f2(c.z, c.w)));
+        hr = t;
       }
-      const float su = au.x + au.y, sv = -(av.x + av.y);
-      if (v) {
-        two_sum_acc(hu, lu, su);
-        two_sum_acc(hv, lv, sv);
-      }
-    } else {
-      const int c0 = q * TREE_FAN, c1 = min(c0 + TREE_FAN, a.lev_cnt[lev - 1]);
-      if (sp + (c1 - c0) > TREE_STACK) {            // cannot happen (depth bound); recorded, not taken
-        if (lane == 0) record_failure(a.status, DEV_ERR_BOUNDS, 1100, wg, sp);
-        break;
-      }
-      if (lane == 0)
-        for (int c = c1 - 1; c >= c0; --c) stk[w][sp + (c1 - 1 - c)] = ((lev - 1) << TREE_LEVBITS) | c;
-      sp += c1 - c0;
+      // (dx - i dy) h / d^2
+      const float2 fr = __fmul2_rn(__ffma2_rn(dx, hr, __fmul2_rn(dy, hi)), inv);
+      const float2 dyn = f2(-dy.x, -dy.y);
+      const float2 fi = __fmul2_rn(__ffma2_rn(dx, hi, __fmul2_rn(dyn, hr)), inv);
+      two_sum2(hu, lu, fi);
+      two_sum2(hv, lv, fr);
+    }
+    // leaves: direct sums, with the core or -- when every pair lies in the core's far regime, the
+    // leaf being too close for its expansion -- with the far form 1/d^2 the core takes there
+    const unsigned farm = __ballot_sync(FULL, far);
+    for (unsigned m = __ballot_sync(FULL, leaf); m; m &= m - 1) {
+      if (turn++ % a.split != part) continue;
+      const int b = __ffs(m) - 1;
+      const int s0 = __shfl_sync(FULL, q, b) * TREE_LEAF;
+      const int cnt = min(TREE_LEAF, a.ns - s0);
       __syncwarp();
+      if (lane < cnt) {
+        const float4 s = a.sp4[s0 + lane];
+        lf.xy[lane] = make_float4(-s.x, -s.x, -s.y, -s.y);
+        lf.gz[lane] = make_float4(-s.w, -s.w, s.z, s.z);
+      }
+      __syncwarp();
+      float2 au = f2(0.0f, 0.0f), av = au;
+      if ((farm >> b) & 1u) tree_leaf_sum<CORE, THICK, true>(lf, cnt, tx, ty, tz, gunif, gcf, gcfl, au, av);
+      else tree_leaf_sum<CORE, THICK, false>(lf, cnt, tx, ty, tz, gunif, gcf, gcfl, au, av);
+      two_sum2(hu, lu, au);
+      two_sum2(hv, lv, f2(-av.x, -av.y));
     }
   }
-  if (!v) return;
-  const int o = a.tperm ? a.tperm[i] : i;
-  if ((unsigned)o >= (unsigned)a.nt) return;        // never taken: tperm is a permutation
+  if (a.split > 1) {                                // the group's warps, added in order by the first
+    red[w][lane] = make_float4(hu.x, lu.x, hv.x, lv.x);
+    red[w][32 + lane] = make_float4(hu.y, lu.y, hv.y, lv.y);
+    __syncthreads();
+    if (part != 0) return;
+    for (int k = 1; k < a.split; ++k) {
+      const float4 p = red[w + k][lane], r = red[w + k][32 + lane];
+      two_sum2(hu, lu, f2(p.x, r.x));
+      two_sum2(hv, lv, f2(p.z, r.z));
+      lu = __fadd2_rn(lu, f2(p.y, r.y));
+      lv = __fadd2_rn(lv, f2(p.w, r.w));
+    }
+  }
   const double f = a.finalize ? kTreeInv2Pi : 1.0;
-  const double su = (double)hu + (double)lu, sv = (double)hv + (double)lv;
-  a.tu[o] = (float)(((double)a.tu[o] + su) * f + (a.finalize ? a.fsx : 0.0));
-  a.tv[o] = (float)(((double)a.tv[o] + sv) * f + (a.finalize ? a.fsy : 0.0));
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    if (!(h ? v1 : v0)) continue;
+    const int i = h ? i1 : i0;
+    const int o = a.tperm ? a.tperm[i] : i;
+    if ((unsigned)o >= (unsigned)a.nt) continue;    // never taken: tperm is a permutation
+    const double su = (double)(h ? hu.y : hu.x) + (double)(h ? lu.y : lu.x);
+    const double sv = (double)(h ? hv.y : hv.x) + (double)(h ? lv.y : lv.x);
+    a.tu[o] = (float)(((double)a.tu[o] + su) * f + (a.finalize ? a.fsx : 0.0));
+    a.tv[o] = (float)(((double)a.tv[o] + sv) * f + (a.finalize ? a.fsy : 0.0));
+  }
 }
 
 template <int CORE>
@@ -383,6 +490,8 @@ cudaError_t tree_eval(int core, bool thick, const TreeArgs& a, int grid, cudaStr
 }
 
 size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
+
+BinCurve tree_curve(int n) { return n > TREE_FINE ? BIN_HILBERT12 : BIN_HILBERT8; }
 
 }  // namespace
 
@@ -416,7 +525,7 @@ int run_tree(obs_context* ctx, int core, int flags, double fsx, double fsy, doub
   const size_t o_geo = o_t + 3 * al256(T * 4);
   const size_t o_box = o_geo + al256((size_t)total * sizeof(float4));
   const size_t o_coef = o_box + al256((size_t)total * sizeof(float4));
-  const size_t o_meta = o_coef + al256((size_t)total * TREE_PMAX * sizeof(float2));
+  const size_t o_meta = o_coef + al256((size_t)total * TREE_PMAX * sizeof(float4));
   const size_t bytes = o_meta + 256;
   int s = ctx->work.ensure(bytes, ctx->stream);
   if (s) return s;
@@ -429,27 +538,18 @@ int run_tree(obs_context* ctx, int core, int flags, double fsx, double fsy, doub
   float* bt[3];
   for (int k = 0; k < 3; ++k) bt[k] = reinterpret_cast<float*>(W + o_t + k * al256(T * 4));
   TreeNodes nd{reinterpret_cast<float4*>(W + o_geo), reinterpret_cast<float4*>(W + o_box),
-               reinterpret_cast<float2*>(W + o_coef)};
+               reinterpret_cast<float4*>(W + o_coef)};
   cudaStream_t st = ctx->stream;
-  // binomial coefficients for the upward shifts (exact in double, rounded once)
-  float binom[TREE_PMAX][TREE_PMAX];
-  for (int k = 0; k < TREE_PMAX; ++k) {
-    double c = 1.0;
-    for (int m = 0; m < TREE_PMAX; ++m) {
-      binom[k][m] = m <= k ? (float)c : 0.0f;
-      c = c * (double)(k - m) / (double)(m + 1);
-    }
-  }
-  cudaError_t e = cudaMemcpyToSymbolAsync(c_binom, binom, sizeof(binom), 0, cudaMemcpyHostToDevice, st);
+  cudaError_t e = cudaSuccess;
   int launches = 0;
-  if (e == cudaSuccess) e = bin_order(sx, sy, ns, W + o_bin, sperm, st, &launches);
+  if (e == cudaSuccess) e = bin_order(sx, sy, ns, W + o_bin, sperm, st, &launches, tree_curve(ns));
   if (e == cudaSuccess) e = bin_gather(sperm, sx, sy, sr, ss, ns, bs[0], bs[1], sr ? bs[2] : nullptr, bs[3], st,
                                        &launches);
   if (e != cudaSuccess) return cuda_status(e);
   const float *ttx = bs[0], *tty = bs[1], *ttr = tr ? bs[2] : nullptr;
   const int* tp = sperm;
   if (!same) {
-    e = bin_order(tx, ty, nt, W + o_bin, tperm, st, &launches);
+    e = bin_order(tx, ty, nt, W + o_bin, tperm, st, &launches, tree_curve(nt));
     if (e == cudaSuccess) e = bin_gather(tperm, tx, ty, tr, nullptr, nt, bt[0], bt[1], tr ? bt[2] : nullptr, nullptr, st,
                                          &launches);
     if (e != cudaSuccess) return cuda_status(e);
@@ -461,8 +561,7 @@ int run_tree(obs_context* ctx, int core, int flags, double fsx, double fsy, doub
                                                                             ns, core, sp4, nd, lev_cnt[0], P);
   ++launches;
   for (int l = 0; l + 1 < nlev; ++l) {
-    tree_up_kernel<<<(lev_cnt[l + 1] + TREE_WARPS - 1) / TREE_WARPS, tb, 0, st>>>(nd, lev_off[l], lev_cnt[l],
-                                                                                lev_off[l + 1], lev_cnt[l + 1], P);
+    tree_up_kernel<<<lev_cnt[l + 1], tb, 0, st>>>(nd, lev_off[l], lev_cnt[l], lev_off[l + 1], P);
     ++launches;
   }
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e);
@@ -476,6 +575,7 @@ int run_tree(obs_context* ctx, int core, int flags, double fsx, double fsy, doub
   for (int l = 0; l < nlev; ++l) { a.lev_off[l] = lev_off[l]; a.lev_cnt[l] = lev_cnt[l]; }
   a.P = P;
   a.theta = (float)theta;
+  a.lterm = (float)((double)P * std::log2(theta) - 2.0);
   a.finalize = (flags & OBS_FLAG_FINALIZE) ? 1 : 0;
   a.fsx = fsx; a.fsy = fsy;
   a.status = ctx->d_status;
@@ -485,14 +585,20 @@ int run_tree(obs_context* ctx, int core, int flags, double fsx, double fsy, doub
   if (core == CORE_GAUSS && sr) {
     if ((e = p2p_launch_target_meta(sr, ns, meta, st)) != cudaSuccess) return cuda_status(e);
     ++launches;
-    if (tr) {
+    if (tr && tr == sr && nt == ns) {
+      e = cudaMemcpyAsync(meta + 4, meta + 2, 2 * sizeof(unsigned), cudaMemcpyDeviceToDevice, st);
+      if (e != cudaSuccess) return cuda_status(e);
+    } else if (tr) {
       if ((e = p2p_launch_target_meta(tr, nt, meta + 2, st)) != cudaSuccess) return cuda_status(e);
       ++launches;
     }
   }
   a.meta = meta;
-  const int nwarps = (nt + 31) / 32;
-  e = tree_eval(core, tr != nullptr, a, (nwarps + TREE_WARPS - 1) / TREE_WARPS, st);
+  // a warp per 64 targets, or two or four where that leaves fewer than 16 warps per SM
+  const int groups = (nt + 63) / 64;
+  a.split = groups >= 16 * ctx->num_sms ? 1 : (groups >= 8 * ctx->num_sms ? 2 : 4);
+  const int gpb = TREE_WARPS / a.split;
+  e = tree_eval(core, tr != nullptr, a, (groups + gpb - 1) / gpb, st);
   ++launches;
   ctx->launches += launches;
   return cuda_status(e);
