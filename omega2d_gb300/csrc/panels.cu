@@ -153,6 +153,31 @@ __device__ __forceinline__ void panel_uv_star_fast2(float2 x0, float2 y0, float2
   if (!(fabsf(sv.y) <= 0.2f)) vs.y = half_log_near(dx0.y, dy0.y, r1.y, diff.y);
 }
 
+// ---- far pairs.  With the panel's midpoint m, half vector h and a target at z, the half-log and the
+// angle are one complex function, v* + i u* = log((z - z0)/(z - z1)) = 2 atanh(q), q = h/(z - m), and
+// where |q| < 0.0178 (targets more than 28 panel lengths away) its odd series ends at q^3: the next
+// term is below 2e-8 relative.  With A + i B = -1/conj(z - m) and n + i m2 = (A + i B)^2 that takes
+// 18 f32x2 operations, one reciprocal and one comparison to the sheet velocity, where the two
+// series of panel_uv_star_fast2 took 30 and two reciprocals.  z - m is formed as (z - z0) - h, so a
+// midpoint is never rounded.  A warp takes this form when all its pairs do (200,000 points around a
+// circle of 2048 panels: every pair; of 128 panels, whose points 28 lengths away are mostly in
+// reach, hardly any).  200,000 x 2048: points on panels 298 us and panels on points 322 us (445 and 490 us
+// with the two series), FMA pipe 72 %, register read ports as for the particle sums; errors against
+// FP64 are equal or smaller.  One kernel per mode: the modes' registers don't add up.
+constexpr float kPanFar = 3163.0f;   // |z - m|^2 > 3163 |h|^2: |q| < 0.01778
+
+// A + i B = -(z - m)/|z - m|^2 and its square n + i m, from d = z - m and d2 = |z - m|^2 (n = 2 A^2 -
+// 1/d2, since A^2 + B^2 = 1/d2)
+__device__ __forceinline__ void pan_far_inverse(float2 dx, float2 dy, float2 d2, float2& A, float2& B, float2& n,
+                                                float2& m) {
+  const float2 nk = f2(rcp_approx(-d2.x), rcp_approx(-d2.y));
+  A = __fmul2_rn(dx, nk);
+  B = __fmul2_rn(dy, nk);
+  const float2 A2 = __fadd2_rn(A, A);
+  n = __ffma2_rn(A, A2, nk);
+  m = __fmul2_rn(A2, B);
+}
+
 struct PanArgs {
   const float* gx;      // the panel set: node coordinates, node-index pairs (mode 0: the
   const float* gy;      //   sources, padded to nsrc with far panels of zero strength; modes 1
@@ -242,11 +267,12 @@ __device__ __forceinline__ void pan_finish(const PanArgs& a, int i, double su, d
 //     B = s tx - g ty, formed once per panel when the tile is staged;
 //   points -> panels: the target panel's tangent is fixed per thread, so the particle sums
 //     are of w u* and w v* and the tangent is applied once at the end.
-template <bool COMP>
+template <int MODE, bool COMP>
 __global__ void __launch_bounds__(PAN_THREADS) pan_kernel(const PanArgs a) {
   // sources pre-duplicated for the packed operands: panels (x0,x0,y0,y0) (x1,x1,y1,y1)
-  // (px,px,py,py) (A,A,B,B); particles (x,x,y,y) (w,w,0,0)
-  __shared__ float4 sE[PAN_TILE][4];
+  // (hx,hx,hy,hy) (A,A,B,B) and, for the far form, d1 = -2 conj(G h), d3 = -2/3 conj(G h^3), G = A + i B,
+  // as (re,re,im,im) and (-im d3, -im d3, far limit on d^2, 0); particles (x,x,y,y) (w,w,-w,-w)
+  __shared__ float4 sE[PAN_TILE][7];
   const int sp = blockIdx.y;
   int ti[2];
   float tx[2] = {0.0f, 0.0f}, ty[2] = {0.0f, 0.0f}, tinv[2] = {0.0f, 0.0f};
@@ -256,7 +282,7 @@ __global__ void __launch_bounds__(PAN_THREADS) pan_kernel(const PanArgs a) {
     ti[h] = blockIdx.x * PAN_TPB + h * PAN_THREADS + threadIdx.x;
     const int ic = ti[h] < a.nt ? ti[h] : a.nt - 1;
     TP[h] = TQ[h] = make_float4(0, 0, 0, 0);
-    if (a.mode == 0) {
+    if constexpr (MODE == 0) {
       tx[h] = a.tx[ic];
       ty[h] = a.ty[ic];
     } else {
@@ -271,6 +297,15 @@ __global__ void __launch_bounds__(PAN_THREADS) pan_kernel(const PanArgs a) {
   const float2 PX = sub2(X1, X0), PY = sub2(Y1, Y0);
   const float2 z2 = f2(0.0f, 0.0f);
   float2 au = z2, av = z2, hu = z2, lu = z2, hv = z2, lv = z2;
+  // mode 1's far form: half vectors, h^3 / 3, limits on d^2 and the block's sums
+  const float2 HX = __fmul2_rn(PX, f2(0.5f, 0.5f)), HY = __fmul2_rn(PY, f2(0.5f, 0.5f));
+  const float2 hh = __ffma2_rn(HX, HX, __fmul2_rn(HY, HY));
+  const float2 LIM = __fmul2_rn(hh, f2(kPanFar, kPanFar));
+  const float2 q2r = __fmul2_rn(sub2(HX, HY), __fadd2_rn(HX, HY)), q2i = __fmul2_rn(__fadd2_rn(HX, HX), HY);
+  const float2 third = f2(1.0f / 3.0f, 1.0f / 3.0f);
+  const float2 H3X = __fmul2_rn(third, sub2(__fmul2_rn(HX, q2r), __fmul2_rn(HY, q2i)));
+  const float2 H3Y = __fmul2_rn(third, __ffma2_rn(HX, q2i, __fmul2_rn(HY, q2r)));
+  float2 t1r = z2, t1i = z2, t3r = z2, t3i = z2;
   // this split's 32-source blocks [b0, b1), staged PAN_TILE sources at a time
   const int b0 = sp * a.blks_per_split;
   const int b1 = min(b0 + a.blks_per_split, a.nblk);
@@ -279,7 +314,7 @@ __global__ void __launch_bounds__(PAN_THREADS) pan_kernel(const PanArgs a) {
     __syncthreads();
     for (int k = threadIdx.x; k < ns; k += PAN_THREADS) {
       const int j = base * PAN_COMP_BLOCK + k;
-      if (a.mode == 0) {
+      if constexpr (MODE == 0) {
         float4 P, Q;
         float len;
         panel_geom(a, j, P, Q, len);
@@ -287,42 +322,86 @@ __global__ void __launch_bounds__(PAN_THREADS) pan_kernel(const PanArgs a) {
         const float A = Q.z * Q.x + Q.w * Q.y, B = Q.w * Q.x - Q.z * Q.y;
         sE[k][0] = make_float4(P.x, P.x, P.y, P.y);
         sE[k][1] = make_float4(P.z, P.z, P.w, P.w);
-        sE[k][2] = make_float4(px, px, py, py);
+        const float hx = 0.5f * px, hy = 0.5f * py;
+        sE[k][2] = make_float4(hx, hx, hy, hy);
         sE[k][3] = make_float4(A, A, B, B);
+        // G h and G h^3 / 3 = (G h) h^2 / 3
+        const float gr = A * hx - B * hy, gi = A * hy + B * hx;
+        const float qr = (hx - hy) * (hx + hy), qi = 2.0f * hx * hy;
+        const float cr = (gr * qr - gi * qi) * (2.0f / 3.0f), ci = (gr * qi + gi * qr) * (2.0f / 3.0f);
+        sE[k][4] = make_float4(-2.0f * gr, -2.0f * gr, 2.0f * gi, 2.0f * gi);
+        sE[k][5] = make_float4(-cr, -cr, ci, ci);
+        sE[k][6] = make_float4(-ci, -ci, kPanFar * (hx * hx + hy * hy), 0.0f);
       } else {
         // (x, y, 0, strength) or, mode 2, (x, y, lu, lv)
-        const float4 q = (a.mode == 2) ? a.pts[j]
+        const float4 q = (MODE == 2) ? a.pts[j]
                          : (j < a.nreal) ? make_float4(a.sx[j], a.sy[j], 0.0f, a.ss[j])
                                          : make_float4(1.0e6f, 1.0e6f, 0.0f, 0.0f);
         sE[k][0] = make_float4(q.x, q.x, q.y, q.y);
-        sE[k][1] = (a.mode == 1) ? make_float4(q.w, q.w, 0.0f, 0.0f) : make_float4(q.z, q.z, q.w, q.w);
+        sE[k][1] = (MODE == 1) ? make_float4(q.w, q.w, -q.w, -q.w) : make_float4(q.z, q.z, q.w, q.w);
       }
     }
     __syncthreads();
     for (int b = 0; b < ns; b += PAN_COMP_BLOCK) {
-      if (a.mode == 0) {
+      if constexpr (MODE == 0) {
 #pragma unroll 2
         for (int k = 0; k < PAN_COMP_BLOCK; ++k) {
-          const float4 E0 = sE[b + k][0], E1 = sE[b + k][1], E2 = sE[b + k][2], E3 = sE[b + k][3];
-          float2 us, vs;
-          panel_uv_star_fast2(f2(E0.x, E0.y), f2(E0.z, E0.w), f2(E1.x, E1.y), f2(E1.z, E1.w), f2(E2.x, E2.y),
-                              f2(E2.z, E2.w), T2x, T2y, us, vs);
-          const float2 A = f2(E3.x, E3.y), B = f2(E3.z, E3.w);
-          au = __ffma2_rn(us, A, __ffma2_rn(vs, B, au));
-          av = __ffma2_rn(vs, A, sub2(av, __fmul2_rn(us, B)));
+          const float4 E0 = sE[b + k][0], E2 = sE[b + k][2], E6 = sE[b + k][6];
+          const float2 dx = sub2(sub2(T2x, f2(E0.x, E0.y)), f2(E2.x, E2.y));
+          const float2 dy = sub2(sub2(T2y, f2(E0.z, E0.w)), f2(E2.z, E2.w));
+          const float2 d2 = __ffma2_rn(dx, dx, __fmul2_rn(dy, dy));
+          if (__all_sync(0xffffffffu, d2.x > E6.z && d2.y > E6.z)) {
+            // v - i u = (A + i B)(d1 + d3 (A + i B)^2)
+            const float4 D1 = sE[b + k][4], D3 = sE[b + k][5];
+            float2 A, B, n, m;
+            pan_far_inverse(dx, dy, d2, A, B, n, m);
+            const float2 d3r = f2(D3.x, D3.y);
+            const float2 er = __ffma2_rn(d3r, n, __ffma2_rn(f2(E6.x, E6.y), m, f2(D1.x, D1.y)));
+            const float2 ei = __ffma2_rn(d3r, m, __ffma2_rn(f2(D3.z, D3.w), n, f2(D1.z, D1.w)));
+            au = sub2(au, __ffma2_rn(A, ei, __fmul2_rn(B, er)));
+            av = __fadd2_rn(av, sub2(__fmul2_rn(A, er), __fmul2_rn(B, ei)));
+          } else {
+            const float4 E1 = sE[b + k][1], E3 = sE[b + k][3];
+            float2 us, vs;
+            panel_uv_star_fast2(f2(E0.x, E0.y), f2(E0.z, E0.w), f2(E1.x, E1.y), f2(E1.z, E1.w),
+                                f2(E2.x + E2.x, E2.x + E2.x), f2(E2.z + E2.z, E2.z + E2.z), T2x, T2y, us, vs);
+            const float2 A = f2(E3.x, E3.y), B = f2(E3.z, E3.w);
+            au = __ffma2_rn(us, A, __ffma2_rn(vs, B, au));
+            av = __ffma2_rn(vs, A, sub2(av, __fmul2_rn(us, B)));
+          }
         }
-      } else if (a.mode == 1) {
+      } else if constexpr (MODE == 1) {
         // the panel is the "source" of kernelu_1v_0p with the particle strength, the particle
         // the "target"; the sum is used with a minus sign (src/Influence.h:737-759)
 #pragma unroll 2
         for (int k = 0; k < PAN_COMP_BLOCK; ++k) {
           const float4 E0 = sE[b + k][0], E1 = sE[b + k][1];
-          float2 us, vs;
-          panel_uv_star_fast2(X0, Y0, X1, Y1, PX, PY, f2(E0.x, E0.y), f2(E0.z, E0.w), us, vs);
           const float2 w = f2(E1.x, E1.y);
-          au = __ffma2_rn(w, us, au);
-          av = __ffma2_rn(w, vs, av);
+          const float2 dx = sub2(sub2(f2(E0.x, E0.y), X0), HX);
+          const float2 dy = sub2(sub2(f2(E0.z, E0.w), Y0), HY);
+          const float2 d2 = __ffma2_rn(dx, dx, __fmul2_rn(dy, dy));
+          if (__all_sync(0xffffffffu, d2.x > LIM.x && d2.y > LIM.y)) {
+            // sums of w (A + i B) and w (A + i B)^3 over the block
+            float2 A, B, n, m;
+            pan_far_inverse(dx, dy, d2, A, B, n, m);
+            const float2 wA = __fmul2_rn(w, A), wB = __fmul2_rn(w, B), nwB = __fmul2_rn(f2(E1.z, E1.w), B);
+            t1r = __fadd2_rn(t1r, wA);
+            t1i = __fadd2_rn(t1i, wB);
+            t3r = __ffma2_rn(wA, n, __ffma2_rn(nwB, m, t3r));
+            t3i = __ffma2_rn(wA, m, __ffma2_rn(wB, n, t3i));
+          } else {
+            float2 us, vs;
+            panel_uv_star_fast2(X0, Y0, X1, Y1, PX, PY, f2(E0.x, E0.y), f2(E0.z, E0.w), us, vs);
+            au = __ffma2_rn(w, us, au);
+            av = __ffma2_rn(w, vs, av);
+          }
         }
+        // v* + i u* = -2 h conj(t1) - 2/3 h^3 conj(t3)
+        const float2 sr = __ffma2_rn(HX, t1r, __ffma2_rn(HY, t1i, __ffma2_rn(H3X, t3r, __fmul2_rn(H3Y, t3i))));
+        const float2 si = __ffma2_rn(HY, t1r, sub2(__ffma2_rn(H3Y, t3r, sub2(z2, __fmul2_rn(H3X, t3i))), __fmul2_rn(HX, t1i)));
+        au = __ffma2_rn(f2(-2.0f, -2.0f), si, au);
+        av = __ffma2_rn(f2(-2.0f, -2.0f), sr, av);
+        t1r = t1i = t3r = t3i = z2;
       } else {
         // VJP of the sheet velocity u = u* A + v* B, v = v* A - u* B at a point with cotangent
         // (lu, lv): P = sum lu u* + lv v*, Q = sum lv u* - lu v*; dL/dA = P, dL/dB = -Q
@@ -635,8 +714,9 @@ int launch_pan(obs_context* ctx, PanArgs& a, bool comp) {
   const int tblocks = (a.nt + PAN_TPB - 1) / PAN_TPB;
   dim3 grid(tblocks, a.nsplit);
   timing_main_begin(ctx);
-  if (comp) pan_kernel<true><<<grid, PAN_THREADS, 0, ctx->stream>>>(a);
-  else pan_kernel<false><<<grid, PAN_THREADS, 0, ctx->stream>>>(a);
+  auto kernel = comp ? (a.mode == 0 ? pan_kernel<0, true> : a.mode == 1 ? pan_kernel<1, true> : pan_kernel<2, true>)
+                     : (a.mode == 0 ? pan_kernel<0, false> : a.mode == 1 ? pan_kernel<1, false> : pan_kernel<2, false>);
+  kernel<<<grid, PAN_THREADS, 0, ctx->stream>>>(a);
   ctx->launches++;
   timing_main_end(ctx);
   cudaError_t e = cudaGetLastError();
