@@ -99,6 +99,10 @@ struct P2PRequest {
   float* extra[4];
 };
 int run_p2p(obs_context* ctx, const P2PRequest& rq);
+// small velocity sums in one launch (p2p_small.cu): whether a request takes it (run_p2p asks first),
+// and the sum
+bool p2p_small_applies(const obs_context* ctx, const P2PRequest& rq);
+int run_p2p_small(obs_context* ctx, const P2PRequest& rq);
 // the velocity of one set on itself, each unordered pair evaluated once (p2p_sym.cu): whether a
 // request takes it (run_p2p asks), and the sum
 bool p2p_sym_applies(const obs_context* ctx, const P2PRequest& rq);
