@@ -21,6 +21,13 @@ int run_adjoint_packed(obs_context* ctx, int accum, int mode, int no, const floa
                        const float* eg, const float* elu, const float* elv, float* gx, float* gy, float* gg,
                        size_t off);
 
+// Small gathers in one launch (adjoint_small.cu), same arguments and results, every core; run_adjoint
+// asks first.
+bool adjoint_small_applies(const obs_context* ctx, int no, int ne);
+int run_adjoint_small(obs_context* ctx, int core, int accum, int mode, int no, const float* ox, const float* oy,
+                      const float* orad, const float* og, int ne, const float* ex, const float* ey, const float* er,
+                      const float* eg, const float* elu, const float* elv, float* gx, float* gy, float* gg);
+
 // Euler (order 1) or Ralston RK2 (order 2) steps of the self-induced velocity, in place on
 // device positions (Convection::advect_1st / advect_2nd_ralston, src/Convection.h:274-466).
 int run_advect(obs_context* ctx, int core, int accum, int order, int n, float* x, float* y,

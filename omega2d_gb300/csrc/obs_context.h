@@ -103,6 +103,9 @@ int run_p2p(obs_context* ctx, const P2PRequest& rq);
 // and the sum
 bool p2p_small_applies(const obs_context* ctx, const P2PRequest& rq);
 int run_p2p_small(obs_context* ctx, const P2PRequest& rq);
+// the same for velocity with gradient, vorticity or shear (p2p_small_res.cu)
+bool p2p_small_res_applies(const obs_context* ctx, const P2PRequest& rq);
+int run_p2p_small_res(obs_context* ctx, const P2PRequest& rq);
 // the velocity of one set on itself, each unordered pair evaluated once (p2p_sym.cu): whether a
 // request takes it (run_p2p asks), and the sum
 bool p2p_sym_applies(const obs_context* ctx, const P2PRequest& rq);

@@ -121,6 +121,7 @@ int run_p2p(obs_context* ctx, const P2PRequest& rq) {
   const bool comp = rq.accum == OBS_COMPENSATED;
   if (rq.ns == 0 || rq.nt == 0) return OBS_OK;
   if (p2p_small_applies(ctx, rq)) return run_p2p_small(ctx, rq);
+  if (p2p_small_res_applies(ctx, rq)) return run_p2p_small_res(ctx, rq);
   if (p2p_sym_applies(ctx, rq)) {
     const int s = run_p2p_sym(ctx, rq);
     if (s != OBS_ERR_ALLOC) return s;             // no room for its partials: the one-sided sum below

@@ -4,20 +4,19 @@
 // The tiled kernels take four or five launches (clear, pack, extrema, sum, reduction) of about 4 us
 // each, which is all the time a thousand particles need.  Here a block owns eight targets, in four
 // f32x2 register pairs of every thread, and its threads stride over the sources, read straight from
-// the caller's arrays (coalesced); the 256 threads' sums are halved over the lanes (16 values in 16
-// shuffles), added over the warps in shared memory and stored.  Nothing is staged, cleared or left
+// the caller's arrays (coalesced); the 256 threads' sums are added over lanes and warps
+// (small_sum.cuh) and stored.  Nothing is staged, cleared or left
 // for a second launch.  Every pair is evaluated one-sided with its own radii.
 #include <cstring>
 
 #include "obs_context.h"
 #include "p2p_sym.cuh"
+#include "small_sum.cuh"
 
 namespace obs {
 
 namespace {
 
-constexpr int SML_THREADS = 256;
-constexpr int SML_WARPS = SML_THREADS / 32;
 constexpr int SML_T = 8;                    // targets per block
 
 struct SmallArgs {
@@ -26,19 +25,11 @@ struct SmallArgs {
   const float* tx; const float* ty; const float* tr;
 };
 
-// (hi, lo) += (bh, bl)
-__device__ __forceinline__ void sml_add(float2& a, float2 b) {
-  two_sum_acc(a.x, a.y, b.x);
-  a.y += b.y;
-}
-
 template <int CORE, bool THICK, bool COMP>
 __global__ void __launch_bounds__(SML_THREADS) p2p_small_kernel(const SmallArgs a, const P2PArgs o) {
   constexpr int NP = SML_T / 2;
-  constexpr unsigned FULL = 0xffffffffu;
   __shared__ float2 red[SML_WARPS][2 * SML_T];
   __shared__ float2 tot[2 * SML_T];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int t0 = blockIdx.x * SML_T;
   float2 nx[NP], ny[NP], zt[NP], u[NP], vn[NP], hu[NP], lu[NP], hv[NP], lv[NP];
 #pragma unroll
@@ -74,39 +65,17 @@ __global__ void __launch_bounds__(SML_THREADS) p2p_small_kernel(const SmallArgs 
       vn[p] = __ffma2_rn(r, dx, vn[p]);
     }
   }
-  // value c of 16: u of targets 0..7, then v; each step keeps the half of the values that the lane's
-  // bit names and adds the other lane's part of it
-  float2 r[2 * SML_T];
+  float2 r[2][SML_T];                              // u, v of the eight targets
 #pragma unroll
   for (int p = 0; p < NP; ++p) {
     two_sum2(hu[p], lu[p], u[p]);
     two_sum2(hv[p], lv[p], vn[p]);
-    r[2 * p] = f2(hu[p].x, lu[p].x);
-    r[2 * p + 1] = f2(hu[p].y, lu[p].y);
-    r[SML_T + 2 * p] = f2(-hv[p].x, -lv[p].x);
-    r[SML_T + 2 * p + 1] = f2(-hv[p].y, -lv[p].y);
+    r[0][2 * p] = f2(hu[p].x, lu[p].x);
+    r[0][2 * p + 1] = f2(hu[p].y, lu[p].y);
+    r[1][2 * p] = f2(-hv[p].x, -lv[p].x);
+    r[1][2 * p + 1] = f2(-hv[p].y, -lv[p].y);
   }
-#pragma unroll
-  for (int h = SML_T; h >= 1; h >>= 1) {           // lane bits 4, 3, 2, 1
-    const int bit = 2 * h;
-    const bool up = (lane & bit) != 0;
-#pragma unroll
-    for (int c = 0; c < h; ++c) {
-      const float2 send = up ? r[c] : r[c + h];
-      float2 keep = up ? r[c + h] : r[c];
-      sml_add(keep, f2(__shfl_xor_sync(FULL, send.x, bit), __shfl_xor_sync(FULL, send.y, bit)));
-      r[c] = keep;
-    }
-  }
-  sml_add(r[0], f2(__shfl_xor_sync(FULL, r[0].x, 1), __shfl_xor_sync(FULL, r[0].y, 1)));
-  if ((lane & 1) == 0) red[w][lane >> 1] = r[0];
-  __syncthreads();
-  if (threadIdx.x < 2 * SML_T) {
-    float2 s = red[0][threadIdx.x];
-    for (int q2 = 1; q2 < SML_WARPS; ++q2) sml_add(s, red[q2][threadIdx.x]);
-    tot[threadIdx.x] = s;
-  }
-  __syncthreads();
+  sml_block_sum<2, SML_T>(r, red, tot);
   const int i = t0 + threadIdx.x;
   if (threadIdx.x < SML_T && i < o.nt) {
     const float2 su = tot[threadIdx.x], sv = tot[SML_T + threadIdx.x];
