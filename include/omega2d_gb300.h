@@ -96,7 +96,7 @@ int obs_selftest_bounded_wait(obs_context* ctx, int which, int max_polls);
 #define OBS_VARIANT_PACKED4 4
 int obs_set_kernel_variant(obs_context* ctx, int variant);
 /* Processing order inside a packed Gaussian or compact-exponential velocity sum.  Binning
- * sorts points into a 256 x 256 Morton-ordered grid over their bounding box (a stable sort), so
+ * sorts points into a 256 x 256 grid along the Hilbert curve over their bounding box (a stable sort), so
  * that each warp's targets and each block of 32 sources lie close together; (warp, block) pairs
  * beyond the core's far radius (4 core radii for the Gaussian, 16^(1/3) for the compact
  * exponential) then take the reference's far-field form G/d^2 without the exponential.
@@ -438,7 +438,7 @@ int obs_points_affect_points_noalloc(void* cuda_stream, int core, int result, in
  * the external solver hook (onbody's treecode, src/Influence.h:31-38, 74-98).  Velocity only
  * (results_t velonly), every core, thick (tr) or field-point (tr == NULL) targets; outputs
  * accumulated like obs_points_affect_points (OBS_FLAG_FINALIZE applies finalize_vels).
- * Sources in Morton order form a tree of 32-source leaves and 4-way nodes carrying `order`
+ * Sources in Hilbert order form a tree of 32-source leaves and 4-way nodes carrying `order`
  * multipole coefficients; a node acts on a warp of 32 targets through its expansion when its
  * radius is at most theta times the distance from its centre to the targets' box and every
  * pair lies where the core equals 1/d^2 (exactly for the Gaussian and compact exponential cut-

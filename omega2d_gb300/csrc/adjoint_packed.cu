@@ -546,11 +546,11 @@ int run_adjoint_packed(obs_context* ctx, int accum, int mode, int no, const floa
   if (e != cudaSuccess) return cuda_status(e);
   int nl = 0;
   if (bin_o) {
-    e = bin_order(ox, oy, no, scratch, operm, st, &nl);
+    e = bin_order(ox, oy, no, scratch, operm, st, &nl, BIN_HILBERT8);
     if (e == cudaSuccess) e = bin_gather(operm, ox, oy, orad, og, no, bx, by, orad ? br : nullptr, og ? bg : nullptr, st, &nl);
     if (e == cudaSuccess && same) e = bin_gather(operm, elu, elv, nullptr, nullptr, no, blu, blv, nullptr, nullptr, st, &nl);
   }
-  if (e == cudaSuccess && bin_e && !(same && bin_o)) e = bin_order(ex, ey, ne, scratch, eperm, st, &nl);
+  if (e == cudaSuccess && bin_e && !(same && bin_o)) e = bin_order(ex, ey, ne, scratch, eperm, st, &nl, BIN_HILBERT8);
   ctx->launches += nl;
   if (e != cudaSuccess) return cuda_status(e);
 

@@ -1,4 +1,4 @@
-// bin_order.cu -- spatial (Morton) order of a point set on the device.
+// bin_order.cu -- spatial (Morton or Hilbert) order of a point set on the device.
 //
 // The packed Gaussian kernel is fastest when the targets of one warp lie close together and
 // the 32 sources of one block lie close together: then most (warp, block) pairs are farther

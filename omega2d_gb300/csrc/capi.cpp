@@ -263,7 +263,7 @@ int obs_morton_order_dev(obs_context* ctx, int n, const float* x, const float* y
   s = ctx->work.ensure(obs::bin_scratch_bytes(n), ctx->stream);
   if (s) return s;
   int nl = 0;
-  s = cuda_status(obs::bin_order(x, y, n, ctx->work.p, perm, ctx->stream, &nl));
+  s = cuda_status(obs::bin_order(x, y, n, ctx->work.p, perm, ctx->stream, &nl, obs::BIN_MORTON8));
   ctx->launches += nl;
   return s;
 }

@@ -139,10 +139,13 @@ cudaError_t packed_launch_pack(const float* sx, const float* sy, const float* sr
 // 256-aligned.  On return perm[k] is the caller's index of the k-th point in the order; the order
 // is stable, so it depends on the input alone.  bin_gather writes x, y (and r, g when given) in
 // that order.
+// The direct sums take BIN_HILBERT8: against the Morton curve the 131,072-particle patch's VJP takes 11.3
+// instead of 12.1 ms, its gradient 8.49 instead of 8.63, the 1M patch's velocity 193.6 instead of 195.8
+// (4096 cells an axis: the same to 1 %, with a third sort pass).
 enum BinCurve { BIN_MORTON8, BIN_HILBERT8, BIN_HILBERT12 };
 size_t bin_scratch_bytes(int n);
 cudaError_t bin_order(const float* x, const float* y, int n, void* scratch, int* perm, cudaStream_t st, int* launches,
-                      BinCurve curve = BIN_MORTON8);
+                      BinCurve curve);
 cudaError_t bin_gather(const int* perm, const float* x, const float* y, const float* r, const float* g, int n,
                        float* bx, float* by, float* br, float* bg, cudaStream_t st, int* launches);
 

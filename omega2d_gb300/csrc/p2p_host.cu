@@ -166,11 +166,11 @@ int run_p2p(obs_context* ctx, const P2PRequest& rq) {
   const int nitems = ntb * nsplit;
   const int grid = std::min(nitems, slots);
   const int nc = ncomp_of(res);
-  // spatial (Morton) order lets the packed Gaussian and compact-exponential kernels skip the
+  // spatial (Hilbert) order lets the packed Gaussian and compact-exponential kernels skip the
   // exponential for far (warp, block) pairs
   const int order = ctx->target_order;
   const bool gauss_packed = packed && masked_core;
-  // Morton order pays from ~3e8 pairs (uniform [-1,1]^2, s = 0.01, Gaussian / compact
+  // spatial order pays from ~3e8 pairs (uniform [-1,1]^2, s = 0.01, Gaussian / compact
   // exponential: 20k +2 % / +25 %, 33k +20 % / +56 %; 8k loses 28 % to the sort)
   const bool big = (double)rq.ns * rq.nt >= 3e8 && rq.nt >= 4096 && rq.ns >= 4096;
   const bool bin_t = gauss_packed && (order == OBS_ORDER_BINNED || order == OBS_ORDER_BINNED_TARGETS ||
@@ -228,10 +228,10 @@ int run_p2p(obs_context* ctx, const P2PRequest& rq) {
   {
     int nl = 0;
     if (bin_t) {
-      e = bin_order(rq.tx, rq.ty, rq.nt, sort_scratch, tperm, st, &nl);
+      e = bin_order(rq.tx, rq.ty, rq.nt, sort_scratch, tperm, st, &nl, BIN_HILBERT8);
       if (e == cudaSuccess) e = bin_gather(tperm, rq.tx, rq.ty, rq.tr, nullptr, rq.nt, bx, by, br, nullptr, st, &nl);
     }
-    if (e == cudaSuccess && bin_s && !same_pts) e = bin_order(rq.sx, rq.sy, rq.ns, sort_scratch, sperm, st, &nl);
+    if (e == cudaSuccess && bin_s && !same_pts) e = bin_order(rq.sx, rq.sy, rq.ns, sort_scratch, sperm, st, &nl, BIN_HILBERT8);
     ctx->launches += nl;
     if (e != cudaSuccess) return cuda_status(e);
   }

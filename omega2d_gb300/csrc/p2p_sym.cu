@@ -161,7 +161,7 @@ int run_p2p_sym(obs_context* ctx, const P2PRequest& rq) {
   timing_begin(ctx);
   cudaError_t e = cudaMemsetAsync(h, 0, sizeof(WorkHeader), st);
   int nl = 0;
-  if (e == cudaSuccess && binned) e = bin_order(rq.sx, rq.sy, n, ctx->work.as<char>(o_sort), perm, st, &nl);
+  if (e == cudaSuccess && binned) e = bin_order(rq.sx, rq.sy, n, ctx->work.as<char>(o_sort), perm, st, &nl, BIN_HILBERT8);
   if (e != cudaSuccess) return cuda_status(e);
   sym_pack_kernel<<<(npad + 255) / 256, 256, 0, st>>>(rq.sx, rq.sy, rq.sr, rq.ss, perm, n, npad, rq.core,
                                                       ctx->work.as<SymGroup>(o_pts), h->meta);
