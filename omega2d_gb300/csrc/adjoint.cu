@@ -299,6 +299,11 @@ int run_adjoint(obs_context* ctx, int core, int accum, int mode,
   if (no == 0 || ne == 0) return OBS_OK;
   if (adjoint_small_applies(ctx, no, ne))
     return run_adjoint_small(ctx, core, accum, mode, no, ox, oy, orad, og, ne, ex, ey, er, eg, elu, elv, gx, gy, gg);
+  if (mode == ADJ_SELF && core == CORE_GAUSS && ctx->kernel_variant == OBS_VARIANT_AUTO &&
+      ctx->target_order == OBS_ORDER_AUTO) {
+    const int s = run_adjoint_self_sym(ctx, accum, no, ox, oy, orad, og, elu, elv, gx, gy, gg, off);
+    if (s != OBS_ERR_ALLOC) return s;
+  }
   if (ctx->kernel_variant != OBS_VARIANT_GENERIC && adjoint_packed_supported(core))
     return run_adjoint_packed(ctx, accum, mode, no, ox, oy, orad, og, ne, ex, ey, er, eg, elu, elv, gx, gy, gg, off);
   const bool comp = accum == OBS_COMPENSATED;

@@ -21,6 +21,11 @@ int run_adjoint_packed(obs_context* ctx, int accum, int mode, int no, const floa
                        const float* eg, const float* elu, const float* elv, float* gx, float* gy, float* gg,
                        size_t off);
 
+// The self-interaction VJP of the Gaussian core, each unordered pair evaluated once (sym_moments.cu);
+// OBS_ERR_ALLOC when its partials find no room (the gathers then serve).
+int run_adjoint_self_sym(obs_context* ctx, int accum, int n, const float* x, const float* y, const float* r,
+                         const float* g, const float* lu, const float* lv, float* gx, float* gy, float* gg, size_t off);
+
 // Small gathers in one launch (adjoint_small.cu), same arguments and results, every core; run_adjoint
 // asks first.
 bool adjoint_small_applies(const obs_context* ctx, int no, int ne);

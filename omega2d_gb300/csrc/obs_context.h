@@ -110,6 +110,9 @@ int run_p2p_small_res(obs_context* ctx, const P2PRequest& rq);
 // request takes it (run_p2p asks), and the sum
 bool p2p_sym_applies(const obs_context* ctx, const P2PRequest& rq);
 int run_p2p_sym(obs_context* ctx, const P2PRequest& rq);
+// the same for velocity with gradient, vorticity or shear, Gaussian core (sym_moments.cu)
+bool p2p_sym_res_applies(const obs_context* ctx, const P2PRequest& rq);
+int run_p2p_sym_res(obs_context* ctx, const P2PRequest& rq);
 double p2p_flops(int core, int result, bool thick, long long ns, long long nt);
 
 // Launch helpers over the same kernels for callers that supply their own scratch.

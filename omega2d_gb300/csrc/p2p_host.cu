@@ -126,6 +126,10 @@ int run_p2p(obs_context* ctx, const P2PRequest& rq) {
     const int s = run_p2p_sym(ctx, rq);
     if (s != OBS_ERR_ALLOC) return s;             // no room for its partials: the one-sided sum below
   }
+  if (p2p_sym_res_applies(ctx, rq)) {
+    const int s = run_p2p_sym_res(ctx, rq);
+    if (s != OBS_ERR_ALLOC) return s;
+  }
   const int res = rq.result;
   const int kcore = (res == RES_PSI) ? CORE_RM : rq.core;
   cudaStream_t st = ctx->stream;

@@ -49,13 +49,8 @@ __global__ void __launch_bounds__(SYM_RED_T * SYM_RED_SUB) sym_reduce_kernel(con
   if (j < a.n) {
     const int k = jb - a.blk0;
     if (k >= 0 && k < a.nblk) {
-      // the pieces of row block k: ranges r0 .. r1 hold its units
-      const int p0 = sym_prefix(a, k), p1 = sym_prefix(a, k + 1) - 1;
-      int r0 = (int)((long long)p0 * a.nrange / a.total), r1 = (int)((long long)p1 * a.nrange / a.total);
-      while (sym_range_begin(a, r0 + 1) <= p0) ++r0;
-      while (sym_range_begin(a, r0) > p0) --r0;
-      while (sym_range_begin(a, r1 + 1) <= p1) ++r1;
-      while (sym_range_begin(a, r1) > p1) --r1;
+      int r0, r1;
+      sym_ranges_of(a, k, r0, r1);
       const float2* rp = a.rowpart + (size_t)k * 2 * SYM_ROWS + (j - jb * SYM_ROWS);
 #pragma unroll 4
       for (int r = r0 + sub; r <= r1; r += SYM_RED_SUB) {
@@ -171,7 +166,7 @@ int run_p2p_sym(obs_context* ctx, const P2PRequest& rq) {
   SymArgs a;
   std::memset(&a, 0, sizeof(a));
   a.grp = ctx->work.as<SymGroup>(o_pts);
-  a.n = n; a.npad = npad; a.ngrp = ngrp;
+  a.n = n; a.npad = npad; a.ngrp = ngrp; a.gpb = SYM_GPB;
   a.counter = &h->counter;
   a.meta = h->meta;
   a.status = ctx->d_status;
@@ -192,12 +187,7 @@ int run_p2p_sym(obs_context* ctx, const P2PRequest& rq) {
     a.nblk = std::min(pass_blk, nblk - b);
     a.first = b == 0;
     a.last = b + a.nblk == nblk;
-    const int K = a.nblk;
-    a.total = K * (ngrp - SYM_GPB * b) - (SYM_GPB / 2) * K * (K - 1);
-    // one range per resident CTA for small sets; up to eight (32 units or more each) for large
-    // ones, whose units differ in cost (near and far column groups)
-    const int per = a.total / slots;
-    a.nrange = std::min(a.total, slots * std::min(8, std::max(1, per / 32)));
+    sym_plan_pass(a, slots);
     if (!a.first && (e = cudaMemsetAsync(&h->counter, 0, sizeof(int), st)) != cudaSuccess) return cuda_status(e);
     if ((e = sym_dispatch(rq.core, comp, a, std::min(a.nrange, slots), st)) != cudaSuccess) return cuda_status(e);
     if (a.last) timing_main_end(ctx);

@@ -61,6 +61,7 @@ struct SymArgs {
   int n;                 // particles
   int npad;              // nblk * SYM_ROWS
   int ngrp;              // 32-column groups holding a particle
+  int gpb;               // groups per row block
   int blk0, nblk;        // row blocks of this pass
   int total;             // (block, group) units of this pass
   int nrange;
@@ -75,10 +76,41 @@ struct SymArgs {
 
 // units of the pass before row block k (of the pass)
 __device__ __forceinline__ int sym_prefix(const SymArgs& a, int k) {
-  return k * (a.ngrp - SYM_GPB * a.blk0) - (SYM_GPB / 2) * k * (k - 1);
+  return k * (a.ngrp - a.gpb * a.blk0) - (a.gpb / 2) * k * (k - 1);
 }
 __device__ __forceinline__ int sym_range_begin(const SymArgs& a, int r) {
   return (int)((long long)a.total * r / a.nrange);
+}
+
+// the row block (of the pass) that unit pos belongs to
+__device__ __forceinline__ int sym_block_of(const SymArgs& a, int pos) {
+  int k = 0, hi = a.nblk - 1;
+  while (k < hi) {
+    const int m = (k + hi + 1) >> 1;
+    if (sym_prefix(a, m) <= pos) k = m;
+    else hi = m - 1;
+  }
+  return k;
+}
+
+// the ranges r0 .. r1 that hold row block k's units
+__device__ __forceinline__ void sym_ranges_of(const SymArgs& a, int k, int& r0, int& r1) {
+  const int p0 = sym_prefix(a, k), p1 = sym_prefix(a, k + 1) - 1;
+  r0 = (int)((long long)p0 * a.nrange / a.total);
+  r1 = (int)((long long)p1 * a.nrange / a.total);
+  while (sym_range_begin(a, r0 + 1) <= p0) ++r0;
+  while (sym_range_begin(a, r0) > p0) --r0;
+  while (sym_range_begin(a, r1 + 1) <= p1) ++r1;
+  while (sym_range_begin(a, r1) > p1) --r1;
+}
+
+// total and nrange of a pass whose blk0 and nblk are set
+inline void sym_plan_pass(SymArgs& a, int slots) {
+  a.total = a.nblk * (a.ngrp - a.gpb * a.blk0) - (a.gpb / 2) * a.nblk * (a.nblk - 1);
+  // one range per resident CTA for small sets; up to eight (32 units or more each) for large
+  // ones, whose units differ in cost (near and far column groups)
+  const int per = a.total / slots, ranges = slots * (per < 64 ? 1 : per >= 256 ? 8 : per / 32);
+  a.nrange = a.total < ranges ? a.total : ranges;
 }
 
 struct SymUni {
@@ -204,15 +236,7 @@ __global__ void __launch_bounds__(SYM_THREADS, 4) p2p_sym_kernel(const SymArgs a
     if (range >= a.nrange) break;
     int pos = sym_range_begin(a, range);
     const int end = sym_range_begin(a, range + 1);
-    int k = 0;
-    {
-      int hi = a.nblk - 1;                         // the block whose units hold pos
-      while (k < hi) {
-        const int m = (k + hi + 1) >> 1;
-        if (sym_prefix(a, m) <= pos) k = m;
-        else hi = m - 1;
-      }
-    }
+    int k = sym_block_of(a, pos);
     for (; pos < end; ++k) {
       const int kbeg = sym_prefix(a, k), kend = min(end, sym_prefix(a, k + 1));
       const int blk = a.blk0 + k;

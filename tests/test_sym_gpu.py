@@ -1,5 +1,6 @@
-"""GPU tests of the self-interaction sum that evaluates each unordered pair once (csrc/p2p_sym.cuh), at the edges of
-its 32-column groups and 1024-row blocks and over several passes, against the FP64 oracle and the one-sided kernels."""
+"""GPU tests of the self-interaction sums that evaluate each unordered pair once (csrc/p2p_sym.cuh, sym_moments.cuh), at
+the edges of their 32-column groups and 1024- or 512-row blocks and over several passes, against the FP64 oracle and the
+one-sided kernels."""
 import numpy as np
 import pytest
 
@@ -53,3 +54,56 @@ def test_several_passes_match_one_sided(ctx, core, n, spread):
     finally:
         ctx.set_kernel_variant(og.VARIANT_AUTO)
     assert rel_err(uo, u) < 2e-6 and rel_err(vo, v) < 2e-6
+
+
+# sizes past the one-launch kernels: one row over a block, an odd remainder
+@pytest.mark.parametrize("accum,tol", [(og.COMPENSATED, 2e-6), (og.PLAIN_F32, 2e-5)])
+@pytest.mark.parametrize("res", [og.VELANDGRAD, og.VELANDVORT, og.VELANDSHEAR])
+@pytest.mark.parametrize("n,spread", [(9217, 0.0), (9999, 0.5), (18_001, 0.0)])
+def test_self_results_match_generic(ctx, accum, tol, res, n, spread):
+    x, y, r, s = cloud(n, n + res, spread)
+    x[n - 1], y[n - 1] = x[1], y[1]    # coincident particles
+    outs = []
+    try:
+        for variant in (og.VARIANT_GENERIC, og.VARIANT_AUTO):
+            ctx.set_kernel_variant(variant)
+            p = og.Points(x, y, r, s)
+            og.points_affect_points(p, p, res, og.ExecEnv(og.CORE_GAUSSIAN, accum, ctx), finalize=True, fs=(1.0, -0.25))
+            outs.append([p.u, p.v] + [a for a in (p.vort, p.shear) if a is not None] + list(p.grad or []))
+    finally:
+        ctx.set_kernel_variant(og.VARIANT_AUTO)
+    for a, b in zip(*outs):
+        assert rel_err(a, b) < tol
+
+
+@pytest.mark.parametrize("accum,tol", [(og.COMPENSATED, 2e-5), (og.PLAIN_F32, 1e-4)])    # as tests/test_adjoint_packed_gpu.py
+@pytest.mark.parametrize("n,spread", [(10_241, 0.0), (12_001, 0.5), (18_001, 0.0)])
+def test_self_vjp_matches_fp64(ctx, restatement, accum, tol, n, spread):
+    x, y, r, s = cloud(n, n, spread)
+    lu, lv = np.random.default_rng(n).normal(0, 1, (2, n)).astype(np.float32)
+    got = og.points_affect_points_vjp_self(og.Points(x, y, r, s), lu, lv, og.ExecEnv(og.CORE_GAUSSIAN, accum, ctx))
+    for a, b in zip(restatement.self_vjp(og.CORE_GAUSSIAN, x, y, r, s, lu, lv), got):
+        assert rel_err(a, b) < tol
+
+
+def test_moment_passes_match_one_sided(ctx):
+    """Gradient and VJP over several passes of row blocks, bit-identical when repeated."""
+    n = 230_001
+    x, y, r, s = cloud(n, n, 0.0, 0.004)
+    lu, lv = np.random.default_rng(n).normal(0, 1, (2, n)).astype(np.float32)
+    env = og.ExecEnv(og.CORE_GAUSSIAN, og.COMPENSATED, ctx)
+
+    def both():
+        p = og.Points(x, y, r, s)
+        og.points_affect_points(p, p, og.VELANDGRAD, env)
+        return [p.u, p.v, *p.grad, *og.points_affect_points_vjp_self(p, lu, lv, env)]
+
+    a, b = both(), both()
+    try:
+        ctx.set_kernel_variant(og.VARIANT_PACKED2)
+        c = both()
+    finally:
+        ctx.set_kernel_variant(og.VARIANT_AUTO)
+    for p, q, t in zip(a, b, c):
+        assert np.array_equal(p, q)
+        assert rel_err(t, p) < 2e-5
