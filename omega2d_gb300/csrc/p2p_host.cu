@@ -141,7 +141,7 @@ int run_p2p(obs_context* ctx, const P2PRequest& rq) {
   // target pairs per thread: one table (packed_np) sizes the target blocks here and picks the
   // kernel instantiation in packed_dispatch
   const bool masked_core = rq.core == CORE_GAUSS || rq.core == CORE_CEXP;
-  int np = packed_np(rq.core, variant, rq.nt);
+  int np = packed_np(rq.core, variant, rq.ns, rq.nt);
   if (packed && res != RES_VEL) np = packed_res_np(res);
   auto launch = [&](const P2PArgs* args, int g, int* occ_out) -> cudaError_t {
     if (!packed) return dispatch(rq.core, thick, res, comp, args, g, st, occ_out);
@@ -174,9 +174,11 @@ int run_p2p(obs_context* ctx, const P2PRequest& rq) {
   // exponential for far (warp, block) pairs
   const int order = ctx->target_order;
   const bool gauss_packed = packed && masked_core;
-  // spatial order pays from ~3e8 pairs (uniform [-1,1]^2, s = 0.01, Gaussian / compact
-  // exponential: 20k +2 % / +25 %, 33k +20 % / +56 %; 8k loses 28 % to the sort)
-  const bool big = (double)rq.ns * rq.nt >= 3e8 && rq.nt >= 4096 && rq.ns >= 4096;
+  // Spatial order pays for the sort from ~7e8 pairs (field points, Gaussian, radius 0.01, binned vs
+  // not: 20,000 of 40,000 particles 368 vs 401 us, 4,000 of 500,000 788 vs 903, 2,000 of 500,000 515 vs
+  // 522, but 5,000 of 100,000 290 vs 274); for the compact exponential's costlier near form from ~3e8
+  const double pairs = (double)rq.ns * rq.nt;
+  const bool big = pairs >= (rq.core == CORE_CEXP ? 3e8 : 7e8) && rq.nt >= 2000 && rq.ns >= 4096;
   const bool bin_t = gauss_packed && (order == OBS_ORDER_BINNED || order == OBS_ORDER_BINNED_TARGETS ||
                                       (order == OBS_ORDER_AUTO && big));
   const bool bin_s = gauss_packed && (order == OBS_ORDER_BINNED || (order == OBS_ORDER_AUTO && big));
