@@ -40,7 +40,9 @@ __device__ __forceinline__ void df_add(float& hi, float& lo, float bh, float bl)
 // own, each in order) to its running sum; the last pass stores the result.  A block takes 64
 // particles; four threads share one, each every fourth partial, added up in thread order.
 constexpr int SYM_RED_T = 64, SYM_RED_SUB = 4;
+template <int NP>
 __global__ void __launch_bounds__(SYM_RED_T * SYM_RED_SUB) sym_reduce_kernel(const SymArgs a, const P2PArgs o) {
+  constexpr int SYM_ROWS = sym_rows(NP);
   __shared__ float4 red[SYM_RED_SUB][SYM_RED_T];
   const int l = threadIdx.x % SYM_RED_T, sub = threadIdx.x / SYM_RED_T;
   const int j = blockIdx.x * SYM_RED_T + l;
@@ -89,27 +91,35 @@ __global__ void __launch_bounds__(SYM_RED_T * SYM_RED_SUB) sym_reduce_kernel(con
   store_target<RES_VEL>(o, j, c);
 }
 
-template <int CORE>
-cudaError_t sym_launch(bool comp, const SymArgs& a, int grid, cudaStream_t st) {
-  if (comp) p2p_sym_kernel<CORE, true><<<grid, SYM_THREADS, 0, st>>>(a);
-  else p2p_sym_kernel<CORE, false><<<grid, SYM_THREADS, 0, st>>>(a);
+// one pass: the sums, then their reduction
+template <int CORE, int NP>
+cudaError_t sym_launch(bool comp, const SymArgs& a, const P2PArgs& o, int grid, cudaStream_t st) {
+  if (comp) p2p_sym_kernel<CORE, true, NP><<<grid, SYM_THREADS, 0, st>>>(a);
+  else p2p_sym_kernel<CORE, false, NP><<<grid, SYM_THREADS, 0, st>>>(a);
+  sym_reduce_kernel<NP><<<(a.n + SYM_RED_T - 1) / SYM_RED_T, SYM_RED_T * SYM_RED_SUB, 0, st>>>(a, o);
   return cudaGetLastError();
 }
 
-cudaError_t sym_dispatch(int core, bool comp, const SymArgs& a, int grid, cudaStream_t st) {
+template <int NP>
+cudaError_t sym_dispatch(int core, bool comp, const SymArgs& a, const P2PArgs& o, int grid, cudaStream_t st) {
   switch (core) {
-    case CORE_RM: return sym_launch<CORE_RM>(comp, a, grid, st);
-    case CORE_GAUSS: return sym_launch<CORE_GAUSS>(comp, a, grid, st);
-    case CORE_V2: return sym_launch<CORE_V2>(comp, a, grid, st);
-    case CORE_WL: return sym_launch<CORE_WL>(comp, a, grid, st);
-    case CORE_V3: return sym_launch<CORE_V3>(comp, a, grid, st);
-    case CORE_SING: return sym_launch<CORE_SING>(comp, a, grid, st);
-    case CORE_CEXP: return sym_launch<CORE_CEXP>(comp, a, grid, st);
+    case CORE_RM: return sym_launch<CORE_RM, NP>(comp, a, o, grid, st);
+    case CORE_GAUSS: return sym_launch<CORE_GAUSS, NP>(comp, a, o, grid, st);
+    case CORE_V2: return sym_launch<CORE_V2, NP>(comp, a, o, grid, st);
+    case CORE_WL: return sym_launch<CORE_WL, NP>(comp, a, o, grid, st);
+    case CORE_V3: return sym_launch<CORE_V3, NP>(comp, a, o, grid, st);
+    case CORE_SING: return sym_launch<CORE_SING, NP>(comp, a, o, grid, st);
+    case CORE_CEXP: return sym_launch<CORE_CEXP, NP>(comp, a, o, grid, st);
     default: return cudaErrorInvalidValue;
   }
 }
 
-constexpr int SYM_OCC = 4;                            // CTAs per SM (__launch_bounds__: 128 registers)
+// Row pairs per thread: eight pass a column's sums on half as often per pair as four, but their row
+// blocks are twice as large (8 vs 4: 20,000 Rosenhead-Moore, ten steps 1220 vs 1204 us; 33,001
+// Vatistas-2 with varying radii 284 vs 306 us; 131,072 plain 3.23 vs 3.49 ms; 400,000 Gaussian 29.8 vs
+// 31.2; the 1M patch 182 vs 194; 200,000 with varying Gaussian radii 13.2 vs 12.9)
+int sym_np(int n) { return n >= 30000 ? 8 : 4; }
+
 constexpr size_t SYM_COL_BYTES = (size_t)1 << 30;     // column partials held at once
 
 }  // namespace
@@ -131,10 +141,11 @@ int run_p2p_sym(obs_context* ctx, const P2PRequest& rq) {
   const int n = rq.nt;
   const bool comp = rq.accum == OBS_COMPENSATED;
   cudaStream_t st = ctx->stream;
-  const int nblk = (n + SYM_ROWS - 1) / SYM_ROWS;
-  const int npad = nblk * SYM_ROWS;
+  const int np = sym_np(n), rows = sym_rows(np);
+  const int nblk = (n + rows - 1) / rows;
+  const int npad = nblk * rows;
   const int ngrp = (n + SYM_GRP - 1) / SYM_GRP;
-  const int slots = SYM_OCC * ctx->num_sms;
+  const int slots = sym_occ(np) * ctx->num_sms;
   const bool binned = (rq.core == CORE_GAUSS || rq.core == CORE_CEXP) && (double)n * n >= 3e8;
   const int pass_blk = std::min(nblk, std::max(1, (int)(SYM_COL_BYTES / ((size_t)npad * sizeof(float2)))));
   const int max_range = 8 * slots;
@@ -145,7 +156,7 @@ int run_p2p_sym(obs_context* ctx, const P2PRequest& rq) {
   const size_t o_run = o_pts + (size_t)(npad / SYM_GRP) * sizeof(SymGroup);
   const size_t o_col = o_run + (pass_blk < nblk ? al((size_t)npad * sizeof(float4)) : 0);
   const size_t o_row = o_col + al((size_t)pass_blk * npad * sizeof(float2));
-  const size_t o_perm = o_row + (size_t)(max_range + pass_blk) * 2 * SYM_ROWS * sizeof(float2);
+  const size_t o_perm = o_row + (size_t)(max_range + pass_blk) * 2 * rows * sizeof(float2);
   const size_t o_sort = o_perm + (binned ? al((size_t)n * sizeof(int)) : 0);
   const size_t bytes = o_sort + (binned ? bin_scratch_bytes(n) : 0);
   int s = ctx->work.ensure(bytes, st);
@@ -166,7 +177,7 @@ int run_p2p_sym(obs_context* ctx, const P2PRequest& rq) {
   SymArgs a;
   std::memset(&a, 0, sizeof(a));
   a.grp = ctx->work.as<SymGroup>(o_pts);
-  a.n = n; a.npad = npad; a.ngrp = ngrp; a.gpb = SYM_GPB;
+  a.n = n; a.npad = npad; a.ngrp = ngrp; a.gpb = sym_gpb(np);
   a.counter = &h->counter;
   a.meta = h->meta;
   a.status = ctx->d_status;
@@ -189,13 +200,12 @@ int run_p2p_sym(obs_context* ctx, const P2PRequest& rq) {
     a.last = b + a.nblk == nblk;
     sym_plan_pass(a, slots);
     if (!a.first && (e = cudaMemsetAsync(&h->counter, 0, sizeof(int), st)) != cudaSuccess) return cuda_status(e);
-    if ((e = sym_dispatch(rq.core, comp, a, std::min(a.nrange, slots), st)) != cudaSuccess) return cuda_status(e);
-    if (a.last) timing_main_end(ctx);
-    // particles before this pass's first row block take nothing from it
-    sym_reduce_kernel<<<(n + SYM_RED_T - 1) / SYM_RED_T, SYM_RED_T * SYM_RED_SUB, 0, st>>>(a, o);
+    const int grid = std::min(a.nrange, slots);
+    e = np == 8 ? sym_dispatch<8>(rq.core, comp, a, o, grid, st) : sym_dispatch<4>(rq.core, comp, a, o, grid, st);
     ctx->launches += 2;
-    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e);
+    if (e != cudaSuccess) return cuda_status(e);
   }
+  timing_main_end(ctx);
   timing_end(ctx);
   return OBS_OK;
 }

@@ -9,20 +9,19 @@
 // f32x2 operation takes 2.1 SM clocks per scheduler with one or two distinct register operands
 // and 3.1 with three (measured; two scalar FMAs in its place take as long), so the four
 // accumulations of a pair of pairs cost half of its 24 clocks; MUFU is at 50 %, the FMA pipe at
-// 67 %.  Other orders and groupings of the same operations, the accumulations as scalars, and 16
-// to 48 rows per thread pair all came within 5 % of one another.  Measured (compensated, one-sided
-// -> here): 1M Gaussian patch 249 -> 196 ms (5.1e12 interactions/s), 131,072 Vatistas-2 plain 4.29
-// -> 3.43 ms, 33,001 Vatistas-2 with varying radii 415 -> 298 us, ten Euler steps of 20,000
-// Rosenhead-Moore 1.65 -> 1.19 ms.
+// 67 %.  Other orders and groupings of the same operations and the accumulations as scalars came
+// within 3 % of one another.  Measured (compensated, one-sided -> here): 1M Gaussian patch 249 -> 182
+// ms (5.5e12 interactions/s), 131,072 Vatistas-2 plain 4.29 -> 3.23 ms, 33,001 Vatistas-2 with varying
+// radii 415 -> 284 us, ten Euler steps of 20,000 Rosenhead-Moore 1.65 -> 1.19 ms.
 //
-// Layout: a row block is 1024 particles, eight per thread of a 128-thread CTA in f32x2 register
-// pairs (a warp owns 256 consecutive ones); columns are taken 32 at a time, one per lane: in
-// step s of 32 lane l meets column l ^ s (a conflict-free shared-memory read) with its eight
-// rows, and the column's running sum (the eight terms added first) moves to the lane that meets it next by shuffle, so after 32
-// steps every lane holds its own column's sum over the warp's 256 rows.  The four warps' sums are
-// added in shared memory and leave as one FP32 pair per (row block, column); a row's own sums
-// stay in registers over a whole run of columns (folded into two-sum pairs every 32 columns when
-// compensated).  Rows against their own block are one-sided.
+// Layout: a row block is 1024 (or 2048) particles, eight (or sixteen) per thread of a 128-thread
+// CTA in f32x2 register pairs (a warp owns 256 or 512 consecutive ones); columns are taken 32 at a
+// time, one per lane: in step s of 32 lane l meets column l ^ s (a conflict-free shared-memory read)
+// with its rows, and the column's running sum (the step's terms added first) moves to the lane that
+// meets it next by shuffle, so after 32 steps every lane holds its own column's sum over the warp's
+// rows.  The four warps' sums are added in shared memory and leave as one FP32 pair per (row block,
+// column); a row's own sums stay in registers over a whole run of columns (folded into two-sum pairs
+// every 32 columns when compensated).  Rows against their own block are one-sided.
 //
 // Work: row block k meets every 32-column group from its own first one on; these (block, group)
 // units in order form a line of `total` units cut into equal ranges that the CTAs take from a
@@ -33,18 +32,19 @@
 // blocks that keep them within a fixed scratch size.
 #pragma once
 
+#include <type_traits>
+
 #include "p2p_kernel.cuh"
 
 namespace obs {
 
 constexpr int SYM_THREADS = 128;
-constexpr int SYM_NP = 4;                          // f32x2 row pairs per thread
-constexpr int SYM_ROWS = SYM_THREADS * 2 * SYM_NP; // 1024 rows per block
-constexpr int SYM_WROWS = 64 * SYM_NP;             // rows per warp
 constexpr int SYM_GRP = 32;                        // columns per group
 constexpr int SYM_TG = 8;                          // groups per staged tile
 constexpr int SYM_TILE = SYM_GRP * SYM_TG;
-constexpr int SYM_GPB = SYM_ROWS / SYM_GRP;        // groups per row block
+// NP f32x2 row pairs per thread: rows and groups per row block
+constexpr int sym_gpb(int np) { return SYM_THREADS / 32 * 2 * np; }
+constexpr int sym_rows(int np) { return sym_gpb(np) * SYM_GRP; }
 constexpr float SYM_FAR = 1.0e18f;                 // padding coordinate: K there is finite and tiny
 
 // A group's 32 columns as staged, every value twice for the packed operands: a warp's reads of
@@ -59,7 +59,7 @@ static_assert(sizeof(SymGroup) == 1024, "group record");
 struct SymArgs {
   const SymGroup* grp;     // the particles in groups of 32, padded to whole row blocks
   int n;                 // particles
-  int npad;              // nblk * SYM_ROWS
+  int npad;              // particles padded to whole row blocks
   int ngrp;              // 32-column groups holding a particle
   int gpb;               // groups per row block
   int blk0, nblk;        // row blocks of this pass
@@ -69,7 +69,7 @@ struct SymArgs {
   const unsigned* meta;  // radius extrema (~min, max bits)
   int* status;
   float2* colpart;       // [nblk][npad] (sum G K dy, sum G K dx)
-  float2* rowpart;       // [nrange + nblk][2][SYM_ROWS] (hi, lo)
+  float2* rowpart;       // [nrange + nblk][2][rows of a block] (hi, lo)
   float4* run;           // [npad] running sums (u hi, u lo, v hi, v lo) over the passes
   int first, last;       // first / last pass
 };
@@ -168,23 +168,24 @@ __device__ __forceinline__ float2 sym_core(float2 d2, float2 zz, const SymUni& q
 }
 
 // one 32-column group against the warp's rows; cu, cv: the column sums, back at their own lane
-// at the end.  zrow: this thread's rows' radius terms in shared memory (FORM 2).
-template <int CORE, int FORM>
+// at the end (COLS; a row block's own columns take none).  zrow: this thread's rows' radius terms in
+// shared memory (FORM 2).
+template <int CORE, int FORM, bool COLS, int NP>
 __device__ __forceinline__ void sym_group(const SymGroup& grp, int lane, const SymUni& q,
-                                          const float2 (&nx)[SYM_NP], const float2 (&ny)[SYM_NP],
-                                          const float2 (&g)[SYM_NP], const float* __restrict__ zrow,
-                                          float2 (&u)[SYM_NP], float2 (&vn)[SYM_NP], float& cu, float& cv) {
+                                          const float2 (&nx)[NP], const float2 (&ny)[NP], const float2 (&g)[NP],
+                                          const float* __restrict__ zrow, float2 (&u)[NP], float2 (&vn)[NP], float& cu,
+                                          float& cv) {
   cu = cv = 0.0f;
 #pragma unroll 4
   for (int s = 0; s < SYM_GRP; ++s) {
-    float2 su = f2(0.0f, 0.0f), sv = f2(0.0f, 0.0f);   // this step's eight rows
+    float2 su = f2(0.0f, 0.0f), sv = f2(0.0f, 0.0f);   // this step's rows
     const int col = lane ^ s;
     const float4 c = grp.xy[col];
     const float2 cx = f2(c.x, c.y), cy = f2(c.z, c.w), cg = grp.g[col];
     float2 cz = f2(0.0f, 0.0f);
     if constexpr (FORM == 2) cz = grp.z[col];
 #pragma unroll
-    for (int p = 0; p < SYM_NP; ++p) {
+    for (int p = 0; p < NP; ++p) {
       const float2 dx = __fadd2_rn(cx, nx[p]);
       const float2 dy = __fadd2_rn(cy, ny[p]);
       float2 zz = f2(q.us2, q.us2);
@@ -193,12 +194,15 @@ __device__ __forceinline__ void sym_group(const SymGroup& grp, int lane, const S
       // Rosenhead-Moore takes d^2 + s^2 in the same two operations
       const float2 d2 = __ffma2_rn(dx, dx, CORE == CORE_RM ? __ffma2_rn(dy, dy, zz) : __fmul2_rn(dy, dy));
       const float2 k = sym_core<CORE, FORM>(d2, zz, q);
-      const float2 rr = __fmul2_rn(cg, k), rc = __fmul2_rn(g[p], k);
+      const float2 rr = __fmul2_rn(cg, k);
       u[p] = __ffma2_rn(rr, dy, u[p]);
       vn[p] = __ffma2_rn(rr, dx, vn[p]);
+      if constexpr (!COLS) continue;
+      const float2 rc = __fmul2_rn(g[p], k);
       su = (p == 0) ? __fmul2_rn(rc, dy) : __ffma2_rn(rc, dy, su);
       sv = (p == 0) ? __fmul2_rn(rc, dx) : __ffma2_rn(rc, dx, sv);
     }
+    if constexpr (!COLS) continue;
     // hand the column's sums to the lane that meets it next (after the last step: to its own)
     const int m = (s ^ (s + 1)) & 31;
     cu = __shfl_xor_sync(0xffffffffu, cu + (su.x + su.y), m);
@@ -206,12 +210,16 @@ __device__ __forceinline__ void sym_group(const SymGroup& grp, int lane, const S
   }
 }
 
-template <int CORE, bool COMP>
-__global__ void __launch_bounds__(SYM_THREADS, 4) p2p_sym_kernel(const SymArgs a) {
+// CTAs per SM: 128 registers a thread for four row pairs, 255 for eight
+constexpr int sym_occ(int np) { return np == 8 ? 2 : 4; }
+
+template <int CORE, bool COMP, int NP>
+__global__ void __launch_bounds__(SYM_THREADS, sym_occ(NP)) p2p_sym_kernel(const SymArgs a) {
+  constexpr int GPB = sym_gpb(NP), ROWS = sym_rows(NP);
   constexpr bool MASKED = CORE == CORE_GAUSS || CORE == CORE_CEXP;
   __shared__ SymGroup tile[NSTAGE][SYM_TG];
   __shared__ float2 csum[SYM_THREADS / 32][SYM_TILE];   // per-warp column sums of the tile
-  __shared__ float zrow[2 * SYM_NP * SYM_THREADS];
+  __shared__ float zrow[2 * NP * SYM_THREADS];
   __shared__ __align__(8) uint64_t bar[NSTAGE];
   __shared__ int s_range;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -240,9 +248,9 @@ __global__ void __launch_bounds__(SYM_THREADS, 4) p2p_sym_kernel(const SymArgs a
     for (; pos < end; ++k) {
       const int kbeg = sym_prefix(a, k), kend = min(end, sym_prefix(a, k + 1));
       const int blk = a.blk0 + k;
-      const int g0 = SYM_GPB * blk + (pos - kbeg);          // first column group of this piece
+      const int g0 = GPB * blk + (pos - kbeg);          // first column group of this piece
       const int ng = kend - pos;
-      const int gdiag = SYM_GPB * (blk + 1);                // groups below this are the block's own
+      const int gdiag = GPB * (blk + 1);                // groups below this are the block's own
       const int ntile = (ng + SYM_TG - 1) / SYM_TG;
       pos = kend;
       auto fetch = [&](int t, int st) {                     // thread 0
@@ -255,16 +263,16 @@ __global__ void __launch_bounds__(SYM_THREADS, 4) p2p_sym_kernel(const SymArgs a
         fence_proxy_async_smem();
         for (int s = 0; s < NSTAGE && s < ntile; ++s) fetch(s, (kt + s) % NSTAGE);
       }
-      float2 nx[SYM_NP], ny[SYM_NP], g[SYM_NP], u[SYM_NP], vn[SYM_NP], hu[SYM_NP], lu[SYM_NP], hv[SYM_NP], lv[SYM_NP];
+      float2 nx[NP], ny[NP], g[NP], u[NP], vn[NP], hu[NP], lu[NP], hv[NP], lv[NP];
       float bx0 = 3.0e38f, bx1 = -3.0e38f, by0 = 3.0e38f, by1 = -3.0e38f;
-      const int row0 = blk * SYM_ROWS + warp * SYM_WROWS + lane;
+      const int row0 = blk * ROWS + warp * 64 * NP + lane;
 #pragma unroll
-      for (int p = 0; p < SYM_NP; ++p) {
+      for (int p = 0; p < NP; ++p) {
         float4 w[2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           // the 32 rows of (p, h) are one group
-          const SymGroup& r = a.grp[blk * SYM_GPB + warp * (SYM_WROWS / 32) + 2 * p + h];
+          const SymGroup& r = a.grp[blk * GPB + warp * 2 * NP + 2 * p + h];
           const float4 xy = r.xy[lane];
           w[h] = make_float4(xy.x, xy.z, r.g[lane].x, r.z[lane].x);
           if (row0 + (2 * p + h) * 32 < a.n) {
@@ -300,24 +308,26 @@ __global__ void __launch_bounds__(SYM_THREADS, 4) p2p_sym_kernel(const SymArgs a
         for (int b = 0; b < cnt; ++b) {
           const SymGroup& grp = tile[st][b];
           float cu, cv;
-          if (!unif) {
-            sym_group<CORE, 2>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, cu, cv);
-          } else if constexpr (MASKED) {
+          bool far = false;
+          if constexpr (MASKED) {
             const float4 c = grp.xy[lane];
             const float ex = fmaxf(0.0f, fmaxf(bx0 - c.x, c.x - bx1));
             const float ey = fmaxf(0.0f, fmaxf(by0 - c.z, c.z - by1));
-            // negated, so that a NaN coordinate takes the near form
-            if (__any_sync(0xffffffffu, !(fmaf(ex, ex, ey * ey) > q.lim)))
-              sym_group<CORE, 1>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, cu, cv);
-            else
-              sym_group<CORE, 0>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, cu, cv);
-          } else {
-            sym_group<CORE, 1>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, cu, cv);
+            // a NaN coordinate takes the near form
+            far = unif && __all_sync(0xffffffffu, fmaf(ex, ex, ey * ey) > q.lim);
           }
+          auto run = [&](auto cols) {
+            constexpr bool COLS = decltype(cols)::value;
+            if (!unif) sym_group<CORE, 2, COLS, NP>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, cu, cv);
+            else if (MASKED && far) sym_group<CORE, MASKED ? 0 : 1, COLS, NP>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, cu, cv);
+            else sym_group<CORE, 1, COLS, NP>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, cu, cv);
+          };
+          if (g0 + t * SYM_TG + b < gdiag) run(std::false_type{});
+          else run(std::true_type{});
           csum[warp][b * SYM_GRP + lane] = make_float2(cu, cv);
           if constexpr (COMP) {
 #pragma unroll
-            for (int p = 0; p < SYM_NP; ++p) {
+            for (int p = 0; p < NP; ++p) {
               two_sum2(hu[p], lu[p], u[p]);
               two_sum2(hv[p], lv[p], vn[p]);
               u[p] = vn[p] = f2(0.0f, 0.0f);
@@ -337,18 +347,18 @@ __global__ void __launch_bounds__(SYM_THREADS, 4) p2p_sym_kernel(const SymArgs a
           a.colpart[(size_t)k * a.npad + c0 + c] = make_float2((s0.x + s1.x) + (s2.x + s3.x), (s0.y + s1.y) + (s2.y + s3.y));
         }
       }
-      float2* rp = a.rowpart + (size_t)(range + k) * 2 * SYM_ROWS;
+      float2* rp = a.rowpart + (size_t)(range + k) * 2 * ROWS;
 #pragma unroll
-      for (int p = 0; p < SYM_NP; ++p) {
+      for (int p = 0; p < NP; ++p) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const int i = warp * SYM_WROWS + (2 * p + h) * 32 + lane;
+          const int i = warp * 64 * NP + (2 * p + h) * 32 + lane;
           if (COMP) {
             rp[i] = h ? make_float2(hu[p].y, lu[p].y) : make_float2(hu[p].x, lu[p].x);
-            rp[SYM_ROWS + i] = h ? make_float2(hv[p].y, lv[p].y) : make_float2(hv[p].x, lv[p].x);
+            rp[ROWS + i] = h ? make_float2(hv[p].y, lv[p].y) : make_float2(hv[p].x, lv[p].x);
           } else {
             rp[i] = make_float2(h ? u[p].y : u[p].x, 0.0f);
-            rp[SYM_ROWS + i] = make_float2(h ? vn[p].y : vn[p].x, 0.0f);
+            rp[ROWS + i] = make_float2(h ? vn[p].y : vn[p].x, 0.0f);
           }
         }
       }
