@@ -37,6 +37,15 @@ struct GmState {
                    // products use the FP32 plane of A (iterative refinement)
 };
 
+// what the host reads after a cycle, in one copy: the true residual norm, ||b||, the cycle's start
+// norm and iteration count, the plane's flag and the context's status word
+struct GmReport {
+  double rn, bnrm, beta;
+  int kd;
+  unsigned range;
+  int status, pad;
+};
+
 // part[c][i] = sum_{j in chunk c} A[j*n + i] * (x[j] * dinv[j])   (column-major A); nothing when
 // nz is given and *nz == 0 (x known to be zero)
 __global__ void __launch_bounds__(GM_THREADS) gemv_part_kernel(const double* __restrict__ A, int n,
@@ -242,11 +251,14 @@ __global__ void __launch_bounds__(GM_THREADS) prep_kernel(const double* __restri
   if (last_block_sum(bb, bpart, cnt, sh, &t) && threadIdx.x == 0) *bnrm = sqrt(t);
 }
 
-// y = b - sum_c part[c] (y = b when nz is given and *nz == 0) and *out = ||y|| (*alt then)
+// y = b - sum_c part[c] (y = b when nz is given and *nz == 0) and *out = ||y|| (*alt = ||b|| then);
+// the report of the cycle before, if there was one
 __global__ void __launch_bounds__(GM_THREADS) gemv_sum_norm_kernel(const double* __restrict__ part, int nchunk, int n,
                                                                    const double* __restrict__ b, double* __restrict__ y,
                                                                    const unsigned* nz, double* bpart, unsigned* cnt,
-                                                                   double* out, const double* alt) {
+                                                                   double* out, const double* alt, const GmState* st,
+                                                                   const unsigned* range, const int* status,
+                                                                   GmReport* rep) {
   __shared__ double sh[32];
   const bool zero = nz && *nz == 0;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -266,7 +278,10 @@ __global__ void __launch_bounds__(GM_THREADS) gemv_sum_norm_kernel(const double*
     return;
   }
   double t;
-  if (last_block_sum(r * r, bpart, cnt, sh, &t) && threadIdx.x == 0) *out = sqrt(t);
+  if (last_block_sum(r * r, bpart, cnt, sh, &t) && threadIdx.x == 0) {
+    *out = sqrt(t);
+    *rep = GmReport{sqrt(t), *alt, st->beta, st->kdone, *range, *status, 0};
+  }
 }
 
 // ---------------------------------------------------------------- one restart cycle in one launch
@@ -889,7 +904,7 @@ int gmres_f64(obs_context* ctx, int n, const double* A, const double* b, double*
     }
   }
   const size_t NP2 = (N + 1) / 2;                  // column pairs
-  const size_t o_bp = o_n + 256;                   // block partials of the fused norms
+  const size_t o_bp = o_n + 256;                   // [norms, report | block partials of the fused norms]
   const size_t o_gp = o_bp + al((size_t)((n + GM_THREADS - 1) / GM_THREADS) * 8);
   const size_t o_gv = o_gp + al((size_t)2 * gc_grid * (m + 2) * 8);
   const size_t o_gl = o_gv + al(NP2 * 16);
@@ -914,6 +929,7 @@ int gmres_f64(obs_context* ctx, int n, const double* A, const double* b, double*
   float4* gvp = ctx->work.as<float4>(o_gv);
   float2* gvl = ctx->work.as<float2>(o_gl);
   double* bpart = ctx->work.as<double>(o_bp);
+  GmReport* report = reinterpret_cast<GmReport*>(nrm + 4);
   // [0] barrier arrivals, [1] plane range flag, [2] x != 0, [3] arrivals of the fused norms
   unsigned* gbar = ctx->work.as<unsigned>(o_gb);
   float2* AH = fused ? ctx->work.as<float2>(o_ap) : nullptr;
@@ -939,32 +955,29 @@ int gmres_f64(obs_context* ctx, int n, const double* A, const double* b, double*
   // (known on the device only) gives r = b and ||b|| without the product
   auto residual = [&](const unsigned* nz) {
     gemv_part_kernel<<<ggrid, GM_THREADS, 0, strm>>>(A, n, x, nullptr, part, nullptr, nz);
-    gemv_sum_norm_kernel<<<gb, GM_THREADS, 0, strm>>>(part, nchunk, n, b, w, nz, bpart, gbar + 3, nrm, nrm + 1);
+    gemv_sum_norm_kernel<<<gb, GM_THREADS, 0, strm>>>(part, nchunk, n, b, w, nz, bpart, gbar + 3, nrm, nrm + 1, st,
+                                                      gbar + 1, ctx->d_status, report);
     launched(2);
   };
   residual(gbar + 2);
   // The first cycle is launched without a host round trip: its start kernel forms the tolerance
   // from ||b|| and stops at once when the initial residual meets it, and the fused cycle returns
   // at once when the plane cannot carry A (the loop then continues with FP64 products).  After
-  // each cycle one round trip reads the true residual norm, the cycle's start norm and
-  // iteration count, ||b||, the plane's flag and the status block (a barrier that gave up
-  // leaves its record there).
+  // each cycle one copy of the report reads the true residual norm, the cycle's start norm and
+  // iteration count, ||b||, the plane's flag and the status word (a barrier that gave up leaves
+  // its record there).
   int total_it = 0;
   double rel = 0.0;
   for (bool check = false;; check = true) {
     if (check) {
-      double rn = 0.0, bnorm = 0.0, beta = 0.0;
-      int kd = 0, flag = 0;
-      unsigned range_bad = 0;
-      e = cudaMemcpyAsync(&rn, nrm, 8, cudaMemcpyDeviceToHost, strm);
-      if (e == cudaSuccess) e = cudaMemcpyAsync(&bnorm, nrm + 1, 8, cudaMemcpyDeviceToHost, strm);
-      if (e == cudaSuccess) e = cudaMemcpyAsync(&beta, &st->beta, 8, cudaMemcpyDeviceToHost, strm);
-      if (e == cudaSuccess) e = cudaMemcpyAsync(&kd, &st->kdone, 4, cudaMemcpyDeviceToHost, strm);
-      if (e == cudaSuccess) e = cudaMemcpyAsync(&range_bad, gbar + 1, 4, cudaMemcpyDeviceToHost, strm);
-      if (e == cudaSuccess) e = cudaMemcpyAsync(&flag, ctx->d_status, 4, cudaMemcpyDeviceToHost, strm);
+      GmReport h{};
+      e = cudaMemcpyAsync(&h, report, sizeof(h), cudaMemcpyDeviceToHost, strm);
       if (e == cudaSuccess) e = cudaStreamSynchronize(strm);
       if (e != cudaSuccess) return cuda_status(e);
-      if (flag) return take_device_status(ctx);
+      if (h.status) return take_device_status(ctx);
+      const double rn = h.rn, bnorm = h.bnrm, beta = h.beta;
+      const int kd = h.kd;
+      const unsigned range_bad = h.range;
       const double bref = (bnorm == 0.0) ? 1.0 : bnorm;   // src/BEM.h:227-229 divides by 1 then
       rel = rn / bref;
       bool stalled = false;

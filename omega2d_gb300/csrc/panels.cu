@@ -568,7 +568,7 @@ __global__ void coeff_kernel(const float4* __restrict__ SP, const float4* __rest
                              const float* __restrict__ SL, int nsrc,
                              const float4* __restrict__ TP, const float4* __restrict__ TQ,
                              const float* __restrict__ TL, int ntarg, int nunk, int self,
-                             float* __restrict__ A32, double* __restrict__ A64) {
+                             float* __restrict__ A32, double* __restrict__ A64, bool wide) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y;
   if (i >= ntarg || j >= nsrc) return;
@@ -617,7 +617,10 @@ __global__ void coeff_kernel(const float4* __restrict__ SP, const float4* __rest
   if (nunk == 2) {
     const size_t c0 = (size_t)(2 * j) * nrows + 2 * i, c1 = (size_t)(2 * j + 1) * nrows + 2 * i;
     if (A32) { A32[c0] = c11; A32[c0 + 1] = c12; A32[c1] = c21; A32[c1 + 1] = c22; }
-    if (A64) {
+    if (A64 && wide) {                        // a column's two entries of this panel in one store
+      *reinterpret_cast<double2*>(A64 + c0) = make_double2(f2d_bits(c11), f2d_bits(c12));
+      *reinterpret_cast<double2*>(A64 + c1) = make_double2(f2d_bits(c21), f2d_bits(c22));
+    } else if (A64) {
       A64[c0] = f2d_bits(c11);
       A64[c0 + 1] = f2d_bits(c12);
       A64[c1] = f2d_bits(c21);
@@ -867,7 +870,8 @@ int run_panels_on_panels_coeff(obs_context* ctx, const PanelSet& src, const Pane
   if (s) return s;
   dim3 grid((targ.npan + 127) / 128, src.npan);
   timing_main_begin(ctx);
-  coeff_kernel<<<grid, 128, 0, ctx->stream>>>(SP, SQ, SL, src.npan, TP, TQ, TL, targ.npan, nunk, self, A32, A64);
+  coeff_kernel<<<grid, 128, 0, ctx->stream>>>(SP, SQ, SL, src.npan, TP, TQ, TL, targ.npan, nunk, self, A32, A64,
+                                                 (reinterpret_cast<uintptr_t>(A64) & 15) == 0);
   ctx->launches++;
   timing_main_end(ctx);
   timing_end(ctx);
