@@ -357,7 +357,8 @@ struct GcArgs {
   float2* vsl;                                  // per column pair: negated lo of Dinv v_j
   double* x;
   float2* P;                                    // partials (double-float): [2][grid][m+2]
-  unsigned* bar;                                // arrival counter, zeroed before each launch
+  unsigned* bar;                                // arrival counter, zeroed before each launch; null:
+                                                // the grid is one cluster
   const unsigned* plane_flag;                   // bit 0: entries out of the plane's range
   GmState* st;
   int* status;
@@ -394,6 +395,15 @@ __device__ bool gc_barrier(unsigned* bar, int* status, unsigned nb, unsigned arr
     }
   }
   return __syncthreads_and(ok) != 0;
+}
+
+// A system of at most GC_CLUSTER row groups runs as one thread-block cluster, whose hardware barrier
+// (release and acquire, so the blocks' global writes are seen) takes about 500 SM clocks; the counter's
+// polls through L2 take 2,500 to 3,500, two of them a fifth of a small system's iteration.  The blocks
+// of a cluster are resident together and none leaves before the others, so the barrier ends.
+constexpr int GC_CLUSTER = 16;
+__device__ __forceinline__ void gc_cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // (S, s) += (T, t) in double-float: two-sum of the leading parts, the trailing parts added to
@@ -506,19 +516,46 @@ __device__ void gc_gram_matvec(const float2* G, int ldg, int n, const float2* x,
   __syncthreads();
 }
 
+// the sum over the warps of red[warp][row], row = this warp's number, in double-float by a fixed
+// shuffle tree: all 32 rows at once, a warp each (one warp adding the 32 partials of its lane's row in
+// turn takes two to four times as long)
+__device__ __forceinline__ float2 gc_cross_sum(float2 (*red)[33]) {
+  __syncthreads();
+  const float2 t = warp_sum_df(red[threadIdx.x & 31][threadIdx.x >> 5]);
+  __syncthreads();
+  return t;
+}
+
 // sum_{k <= j} V_k[r] c[k] for local row group q in double-float (warps split k, fixed-order
-// sum); valid in warp 0
-__device__ float2 gc_vsum(const GcRows& R, int j, int q, const float2* c, float2 (*red)[32]) {
+// sum); every lane of warp r gets row r
+__device__ float2 gc_vsum(const GcRows& R, int j, int q, const float2* c, float2 (*red)[33]) {
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
   float2 s = make_float2(0.0f, 0.0f);
   for (int k = wp; k <= j; k += GC_WARPS) s = df_sum(s, df_mul(R.Vs[(size_t)k * R.RB + q * 32 + lane], c[k]));
   red[wp][lane] = s;
-  __syncthreads();
-  float2 t = make_float2(0.0f, 0.0f);
-  if (wp == 0)
-    for (int p = 0; p < GC_WARPS; ++p) t = df_sum(t, red[p][lane]);
-  __syncthreads();
-  return t;
+  return gc_cross_sum(red);
+}
+
+// c = x / r, s = y / r, r = sqrt(x^2 + y^2) for a Givens rotation: an FP32 reciprocal square root
+// and two Newton steps y <- y + y (1/2 - (s/2) y^2) in FP64 (2^-23 -> 2^-45 -> 2^-88), then one step on r =
+// s y; a third of the FP64 operations of hypot and two divisions, whose chain is on the critical path of
+// small systems (FP64 latency).  Sums of squares outside FP32's safe range take hypot.
+__device__ __forceinline__ void gc_rotation(double x, double y, double& c, double& s, double& r) {
+  const double q = fma(x, x, y * y);
+  if (q > 1.0e-30 && q < 1.0e30) {
+    double v = (double)rsqrtf((float)q);
+    const double h = 0.5 * q;
+    v = fma(v, fma(-h * v, v, 0.5), v);
+    v = fma(v, fma(-h * v, v, 0.5), v);
+    r = q * v;
+    r = fma(0.5 * v, fma(-r, r, q), r);
+    c = x * v;
+    s = y * v;
+    return;
+  }
+  r = hypot(x, y);
+  c = (r == 0.0) ? 1.0 : x / r;
+  s = (r == 0.0) ? 0.0 : y / r;
 }
 
 // Two columns at once (f32x2): (NS, Ns) -= a * (xh + xl) in double-float, kept negated so that
@@ -556,7 +593,7 @@ __device__ __forceinline__ void df2_acc(float2 a, float2 xh, float2 nxh, float2 
 // GPU makes a sequential chain of 2 j operations slow).  All sums over blocks run in a fixed
 // order, so the result does not depend on timing.
 __global__ void __launch_bounds__(GC_THREADS, 1) gmres_cycle_kernel(const GcArgs a) {
-  __shared__ float2 redf[GC_WARPS][32];
+  __shared__ float2 redf[GC_WARPS][33];
   __shared__ double Hs[GC_MAXM][GC_MAXM + 1];   // Hs[j][k]: rotated column j (R factor)
   __shared__ float2 h1[GC_MAXM + 2];
   __shared__ float2 sh[2 * GC_MAXM + 3];
@@ -599,6 +636,11 @@ __global__ void __launch_bounds__(GC_THREADS, 1) gmres_cycle_kernel(const GcArgs
     lp[i & 1] = -e;
   };
   unsigned nb = 0;
+  auto grid_barrier = [&]() {
+    if (a.bar) return gc_barrier(a.bar, a.status, nb++);
+    gc_cluster_barrier();
+    return true;
+  };
   // entries the plane cannot carry: nothing is done, and the host finishes with FP64 products
   if (*a.plane_flag & 1u) {
     if (blockIdx.x == 0 && threadIdx.x == 0) a.st->kdone = 0;
@@ -627,7 +669,7 @@ __global__ void __launch_bounds__(GC_THREADS, 1) gmres_cycle_kernel(const GcArgs
       R.ds[q * 32 + lane] = d;
       if (i < a.n) put_split(i, v, d);
     }
-  if (!gc_barrier(a.bar, a.status, nb++)) return;
+  if (!grid_barrier()) return;
 
   int kd = 0;
   for (int j = 0;; ++j) {
@@ -665,8 +707,8 @@ __global__ void __launch_bounds__(GC_THREADS, 1) gmres_cycle_kernel(const GcArgs
       double xK = __shfl_sync(FULL, cand, K > 0 ? ((K - 1) >> 1) : 0);
       if (K == 0) xK = x0;
       if (lane == 0) {
-        const double r = hypot(xK, xn);
-        const double c = (r == 0.0) ? 1.0 : xK / r, sg = (r == 0.0) ? 0.0 : xn / r;
+        double r, c, sg;
+        gc_rotation(xK, xn, c, sg, r);
         css[K] = c;
         sns[K] = sg;
         hc[K] = r;
@@ -701,15 +743,12 @@ __global__ void __launch_bounds__(GC_THREADS, 1) gmres_cycle_kernel(const GcArgs
       df_add(S, s, NS0.y, Ns0.y);
       df_add(S, s, NS1.x, Ns1.x);
       df_add(S, s, NS1.y, Ns1.y);
-      redf[wp][lane] = make_float2(S, s);
-      __syncthreads();
-      if (wp == 0) {
-        float2 t = redf[0][lane];
-        for (int p = 1; p < GC_WARPS - 1; ++p) df_add(t.x, t.y, redf[p][lane].x, redf[p][lane].y);
-        const float h = -__fadd_rn(t.x, t.y);   // -(S + s), renormalised
-        R.ws[q * 32 + lane] = (i < a.n) ? make_float2(h, __fsub_rn(-t.y, __fadd_rn(h, t.x))) : make_float2(0.f, 0.f);
+      redf[wp][lane] = make_float2(S, s);          // the last warp's is zero
+      const float2 t = gc_cross_sum(redf);          // row wp of the group
+      if (lane == 0) {
+        const bool real = ((int)blockIdx.x + q * (int)gridDim.x) * 32 + wp < a.n;
+        R.ws[q * 32 + wp] = real ? make_float2(-t.x, -t.y) : make_float2(0.f, 0.f);
       }
-      __syncthreads();
     }
     __syncthreads();
     if (sdone || !more) {   // converged at column j-1 (the last product is discarded), or m steps
@@ -718,7 +757,7 @@ __global__ void __launch_bounds__(GC_THREADS, 1) gmres_cycle_kernel(const GcArgs
     }
     // (2) one pass of dot products: c = V^T w, the Gram column of v_j, w . w, v_j . v_j
     gc_partial_dots_gram(R, j, ld, P1, sh);
-    if (!gc_barrier(a.bar, a.status, nb++)) return;
+    if (!grid_barrier()) return;
     gc_sum_partials(P1, ld, 2 * j + 3, sh);
     for (int k = threadIdx.x; k <= j; k += GC_THREADS) {
       const float2 g = (k < j) ? sh[j + 1 + k] : sh[2 * j + 2];
@@ -756,18 +795,18 @@ __global__ void __launch_bounds__(GC_THREADS, 1) gmres_cycle_kernel(const GcArgs
     const float inv = nrm_inv[1];
     for (int q = 0; q < R.nq; ++q) {
       const float2 t = gc_vsum(R, j, q, gx, redf);
-      if (wp == 0) {
-        const int i = row(q);
-        const float2 w2 = df_sum(R.ws[q * 32 + lane], make_float2(-t.x, -t.y));
+      if (lane == 0) {
+        const int l = q * 32 + wp, i = ((int)blockIdx.x + q * (int)gridDim.x) * 32 + wp;
+        const float2 w2 = df_sum(R.ws[l], make_float2(-t.x, -t.y));
         const float2 v = df_scale(inv, w2);       // w2 * inv; H[j+1][j] = 1 / inv, so that
                                                   // H[j+1][j] v_{j+1} = w2 to double-float
-        R.Vs[(size_t)(j + 1) * R.RB + q * 32 + lane] = v;
-        if (i < a.n) put_split(i, v, R.ds[q * 32 + lane]);
+        R.Vs[(size_t)(j + 1) * R.RB + l] = v;
+        if (i < a.n) put_split(i, v, R.ds[l]);
       }
     }
     for (int k = threadIdx.x; k <= j; k += GC_THREADS) Hs[j][k] = (double)gx[k].x + (double)gx[k].y;
     if (threadIdx.x == 0) Hs[j][j + 1] = (inv > 0.0f) ? 1.0 / (double)inv : 0.0;
-    if (!gc_barrier(a.bar, a.status, nb++)) return;
+    if (!grid_barrier()) return;
   }
   // y = R^{-1} g on one warp (every block): a column sweep from the last unknown, the
   // reciprocals of the diagonal formed in parallel first; R[k][i] = Hs[i][k]
@@ -791,7 +830,7 @@ __global__ void __launch_bounds__(GC_THREADS, 1) gmres_cycle_kernel(const GcArgs
   __syncthreads();
   // x += Dinv V y on the owned rows, in FP64: an FP32 rounding of the correction would come
   // back in the next residual amplified by the condition number of A Dinv
-  double (*redd)[32] = reinterpret_cast<double (*)[32]>(redf);
+  double (*redd)[33] = reinterpret_cast<double (*)[33]>(redf);
   if (kd > 0)
     for (int q = 0; q < R.nq; ++q) {
       double t = 0.0;
@@ -828,6 +867,21 @@ __global__ void selftest_mbar_kernel(int* status, unsigned max_polls) {
 
 __global__ void selftest_grid_barrier_kernel(unsigned* bar, int* status, unsigned max_polls) {
   (void)gc_barrier(bar, status, 0, gridDim.x + 1, max_polls);
+}
+
+// the cycle kernel's launch as one cluster of the whole grid (attr outlives the launch)
+cudaLaunchConfig_t cluster_config(int grid, size_t smem, cudaStream_t st, cudaLaunchAttribute* attr) {
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = (unsigned)grid;
+  attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(GC_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cfg;
 }
 
 }  // namespace
@@ -887,6 +941,8 @@ int gmres_f64(obs_context* ctx, int n, const double* A, const double* b, double*
   const int gc_gpb = (ngroups + gc_grid - 1) / gc_grid;
   const size_t gc_smem = (size_t)(2 * (m + 2) + 1) * 32 * gc_gpb * sizeof(float) +
                          (size_t)(m + 1) * (m + 1) * sizeof(float2);
+  bool cluster = false;
+  cudaLaunchAttribute cluster_attr{};
   bool fused = coop && gc_occ > 0 && m <= GC_MAXM && ctx->kernel_variant != OBS_VARIANT_GENERIC;
   if (fused) {
     cudaFuncAttributes fa{};
@@ -901,6 +957,15 @@ int gmres_f64(obs_context* ctx, int n, const double* A, const double* b, double*
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ2, gmres_cycle_kernel, GC_THREADS, gc_smem);
       if (e != cudaSuccess) return cuda_status(e);
       fused = occ2 * ctx->num_sms >= gc_grid;
+      if (fused && gc_grid > 1 && gc_grid <= GC_CLUSTER) {
+        // one cluster, where the device places clusters of that size
+        cudaLaunchConfig_t cfg = cluster_config(gc_grid, gc_smem, ctx->stream, &cluster_attr);
+        int nclus = 0;
+        e = cudaFuncSetAttribute(gmres_cycle_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&nclus, (const void*)gmres_cycle_kernel, &cfg);
+        cluster = e == cudaSuccess && nclus > 0;
+        if (e != cudaSuccess) cudaGetLastError();
+      }
     }
   }
   const size_t NP2 = (N + 1) / 2;                  // column pairs
@@ -997,10 +1062,15 @@ int gmres_f64(obs_context* ctx, int n, const double* A, const double* b, double*
     launched(1);
     const int mc = std::min(m, maxiter - total_it);
     if (fused) {
-      GcArgs ga{AH, dinv, n, m, mc, gc_gpb, V, gvp, gvl, x, gpart, gbar, gbar + 1, st, ctx->d_status};
+      GcArgs ga{AH, dinv, n, m, mc, gc_gpb, V, gvp, gvl, x, gpart, cluster ? nullptr : gbar, gbar + 1, st, ctx->d_status};
       void* args[] = {&ga};
-      e = cudaLaunchCooperativeKernel((const void*)gmres_cycle_kernel, dim3(gc_grid), dim3(GC_THREADS), args, gc_smem,
-                                      strm);
+      if (cluster) {
+        cudaLaunchConfig_t cfg = cluster_config(gc_grid, gc_smem, strm, &cluster_attr);
+        e = cudaLaunchKernelExC(&cfg, (const void*)gmres_cycle_kernel, args);
+      } else {
+        e = cudaLaunchCooperativeKernel((const void*)gmres_cycle_kernel, dim3(gc_grid), dim3(GC_THREADS), args, gc_smem,
+                                        strm);
+      }
       if (e != cudaSuccess) return cuda_status(e);
       launched(1);
     } else {
