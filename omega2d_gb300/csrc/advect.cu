@@ -90,11 +90,8 @@ int grid_of(int n) { return (n + 255) / 256; }
 // finalized self-induced velocity into (u, v)
 int velocity(obs_context* ctx, int core, int accum, int n, const float* x, const float* y, const float* r,
              const float* s, double fsx, double fsy, float* u, float* v) {
-  cudaError_t e = cudaMemsetAsync(u, 0, (size_t)n * 4, ctx->stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(v, 0, (size_t)n * 4, ctx->stream);
-  if (e != cudaSuccess) return cuda_status(e);
-  P2PRequest rq;
-  std::memset(&rq, 0, sizeof(rq));
+  P2PRequest rq{};
+  rq.overwrite = true;
   rq.core = core; rq.result = OBS_VELONLY; rq.accum = accum; rq.flags = OBS_FLAG_FINALIZE;
   rq.fsx = fsx; rq.fsy = fsy;
   rq.ns = n; rq.sx = x; rq.sy = y; rq.sr = r; rq.ss = s;

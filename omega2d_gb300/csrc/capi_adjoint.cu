@@ -87,10 +87,8 @@ int obs_points_affect_points_vjp_dev(obs_context* ctx, int core, int accum,
     s = ctx->state.ensure(6 * N * 4 + 1024, ctx->stream);
     if (s) return s;
     float* g = ctx->state.as<float>();
-    cudaError_t e = cudaMemsetAsync(g, 0, 6 * N * 4, ctx->stream);
-    if (e != cudaSuccess) return obs::cuda_status(e);
-    obs::P2PRequest rq;
-    std::memset(&rq, 0, sizeof(rq));
+    obs::P2PRequest rq{};
+    rq.overwrite = true;
     rq.core = core; rq.result = OBS_VELANDGRAD; rq.accum = accum;
     rq.ns = ns; rq.sx = sx; rq.sy = sy; rq.sr = sr; rq.ss = ss;
     rq.nt = nt; rq.tx = tx; rq.ty = ty; rq.tr = tr;

@@ -18,8 +18,7 @@ int check_vort(int accum, int ns, const float* sx, const float* sy, const float*
 
 obs::P2PRequest vort_request(int accum, int flags, int ns, const float* sx, const float* sy, const float* sr,
                              const float* ss, int nt, const float* tx, const float* ty, float* tw) {
-  obs::P2PRequest rq;
-  std::memset(&rq, 0, sizeof(rq));
+  obs::P2PRequest rq{};
   rq.core = obs::CORE_GAUSS;
   rq.result = obs::RES_BLOBVORT;
   rq.accum = accum;

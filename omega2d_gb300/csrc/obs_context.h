@@ -97,6 +97,7 @@ struct P2PRequest {
   const float *tx, *ty, *tr;
   float *tu, *tv;
   float* extra[4];
+  bool overwrite = false;   // the outputs' contents are not added to (they need no clearing)
 };
 int run_p2p(obs_context* ctx, const P2PRequest& rq);
 // small velocity sums in one launch (p2p_small.cu): whether a request takes it (run_p2p asks first),

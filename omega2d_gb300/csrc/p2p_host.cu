@@ -280,6 +280,7 @@ int run_p2p(obs_context* ctx, const P2PRequest& rq) {
   a.direct = nsplit == 1;
   a.finalize = (rq.flags & OBS_FLAG_FINALIZE) ? 1 : 0;
   a.fsx = rq.fsx; a.fsy = rq.fsy;
+  a.overwrite = rq.overwrite;
   a.blkcnt = blkcnt;
 
   timing_main_begin(ctx);

@@ -48,6 +48,7 @@ struct P2PArgs {
   int direct;            // nsplit == 1: write outputs from the main kernel
   int finalize;          // apply fs + (1/2pi) in the epilogue
   double fsx, fsy;
+  int overwrite;         // outputs = sum instead of += sum
   // Non-null (packed velocity kernel, 1 < nsplit <= 64): per target block arrival counts,
   // zeroed before launch.  Items then run target-block-major, the partials' row stride is
   // ntb * TB (compensated partials as (hi, lo) FP32 pairs), and the last split of a block to
@@ -78,7 +79,7 @@ __device__ __forceinline__ void store_target(const P2PArgs& a, int ib, const dou
   if ((unsigned)i >= (unsigned)a.nt) return;      // never taken: perm is a permutation of 0..nt-1
   auto put = [&](int k, double add, double fs) {
     float* p = a.out[k];
-    const double v = ((double)p[i] + add) * f + fs;
+    const double v = ((a.overwrite ? 0.0 : (double)p[i]) + add) * f + fs;
     p[i] = (float)v;
   };
   if constexpr (RES == RES_PSI || RES == RES_BLOBVORT) {

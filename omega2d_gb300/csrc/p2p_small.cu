@@ -115,6 +115,7 @@ int run_p2p_small(obs_context* ctx, const P2PRequest& rq) {
   o.out[0] = rq.tu; o.out[1] = rq.tv;
   o.finalize = (rq.flags & OBS_FLAG_FINALIZE) ? 1 : 0;
   o.fsx = rq.fsx; o.fsy = rq.fsy;
+  o.overwrite = rq.overwrite;
   const bool thick = rq.tr != nullptr, comp = rq.accum == OBS_COMPENSATED;
   const int grid = (rq.nt + SML_T - 1) / SML_T;
   timing_begin(ctx);

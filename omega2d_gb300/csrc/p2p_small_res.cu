@@ -126,6 +126,7 @@ int run_p2p_small_res(obs_context* ctx, const P2PRequest& rq) {
   for (int k = 0; k < 4; ++k) o.out[2 + k] = rq.extra[k];
   o.finalize = (rq.flags & OBS_FLAG_FINALIZE) ? 1 : 0;
   o.fsx = rq.fsx; o.fsy = rq.fsy;
+  o.overwrite = rq.overwrite;
   const bool thick = rq.tr != nullptr, comp = rq.accum == OBS_COMPENSATED;
   const int grid = (rq.nt + SMR_T - 1) / SMR_T;
   timing_begin(ctx);

@@ -191,6 +191,7 @@ int run_p2p_sym(obs_context* ctx, const P2PRequest& rq) {
   o.out[0] = rq.tu; o.out[1] = rq.tv;
   o.finalize = (rq.flags & OBS_FLAG_FINALIZE) ? 1 : 0;
   o.fsx = rq.fsx; o.fsy = rq.fsy;
+  o.overwrite = rq.overwrite;
 
   timing_main_begin(ctx);
   for (int b = 0; b < nblk; b += pass_blk) {

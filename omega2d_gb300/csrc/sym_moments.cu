@@ -208,6 +208,7 @@ int run_p2p_sym_res(obs_context* ctx, const P2PRequest& rq) {
   for (int k = 0; k < 4; ++k) o.p.out[2 + k] = rq.extra[k];
   o.p.finalize = (rq.flags & OBS_FLAG_FINALIZE) ? 1 : 0;
   o.p.fsx = rq.fsx; o.p.fsy = rq.fsy;
+  o.p.overwrite = rq.overwrite;
   const bool comp = rq.accum == OBS_COMPENSATED;
   if (rq.result == RES_GRAD) return run_moments<MomGrad, RES_GRAD>(ctx, comp, rq.nt, rq.sx, rq.sy, rq.sr, rq.ss, nullptr, nullptr, o, 0);
   if (rq.result == RES_VORT) return run_moments<MomVort, RES_VORT>(ctx, comp, rq.nt, rq.sx, rq.sy, rq.sr, rq.ss, nullptr, nullptr, o, 0);
