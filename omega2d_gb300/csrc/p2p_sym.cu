@@ -146,7 +146,10 @@ int run_p2p_sym(obs_context* ctx, const P2PRequest& rq) {
   const int npad = nblk * rows;
   const int ngrp = (n + SYM_GRP - 1) / SYM_GRP;
   const int slots = sym_occ(np) * ctx->num_sms;
-  const bool binned = (rq.core == CORE_GAUSS || rq.core == CORE_CEXP) && (double)n * n >= 3e8;
+  // The near form costs little more here (MUFU under the register reads), so the sort (nine launches, 60 us)
+  // pays late (Gaussian, binned vs not): 20,000 173-187 vs 155 us, 40,000 458-507 vs 469-483, 60,000
+  // 982-1068 vs 995-1028
+  const bool binned = (rq.core == CORE_GAUSS || rq.core == CORE_CEXP) && (double)n * n >= 4e9;
   const int pass_blk = std::min(nblk, std::max(1, (int)(SYM_COL_BYTES / ((size_t)npad * sizeof(float2)))));
   const int max_range = 8 * slots;
 
