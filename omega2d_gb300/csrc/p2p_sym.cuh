@@ -11,8 +11,8 @@
 // accumulations of a pair of pairs cost half of its 24 clocks; MUFU is at 50 %, the FMA pipe at
 // 67 %.  Other orders and groupings of the same operations and the accumulations as scalars came
 // within 3 % of one another.  Measured (compensated, one-sided -> here): 1M Gaussian patch 249 -> 182
-// ms (5.5e12 interactions/s), 131,072 Vatistas-2 plain 4.29 -> 3.23 ms, 33,001 Vatistas-2 with varying
-// radii 415 -> 284 us, ten Euler steps of 20,000 Rosenhead-Moore 1.65 -> 1.19 ms.
+// ms (5.5e12 interactions/s), 131,072 Vatistas-2 plain 4.29 -> 3.28 ms, 33,001 Vatistas-2 with varying
+// radii 415 -> 274 us, ten Euler steps of 20,000 Rosenhead-Moore 1.65 -> 1.13 ms.
 //
 // Layout: a row block is 1024 (or 2048) particles, eight (or sixteen) per thread of a 128-thread
 // CTA in f32x2 register pairs (a warp owns 256 or 512 consecutive ones); columns are taken 32 at a
@@ -21,7 +21,7 @@
 // meets it next by shuffle, so after 32 steps every lane holds its own column's sum over the warp's
 // rows.  The four warps' sums are added in shared memory and leave as one FP32 pair per (row block,
 // column); a row's own sums stay in registers over a whole run of columns (folded into two-sum pairs
-// every 32 columns when compensated).  Rows against their own block are one-sided.
+// every 32 columns when compensated, every 256 otherwise).  Rows against their own block are one-sided.
 //
 // Work: row block k meets every 32-column group from its own first one on; these (block, group)
 // units in order form a line of `total` units cut into equal ranges that the CTAs take from a
@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(SYM_THREADS, sym_occ(NP)) p2p_sym_kernel(const
           if (g0 + t * SYM_TG + b < gdiag) run(std::false_type{});
           else run(std::true_type{});
           csum[warp][b * SYM_GRP + lane] = make_float2(cu, cv);
-          if constexpr (COMP) {
+          if (COMP || b == cnt - 1) {              // plain sums fold once per tile
 #pragma unroll
             for (int p = 0; p < NP; ++p) {
               two_sum2(hu[p], lu[p], u[p]);
@@ -353,13 +353,8 @@ __global__ void __launch_bounds__(SYM_THREADS, sym_occ(NP)) p2p_sym_kernel(const
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int i = warp * 64 * NP + (2 * p + h) * 32 + lane;
-          if (COMP) {
-            rp[i] = h ? make_float2(hu[p].y, lu[p].y) : make_float2(hu[p].x, lu[p].x);
-            rp[ROWS + i] = h ? make_float2(hv[p].y, lv[p].y) : make_float2(hv[p].x, lv[p].x);
-          } else {
-            rp[i] = make_float2(h ? u[p].y : u[p].x, 0.0f);
-            rp[ROWS + i] = make_float2(h ? vn[p].y : vn[p].x, 0.0f);
-          }
+          rp[i] = h ? make_float2(hu[p].y, lu[p].y) : make_float2(hu[p].x, lu[p].x);
+          rp[ROWS + i] = h ? make_float2(hv[p].y, lv[p].y) : make_float2(hv[p].x, lv[p].x);
         }
       }
     }

@@ -31,7 +31,7 @@ __global__ void mom_pack_kernel(const float* __restrict__ x, const float* __rest
     o.z[l] = make_float2(z, z);
     if constexpr (VJP) {
       const float U = real ? lu[j] : 0.0f, V = real ? lv[j] : 0.0f;
-      o.l[l] = make_float4(U, U, V, V);
+      o.l[l] = make_float4(-U, -U, V, V);
     }
   }
   fold_extrema_block(i < n ? __float_as_uint(rr) : ~0u, i < n ? __float_as_uint(rr) : 0u, meta);

@@ -12,10 +12,10 @@
 //              the other sign, to the column, and a lv - b lu of the other particle to dL/dG
 // Beyond the core's far radius K = 1/d^2 and B = -2 K^2, so n = b^2 - K/2, h = a b, e = 0,
 // X / 2 = n wv + h wu, Y / 2 = n wu - h wv: far groups need no exponential and drop the sums of e.  A pair
-// of pairs takes 17 f32x2 operations for two gradient interactions (one-sided: 24) and 25 for two VJP
+// of pairs takes 17 f32x2 operations for two gradient interactions (one-sided: 24) and 23 for two VJP
 // interactions (one-sided: 34); bound by the registers' read ports like the velocity sum.
 // Measured, 131,072-particle patch, compensated (one-sided -> here): gradient 8.68 -> 6.7 ms, vorticity 5.7
-// -> 4.3, shear 6.2 -> 5.1, self VJP 12.1 -> 8.8 (11.3 in Hilbert order); 3 and 4 row pairs per thread take
+// -> 4.3, shear 6.2 -> 5.1, self VJP 12.1 -> 8.5 (11.3 in Hilbert order); 3 and 4 row pairs per thread take
 // 2 to 20 % longer (fewer, larger row blocks; 128 registers either way), 5 and 6 CTAs per SM as long.
 #pragma once
 
@@ -45,7 +45,7 @@ template <> struct __align__(128) MomGroup<false> {
 template <> struct __align__(128) MomGroup<true> {
   float4 xy[SYM_GRP];
   float2 g[SYM_GRP], z[SYM_GRP];
-  float4 l[SYM_GRP];       // (lu, lu, lv, lv)
+  float4 l[SYM_GRP];       // (-lu, -lu, lv, lv): the strength term is then two fused operations
 };
 
 struct MomArgs {
@@ -56,9 +56,9 @@ struct MomArgs {
   float2* run;             // [NF + NN][npad] running sums over the passes
 };
 
-// a particle's weights: strength and, for the VJP, cotangents
+// a particle's weights: strength and, for the VJP, cotangents (the first one negated)
 struct MomW {
-  float2 g, lu, lv;
+  float2 g, mlu, lv;
 };
 
 __device__ __forceinline__ float2 abs2(float2 v) { return f2(fabsf(v.x), fabsf(v.y)); }
@@ -84,10 +84,10 @@ __device__ __forceinline__ void mom_group(const MomGroup<OP::VJP>& grp, int lane
     const int col = lane ^ s;
     const float4 c4 = grp.xy[col];
     const float2 cx = f2(c4.x, c4.y), cy = f2(c4.z, c4.w), cg = grp.g[col];
-    float2 clu = f2(0.0f, 0.0f), clv = clu;
+    float2 cmlu = f2(0.0f, 0.0f), clv = cmlu;
     if constexpr (OP::VJP) {
       const float4 l = grp.l[col];
-      clu = f2(l.x, l.y);
+      cmlu = f2(l.x, l.y);
       clv = f2(l.z, l.w);
     }
     float2 t[OP::NF + OP::NN];                     // this step's rows for the column
@@ -119,7 +119,7 @@ __device__ __forceinline__ void mom_group(const MomGroup<OP::VJP>& grp, int lane
       }
       const float2 a = mul2(k, dx), b = mul2(k, dy);
       if constexpr (OP::VJP) {
-        const float2 wu = nfma2(w[p].g, clu, mul2(cg, w[p].lu)), wv = nfma2(w[p].g, clv, mul2(cg, w[p].lv));
+        const float2 wu = nfma2(cg, w[p].mlu, mul2(w[p].g, cmlu)), wv = nfma2(w[p].g, clv, mul2(cg, w[p].lv));
         float2 X, Y;                               // halved
         if constexpr (FAR) {
           const float2 n = __ffma2_rn(b, b, mul2(k, mhalf)), h = mul2(a, b);
@@ -134,8 +134,8 @@ __device__ __forceinline__ void mom_group(const MomGroup<OP::VJP>& grp, int lane
         acc[p][1] = __fadd2_rn(acc[p][1], Y);
         t[0] = (p == 0) ? X : __fadd2_rn(t[0], X);
         t[1] = (p == 0) ? Y : __fadd2_rn(t[1], Y);
-        acc[p][2] = nfma2(b, clu, __ffma2_rn(a, clv, acc[p][2]));
-        t[2] = nfma2(b, w[p].lu, (p == 0) ? mul2(a, w[p].lv) : __ffma2_rn(a, w[p].lv, t[2]));
+        acc[p][2] = __ffma2_rn(b, cmlu, __ffma2_rn(a, clv, acc[p][2]));
+        t[2] = __ffma2_rn(b, w[p].mlu, (p == 0) ? mul2(a, w[p].lv) : __ffma2_rn(a, w[p].lv, t[2]));
       } else {
         both(p, 0, b, cg, w[p].g);
         both(p, 1, a, cg, w[p].g);
@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(SYM_THREADS, 4) sym_moments_kernel(const MomAr
           zrow[(2 * p + 1) * SYM_THREADS + tid] = r1.z[lane].x;
         }
         if constexpr (OP::VJP) {
-          w[p].lu = f2(r0.l[lane].x, r1.l[lane].x);
+          w[p].mlu = f2(r0.l[lane].x, r1.l[lane].x);
           w[p].lv = f2(r0.l[lane].z, r1.l[lane].z);
         }
 #pragma unroll
@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(SYM_THREADS, 4) sym_moments_kernel(const MomAr
           }
 #pragma unroll
           for (int c = 0; c < NC; ++c) csum[warp][c][b * SYM_GRP + lane] = cs[c];
-          if constexpr (COMP) {
+          if (COMP || b == cnt - 1) {              // plain sums fold once per tile
 #pragma unroll
             for (int p = 0; p < NP; ++p)
 #pragma unroll
@@ -334,8 +334,7 @@ __global__ void __launch_bounds__(SYM_THREADS, 4) sym_moments_kernel(const MomAr
           const int i = warp * 64 * NP + (2 * p + h) * 32 + lane;
 #pragma unroll
           for (int c = 0; c < NF; ++c)
-            rp[(size_t)c * ROWS + i] = COMP ? (h ? f2(hi[p][c].y, lo[p][c].y) : f2(hi[p][c].x, lo[p][c].x))
-                                                : f2(h ? acc[p][c].y : acc[p][c].x, 0.0f);
+            rp[(size_t)c * ROWS + i] = h ? f2(hi[p][c].y, lo[p][c].y) : f2(hi[p][c].x, lo[p][c].x);
 #pragma unroll
           for (int c = 0; c < NN; ++c) rp[(size_t)(NF + c) * ROWS + i] = met_near ? nsum[c][2 * p + h][tid] : f2(0.0f, 0.0f);
         }
