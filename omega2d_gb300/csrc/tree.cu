@@ -39,7 +39,7 @@
 // leaf (twenty times the mean cost in a sample of such groups, more at worst); along the Hilbert
 // curve the worst group costs 1.7 times the mean and the mean group accepts half as many nodes.
 // What is left is the near leaves (about 170 per group, three quarters of the instructions): issue
-// active 62 %, FMA pipe 43 %, MUFU 34 %.  Sorting, tree and extrema take 0.35 ms.
+// active 63 %, FMA pipe 55 %, MUFU 43 %.  Sorting, tree and extrema take 0.35 ms.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -101,7 +101,7 @@ struct TreeArgs {
   int P;
   float theta;
   float lterm;       // log2(theta^P / 4): a node stops at the first p with p log2|w| below it
-  int split;         // warps per target group (1, 2 or 4)
+  int one, two;      // blocks with a warp per target group, then blocks with two, then four
   int finalize;
   double fsx, fsy;
   int* status;
@@ -268,45 +268,52 @@ struct TreeLeaf {
 template <int CORE, bool THICK, bool FAR>
 __device__ __forceinline__ void tree_leaf_sum(const TreeLeaf& lf, int cnt, float2 tx, float2 ty, float2 tz, bool unif,
                                               float cf, float cfl, float2& au, float2& av) {
+  float2 su[2] = {au, au}, sv[2] = {av, av};       // the odd and the even sources apart: half the rounding
   if (!FAR && CORE == CORE_GAUSS && unif) {
     // (1 - e^-x)/d^2; x < 0.001 -> 1/s^2 (src/CoreFunc.h:111-181).  The reference's 1/d^2 for
     // x > 16 is within 1.2e-7 of this form, one ulp, so it needs no select here
     const float thr_small = -0.001f * kLog2e;
     const float2 cfl2 = f2(cfl, cfl), m1 = f2(-1.0f, -1.0f), one = f2(1.0f, 1.0f);
 #pragma unroll 4
-    for (int k = 0; k < cnt; ++k) {
-      const float4 P = lf.xy[k], Q = lf.gz[k];
-      const float2 dx = __fadd2_rn(tx, f2(P.x, P.y)), dy = __fadd2_rn(ty, f2(P.z, P.w));
-      const float2 d2 = __ffma2_rn(dx, dx, __fmul2_rn(dy, dy));
-      const float2 t = __fmul2_rn(d2, cfl2);
-      const float2 ood2 = f2(rcp_a(d2.x), rcp_a(d2.y));
-      const float2 ome = __ffma2_rn(f2(ex2_a(t.x), ex2_a(t.y)), m1, one);
-      float2 K = __fmul2_rn(ood2, ome);
-      K.x = (t.x > thr_small) ? cf : K.x;
-      K.y = (t.y > thr_small) ? cf : K.y;
-      const float2 fn = __fmul2_rn(f2(Q.x, Q.y), K);
-      au = __ffma2_rn(fn, dy, au);
-      av = __ffma2_rn(fn, dx, av);
-    }
-  } else {
-#pragma unroll 4
-    for (int k = 0; k < cnt; ++k) {
-      const float4 P = lf.xy[k], Q = lf.gz[k];
-      const float2 dx = __fadd2_rn(tx, f2(P.x, P.y)), dy = __fadd2_rn(ty, f2(P.z, P.w));
-      const float2 d2 = __ffma2_rn(dx, dx, __fmul2_rn(dy, dy));
-      float K0, K1, B;
-      if constexpr (FAR) {
-        K0 = rcp_a(d2.x);
-        K1 = rcp_a(d2.y);
-      } else {
-        core_eval<CORE, THICK, false, false>(d2.x, Q.z, tz.x, 0.0f, 0.0f, K0, B);
-        core_eval<CORE, THICK, false, false>(d2.y, Q.z, tz.y, 0.0f, 0.0f, K1, B);
+    for (int k0 = 0; k0 < cnt; k0 += 2)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float4 P = lf.xy[k0 + h], Q = lf.gz[k0 + h];
+        const float2 dx = __fadd2_rn(tx, f2(P.x, P.y)), dy = __fadd2_rn(ty, f2(P.z, P.w));
+        const float2 d2 = __ffma2_rn(dx, dx, __fmul2_rn(dy, dy));
+        const float2 t = __fmul2_rn(d2, cfl2);
+        const float2 ood2 = f2(rcp_a(d2.x), rcp_a(d2.y));
+        const float2 ome = __ffma2_rn(f2(ex2_a(t.x), ex2_a(t.y)), m1, one);
+        float2 K = __fmul2_rn(ood2, ome);
+        K.x = (t.x > thr_small) ? cf : K.x;
+        K.y = (t.y > thr_small) ? cf : K.y;
+        const float2 fn = __fmul2_rn(f2(Q.x, Q.y), K);
+        su[h] = __ffma2_rn(fn, dy, su[h]);
+        sv[h] = __ffma2_rn(fn, dx, sv[h]);
       }
-      const float2 fn = __fmul2_rn(f2(Q.x, Q.y), f2(K0, K1));
-      au = __ffma2_rn(fn, dy, au);
-      av = __ffma2_rn(fn, dx, av);
-    }
+  } else {
+#pragma unroll 2
+    for (int k0 = 0; k0 < cnt; k0 += 2)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float4 P = lf.xy[k0 + h], Q = lf.gz[k0 + h];
+        const float2 dx = __fadd2_rn(tx, f2(P.x, P.y)), dy = __fadd2_rn(ty, f2(P.z, P.w));
+        const float2 d2 = __ffma2_rn(dx, dx, __fmul2_rn(dy, dy));
+        float K0, K1, B;
+        if constexpr (FAR) {
+          K0 = rcp_a(d2.x);
+          K1 = rcp_a(d2.y);
+        } else {
+          core_eval<CORE, THICK, false, false>(d2.x, Q.z, tz.x, 0.0f, 0.0f, K0, B);
+          core_eval<CORE, THICK, false, false>(d2.y, Q.z, tz.y, 0.0f, 0.0f, K1, B);
+        }
+        const float2 fn = __fmul2_rn(f2(Q.x, Q.y), f2(K0, K1));
+        su[h] = __ffma2_rn(fn, dy, su[h]);
+        sv[h] = __ffma2_rn(fn, dx, sv[h]);
+      }
   }
+  au = __fadd2_rn(su[0], su[1]);
+  av = __fadd2_rn(sv[0], sv[1]);
 }
 
 template <int CORE, bool THICK>
@@ -318,8 +325,10 @@ __global__ void __launch_bounds__(TREE_WARPS * 32, 6) tree_eval_kernel(const Tre
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int* stk = stk_all[w];
   TreeLeaf& lf = leafs[w];
-  const int part = w % a.split;
-  const int grp = blockIdx.x * (TREE_WARPS / a.split) + w / a.split;
+  const int blk = blockIdx.x;
+  const int split = blk < a.one ? 1 : (blk < a.one + a.two ? 2 : 4);
+  const int part = w % split;
+  const int grp = blk * 4 / split + w / split + (split > 1 ? 2 * a.one : 0) + (split > 2 ? a.one + a.two : 0);
   const bool live = grp * 64 < a.nt;                // warp-uniform
   const int i0 = grp * 64 + lane, i1 = i0 + 32;
   const bool v0 = live && i0 < a.nt, v1 = live && i1 < a.nt;
@@ -392,7 +401,7 @@ __global__ void __launch_bounds__(TREE_WARPS * 32, 6) tree_eval_kernel(const Tre
     sp += total;
     __syncwarp();
     for (unsigned m = __ballot_sync(FULL, accept); m; m &= m - 1) {
-      if (turn++ % a.split != part) continue;
+      if (turn++ % split != part) continue;
       // F = (1/(z - c)) sum_k b_k w^k, w = rn/(z - c); u += Im F, v += Re F
       const int b = __ffs(m) - 1;
       const float4* cf = a.nodes.coef + (size_t)__shfl_sync(FULL, node, b) * TREE_PMAX;
@@ -425,15 +434,16 @@ __global__ void __launch_bounds__(TREE_WARPS * 32, 6) tree_eval_kernel(const Tre
     // leaf being too close for its expansion -- with the far form 1/d^2 the core takes there
     const unsigned farm = __ballot_sync(FULL, far);
     for (unsigned m = __ballot_sync(FULL, leaf); m; m &= m - 1) {
-      if (turn++ % a.split != part) continue;
+      if (turn++ % split != part) continue;
       const int b = __ffs(m) - 1;
       const int s0 = __shfl_sync(FULL, q, b) * TREE_LEAF;
       const int cnt = min(TREE_LEAF, a.ns - s0);
       __syncwarp();
-      if (lane < cnt) {
-        const float4 s = a.sp4[s0 + lane];
+      {
+        const float4 s = a.sp4[s0 + min(lane, cnt - 1)];
+        const float g = lane < cnt ? -s.w : 0.0f;   // an odd count: the last source again, without strength
         lf.xy[lane] = make_float4(-s.x, -s.x, -s.y, -s.y);
-        lf.gz[lane] = make_float4(-s.w, -s.w, s.z, s.z);
+        lf.gz[lane] = make_float4(g, g, s.z, s.z);
       }
       __syncwarp();
       float2 au = f2(0.0f, 0.0f), av = au;
@@ -443,12 +453,12 @@ __global__ void __launch_bounds__(TREE_WARPS * 32, 6) tree_eval_kernel(const Tre
       two_sum2(hv, lv, f2(-av.x, -av.y));
     }
   }
-  if (a.split > 1) {                                // the group's warps, added in order by the first
+  if (split > 1) {                                  // the group's warps, added in order by the first
     red[w][lane] = make_float4(hu.x, lu.x, hv.x, lv.x);
     red[w][32 + lane] = make_float4(hu.y, lu.y, hv.y, lv.y);
     __syncthreads();
     if (part != 0) return;
-    for (int k = 1; k < a.split; ++k) {
+    for (int k = 1; k < split; ++k) {
       const float4 p = red[w + k][lane], r = red[w + k][32 + lane];
       two_sum2(hu, lu, f2(p.x, r.x));
       two_sum2(hv, lv, f2(p.z, r.z));
@@ -596,9 +606,11 @@ int run_tree(obs_context* ctx, int core, int flags, double fsx, double fsy, doub
   a.meta = meta;
   // a warp per 64 targets, or two or four where that leaves fewer than 16 warps per SM
   const int groups = (nt + 63) / 64;
-  a.split = groups >= 16 * ctx->num_sms ? 1 : (groups >= 8 * ctx->num_sms ? 2 : 4);
-  const int gpb = TREE_WARPS / a.split;
-  e = tree_eval(core, tr != nullptr, a, (groups + gpb - 1) / gpb, st);
+  constexpr int FOUR = 6, TWO = 6;
+  const int four = std::min(groups, FOUR * ctx->num_sms), two = std::min(groups - four, TWO * ctx->num_sms);
+  a.one = (groups - four - two) / 4;
+  a.two = (groups - four - 4 * a.one) / 2;
+  e = tree_eval(core, tr != nullptr, a, groups - 3 * a.one - a.two, st);
   ++launches;
   ctx->launches += launches;
   return cuda_status(e);
