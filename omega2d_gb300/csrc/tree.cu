@@ -29,11 +29,11 @@
 //
 // With u + i v = i conj(F), F = sum_j G_j / (z - z_j): u = Im F, v = Re F (unscaled, as the
 // direct sums; finalize_vels semantics optional).  Per-node contributions are accumulated with
-// two-sums.  Small target sets split a group's nodes over two or four warps, every one of them
-// walking the same tree and taking its share in turn.  Results are deterministic: the traversal
+// two-sums.  The last groups, all of a small set, split their nodes over two or four warps, every
+// one of them walking the same tree and taking its share in turn.  Results are deterministic: the traversal
 // order is a function of the inputs.
 //
-// 1M Gaussian patch, self interaction: 4.4 ms (44 ms in Morton order with 32 targets per warp and
+// 1M Gaussian patch, self interaction: 4.1 ms (44 ms in Morton order with 32 targets per warp and
 // every node at full order).  Most of the 44 ms was a tail: a run of targets or sources across one
 // of the Morton curve's jumps has a box the size of the domain, and its warp opened nearly every
 // leaf (twenty times the mean cost in a sample of such groups, more at worst); along the Hilbert
@@ -265,11 +265,14 @@ struct TreeLeaf {
 };
 
 // sums of -G K dy (= u) and -G K dx (= -v) of a leaf's cnt sources at the lane's two targets
-template <int CORE, bool THICK, bool FAR>
+// FORM 0: every pair in the core's far regime; 1: any pair; 2: unif, and no pair inside x < 0.001 (most near
+// leaves: without the select a million-particle patch takes 4.1 instead of 4.35 ms)
+template <int CORE, bool THICK, int FORM>
 __device__ __forceinline__ void tree_leaf_sum(const TreeLeaf& lf, int cnt, float2 tx, float2 ty, float2 tz, bool unif,
                                               float cf, float cfl, float2& au, float2& av) {
   float2 su[2] = {au, au}, sv[2] = {av, av};       // the odd and the even sources apart: half the rounding
-  if (!FAR && CORE == CORE_GAUSS && unif) {
+  constexpr bool FAR = FORM == 0;
+  if (!FAR && CORE == CORE_GAUSS && (FORM == 2 || unif)) {
     // (1 - e^-x)/d^2; x < 0.001 -> 1/s^2 (src/CoreFunc.h:111-181).  The reference's 1/d^2 for
     // x > 16 is within 1.2e-7 of this form, one ulp, so it needs no select here
     const float thr_small = -0.001f * kLog2e;
@@ -285,8 +288,10 @@ __device__ __forceinline__ void tree_leaf_sum(const TreeLeaf& lf, int cnt, float
         const float2 ood2 = f2(rcp_a(d2.x), rcp_a(d2.y));
         const float2 ome = __ffma2_rn(f2(ex2_a(t.x), ex2_a(t.y)), m1, one);
         float2 K = __fmul2_rn(ood2, ome);
-        K.x = (t.x > thr_small) ? cf : K.x;
-        K.y = (t.y > thr_small) ? cf : K.y;
+        if constexpr (FORM != 2) {
+          K.x = (t.x > thr_small) ? cf : K.x;
+          K.y = (t.y > thr_small) ? cf : K.y;
+        }
         const float2 fn = __fmul2_rn(f2(Q.x, Q.y), K);
         su[h] = __ffma2_rn(fn, dy, su[h]);
         sv[h] = __ffma2_rn(fn, dx, sv[h]);
@@ -432,7 +437,7 @@ __global__ void __launch_bounds__(TREE_WARPS * 32, 6) tree_eval_kernel(const Tre
     }
     // leaves: direct sums, with the core or -- when every pair lies in the core's far regime, the
     // leaf being too close for its expansion -- with the far form 1/d^2 the core takes there
-    const unsigned farm = __ballot_sync(FULL, far);
+    const unsigned farm = __ballot_sync(FULL, far), outm = __ballot_sync(FULL, gunif && dmin2 * gcf > 0.00101f);
     for (unsigned m = __ballot_sync(FULL, leaf); m; m &= m - 1) {
       if (turn++ % split != part) continue;
       const int b = __ffs(m) - 1;
@@ -447,8 +452,10 @@ __global__ void __launch_bounds__(TREE_WARPS * 32, 6) tree_eval_kernel(const Tre
       }
       __syncwarp();
       float2 au = f2(0.0f, 0.0f), av = au;
-      if ((farm >> b) & 1u) tree_leaf_sum<CORE, THICK, true>(lf, cnt, tx, ty, tz, gunif, gcf, gcfl, au, av);
-      else tree_leaf_sum<CORE, THICK, false>(lf, cnt, tx, ty, tz, gunif, gcf, gcfl, au, av);
+      if ((farm >> b) & 1u) tree_leaf_sum<CORE, THICK, 0>(lf, cnt, tx, ty, tz, gunif, gcf, gcfl, au, av);
+      else if (CORE == CORE_GAUSS && ((outm >> b) & 1u))
+        tree_leaf_sum<CORE, THICK, 2>(lf, cnt, tx, ty, tz, true, gcf, gcfl, au, av);
+      else tree_leaf_sum<CORE, THICK, 1>(lf, cnt, tx, ty, tz, gunif, gcf, gcfl, au, av);
       two_sum2(hu, lu, au);
       two_sum2(hv, lv, f2(-av.x, -av.y));
     }
@@ -604,7 +611,10 @@ int run_tree(obs_context* ctx, int core, int flags, double fsx, double fsy, doub
     }
   }
   a.meta = meta;
-  // a warp per 64 targets, or two or four where that leaves fewer than 16 warps per SM
+  // A warp per 64 targets, but four for the last 6 groups per SM (one resident wave of blocks) and two for the 6
+  // per SM before them: whole groups started last would leave most of the chip idle at the end.  Every split warp
+  // walks the tree again: measured with four for the last 0, 6, 12, 24, 48 per SM, 1,000,000 targets take 4.35, 4.31,
+  // 4.34, 4.44, 4.68 ms and 300,000 1.44, 0.97, 1.04, 1.11, 1.15 ms; with none of two, 60,000 take 0.44 ms, not 0.33.
   const int groups = (nt + 63) / 64;
   constexpr int FOUR = 6, TWO = 6;
   const int four = std::min(groups, FOUR * ctx->num_sms), two = std::min(groups - four, TWO * ctx->num_sms);

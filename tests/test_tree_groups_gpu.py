@@ -36,3 +36,17 @@ def test_tree_matches_direct(ctx, n):
     og.points_affect_points_tree(a, a, env)
     og.points_affect_points(b, b, og.VELONLY, env)
     assert rel_err(b.u, a.u) < TOL and rel_err(b.v, a.v) < TOL
+
+
+@pytest.mark.parametrize("x", [0.0, 0.0009, 0.00095, 0.00103, 0.0011, 0.01])
+def test_tree_leaves_about_the_core(ctx, restatement, x):
+    # a leaf at d^2 / s^2 = x from the targets: below 0.001 the Gaussian core is the constant 1 / s^2, which is 4.7e-4
+    # off (1 - e^-x) / d^2 there; that formula in FP32 carries 2^-23 / x <= 1.2e-4 (the FP64 oracle none)
+    rad = np.float32(0.02)
+    d = np.float32(np.sqrt(2 * x) * rad)
+    sx = np.concatenate([np.full(32, d), np.full(32, 0.3)]).astype(np.float32)
+    sy, r, s = np.zeros(64, np.float32), np.full(64, rad), np.full(64, 1 / 64, np.float32)
+    t = og.Points(np.zeros(64, np.float32), np.full(64, 1e-7, np.float32), r)
+    og.points_affect_points_tree(og.Points(sx, sy, r, s), t, og.ExecEnv(og.CORE_GAUSSIAN, context=ctx))
+    u, v, _ = restatement.points_affect_points(og.CORE_GAUSSIAN, 1, sx, sy, r, s, t.x, t.y, r, fp64=True)
+    assert np.isfinite(t.u).all() and rel_err(v, t.v) < 2e-4
