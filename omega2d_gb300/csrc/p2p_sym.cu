@@ -38,8 +38,9 @@ __device__ __forceinline__ void df_add(float& hi, float& lo, float bh, float bl)
 
 // Adds a particle's partials of this pass (its row block's pieces, then the row blocks before its
 // own, each in order) to its running sum; the last pass stores the result.  A block takes 64
-// particles; four threads share one, each every fourth partial, added up in thread order.
-constexpr int SYM_RED_T = 64, SYM_RED_SUB = 4;
+// particles; eight threads share one, each every eighth partial, added up in thread order (with four ten
+// steps of 20,000 particles take 20 us longer, with sixteen as long as with four).
+constexpr int SYM_RED_T = 64, SYM_RED_SUB = 8;
 template <int NP>
 __global__ void __launch_bounds__(SYM_RED_T * SYM_RED_SUB) sym_reduce_kernel(const SymArgs a, const P2PArgs o) {
   constexpr int SYM_ROWS = sym_rows(NP);
