@@ -50,9 +50,9 @@ bool scheme_of(int order, Scheme* sc) {
 }
 
 // ElementBase::move with one weight 1.0: x += (S)h * 1.0 * u, the product formed in double
-__global__ void move1_kernel(int n, const float* __restrict__ x, const float* __restrict__ y,
-                             const float* __restrict__ u, const float* __restrict__ v, float h,
-                             float* __restrict__ xo, float* __restrict__ yo) {
+__global__ void move1_kernel(int n, const float* x, const float* y, const float* u, const float* v, float h, float* xo,
+                             float* yo) {
+  wait_for_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   xo[i] = (float)((double)x[i] + (double)h * (double)u[i]);
@@ -119,9 +119,8 @@ int step(const Step& p, const float* x, float* xo, float* vel, float* stages, bo
   for (int s = 0; s < S; ++s) {
     if (s > 0) {
       float* y = stages + (size_t)(s - 1) * 2 * N;
-      move1_kernel<<<grid_of(p.n), 256, 0, ctx->stream>>>(p.n, x, x + N, vel + (size_t)(s - 1) * 2 * N,
-                                                          vel + (size_t)(s - 1) * 2 * N + N,
-                                                          (float)(p.sc.a[s] * p.dt), y, y + N);
+      launch_early(move1_kernel, grid_of(p.n), 256, ctx->stream, p.n, x, x + N, vel + (size_t)(s - 1) * 2 * N,
+                   vel + (size_t)(s - 1) * 2 * N + N, (float)(p.sc.a[s] * p.dt), y, y + N);
       ctx->launches++;
       ys = y;
     }
@@ -132,7 +131,7 @@ int step(const Step& p, const float* x, float* xo, float* vel, float* stages, bo
   }
   if (!want_end) return cuda_status(cudaGetLastError());
   if (S == 1) {
-    move1_kernel<<<grid_of(p.n), 256, 0, ctx->stream>>>(p.n, x, x + N, vel, vel + N, (float)p.dt, xo, xo + N);
+    launch_early(move1_kernel, grid_of(p.n), 256, ctx->stream, p.n, x, x + N, vel, vel + N, (float)p.dt, xo, xo + N);
   } else {
     if (xo != x) {
       cudaError_t e = cudaMemcpyAsync(xo, x, 2 * N * 4, cudaMemcpyDeviceToDevice, ctx->stream);

@@ -12,9 +12,9 @@ namespace {
 
 // Particles in groups of 32 in processing order, padded to whole row blocks with far particles of
 // zero strength, and the radius extrema (meta[0] = ~min, meta[1] = max bits).
-__global__ void sym_pack_kernel(const float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ r,
-                                const float* __restrict__ g, const int* __restrict__ perm, int n, int npad, int core,
-                                SymGroup* __restrict__ out, unsigned* __restrict__ meta) {
+__global__ void sym_pack_kernel(const float* x, const float* y, const float* r, const float* g, const int* perm, int n,
+                                int npad, int core, SymGroup* out, unsigned* meta) {
+  wait_for_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   int j = (i < n && perm) ? perm[i] : i;
   if ((unsigned)j >= (unsigned)n) j = 0;          // never taken for i < n: perm is a permutation
@@ -44,6 +44,7 @@ constexpr int SYM_RED_T = 64, SYM_RED_SUB = 8;
 template <int NP>
 __global__ void __launch_bounds__(SYM_RED_T * SYM_RED_SUB) sym_reduce_kernel(const SymArgs a, const P2PArgs o) {
   constexpr int SYM_ROWS = sym_rows(NP);
+  wait_for_previous();
   __shared__ float4 red[SYM_RED_SUB][SYM_RED_T];
   const int l = threadIdx.x % SYM_RED_T, sub = threadIdx.x / SYM_RED_T;
   const int j = blockIdx.x * SYM_RED_T + l;
@@ -95,9 +96,9 @@ __global__ void __launch_bounds__(SYM_RED_T * SYM_RED_SUB) sym_reduce_kernel(con
 // one pass: the sums, then their reduction
 template <int CORE, int NP>
 cudaError_t sym_launch(bool comp, const SymArgs& a, const P2PArgs& o, int grid, cudaStream_t st) {
-  if (comp) p2p_sym_kernel<CORE, true, NP><<<grid, SYM_THREADS, 0, st>>>(a);
-  else p2p_sym_kernel<CORE, false, NP><<<grid, SYM_THREADS, 0, st>>>(a);
-  sym_reduce_kernel<NP><<<(a.n + SYM_RED_T - 1) / SYM_RED_T, SYM_RED_T * SYM_RED_SUB, 0, st>>>(a, o);
+  if (comp) launch_early(p2p_sym_kernel<CORE, true, NP>, grid, SYM_THREADS, st, a);
+  else launch_early(p2p_sym_kernel<CORE, false, NP>, grid, SYM_THREADS, st, a);
+  launch_early(sym_reduce_kernel<NP>, (a.n + SYM_RED_T - 1) / SYM_RED_T, SYM_RED_T * SYM_RED_SUB, st, a, o);
   return cudaGetLastError();
 }
 
@@ -173,8 +174,8 @@ int run_p2p_sym(obs_context* ctx, const P2PRequest& rq) {
   int nl = 0;
   if (e == cudaSuccess && binned) e = bin_order(rq.sx, rq.sy, n, ctx->work.as<char>(o_sort), perm, st, &nl, BIN_HILBERT8);
   if (e != cudaSuccess) return cuda_status(e);
-  sym_pack_kernel<<<(npad + 255) / 256, 256, 0, st>>>(rq.sx, rq.sy, rq.sr, rq.ss, perm, n, npad, rq.core,
-                                                      ctx->work.as<SymGroup>(o_pts), h->meta);
+  launch_early(sym_pack_kernel, (npad + 255) / 256, 256, st, rq.sx, rq.sy, rq.sr, rq.ss, perm, n, npad, rq.core,
+               ctx->work.as<SymGroup>(o_pts), h->meta);
   ctx->launches += nl + 1;
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e);
 

@@ -12,7 +12,7 @@
 // 67 %.  Other orders and groupings of the same operations and the accumulations as scalars came
 // within 3 % of one another.  Measured (compensated, one-sided -> here): 1M Gaussian patch 249 -> 182
 // ms (5.5e12 interactions/s), 131,072 Vatistas-2 plain 4.29 -> 3.28 ms, 33,001 Vatistas-2 with varying
-// radii 415 -> 274 us, ten Euler steps of 20,000 Rosenhead-Moore 1.65 -> 1.13 ms.
+// radii 415 -> 271 us, ten Euler steps of 20,000 Rosenhead-Moore 1.65 -> 1.04 ms.
 //
 // Layout: a row block is 1024 (or 2048) particles, eight (or sixteen) per thread of a 128-thread
 // CTA in f32x2 register pairs (a warp owns 256 or 512 consecutive ones); columns are taken 32 at a
@@ -217,6 +217,7 @@ template <int CORE, bool COMP, int NP>
 __global__ void __launch_bounds__(SYM_THREADS, sym_occ(NP)) p2p_sym_kernel(const SymArgs a) {
   constexpr int GPB = sym_gpb(NP), ROWS = sym_rows(NP);
   constexpr bool MASKED = CORE == CORE_GAUSS || CORE == CORE_CEXP;
+  wait_for_previous();
   __shared__ SymGroup tile[NSTAGE][SYM_TG];
   __shared__ float2 csum[SYM_THREADS / 32][SYM_TILE];   // per-warp column sums of the tile
   __shared__ float zrow[2 * NP * SYM_THREADS];

@@ -269,6 +269,7 @@ __device__ __forceinline__ void pan_finish(const PanArgs& a, int i, double su, d
 //     are of w u* and w v* and the tangent is applied once at the end.
 template <int MODE, bool COMP>
 __global__ void __launch_bounds__(PAN_THREADS) pan_kernel(const PanArgs a) {
+  wait_for_previous();
   // sources pre-duplicated for the packed operands: panels (x0,x0,y0,y0) (x1,x1,y1,y1)
   // (hx,hx,hy,hy) (A,A,B,B) and, for the far form, d1 = -2 conj(G h), d3 = -2/3 conj(G h^3), G = A + i B,
   // as (re,re,im,im) and (-im d3, -im d3, far limit on d^2, 0); particles (x,x,y,y) (w,w,-w,-w)
@@ -472,6 +473,7 @@ __device__ __forceinline__ void pan_finish_sum(const PanArgs& a, int i, float4 t
 // consecutive targets): double-float sums when compensated; for a few splits
 template <bool COMP>
 __global__ void pan_reduce_kernel(const PanArgs a) {
+  wait_for_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.nt) return;
   float4 t = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -499,6 +501,7 @@ __global__ void pan_reduce_kernel(const PanArgs a) {
 constexpr int PAN_RED_WARPS = 32;
 template <bool COMP>
 __global__ void __launch_bounds__(32 * PAN_RED_WARPS) pan_reduce_wide_kernel(const PanArgs a) {
+  wait_for_previous();
   __shared__ float4 red[PAN_RED_WARPS][32];
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
   const int i = blockIdx.x * 32 + lane;
@@ -719,19 +722,19 @@ int launch_pan(obs_context* ctx, PanArgs& a, bool comp) {
   timing_main_begin(ctx);
   auto kernel = comp ? (a.mode == 0 ? pan_kernel<0, true> : a.mode == 1 ? pan_kernel<1, true> : pan_kernel<2, true>)
                      : (a.mode == 0 ? pan_kernel<0, false> : a.mode == 1 ? pan_kernel<1, false> : pan_kernel<2, false>);
-  kernel<<<grid, PAN_THREADS, 0, ctx->stream>>>(a);
+  launch_early(kernel, grid, PAN_THREADS, ctx->stream, a);
   ctx->launches++;
   timing_main_end(ctx);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess && a.nsplit > 16) {
     const unsigned blocks = (unsigned)((a.nt + 31) / 32);
-    if (comp) pan_reduce_wide_kernel<true><<<blocks, 32 * PAN_RED_WARPS, 0, ctx->stream>>>(a);
-    else pan_reduce_wide_kernel<false><<<blocks, 32 * PAN_RED_WARPS, 0, ctx->stream>>>(a);
+    if (comp) launch_early(pan_reduce_wide_kernel<true>, blocks, 32 * PAN_RED_WARPS, ctx->stream, a);
+    else launch_early(pan_reduce_wide_kernel<false>, blocks, 32 * PAN_RED_WARPS, ctx->stream, a);
     ctx->launches++;
     e = cudaGetLastError();
   } else if (e == cudaSuccess && a.nsplit > 1) {
-    if (comp) pan_reduce_kernel<true><<<(a.nt + 255) / 256, 256, 0, ctx->stream>>>(a);
-    else pan_reduce_kernel<false><<<(a.nt + 255) / 256, 256, 0, ctx->stream>>>(a);
+    if (comp) launch_early(pan_reduce_kernel<true>, (a.nt + 255) / 256, 256, ctx->stream, a);
+    else launch_early(pan_reduce_kernel<false>, (a.nt + 255) / 256, 256, ctx->stream, a);
     ctx->launches++;
     e = cudaGetLastError();
   }

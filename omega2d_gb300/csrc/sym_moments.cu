@@ -12,10 +12,9 @@ namespace obs {
 namespace {
 
 template <bool VJP>
-__global__ void mom_pack_kernel(const float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ r,
-                                const float* __restrict__ g, const float* __restrict__ lu, const float* __restrict__ lv,
-                                const int* __restrict__ perm, int n, int npad, MomGroup<VJP>* __restrict__ out,
-                                unsigned* __restrict__ meta) {
+__global__ void mom_pack_kernel(const float* x, const float* y, const float* r, const float* g, const float* lu,
+                                const float* lv, const int* perm, int n, int npad, MomGroup<VJP>* out, unsigned* meta) {
+  wait_for_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   int j = (i < n && perm) ? perm[i] : i;
   if ((unsigned)j >= (unsigned)n) j = 0;          // never taken for i < n: perm is a permutation
@@ -54,6 +53,7 @@ constexpr int MOM_RED_T = 64, MOM_RED_SUB = 4;
 template <class OP, int RES>
 __global__ void __launch_bounds__(MOM_RED_T * MOM_RED_SUB) mom_reduce_kernel(const MomArgs m, const MomOut o) {
   constexpr int NC = OP::NF + OP::NN, ROWS = mom_rows<OP>();
+  wait_for_previous();
   __shared__ float2 red[MOM_RED_SUB][NC][MOM_RED_T];
   const SymArgs& a = m.s;
   const int l = threadIdx.x % MOM_RED_T, sub = threadIdx.x / MOM_RED_T;
@@ -157,7 +157,7 @@ int run_moments(obs_context* ctx, bool comp, int n, const float* x, const float*
   int nl = 0;
   if (e == cudaSuccess && binned) e = bin_order(x, y, n, ctx->work.as<char>(o_sort), perm, st, &nl, BIN_HILBERT8);
   if (e != cudaSuccess) return cuda_status(e);
-  mom_pack_kernel<OP::VJP><<<(npad + 255) / 256, 256, 0, st>>>(x, y, r, g, lu, lv, perm, n, npad, grp, h->meta);
+  launch_early(mom_pack_kernel<OP::VJP>, (npad + 255) / 256, 256, st, x, y, r, g, lu, lv, perm, n, npad, grp, h->meta);
   ctx->launches += nl + 1;
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e);
 
@@ -184,10 +184,10 @@ int run_moments(obs_context* ctx, bool comp, int n, const float* x, const float*
     sym_plan_pass(m.s, slots);
     if (b > 0 && (e = cudaMemsetAsync(&h->counter, 0, sizeof(int), st)) != cudaSuccess) return cuda_status(e);
     const int grid = std::min(m.s.nrange, slots);
-    if (comp) sym_moments_kernel<OP, true><<<grid, SYM_THREADS, 0, st>>>(m);
-    else sym_moments_kernel<OP, false><<<grid, SYM_THREADS, 0, st>>>(m);
+    if (comp) launch_early(sym_moments_kernel<OP, true>, grid, SYM_THREADS, st, m);
+    else launch_early(sym_moments_kernel<OP, false>, grid, SYM_THREADS, st, m);
     if (m.s.last) timing_main_end(ctx);
-    mom_reduce_kernel<OP, RES><<<(n + MOM_RED_T - 1) / MOM_RED_T, MOM_RED_T * MOM_RED_SUB, 0, st>>>(m, out);
+    launch_early(mom_reduce_kernel<OP, RES>, (n + MOM_RED_T - 1) / MOM_RED_T, MOM_RED_T * MOM_RED_SUB, st, m, out);
     ctx->launches += 2;
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e);
   }

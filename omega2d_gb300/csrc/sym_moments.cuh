@@ -170,6 +170,7 @@ __global__ void __launch_bounds__(SYM_THREADS, 4) sym_moments_kernel(const MomAr
   constexpr int NP = OP::NP, NF = OP::NF, NN = OP::NN, NC = NF + NN;
   constexpr int GPB = mom_gpb<OP>(), ROWS = mom_rows<OP>();
   using Group = MomGroup<OP::VJP>;
+  wait_for_previous();
   const SymArgs& a = m.s;
   __shared__ Group tile[NSTAGE][MOM_TG];
   __shared__ float csum[SYM_THREADS / 32][NC][MOM_TILE];
