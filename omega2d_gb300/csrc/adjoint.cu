@@ -318,7 +318,9 @@ int run_adjoint(obs_context* ctx, int core, int accum, int mode,
   const int nob = (no + tb - 1) / tb;
   const int nst = (ne + ADJ_TILE - 1) / ADJ_TILE;
   int nsplit = std::max(1, (24 * slots + nob - 1) / nob);
-  nsplit = std::min(nsplit, std::max(1, nst / 4));
+  // splits of four tiles or more, but down to one tile where the blocks would not fill the SMs: Vatistas-2,
+  // 33,000 sources x 3,200 probes 142 -> 117 us, 80,590 x 812 112 -> 92
+  nsplit = std::max(std::min(nsplit, std::max(1, nst / 4)), std::min(nst, (slots + nob - 1) / nob));
   const int tps = (nst + nsplit - 1) / nsplit;
   nsplit = (nst + tps - 1) / tps;
   const size_t hdr = 256;

@@ -498,7 +498,10 @@ int run_adjoint_packed(obs_context* ctx, int accum, int mode, int no, const floa
   const int nob = (no + tb - 1) / tb;
   const int nst = (ne + PA_TILE - 1) / PA_TILE;
   int nsplit = std::max(1, (4 * slots + nob - 1) / nob);
-  nsplit = std::min(nsplit, std::max(1, nst / 4));
+  // splits of four tiles or more, but down to one tile where the blocks would not fill the SMs: 80,590 sources x
+  // 812 probes 254 -> 117 us, 40,000 x 600 165 -> 68, 33,000 x 3,200 217 -> 159; two SM fills instead of one take
+  // 0 to 15 % longer in half of those
+  nsplit = std::max(std::min(nsplit, std::max(1, nst / 4)), std::min(nst, (slots + nob - 1) / nob));
   const int tps = (nst + nsplit - 1) / nsplit;
   nsplit = (nst + tps - 1) / tps;
 

@@ -96,3 +96,17 @@ def test_probe_vjp_binned_reproducible(ctx):
     b = _with(ctx, og.VARIANT_AUTO, og.ORDER_BINNED, lambda: og.points_affect_points_vjp(src, probes, lu, lv, env))
     for ga, gb in zip(a, b):
         assert np.array_equal(ga, gb)
+
+
+@pytest.mark.parametrize("core", [og.CORE_GAUSSIAN, og.CORE_V2])
+@pytest.mark.parametrize("nt", [3, 129, 600, 1500])
+def test_probe_vjp_splits_down_to_a_tile(ctx, restatement, core, nt):
+    # 33,001 sources take the tiled gathers at every size; few probes are split to single tiles
+    rng = np.random.default_rng(nt)
+    sx, sy, sr, ss = _sources(rng, 33_001, 0.02)
+    px, py = rng.uniform(-1, 1, (2, nt)).astype(np.float32)
+    lu, lv = rng.normal(size=(2, nt)).astype(np.float32)
+    gx, gy, gs = og.points_affect_points_vjp(og.Points(sx, sy, sr, ss), og.Points(px, py), lu, lv,
+                                             og.ExecEnv(core, og.COMPENSATED, ctx))
+    rx, ry, rs = restatement.probe_vjp(core, sx, sy, sr, ss, px, py, lu, lv)
+    assert rel_err(rs, gs) < 1e-5 and rel_err(rx, gx) < 1e-5 and rel_err(ry, gy) < 1e-5      # as above
