@@ -140,13 +140,13 @@ def aggregate_rate(units_per_rank: float, world_size: int, max_ms: float) -> flo
 
 
 def time_gradient(og, torch, ctx, stream, dev, flush, X, Y, R, S, args):
-    """Velocity + velocity gradient of the headline patch (VELANDGRAD, generic kernel):
+    """Velocity + velocity gradient of the headline patch (VELANDGRAD):
     one timed call per accumulation mode after one warm-up, CUDA events, L2 flushed."""
     n = X.numel()
     U, V = torch.zeros(n, device=dev), torch.zeros(n, device=dev)
     G = [torch.zeros(n, device=dev) for _ in range(4)]
-    out = {"kernel": "p2p_packed_res_kernel<thick, compensated, GRAD> (Morton-ordered; far blocks d^2/s^2 > 25 "
-                     "without the exponential)", "flops_per_interaction": 41}
+    out = {"kernel": "sym_moments_kernel<MomGrad, compensated> (each unordered pair once, Hilbert-ordered; far groups "
+                     "d^2/s^2 > 25 without the exponential)", "flops_per_interaction": 41}
     for name, accum in (("compensated", og.COMPENSATED), ("plain", og.PLAIN_F32)):
         def call():
             for t in (U, V, *G):
@@ -171,7 +171,7 @@ def time_tree(og, torch, ctx, stream, flush, X, Y, R, S, args):
         V.zero_()
         og.points_affect_points_tree_dev(ctx, og.CORE_GAUSSIAN, X, Y, R, S, X, Y, R, U, V)
     ms = _event_time(torch, stream, flush, call, max(1, args.steps // 2), 2)
-    return {"kernel": "tree_eval_kernel (Morton-ordered tree of 32-source leaves, 4-way nodes, 24-term "
+    return {"kernel": "tree_eval_kernel (Hilbert-ordered tree of 32-source leaves, 4-way nodes, up to 24-term "
                       "multipole expansions; theta 0.5)", "ms": ms,
             "effective_ginter_s": float(n) * n / (ms * 1e-3) / 1e9,
             "_uv": (U, V)}
@@ -463,10 +463,11 @@ def run_engine(args):
                 "ms_per_step": float(np.mean(e2e_ms))},
         "roofline": {"bound": "fp32", "achieved": achieved, "peak": fp32_peak, "unit": "TFLOP/s",
                      "frac": achieved / fp32_peak, "traffic": traffic,
-                     "kernel": "p2p_packed_kernel<GAUSS,thick,compensated,4> (Morton-ordered targets and sources)",
+                     "kernel": "p2p_sym_kernel<GAUSS, compensated, 8> (each unordered pair once, Hilbert-ordered particles)",
                      "flops_per_interaction": FLOPS_PER_PAIR,
                      "flops_note": "the reference's count for the Gaussian thick-target velocity kernel; far "
-                                   "(warp, block) pairs execute 7 FP32 lane-ops + 1 MUFU.RCP per interaction",
+                                   "(warp, group) pairs execute 10 FP32 lane-ops + 1 MUFU.RCP per unordered pair, "
+                                   "two interactions, so the fraction can exceed 1",
                      "peak_note": f"2 x {FMA_PER_CLK_PER_SM} FP32 lanes x {nsm} SMs x {sm_max:.0f} MHz (max SM clock of measured)",
                      "frac_at_median_clock": (achieved / (fp32_peak * clocks["sm_mhz"] / sm_max)) if clocks.get("sm_mhz") else None,
                      "main_kernel_ms": main_comp},
