@@ -41,8 +41,8 @@ __device__ __forceinline__ float ord_val(unsigned k) {
 
 // bb[0] = ~min key x, bb[1] = max key x, bb[2] = ~min key y, bb[3] = max key y (zeroed first);
 // one set of atomics per block
-__global__ void __launch_bounds__(256) bin_bbox_kernel(const float* __restrict__ x, const float* __restrict__ y,
-                                                       int n, unsigned* __restrict__ bb) {
+__global__ void __launch_bounds__(256) bin_bbox_kernel(const float* x, const float* y, int n, unsigned* bb) {
+  wait_for_previous();
   __shared__ unsigned red[4][8];
   unsigned v[4] = {0u, 0u, 0u, 0u};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -97,8 +97,9 @@ __device__ __forceinline__ unsigned cell_of(float v, float lo, float scale, floa
   return (unsigned)c;
 }
 
-__global__ void bin_key_kernel(const float* __restrict__ x, const float* __restrict__ y, int n,
-                               const unsigned* __restrict__ bb, int bits, bool hilbert, unsigned* __restrict__ keys) {
+__global__ void bin_key_kernel(const float* x, const float* y, int n, const unsigned* bb, int bits, bool hilbert,
+                               unsigned* keys) {
+  wait_for_previous();
   const float cells = (float)(1 << bits);
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -112,9 +113,9 @@ __global__ void bin_key_kernel(const float* __restrict__ x, const float* __restr
 }
 
 // digit counts of one tile: table[digit * ntiles + tile]; digit totals into tot[256] (zeroed)
-__global__ void __launch_bounds__(RS_THREADS) rs_count_kernel(const unsigned* __restrict__ keys, int n, int shift,
-                                                             unsigned* __restrict__ table, int ntiles,
-                                                             unsigned* __restrict__ tot) {
+__global__ void __launch_bounds__(RS_THREADS) rs_count_kernel(const unsigned* keys, int n, int shift, unsigned* table,
+                                                             int ntiles, unsigned* tot) {
+  wait_for_previous();
   __shared__ unsigned cnt[RS_THREADS];
   cnt[threadIdx.x] = 0;
   __syncthreads();
@@ -132,8 +133,8 @@ __global__ void __launch_bounds__(RS_THREADS) rs_count_kernel(const unsigned* __
 
 // exclusive offsets in place: table[d][t] <- sum of all counts of digits < d + counts of digit d
 // in tiles < t.  One warp per digit; the row is scanned 32 tiles at a time (coalesced).
-__global__ void __launch_bounds__(256) rs_offsets_kernel(unsigned* __restrict__ table, int ntiles,
-                                                         const unsigned* __restrict__ tot) {
+__global__ void __launch_bounds__(256) rs_offsets_kernel(unsigned* table, int ntiles, const unsigned* tot) {
+  wait_for_previous();
   const int lane = threadIdx.x & 31;
   const int d = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (d >= RS_THREADS) return;
@@ -155,10 +156,10 @@ __global__ void __launch_bounds__(256) rs_offsets_kernel(unsigned* __restrict__ 
 }
 
 // stable scatter of one tile; vin == nullptr means the identity payload (the point's index)
-__global__ void __launch_bounds__(RS_THREADS) rs_scatter_kernel(const unsigned* __restrict__ kin,
-                                                               const int* __restrict__ vin, int n, int shift,
-                                                               const unsigned* __restrict__ table, int ntiles,
-                                                               unsigned* __restrict__ kout, int* __restrict__ vout) {
+__global__ void __launch_bounds__(RS_THREADS) rs_scatter_kernel(const unsigned* kin, const int* vin, int n, int shift,
+                                                               const unsigned* table, int ntiles, unsigned* kout,
+                                                               int* vout) {
+  wait_for_previous();
   __shared__ unsigned run[RS_THREADS];            // next output slot per digit for this tile
   __shared__ unsigned wcnt[RS_WARPS][RS_THREADS]; // per-warp counts of the chunk, then their prefix
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
@@ -197,10 +198,9 @@ __global__ void __launch_bounds__(RS_THREADS) rs_scatter_kernel(const unsigned* 
   }
 }
 
-__global__ void bin_gather_kernel(const int* __restrict__ perm, const float* __restrict__ x,
-                                  const float* __restrict__ y, const float* __restrict__ r,
-                                  const float* __restrict__ g, int n, float* __restrict__ bx,
-                                  float* __restrict__ by, float* __restrict__ br, float* __restrict__ bg) {
+__global__ void bin_gather_kernel(const int* perm, const float* x, const float* y, const float* r, const float* g, int n,
+                                  float* bx, float* by, float* br, float* bg) {
+  wait_for_previous();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   int i = perm[k];
@@ -238,15 +238,15 @@ cudaError_t bin_order(const float* x, const float* y, int n, void* scratch, int*
   if (e != cudaSuccess) return e;
   const int threads = 256;
   const int blocks = (n + threads - 1) / threads;
-  bin_bbox_kernel<<<blocks < 512 ? blocks : 512, threads, 0, st>>>(x, y, n, bb);
-  bin_key_kernel<<<blocks, threads, 0, st>>>(x, y, n, bb, bits, curve != BIN_MORTON8, ka);
+  launch_early(bin_bbox_kernel, blocks < 512 ? blocks : 512, threads, st, x, y, n, bb);
+  launch_early(bin_key_kernel, blocks, threads, st, x, y, n, bb, bits, curve != BIN_MORTON8, ka);
   // low digit first; the first pass has the identity payload, the last one writes perm
   const int* vin = nullptr;
   for (int q = 0; q < passes; ++q) {
     int* vout = ((passes - 1 - q) & 1) ? vb : perm;
-    rs_count_kernel<<<ntiles, RS_THREADS, 0, st>>>(ka, n, q * RS_BITS, table, ntiles, tot + q * RS_THREADS);
-    rs_offsets_kernel<<<RS_THREADS / 8, 256, 0, st>>>(table, ntiles, tot + q * RS_THREADS);
-    rs_scatter_kernel<<<ntiles, RS_THREADS, 0, st>>>(ka, vin, n, q * RS_BITS, table, ntiles, kb, vout);
+    launch_early(rs_count_kernel, ntiles, RS_THREADS, st, ka, n, q * RS_BITS, table, ntiles, tot + q * RS_THREADS);
+    launch_early(rs_offsets_kernel, RS_THREADS / 8, 256, st, table, ntiles, tot + q * RS_THREADS);
+    launch_early(rs_scatter_kernel, ntiles, RS_THREADS, st, ka, vin, n, q * RS_BITS, table, ntiles, kb, vout);
     unsigned* t = ka;
     ka = kb;
     kb = t;
@@ -259,7 +259,7 @@ cudaError_t bin_order(const float* x, const float* y, int n, void* scratch, int*
 cudaError_t bin_gather(const int* perm, const float* x, const float* y, const float* r, const float* g, int n,
                        float* bx, float* by, float* br, float* bg, cudaStream_t st, int* launches) {
   if (n <= 0) return cudaSuccess;
-  bin_gather_kernel<<<(n + 255) / 256, 256, 0, st>>>(perm, x, y, r, g, n, bx, by, br, bg);
+  launch_early(bin_gather_kernel, (n + 255) / 256, 256, st, perm, x, y, r, g, n, bx, by, br, bg);
   if (launches) *launches += 1;
   return cudaGetLastError();
 }

@@ -208,7 +208,7 @@ __device__ __forceinline__ void fold_extrema_block(unsigned rmin, unsigned rmax,
 // ---------------------------------------------------------------- launches ahead of their predecessor
 // A kernel launched with launch_early may be brought onto the SMs while the kernel before it in the
 // stream drains, which hides most of a launch's latency (ten time steps of 20,000 particles, four launches
-// a step: 1100 -> 1041 us).  It has to call wait_for_previous() before it touches memory: that returns when the
+// a step: 1100 -> 1041 us; a treecode sum of 40,000, 21 launches: 237 -> 197).  It has to call wait_for_previous() before it touches memory: that returns when the
 // kernel before is complete and its writes are seen.  Every kernel launched so does it first, so that the
 // kernels before that one are complete as well; a plain launch, copy or event after it waits for all of it.
 // Its pointers to what earlier kernels write are not const __restrict__, nor read by __ldg: such loads may be

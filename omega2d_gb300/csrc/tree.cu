@@ -122,12 +122,10 @@ __device__ __forceinline__ float warp_add(float v) {
 }
 
 // leaves: one warp per 32 sorted sources; also packs each source as (x, y, radius term, G)
-__global__ void __launch_bounds__(TREE_WARPS * 32) tree_leaf_kernel(const float* __restrict__ sx,
-                                                                    const float* __restrict__ sy,
-                                                                    const float* __restrict__ sr,
-                                                                    const float* __restrict__ sg, int ns, int core,
-                                                                    float4* __restrict__ sp4, TreeNodes nd, int nleaf,
-                                                                    int P) {
+__global__ void __launch_bounds__(TREE_WARPS * 32) tree_leaf_kernel(const float* sx, const float* sy, const float* sr,
+                                                                    const float* sg, int ns, int core, float4* sp4,
+                                                                    TreeNodes nd, int nleaf, int P) {
+  wait_for_previous();
   const int leaf = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (leaf >= nleaf) return;                        // warp-uniform
@@ -172,6 +170,7 @@ __global__ void __launch_bounds__(TREE_WARPS * 32) tree_up_kernel(TreeNodes nd, 
   __shared__ float2 cc[TREE_WARPS][TREE_PMAX];
   __shared__ float2 sum[TREE_WARPS][TREE_PMAX];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  wait_for_previous();
   const int q = blockIdx.x;
   const int c0 = q * TREE_FAN, nc = min(TREE_FAN, cnt_c - c0);
   const bool have = w < nc;                         // warp-uniform
@@ -328,6 +327,7 @@ __global__ void __launch_bounds__(TREE_WARPS * 32, 6) tree_eval_kernel(const Tre
   __shared__ TreeLeaf leafs[TREE_WARPS];
   __shared__ float4 red[TREE_WARPS][64];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  wait_for_previous();
   int* stk = stk_all[w];
   TreeLeaf& lf = leafs[w];
   const int blk = blockIdx.x;
@@ -489,8 +489,8 @@ __global__ void __launch_bounds__(TREE_WARPS * 32, 6) tree_eval_kernel(const Tre
 
 template <int CORE>
 cudaError_t tree_eval_core(bool thick, const TreeArgs& a, int grid, cudaStream_t st) {
-  if (thick) tree_eval_kernel<CORE, true><<<grid, TREE_WARPS * 32, 0, st>>>(a);
-  else tree_eval_kernel<CORE, false><<<grid, TREE_WARPS * 32, 0, st>>>(a);
+  if (thick) launch_early(tree_eval_kernel<CORE, true>, grid, TREE_WARPS * 32, st, a);
+  else launch_early(tree_eval_kernel<CORE, false>, grid, TREE_WARPS * 32, st, a);
   return cudaGetLastError();
 }
 
@@ -559,6 +559,21 @@ int run_tree(obs_context* ctx, int core, int flags, double fsx, double fsy, doub
   cudaStream_t st = ctx->stream;
   cudaError_t e = cudaSuccess;
   int launches = 0;
+  // radius extrema for the Gaussian's uniform-radius leaf sums (zeroed: "not uniform"), before the sort so that
+  // the kernels from there to the evaluation follow one another directly
+  unsigned* meta = reinterpret_cast<unsigned*>(W + o_meta);
+  if ((e = cudaMemsetAsync(meta, 0, 6 * sizeof(unsigned), st)) != cudaSuccess) return cuda_status(e);
+  if (core == CORE_GAUSS && sr) {
+    if ((e = p2p_launch_target_meta(sr, ns, meta, st)) != cudaSuccess) return cuda_status(e);
+    ++launches;
+    if (tr && tr == sr && nt == ns) {
+      e = cudaMemcpyAsync(meta + 4, meta + 2, 2 * sizeof(unsigned), cudaMemcpyDeviceToDevice, st);
+      if (e != cudaSuccess) return cuda_status(e);
+    } else if (tr) {
+      if ((e = p2p_launch_target_meta(tr, nt, meta + 2, st)) != cudaSuccess) return cuda_status(e);
+      ++launches;
+    }
+  }
   if (e == cudaSuccess) e = bin_order(sx, sy, ns, W + o_bin, sperm, st, &launches, tree_curve(ns));
   if (e == cudaSuccess) e = bin_gather(sperm, sx, sy, sr, ss, ns, bs[0], bs[1], sr ? bs[2] : nullptr, bs[3], st,
                                        &launches);
@@ -574,11 +589,11 @@ int run_tree(obs_context* ctx, int core, int flags, double fsx, double fsy, doub
     tp = tperm;
   }
   const int tb = TREE_WARPS * 32;
-  tree_leaf_kernel<<<(lev_cnt[0] + TREE_WARPS - 1) / TREE_WARPS, tb, 0, st>>>(bs[0], bs[1], sr ? bs[2] : nullptr, bs[3],
-                                                                            ns, core, sp4, nd, lev_cnt[0], P);
+  launch_early(tree_leaf_kernel, (lev_cnt[0] + TREE_WARPS - 1) / TREE_WARPS, tb, st, bs[0], bs[1], sr ? bs[2] : nullptr,
+               bs[3], ns, core, sp4, nd, lev_cnt[0], P);
   ++launches;
   for (int l = 0; l + 1 < nlev; ++l) {
-    tree_up_kernel<<<lev_cnt[l + 1], tb, 0, st>>>(nd, lev_off[l], lev_cnt[l], lev_off[l + 1], P);
+    launch_early(tree_up_kernel, lev_cnt[l + 1], tb, st, nd, lev_off[l], lev_cnt[l], lev_off[l + 1], P);
     ++launches;
   }
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e);
@@ -596,20 +611,6 @@ int run_tree(obs_context* ctx, int core, int flags, double fsx, double fsy, doub
   a.finalize = (flags & OBS_FLAG_FINALIZE) ? 1 : 0;
   a.fsx = fsx; a.fsy = fsy;
   a.status = ctx->d_status;
-  // radius extrema for the Gaussian's uniform-radius leaf sums (zeroed: "not uniform")
-  unsigned* meta = reinterpret_cast<unsigned*>(W + o_meta);
-  if ((e = cudaMemsetAsync(meta, 0, 6 * sizeof(unsigned), st)) != cudaSuccess) return cuda_status(e);
-  if (core == CORE_GAUSS && sr) {
-    if ((e = p2p_launch_target_meta(sr, ns, meta, st)) != cudaSuccess) return cuda_status(e);
-    ++launches;
-    if (tr && tr == sr && nt == ns) {
-      e = cudaMemcpyAsync(meta + 4, meta + 2, 2 * sizeof(unsigned), cudaMemcpyDeviceToDevice, st);
-      if (e != cudaSuccess) return cuda_status(e);
-    } else if (tr) {
-      if ((e = p2p_launch_target_meta(tr, nt, meta + 2, st)) != cudaSuccess) return cuda_status(e);
-      ++launches;
-    }
-  }
   a.meta = meta;
   // A warp per 64 targets, but four for the last 6 groups per SM (one resident wave of blocks) and two for the 6
   // per SM before them: whole groups started last would leave most of the chip idle at the end.  Every split warp
