@@ -10,16 +10,16 @@
 // and 3.1 with three (measured; two scalar FMAs in its place take as long), so the four
 // accumulations of a pair of pairs cost half of its 24 clocks; MUFU is at 50 %, the FMA pipe at
 // 67 %.  Other orders and groupings of the same operations and the accumulations as scalars came
-// within 3 % of one another.  Measured (compensated, one-sided -> here): 1M Gaussian patch 249 -> 182
-// ms (5.5e12 interactions/s), 131,072 Vatistas-2 plain 4.29 -> 3.28 ms, 33,001 Vatistas-2 with varying
-// radii 415 -> 271 us, ten Euler steps of 20,000 Rosenhead-Moore 1.65 -> 1.04 ms.
+// within 3 % of one another.  Measured (compensated, one-sided -> here): 1M Gaussian patch 249 -> 183
+// ms (5.5e12 interactions/s), 131,072 Vatistas-2 plain 4.29 -> 3.25 ms, 33,001 Vatistas-2 with varying
+// radii 415 -> 274 us, ten Euler steps of 20,000 Rosenhead-Moore 1.65 -> 1.08 ms.
 //
 // Layout: a row block is 1024 (or 2048) particles, eight (or sixteen) per thread of a 128-thread
 // CTA in f32x2 register pairs (a warp owns 256 or 512 consecutive ones); columns are taken 32 at a
 // time, one per lane: in step s of 32 lane l meets column l ^ s (a conflict-free shared-memory read)
 // with its rows, and the column's running sum (the step's terms added first) moves to the lane that
 // meets it next by shuffle, so after 32 steps every lane holds its own column's sum over the warp's
-// rows.  The four warps' sums are added in shared memory and leave as one FP32 pair per (row block,
+// rows (half of the rows apart from the other half, sym_group).  The four warps' sums are added in shared memory and leave as one FP32 pair per (row block,
 // column); a row's own sums stay in registers over a whole run of columns (folded into two-sum pairs
 // every 32 columns when compensated, every 256 otherwise).  Rows against their own block are one-sided.
 //
@@ -167,46 +167,61 @@ __device__ __forceinline__ float2 sym_core(float2 d2, float2 zz, const SymUni& q
   }
 }
 
-// one 32-column group against the warp's rows; cu, cv: the column sums, back at their own lane
-// at the end (COLS; a row block's own columns take none).  zrow: this thread's rows' radius terms in
-// shared memory (FORM 2).
+// one 32-column group against the warp's rows; csum: the warp's sums of the columns (COLS; a row block's own
+// columns take none), as two sums of half the rows in turn: one running sum over all of them has 8 % more
+// rounding error than the one-sided sums (the two 0 to 4 %; 0.5 % of the time at a million particles, 3 % at 20,000).
+// zrow: this thread's rows' radius terms in shared memory (FORM 2).
 template <int CORE, int FORM, bool COLS, int NP>
 __device__ __forceinline__ void sym_group(const SymGroup& grp, int lane, const SymUni& q,
                                           const float2 (&nx)[NP], const float2 (&ny)[NP], const float2 (&g)[NP],
-                                          const float* __restrict__ zrow, float2 (&u)[NP], float2 (&vn)[NP], float& cu,
-                                          float& cv) {
-  cu = cv = 0.0f;
-#pragma unroll 4
-  for (int s = 0; s < SYM_GRP; ++s) {
-    float2 su = f2(0.0f, 0.0f), sv = f2(0.0f, 0.0f);   // this step's rows
-    const int col = lane ^ s;
-    const float4 c = grp.xy[col];
-    const float2 cx = f2(c.x, c.y), cy = f2(c.z, c.w), cg = grp.g[col];
-    float2 cz = f2(0.0f, 0.0f);
-    if constexpr (FORM == 2) cz = grp.z[col];
-#pragma unroll
-    for (int p = 0; p < NP; ++p) {
-      const float2 dx = __fadd2_rn(cx, nx[p]);
-      const float2 dy = __fadd2_rn(cy, ny[p]);
-      float2 zz = f2(q.us2, q.us2);
-      if constexpr (FORM == 2)
-        zz = __fadd2_rn(cz, f2(zrow[(2 * p) * SYM_THREADS], zrow[(2 * p + 1) * SYM_THREADS]));
-      // Rosenhead-Moore takes d^2 + s^2 in the same two operations
-      const float2 d2 = __ffma2_rn(dx, dx, CORE == CORE_RM ? __ffma2_rn(dy, dy, zz) : __fmul2_rn(dy, dy));
-      const float2 k = sym_core<CORE, FORM>(d2, zz, q);
-      const float2 rr = __fmul2_rn(cg, k);
-      u[p] = __ffma2_rn(rr, dy, u[p]);
-      vn[p] = __ffma2_rn(rr, dx, vn[p]);
-      if constexpr (!COLS) continue;
-      const float2 rc = __fmul2_rn(g[p], k);
-      su = (p == 0) ? __fmul2_rn(rc, dy) : __ffma2_rn(rc, dy, su);
-      sv = (p == 0) ? __fmul2_rn(rc, dx) : __ffma2_rn(rc, dx, sv);
+                                          const float* __restrict__ zrow, float2 (&u)[NP], float2 (&vn)[NP],
+                                          float2* csum) {
+  float cu = 0.0f, cv = 0.0f;
+#pragma unroll 1
+  for (int s0 = 0; s0 < SYM_GRP; s0 += SYM_GRP / 2) {
+    if (COLS && s0) {                              // the first half's sums, at the lanes half a group away
+      csum[lane ^ s0] = make_float2(cu, cv);
+      cu = cv = 0.0f;
     }
-    if constexpr (!COLS) continue;
-    // hand the column's sums to the lane that meets it next (after the last step: to its own)
-    const int m = (s ^ (s + 1)) & 31;
-    cu = __shfl_xor_sync(0xffffffffu, cu + (su.x + su.y), m);
-    cv = __shfl_xor_sync(0xffffffffu, cv + (sv.x + sv.y), m);
+#pragma unroll 4
+    for (int s = s0; s < s0 + SYM_GRP / 2; ++s) {
+      float2 su = f2(0.0f, 0.0f), sv = f2(0.0f, 0.0f);   // this step's rows
+      const int col = lane ^ s;
+      const float4 c = grp.xy[col];
+      const float2 cx = f2(c.x, c.y), cy = f2(c.z, c.w), cg = grp.g[col];
+      float2 cz = f2(0.0f, 0.0f);
+      if constexpr (FORM == 2) cz = grp.z[col];
+#pragma unroll
+      for (int p = 0; p < NP; ++p) {
+        const float2 dx = __fadd2_rn(cx, nx[p]);
+        const float2 dy = __fadd2_rn(cy, ny[p]);
+        float2 zz = f2(q.us2, q.us2);
+        if constexpr (FORM == 2)
+          zz = __fadd2_rn(cz, f2(zrow[(2 * p) * SYM_THREADS], zrow[(2 * p + 1) * SYM_THREADS]));
+        // Rosenhead-Moore takes d^2 + s^2 in the same two operations
+        const float2 d2 = __ffma2_rn(dx, dx, CORE == CORE_RM ? __ffma2_rn(dy, dy, zz) : __fmul2_rn(dy, dy));
+        const float2 k = sym_core<CORE, FORM>(d2, zz, q);
+        const float2 rr = __fmul2_rn(cg, k);
+        u[p] = __ffma2_rn(rr, dy, u[p]);
+        vn[p] = __ffma2_rn(rr, dx, vn[p]);
+        if constexpr (!COLS) continue;
+        const float2 rc = __fmul2_rn(g[p], k);
+        su = (p == 0) ? __fmul2_rn(rc, dy) : __ffma2_rn(rc, dy, su);
+        sv = (p == 0) ? __fmul2_rn(rc, dx) : __ffma2_rn(rc, dx, sv);
+      }
+      if constexpr (!COLS) continue;
+      // hand the column's sums to the lane that meets it next (after the last step: to its own)
+      const int m = (s ^ (s + 1)) & 31;
+      cu = __shfl_xor_sync(0xffffffffu, cu + (su.x + su.y), m);
+      cv = __shfl_xor_sync(0xffffffffu, cv + (sv.x + sv.y), m);
+    }
+  }
+  if constexpr (COLS) {
+    __syncwarp();
+    const float2 h = csum[lane];
+    csum[lane] = make_float2(h.x + cu, h.y + cv);
+  } else {
+    csum[lane] = make_float2(0.0f, 0.0f);
   }
 }
 
@@ -308,7 +323,6 @@ __global__ void __launch_bounds__(SYM_THREADS, sym_occ(NP)) p2p_sym_kernel(const
         const int cnt = min(SYM_TG, ng - t * SYM_TG);
         for (int b = 0; b < cnt; ++b) {
           const SymGroup& grp = tile[st][b];
-          float cu, cv;
           bool far = false;
           if constexpr (MASKED) {
             const float4 c = grp.xy[lane];
@@ -319,13 +333,12 @@ __global__ void __launch_bounds__(SYM_THREADS, sym_occ(NP)) p2p_sym_kernel(const
           }
           auto run = [&](auto cols) {
             constexpr bool COLS = decltype(cols)::value;
-            if (!unif) sym_group<CORE, 2, COLS, NP>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, cu, cv);
-            else if (MASKED && far) sym_group<CORE, MASKED ? 0 : 1, COLS, NP>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, cu, cv);
-            else sym_group<CORE, 1, COLS, NP>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, cu, cv);
+            if (!unif) sym_group<CORE, 2, COLS, NP>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, csum[warp] + b * SYM_GRP);
+            else if (MASKED && far) sym_group<CORE, MASKED ? 0 : 1, COLS, NP>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, csum[warp] + b * SYM_GRP);
+            else sym_group<CORE, 1, COLS, NP>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, csum[warp] + b * SYM_GRP);
           };
           if (g0 + t * SYM_TG + b < gdiag) run(std::false_type{});
           else run(std::true_type{});
-          csum[warp][b * SYM_GRP + lane] = make_float2(cu, cv);
           if (COMP || b == cnt - 1) {              // plain sums fold once per tile
 #pragma unroll
             for (int p = 0; p < NP; ++p) {

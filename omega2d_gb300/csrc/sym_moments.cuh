@@ -14,7 +14,7 @@
 // X / 2 = n wv + h wu, Y / 2 = n wu - h wv: far groups need no exponential and drop the sums of e.  A pair
 // of pairs takes 17 f32x2 operations for two gradient interactions (one-sided: 24) and 23 for two VJP
 // interactions (one-sided: 34); bound by the registers' read ports like the velocity sum.
-// Measured, 131,072-particle patch, compensated (one-sided -> here): gradient 8.68 -> 6.7 ms, vorticity 5.7
+// Measured, 131,072-particle patch, compensated (one-sided -> here): gradient 8.68 -> 6.85 ms, vorticity 5.7
 // -> 4.3, shear 6.2 -> 5.1, self VJP 12.1 -> 8.5 (11.3 in Hilbert order); 3 and 4 row pairs per thread take
 // 2 to 20 % longer (fewer, larger row blocks; 128 registers either way), 5 and 6 CTAs per SM as long.
 #pragma once
@@ -67,102 +67,116 @@ __device__ __forceinline__ float2 nfma2(float2 a, float2 b, float2 c) {   // c -
   return __ffma2_rn(__fmul2_rn(a, b), f2(-1.0f, -1.0f), c);
 }
 
-// one group against the warp's rows; FORM as sym_core's; cs: the columns' sums, back at their own
-// lane at the end (velocity, X, Y and the dL/dG term as the row sees them: the reduction turns the signs)
+// one group against the warp's rows; FORM as sym_core's; csum: the warp's sums of the columns, as in sym_group
+// (velocity, X, Y and the dL/dG term as the row sees them: the reduction turns the signs)
 template <class OP, int FORM>
 __device__ __forceinline__ void mom_group(const MomGroup<OP::VJP>& grp, int lane, float us2, float ucf,
                                           const float2 (&nx)[OP::NP], const float2 (&ny)[OP::NP], const MomW (&w)[OP::NP],
                                           const float* __restrict__ zrow, float2 (&acc)[OP::NP][OP::NF + OP::NN],
-                                          float (&cs)[OP::NF + OP::NN]) {
+                                          float (*csum)[MOM_TILE]) {
   constexpr bool FAR = FORM == 0;
   constexpr int NC = OP::NF + (FAR ? 0 : OP::NN);
   const float2 half = f2(0.5f, 0.5f), mhalf = f2(-0.5f, -0.5f);
+  float cs[OP::NF + OP::NN];
 #pragma unroll
   for (int c = 0; c < OP::NF + OP::NN; ++c) cs[c] = 0.0f;
+#pragma unroll 1
+  for (int s0 = 0; s0 < SYM_GRP; s0 += SYM_GRP / 2) {
+    if (s0) {                                      // the first half's sums, at the lanes half a group away
+#pragma unroll
+      for (int c = 0; c < OP::NF + OP::NN; ++c) {
+        csum[c][lane ^ s0] = cs[c];
+        cs[c] = 0.0f;
+      }
+    }
 #pragma unroll 4
-  for (int s = 0; s < SYM_GRP; ++s) {
-    const int col = lane ^ s;
-    const float4 c4 = grp.xy[col];
-    const float2 cx = f2(c4.x, c4.y), cy = f2(c4.z, c4.w), cg = grp.g[col];
-    float2 cmlu = f2(0.0f, 0.0f), clv = cmlu;
-    if constexpr (OP::VJP) {
-      const float4 l = grp.l[col];
-      cmlu = f2(l.x, l.y);
-      clv = f2(l.z, l.w);
-    }
-    float2 t[OP::NF + OP::NN];                     // this step's rows for the column
-#pragma unroll
-    for (int c = 0; c < OP::NF + OP::NN; ++c) t[c] = f2(0.0f, 0.0f);
-    // to both particles of a pair, value v times the other one's weight
-    auto both = [&](int p, int c, float2 v, float2 wc, float2 wr) {
-      acc[p][c] = __ffma2_rn(wc, v, acc[p][c]);
-      t[c] = (p == 0) ? __fmul2_rn(wr, v) : __ffma2_rn(wr, v, t[c]);
-    };
-#pragma unroll
-    for (int p = 0; p < OP::NP; ++p) {
-      const float2 dx = __fadd2_rn(cx, nx[p]), dy = __fadd2_rn(cy, ny[p]);
-      const float2 d2 = __ffma2_rn(dx, dx, __fmul2_rn(dy, dy));
-      float2 k, B = f2(0.0f, 0.0f);
-      if constexpr (FAR) {
-        k = f2(rcp_a(d2.x), rcp_a(d2.y));
-      } else {
-        const float2 cz = (FORM == 2) ? grp.z[col] : f2(0.0f, 0.0f);
-        const float z0 = (FORM == 2) ? zrow[(2 * p) * SYM_THREADS] : 0.0f;
-        const float z1 = (FORM == 2) ? zrow[(2 * p + 1) * SYM_THREADS] : 0.0f;
-        core_eval<CORE_GAUSS, true, true, FORM == 1>(d2.x, cz.x, z0, us2, ucf, k.x, B.x);
-        core_eval<CORE_GAUSS, true, true, FORM == 1>(d2.y, cz.y, z1, us2, ucf, k.y, B.y);
-        if constexpr (OP::VJP && FORM == 1) {
-          // the exact derivative of the forward's far branch
-          B.x = (d2.x * ucf > 16.0f) ? -2.0f * k.x * k.x : B.x;
-          B.y = (d2.y * ucf > 16.0f) ? -2.0f * k.y * k.y : B.y;
-        }
-      }
-      const float2 a = mul2(k, dx), b = mul2(k, dy);
+    for (int s = s0; s < s0 + SYM_GRP / 2; ++s) {
+      const int col = lane ^ s;
+      const float4 c4 = grp.xy[col];
+      const float2 cx = f2(c4.x, c4.y), cy = f2(c4.z, c4.w), cg = grp.g[col];
+      float2 cmlu = f2(0.0f, 0.0f), clv = cmlu;
       if constexpr (OP::VJP) {
-        const float2 wu = nfma2(cg, w[p].mlu, mul2(w[p].g, cmlu)), wv = nfma2(w[p].g, clv, mul2(cg, w[p].lv));
-        float2 X, Y;                               // halved
+        const float4 l = grp.l[col];
+        cmlu = f2(l.x, l.y);
+        clv = f2(l.z, l.w);
+      }
+      float2 t[OP::NF + OP::NN];                     // this step's rows for the column
+#pragma unroll
+      for (int c = 0; c < OP::NF + OP::NN; ++c) t[c] = f2(0.0f, 0.0f);
+      // to both particles of a pair, value v times the other one's weight
+      auto both = [&](int p, int c, float2 v, float2 wc, float2 wr) {
+        acc[p][c] = __ffma2_rn(wc, v, acc[p][c]);
+        t[c] = (p == 0) ? __fmul2_rn(wr, v) : __ffma2_rn(wr, v, t[c]);
+      };
+#pragma unroll
+      for (int p = 0; p < OP::NP; ++p) {
+        const float2 dx = __fadd2_rn(cx, nx[p]), dy = __fadd2_rn(cy, ny[p]);
+        const float2 d2 = __ffma2_rn(dx, dx, __fmul2_rn(dy, dy));
+        float2 k, B = f2(0.0f, 0.0f);
         if constexpr (FAR) {
-          const float2 n = __ffma2_rn(b, b, mul2(k, mhalf)), h = mul2(a, b);
-          X = __ffma2_rn(n, wv, mul2(h, wu));
-          Y = nfma2(h, wv, mul2(n, wu));
+          k = f2(rcp_a(d2.x), rcp_a(d2.y));
         } else {
-          const float2 q = nfma2(dy, wu, mul2(dx, wv)), bq = mul2(mul2(B, half), q), kh = mul2(k, half);
-          X = __ffma2_rn(bq, dx, mul2(kh, wv));
-          Y = nfma2(kh, wu, mul2(bq, dy));
-        }
-        acc[p][0] = __fadd2_rn(acc[p][0], X);
-        acc[p][1] = __fadd2_rn(acc[p][1], Y);
-        t[0] = (p == 0) ? X : __fadd2_rn(t[0], X);
-        t[1] = (p == 0) ? Y : __fadd2_rn(t[1], Y);
-        acc[p][2] = __ffma2_rn(b, cmlu, __ffma2_rn(a, clv, acc[p][2]));
-        t[2] = __ffma2_rn(b, w[p].mlu, (p == 0) ? mul2(a, w[p].lv) : __ffma2_rn(a, w[p].lv, t[2]));
-      } else {
-        both(p, 0, b, cg, w[p].g);
-        both(p, 1, a, cg, w[p].g);
-        const float2 q = mul2(B, half);            // near: B / 2
-        if constexpr (OP::NF == 4) {
-          float2 n, h;
-          if constexpr (FAR) {
-            n = __ffma2_rn(b, b, mul2(k, mhalf));
-            h = mul2(a, b);
-          } else {
-            n = mul2(q, __ffma2_rn(dx, dx, mul2(d2, mhalf)));
-            h = mul2(mul2(B, mhalf), mul2(dx, dy));
-            both(p, 4, __ffma2_rn(q, d2, k), cg, w[p].g);
+          const float2 cz = (FORM == 2) ? grp.z[col] : f2(0.0f, 0.0f);
+          const float z0 = (FORM == 2) ? zrow[(2 * p) * SYM_THREADS] : 0.0f;
+          const float z1 = (FORM == 2) ? zrow[(2 * p + 1) * SYM_THREADS] : 0.0f;
+          core_eval<CORE_GAUSS, true, true, FORM == 1>(d2.x, cz.x, z0, us2, ucf, k.x, B.x);
+          core_eval<CORE_GAUSS, true, true, FORM == 1>(d2.y, cz.y, z1, us2, ucf, k.y, B.y);
+          if constexpr (OP::VJP && FORM == 1) {
+            // the exact derivative of the forward's far branch
+            B.x = (d2.x * ucf > 16.0f) ? -2.0f * k.x * k.x : B.x;
+            B.y = (d2.y * ucf > 16.0f) ? -2.0f * k.y * k.y : B.y;
           }
-          both(p, 2, h, cg, w[p].g);
-          both(p, 3, n, cg, w[p].g);
-        } else if constexpr (OP::NF == 3) {
-          both(p, 2, FAR ? k : mul2(abs2(q), d2), abs2(cg), abs2(w[p].g));
-        } else if constexpr (!FAR) {
-          both(p, 2, __ffma2_rn(q, d2, k), cg, w[p].g);
+        }
+        const float2 a = mul2(k, dx), b = mul2(k, dy);
+        if constexpr (OP::VJP) {
+          const float2 wu = nfma2(cg, w[p].mlu, mul2(w[p].g, cmlu)), wv = nfma2(w[p].g, clv, mul2(cg, w[p].lv));
+          float2 X, Y;                               // halved
+          if constexpr (FAR) {
+            const float2 n = __ffma2_rn(b, b, mul2(k, mhalf)), h = mul2(a, b);
+            X = __ffma2_rn(n, wv, mul2(h, wu));
+            Y = nfma2(h, wv, mul2(n, wu));
+          } else {
+            const float2 q = nfma2(dy, wu, mul2(dx, wv)), bq = mul2(mul2(B, half), q), kh = mul2(k, half);
+            X = __ffma2_rn(bq, dx, mul2(kh, wv));
+            Y = nfma2(kh, wu, mul2(bq, dy));
+          }
+          acc[p][0] = __fadd2_rn(acc[p][0], X);
+          acc[p][1] = __fadd2_rn(acc[p][1], Y);
+          t[0] = (p == 0) ? X : __fadd2_rn(t[0], X);
+          t[1] = (p == 0) ? Y : __fadd2_rn(t[1], Y);
+          acc[p][2] = __ffma2_rn(b, cmlu, __ffma2_rn(a, clv, acc[p][2]));
+          t[2] = __ffma2_rn(b, w[p].mlu, (p == 0) ? mul2(a, w[p].lv) : __ffma2_rn(a, w[p].lv, t[2]));
+        } else {
+          both(p, 0, b, cg, w[p].g);
+          both(p, 1, a, cg, w[p].g);
+          const float2 q = mul2(B, half);            // near: B / 2
+          if constexpr (OP::NF == 4) {
+            float2 n, h;
+            if constexpr (FAR) {
+              n = __ffma2_rn(b, b, mul2(k, mhalf));
+              h = mul2(a, b);
+            } else {
+              n = mul2(q, __ffma2_rn(dx, dx, mul2(d2, mhalf)));
+              h = mul2(mul2(B, mhalf), mul2(dx, dy));
+              both(p, 4, __ffma2_rn(q, d2, k), cg, w[p].g);
+            }
+            both(p, 2, h, cg, w[p].g);
+            both(p, 3, n, cg, w[p].g);
+          } else if constexpr (OP::NF == 3) {
+            both(p, 2, FAR ? k : mul2(abs2(q), d2), abs2(cg), abs2(w[p].g));
+          } else if constexpr (!FAR) {
+            both(p, 2, __ffma2_rn(q, d2, k), cg, w[p].g);
+          }
         }
       }
-    }
-    const int m = (s ^ (s + 1)) & 31;
+      const int m = (s ^ (s + 1)) & 31;
 #pragma unroll
-    for (int c = 0; c < NC; ++c) cs[c] = __shfl_xor_sync(0xffffffffu, cs[c] + (t[c].x + t[c].y), m);
+      for (int c = 0; c < NC; ++c) cs[c] = __shfl_xor_sync(0xffffffffu, cs[c] + (t[c].x + t[c].y), m);
+    }
   }
+  __syncwarp();
+#pragma unroll
+  for (int c = 0; c < OP::NF + OP::NN; ++c) csum[c][lane] += cs[c];
 }
 
 template <class OP, bool COMP>
@@ -271,7 +285,7 @@ __global__ void __launch_bounds__(SYM_THREADS, 4) sym_moments_kernel(const MomAr
         const int cnt = min(MOM_TG, ng - t * MOM_TG);
         for (int b = 0; b < cnt; ++b) {
           const Group& grp = tile[st][b];
-          float cs[NC];
+          float (*cw)[MOM_TILE] = reinterpret_cast<float (*)[MOM_TILE]>(&csum[warp][0][b * SYM_GRP]);
           bool near = true;
           if (unif) {
             const float4 c = grp.xy[lane];
@@ -280,10 +294,10 @@ __global__ void __launch_bounds__(SYM_THREADS, 4) sym_moments_kernel(const MomAr
             near = __any_sync(0xffffffffu, !(fmaf(ex, ex, ey * ey) > lim));   // a NaN coordinate is near
           }
           if (!near) {
-            mom_group<OP, 0>(grp, lane, us2, ucf, nx, ny, w, zrow + tid, acc, cs);
+            mom_group<OP, 0>(grp, lane, us2, ucf, nx, ny, w, zrow + tid, acc, cw);
           } else {
-            if (unif) mom_group<OP, 1>(grp, lane, us2, ucf, nx, ny, w, zrow + tid, acc, cs);
-            else mom_group<OP, 2>(grp, lane, us2, ucf, nx, ny, w, zrow + tid, acc, cs);
+            if (unif) mom_group<OP, 1>(grp, lane, us2, ucf, nx, ny, w, zrow + tid, acc, cw);
+            else mom_group<OP, 2>(grp, lane, us2, ucf, nx, ny, w, zrow + tid, acc, cw);
             if constexpr (NN > 0) {
               // fold this group's near-only row sums into shared memory, compensated in both modes
 #pragma unroll
@@ -300,8 +314,6 @@ __global__ void __launch_bounds__(SYM_THREADS, 4) sym_moments_kernel(const MomAr
               met_near = true;
             }
           }
-#pragma unroll
-          for (int c = 0; c < NC; ++c) csum[warp][c][b * SYM_GRP + lane] = cs[c];
           if (COMP || b == cnt - 1) {              // plain sums fold once per tile
 #pragma unroll
             for (int p = 0; p < NP; ++p)
