@@ -395,7 +395,7 @@ def run_engine(args):
         t1 = time.perf_counter()
         if k > 0:
             e2e_ms.append(1e3 * (t1 - t0))
-    h2d = 4 * N * 4 + 3 * N * 4 + 2 * N * 4
+    h2d = 4 * N * 4 + 2 * N * 4            # targets equal to the sources share their device copy
     d2h = 2 * N * 4
 
     value = aggregate_rate(pairs, ws, ms_comp)

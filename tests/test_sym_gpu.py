@@ -107,3 +107,24 @@ def test_moment_passes_match_one_sided(ctx):
     for p, q, t in zip(a, b, c):
         assert np.array_equal(p, q)
         assert rel_err(t, p) < 2e-5
+
+
+@pytest.mark.parametrize("res", [og.VELONLY, og.VELANDGRAD])
+@pytest.mark.parametrize("n", [300, 9001])
+def test_equal_host_targets_are_the_set_itself(ctx, restatement, res, n):
+    rng = np.random.default_rng(n)
+    x, y = rng.uniform(-1, 1, (2, n)).astype(np.float32)
+    r, s = np.full(n, 0.02, np.float32), rng.normal(0, 1 / np.sqrt(n), n).astype(np.float32)
+    env = og.ExecEnv(og.CORE_GAUSSIAN, og.COMPENSATED, ctx)
+    same = og.Points(x, y, r, s)
+    og.points_affect_points(same, same, res, env)
+    copy = og.Points(x, y, r)
+    og.points_affect_points(og.Points(x, y, r, s), copy, res, env)
+    assert np.array_equal(same.u, copy.u) and np.array_equal(same.v, copy.v)
+    tx = x.copy()
+    tx[-1] += 0.25                                   # the last of them elsewhere: two sets
+    other = og.Points(tx, y, r)
+    og.points_affect_points(og.Points(x, y, r, s), other, res, env)
+    u, v, _ = restatement.points_affect_points(og.CORE_GAUSSIAN, 1, x, y, r, s, tx, y, r, fp64=True)
+    assert rel_err(u, other.u) < 2e-6 and rel_err(v, other.v) < 2e-6      # the tolerance of the sums above
+    assert rel_err(u[-1:], other.u[-1:]) < 1e-4
