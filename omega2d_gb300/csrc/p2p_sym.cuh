@@ -180,7 +180,7 @@ __device__ __forceinline__ void sym_group(const SymGroup& grp, int lane, const S
 #pragma unroll 1
   for (int s0 = 0; s0 < SYM_GRP; s0 += SYM_GRP / 2) {
     if (COLS && s0) {                              // the first half's sums, at the lanes half a group away
-      csum[lane ^ s0] = make_float2(cu, cv);
+      csum[lane ^ (SYM_GRP / 2)] = make_float2(cu, cv);
       cu = cv = 0.0f;
     }
 #pragma unroll 4
