@@ -195,9 +195,10 @@ __global__ void __launch_bounds__(TREE_WARPS * 32) tree_up_kernel(TreeNodes nd, 
   float ar = 0.0f, ai = 0.0f;
   if (have) {
     const float4 gc = nd.geo[off_c + c0 + w];
-    const float rnc = gc.z > 0.0f ? gc.z : 1.0f;
-    // (z - c)/rn = s (z - c_child)/rnc + t; lane m: s^m and t^m by squaring
-    float s = rnc / rn, tr = (gc.x - cx) / rn, ti = (gc.y - cy) / rn;
+    // (z - c)/rn = s (z - c_child)/rho_child + t, |s| + |t| <= 1; lane m: s^m and t^m by squaring.  A child of
+    // radius 0 (one source, or coincident ones) has no coefficient but the first, so s = 0 does for it; taken
+    // as radius 1 its s^m = rn^-m left FP32's range in small parents, and inf times those zeros was NaN
+    float s = gc.z / rn, tr = (gc.x - cx) / rn, ti = (gc.y - cy) / rn;
     float pws = 1.0f, pwr = 1.0f, pwi = 0.0f;
 #pragma unroll
     for (int b = 0; b < 5; ++b) {
