@@ -400,10 +400,13 @@ __device__ bool gc_barrier(unsigned* bar, int* status, unsigned nb, unsigned arr
 // A system of at most GC_CLUSTER row groups runs as one thread-block cluster, whose hardware barrier
 // (release and acquire, so the blocks' global writes are seen) takes about 500 SM clocks; the counter's
 // polls through L2 take 2,500 to 3,500, two of them a fifth of a small system's iteration.  The blocks
-// of a cluster are resident together and none leaves before the others, so the barrier ends.
+// of a cluster are resident together and none leaves before the others, so the barrier ends.  Not the
+// .aligned forms: those need every warp to arrive as one, and nothing in the language brings its threads
+// together after the branches before the calls.
 constexpr int GC_CLUSTER = 16;
 __device__ __forceinline__ void gc_cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 
 // (S, s) += (T, t) in double-float: two-sum of the leading parts, the trailing parts added to
