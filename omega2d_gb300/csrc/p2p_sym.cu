@@ -41,7 +41,7 @@ __device__ __forceinline__ void df_add(float& hi, float& lo, float bh, float bl)
 // particles; eight threads share one, each every eighth partial, added up in thread order (with four ten
 // steps of 20,000 particles take 20 us longer, with sixteen as long as with four).
 constexpr int SYM_RED_T = 64, SYM_RED_SUB = 8;
-template <int NP>
+template <bool COMP, int NP>
 __global__ void __launch_bounds__(SYM_RED_T * SYM_RED_SUB) sym_reduce_kernel(const SymArgs a, const P2PArgs o) {
   constexpr int SYM_ROWS = sym_rows(NP);
   wait_for_previous();
@@ -64,12 +64,18 @@ __global__ void __launch_bounds__(SYM_RED_T * SYM_RED_SUB) sym_reduce_kernel(con
       }
     }
     const int kc = min(a.nblk, jb - a.blk0);       // row blocks of this pass before the particle's own
-    const float2* cp = a.colpart + j;
 #pragma unroll 8
     for (int m = sub; m < kc; m += SYM_RED_SUB) {
-      const float2 c = __ldcg(cp + (size_t)m * a.npad);
-      two_sum_acc(s.x, s.y, -c.x);
-      two_sum_acc(s.z, s.w, c.y);
+      const size_t at = sym_base(a, m) + (j - sym_first(a, m));
+      if constexpr (COMP) {
+        const float4 c = __ldcg(static_cast<const float4*>(a.colpart) + at);
+        df_add(s.x, s.y, -c.x, -c.y);
+        df_add(s.z, s.w, c.z, c.w);
+      } else {
+        const float2 c = __ldcg(static_cast<const float2*>(a.colpart) + at);
+        two_sum_acc(s.x, s.y, -c.x);
+        two_sum_acc(s.z, s.w, c.y);
+      }
     }
   }
   red[sub][l] = s;
@@ -96,9 +102,9 @@ __global__ void __launch_bounds__(SYM_RED_T * SYM_RED_SUB) sym_reduce_kernel(con
 // one pass: the sums, then their reduction
 template <int CORE, int NP>
 cudaError_t sym_launch(bool comp, const SymArgs& a, const P2PArgs& o, int grid, cudaStream_t st) {
-  if (comp) launch_early(p2p_sym_kernel<CORE, true, NP>, grid, SYM_THREADS, st, a);
-  else launch_early(p2p_sym_kernel<CORE, false, NP>, grid, SYM_THREADS, st, a);
-  launch_early(sym_reduce_kernel<NP>, (a.n + SYM_RED_T - 1) / SYM_RED_T, SYM_RED_T * SYM_RED_SUB, st, a, o);
+  launch_early(comp ? p2p_sym_kernel<CORE, true, NP> : p2p_sym_kernel<CORE, false, NP>, grid, SYM_THREADS, st, a);
+  launch_early(comp ? sym_reduce_kernel<true, NP> : sym_reduce_kernel<false, NP>, (a.n + SYM_RED_T - 1) / SYM_RED_T,
+               SYM_RED_T * SYM_RED_SUB, st, a, o);
   return cudaGetLastError();
 }
 
@@ -152,16 +158,19 @@ int run_p2p_sym(obs_context* ctx, const P2PRequest& rq) {
   // pays late (Gaussian, binned vs not): 20,000 173-187 vs 155 us, 40,000 458-507 vs 469-483, 60,000
   // 982-1068 vs 995-1028
   const bool binned = (rq.core == CORE_GAUSS || rq.core == CORE_CEXP) && (double)n * n >= 4e9;
-  const int pass_blk = std::min(nblk, std::max(1, (int)(SYM_COL_BYTES / ((size_t)npad * sizeof(float2)))));
-  const int max_range = 8 * slots;
+  SymArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.n = n; a.npad = npad; a.ngrp = ngrp; a.gpb = sym_gpb(np);
+  const size_t col = comp ? sizeof(float4) : sizeof(float2);
+  const SymScratch m = sym_scratch(a, nblk, slots, SYM_COL_BYTES / col);
 
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t hdr = 256;
   const size_t o_pts = hdr;
   const size_t o_run = o_pts + (size_t)(npad / SYM_GRP) * sizeof(SymGroup);
-  const size_t o_col = o_run + (pass_blk < nblk ? al((size_t)npad * sizeof(float4)) : 0);
-  const size_t o_row = o_col + al((size_t)pass_blk * npad * sizeof(float2));
-  const size_t o_perm = o_row + (size_t)(max_range + pass_blk) * 2 * rows * sizeof(float2);
+  const size_t o_col = o_run + (m.passes > 1 ? al((size_t)npad * sizeof(float4)) : 0);
+  const size_t o_row = o_col + al(m.cols * col);
+  const size_t o_perm = o_row + m.rows * 2 * rows * sizeof(float2);
   const size_t o_sort = o_perm + (binned ? al((size_t)n * sizeof(int)) : 0);
   const size_t bytes = o_sort + (binned ? bin_scratch_bytes(n) : 0);
   int s = ctx->work.ensure(bytes, st);
@@ -179,14 +188,11 @@ int run_p2p_sym(obs_context* ctx, const P2PRequest& rq) {
   ctx->launches += nl + 1;
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e);
 
-  SymArgs a;
-  std::memset(&a, 0, sizeof(a));
   a.grp = ctx->work.as<SymGroup>(o_pts);
-  a.n = n; a.npad = npad; a.ngrp = ngrp; a.gpb = sym_gpb(np);
   a.counter = &h->counter;
   a.meta = h->meta;
   a.status = ctx->d_status;
-  a.colpart = ctx->work.as<float2>(o_col);
+  a.colpart = ctx->work.as<char>(o_col);
   a.rowpart = ctx->work.as<float2>(o_row);
   a.run = ctx->work.as<float4>(o_run);
   P2PArgs o;
@@ -199,12 +205,8 @@ int run_p2p_sym(obs_context* ctx, const P2PRequest& rq) {
   o.overwrite = rq.overwrite;
 
   timing_main_begin(ctx);
-  for (int b = 0; b < nblk; b += pass_blk) {
-    a.blk0 = b;
-    a.nblk = std::min(pass_blk, nblk - b);
-    a.first = b == 0;
-    a.last = b + a.nblk == nblk;
-    sym_plan_pass(a, slots);
+  for (; a.blk0 < nblk; a.blk0 += a.nblk) {
+    sym_next_pass(a, nblk, slots, SYM_COL_BYTES / col);
     if (!a.first && (e = cudaMemsetAsync(&h->counter, 0, sizeof(int), st)) != cudaSuccess) return cuda_status(e);
     const int grid = std::min(a.nrange, slots);
     e = np == 8 ? sym_dispatch<8>(rq.core, comp, a, o, grid, st) : sym_dispatch<4>(rq.core, comp, a, o, grid, st);

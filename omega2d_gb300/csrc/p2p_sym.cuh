@@ -10,26 +10,27 @@
 // and 3.1 with three (measured; two scalar FMAs in its place take as long), so the four
 // accumulations of a pair of pairs cost half of its 24 clocks; MUFU is at 50 %, the FMA pipe at
 // 67 %.  Other orders and groupings of the same operations and the accumulations as scalars came
-// within 3 % of one another.  Measured (compensated, one-sided -> here): 1M Gaussian patch 249 -> 183
-// ms (5.5e12 interactions/s), 131,072 Vatistas-2 plain 4.29 -> 3.25 ms, 33,001 Vatistas-2 with varying
-// radii 415 -> 274 us, ten Euler steps of 20,000 Rosenhead-Moore 1.65 -> 1.08 ms.
+// within 3 % of one another.  Measured (compensated, one-sided -> here): 1M Gaussian patch 249 -> 185.6
+// ms (5.4e12 interactions/s), 131,072 Vatistas-2 plain 4.29 -> 3.26 ms, 33,001 Vatistas-2 with varying
+// radii 415 -> 274 us, ten Euler steps of 20,000 Rosenhead-Moore 1.65 -> 1.06 ms.
 //
 // Layout: a row block is 1024 (or 2048) particles, eight (or sixteen) per thread of a 128-thread
 // CTA in f32x2 register pairs (a warp owns 256 or 512 consecutive ones); columns are taken 32 at a
 // time, one per lane: in step s of 32 lane l meets column l ^ s (a conflict-free shared-memory read)
 // with its rows, and the column's running sum (the step's terms added first) moves to the lane that
 // meets it next by shuffle, so after 32 steps every lane holds its own column's sum over the warp's
-// rows (half of the rows apart from the other half, sym_group).  The four warps' sums are added in shared memory and leave as one FP32 pair per (row block,
-// column); a row's own sums stay in registers over a whole run of columns (folded into two-sum pairs
-// every 32 columns when compensated, every 256 otherwise).  Rows against their own block are one-sided.
+// rows (half of the rows apart from the other half, sym_group).  The four warps' sums are added in
+// shared memory and leave as one pair per (row block, column), (hi, lo) of each when compensated; a row's
+// own sums stay in registers over a whole run of columns (folded into two-sum pairs every 32 columns when
+// compensated, every 256 otherwise).  Rows against their own block are one-sided.
 //
 // Work: row block k meets every 32-column group from its own first one on; these (block, group)
 // units in order form a line of `total` units cut into equal ranges that the CTAs take from a
 // counter.  A range may cross blocks; each (range, block) piece writes one row partial at slot
 // range + block (strictly increasing along the line, so unique).  sym_reduce_kernel adds a
 // particle's row partials and column partials in a fixed order: results do not depend on timing.
-// Column partials take 8 bytes per (row block, particle); large sets run in passes over the row
-// blocks that keep them within a fixed scratch size.
+// Column partials take 16 bytes (8 when plain) per row block and later particle; large sets run in passes over
+// the row blocks that keep them within a fixed scratch size.
 #pragma once
 
 #include <type_traits>
@@ -68,7 +69,8 @@ struct SymArgs {
   int* counter;
   const unsigned* meta;  // radius extrema (~min, max bits)
   int* status;
-  float2* colpart;       // [nblk][npad] (sum G K dy, sum G K dx)
+  void* colpart;         // per row block, its later columns: (sum G K dy, sum G K dx) as float4, each (hi, lo),
+                         // when compensated, else float2
   float2* rowpart;       // [nrange + nblk][2][rows of a block] (hi, lo)
   float4* run;           // [npad] running sums (u hi, u lo, v hi, v lo) over the passes
   int first, last;       // first / last pass
@@ -104,13 +106,46 @@ __device__ __forceinline__ void sym_ranges_of(const SymArgs& a, int k, int& r0, 
   while (sym_range_begin(a, r1) > p1) --r1;
 }
 
+// Column partials are kept for the columns after a row block only: row block k (of the pass) has sym_width
+// of them, from column sym_first on, after those of the blocks before it (sym_base).
+__host__ __device__ __forceinline__ int sym_first(const SymArgs& a, int k) { return (a.blk0 + k + 1) * a.gpb * SYM_GRP; }
+__host__ __device__ __forceinline__ int sym_width(const SymArgs& a, int k) { return a.npad - sym_first(a, k); }
+__host__ __device__ __forceinline__ size_t sym_base(const SymArgs& a, int k) {
+  return (size_t)k * a.npad - (size_t)a.gpb * SYM_GRP * ((size_t)k * a.blk0 + (size_t)k * (k + 1) / 2);
+}
+
 // total and nrange of a pass whose blk0 and nblk are set
 inline void sym_plan_pass(SymArgs& a, int slots) {
   a.total = a.nblk * (a.ngrp - a.gpb * a.blk0) - (a.gpb / 2) * a.nblk * (a.nblk - 1);
-  // one range per resident CTA for small sets; up to eight (32 units or more each) for large
-  // ones, whose units differ in cost (near and far column groups)
-  const int per = a.total / slots, ranges = slots * (per < 64 ? 1 : per >= 256 ? 8 : per / 32);
+  // one range per resident CTA for small sets; up to sixteen (32 units or more each) for large
+  // ones, whose units differ in cost (near and far column groups; eight: the 1M patch takes 186.8 instead of 185.5 ms)
+  const int per = a.total / slots, ranges = slots * (per < 64 ? 1 : per >= 1024 ? 16 : per >= 256 ? 8 : per / 32);
   a.nrange = a.total < ranges ? a.total : ranges;
+}
+
+// a pass from row block a.blk0 of nblk on: as many row blocks as have their column partials within cap columns, one
+// at least
+inline void sym_next_pass(SymArgs& a, int nblk, int slots, size_t cap) {
+  a.nblk = 1;
+  while (a.blk0 + a.nblk < nblk && sym_base(a, a.nblk + 1) <= cap) ++a.nblk;
+  a.first = a.blk0 == 0;
+  a.last = a.blk0 + a.nblk == nblk;
+  sym_plan_pass(a, slots);
+}
+// most columns and row partials of any pass
+struct SymScratch {
+  size_t cols = 0, rows = 0;
+  int passes = 0;
+};
+inline SymScratch sym_scratch(SymArgs a, int nblk, int slots, size_t cap) {
+  SymScratch m;
+  for (a.blk0 = 0; a.blk0 < nblk; a.blk0 += a.nblk, ++m.passes) {
+    sym_next_pass(a, nblk, slots, cap);
+    const size_t c = sym_base(a, a.nblk), r = (size_t)a.nrange + a.nblk;
+    m.cols = c > m.cols ? c : m.cols;
+    m.rows = r > m.rows ? r : m.rows;
+  }
+  return m;
 }
 
 struct SymUni {
@@ -168,10 +203,13 @@ __device__ __forceinline__ float2 sym_core(float2 d2, float2 zz, const SymUni& q
 }
 
 // one 32-column group against the warp's rows; csum: the warp's sums of the columns (COLS; a row block's own
-// columns take none), as two sums of half the rows in turn: one running sum over all of them has 8 % more
-// rounding error than the one-sided sums (the two 0 to 4 %; 0.5 % of the time at a million particles, 3 % at 20,000).
+// columns take none), two sums of half the rows in turn: kept apart in the two planes of csum when compensated
+// (the tile's end adds all halves and warps in two-sums), added up otherwise.  Errors of v against FP64, one FP32
+// number per row block and column -> this (one-sided): 33,001 Vatistas-2 1.25e-7 -> 1.20e-7 (1.23e-7), 131,072
+// Gaussian patch 2.77e-8 -> 2.64e-8 (2.60e-8); time of the 1M patch 183.3 -> 185.6 ms.  Four sums of eight steps
+// each: 1.14e-7 and 2.60e-8, 189.6 ms.
 // zrow: this thread's rows' radius terms in shared memory (FORM 2).
-template <int CORE, int FORM, bool COLS, int NP>
+template <int CORE, int FORM, bool COLS, bool COMP, int NP>
 __device__ __forceinline__ void sym_group(const SymGroup& grp, int lane, const SymUni& q,
                                           const float2 (&nx)[NP], const float2 (&ny)[NP], const float2 (&g)[NP],
                                           const float* __restrict__ zrow, float2 (&u)[NP], float2 (&vn)[NP],
@@ -216,12 +254,12 @@ __device__ __forceinline__ void sym_group(const SymGroup& grp, int lane, const S
       cv = __shfl_xor_sync(0xffffffffu, cv + (sv.x + sv.y), m);
     }
   }
-  if constexpr (COLS) {
+  if constexpr (COLS && COMP) {
+    csum[SYM_TILE + lane] = make_float2(cu, cv);
+  } else if constexpr (COLS) {
     __syncwarp();
     const float2 h = csum[lane];
     csum[lane] = make_float2(h.x + cu, h.y + cv);
-  } else {
-    csum[lane] = make_float2(0.0f, 0.0f);
   }
 }
 
@@ -234,7 +272,8 @@ __global__ void __launch_bounds__(SYM_THREADS, sym_occ(NP)) p2p_sym_kernel(const
   constexpr bool MASKED = CORE == CORE_GAUSS || CORE == CORE_CEXP;
   wait_for_previous();
   __shared__ SymGroup tile[NSTAGE][SYM_TG];
-  __shared__ float2 csum[SYM_THREADS / 32][SYM_TILE];   // per-warp column sums of the tile
+  constexpr int PLANES = COMP ? 2 : 1;
+  __shared__ float2 csum[SYM_THREADS / 32][PLANES * SYM_TILE];   // per-warp column sums of the tile
   __shared__ float zrow[2 * NP * SYM_THREADS];
   __shared__ __align__(8) uint64_t bar[NSTAGE];
   __shared__ int s_range;
@@ -333,9 +372,9 @@ __global__ void __launch_bounds__(SYM_THREADS, sym_occ(NP)) p2p_sym_kernel(const
           }
           auto run = [&](auto cols) {
             constexpr bool COLS = decltype(cols)::value;
-            if (!unif) sym_group<CORE, 2, COLS, NP>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, csum[warp] + b * SYM_GRP);
-            else if (MASKED && far) sym_group<CORE, MASKED ? 0 : 1, COLS, NP>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, csum[warp] + b * SYM_GRP);
-            else sym_group<CORE, 1, COLS, NP>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, csum[warp] + b * SYM_GRP);
+            if (!unif) sym_group<CORE, 2, COLS, COMP, NP>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, csum[warp] + b * SYM_GRP);
+            else if (MASKED && far) sym_group<CORE, MASKED ? 0 : 1, COLS, COMP, NP>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, csum[warp] + b * SYM_GRP);
+            else sym_group<CORE, 1, COLS, COMP, NP>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, csum[warp] + b * SYM_GRP);
           };
           if (g0 + t * SYM_TG + b < gdiag) run(std::false_type{});
           else run(std::true_type{});
@@ -357,8 +396,18 @@ __global__ void __launch_bounds__(SYM_THREADS, sym_occ(NP)) p2p_sym_kernel(const
         const int c0 = (g0 + t * SYM_TG) * SYM_GRP;
         for (int c = tid; c < cnt * SYM_GRP; c += SYM_THREADS) {
           if (c0 + c < gdiag * SYM_GRP || c0 + c >= a.n) continue;
-          const float2 s0 = csum[0][c], s1 = csum[1][c], s2 = csum[2][c], s3 = csum[3][c];
-          a.colpart[(size_t)k * a.npad + c0 + c] = make_float2((s0.x + s1.x) + (s2.x + s3.x), (s0.y + s1.y) + (s2.y + s3.y));
+          const size_t at = sym_base(a, k) + (c0 + c - sym_first(a, k));
+          if constexpr (COMP) {
+            float2 hi = csum[0][c], lo = f2(0.0f, 0.0f);
+#pragma unroll
+            for (int w = 0; w < SYM_THREADS / 32; ++w)
+#pragma unroll
+              for (int h = w ? 0 : 1; h < PLANES; ++h) two_sum2(hi, lo, csum[w][h * SYM_TILE + c]);
+            static_cast<float4*>(a.colpart)[at] = make_float4(hi.x, lo.x, hi.y, lo.y);
+          } else {
+            const float2 s0 = csum[0][c], s1 = csum[1][c], s2 = csum[2][c], s3 = csum[3][c];
+            static_cast<float2*>(a.colpart)[at] = make_float2((s0.x + s1.x) + (s2.x + s3.x), (s0.y + s1.y) + (s2.y + s3.y));
+          }
         }
       }
       float2* rp = a.rowpart + (size_t)(range + k) * 2 * ROWS;

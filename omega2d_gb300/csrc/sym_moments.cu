@@ -50,7 +50,7 @@ struct MomOut {
 // As sym_reduce_kernel: a particle's pieces of its own row block, then the row blocks before it, four
 // threads each every fourth, then the passes before; the last pass forms and stores the results.
 constexpr int MOM_RED_T = 64, MOM_RED_SUB = 4;
-template <class OP, int RES>
+template <class OP, int RES, bool COMP>
 __global__ void __launch_bounds__(MOM_RED_T * MOM_RED_SUB) mom_reduce_kernel(const MomArgs m, const MomOut o) {
   constexpr int NC = OP::NF + OP::NN, ROWS = mom_rows<OP>();
   wait_for_previous();
@@ -65,11 +65,14 @@ __global__ void __launch_bounds__(MOM_RED_T * MOM_RED_SUB) mom_reduce_kernel(con
   if (j < a.n) {
     const int k = jb - a.blk0;
     const int kc = min(a.nblk, k);                 // row blocks of this pass before the particle's own
-    const float* cp = m.colpart + j;
 #pragma unroll 4
     for (int q = sub; q < kc; q += MOM_RED_SUB)
 #pragma unroll
-      for (int c = 0; c < NC; ++c) two_sum_acc(s[c].x, s[c].y, __ldcg(cp + ((size_t)q * NC + c) * a.npad));
+      for (int c = 0; c < NC; ++c) {
+        const size_t at = NC * sym_base(a, q) + (size_t)c * sym_width(a, q) + (j - sym_first(a, q));
+        if constexpr (COMP) df_add(s[c], __ldcg(static_cast<const float2*>(m.colpart) + at));
+        else two_sum_acc(s[c].x, s[c].y, __ldcg(static_cast<const float*>(m.colpart) + at));
+      }
     // the column sees velocity, X, Y and the strength term with the other sign
 #pragma unroll
     for (int c = 0; c < NC; ++c)
@@ -101,8 +104,8 @@ __global__ void __launch_bounds__(MOM_RED_T * MOM_RED_SUB) mom_reduce_kernel(con
   if constexpr (OP::VJP) {
     const int i = o.perm ? o.perm[j] : j;
     if ((unsigned)i >= (unsigned)a.n) return;      // never taken: perm is a permutation
-    if (o.gx) o.gx[i] = (float)((double)o.gx[i] + 2.0 * v[0] * kInv2Pi);
-    if (o.gy) o.gy[i] = (float)((double)o.gy[i] + 2.0 * v[1] * kInv2Pi);
+    if (o.gx) o.gx[i] = (float)((double)o.gx[i] - 2.0 * v[0] * kInv2Pi);
+    if (o.gy) o.gy[i] = (float)((double)o.gy[i] - 2.0 * v[1] * kInv2Pi);
     if (o.gg) o.gg[i] = (float)((double)o.gg[i] + v[2] * kInv2Pi);
   } else {
     double c[NComp<RES>::v];
@@ -138,13 +141,17 @@ int run_moments(obs_context* ctx, bool comp, int n, const float* x, const float*
   // binned vs not, us: 20,000 gradient 380 vs 369, VJP 399 vs 380; 30,000 gradient 691 vs 752, VJP 761 vs
   // 794, shear at a wide core 717 vs 621; 40,000 918 vs 1298, 1103 vs 1487, 903 vs 1077
   const bool binned = (double)n * n >= 7e8;
-  const int pass_blk = std::min(nblk, std::max(1, (int)(MOM_COL_BYTES / ((size_t)npad * NC * sizeof(float)))));
+  MomArgs m;
+  std::memset(&m, 0, sizeof(m));
+  m.s.n = n; m.s.npad = npad; m.s.ngrp = ngrp; m.s.gpb = mom_gpb<OP>();
+  const size_t col = NC * (comp ? sizeof(float2) : sizeof(float));
+  const SymScratch need = sym_scratch(m.s, nblk, slots, MOM_COL_BYTES / col);
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t o_grp = off + 256;
   const size_t o_run = o_grp + (size_t)(npad / SYM_GRP) * sizeof(Group);
-  const size_t o_col = o_run + (pass_blk < nblk ? al((size_t)npad * NC * sizeof(float2)) : 0);
-  const size_t o_row = o_col + al((size_t)pass_blk * npad * NC * sizeof(float));
-  const size_t o_perm = o_row + (size_t)(8 * slots + pass_blk) * NC * ROWS * sizeof(float2);
+  const size_t o_col = o_run + (need.passes > 1 ? al((size_t)npad * NC * sizeof(float2)) : 0);
+  const size_t o_row = o_col + al(need.cols * col);
+  const size_t o_perm = o_row + need.rows * NC * ROWS * sizeof(float2);
   const size_t o_sort = o_perm + (binned ? al((size_t)n * sizeof(int)) : 0);
   int s = ctx->work.ensure(o_sort + (binned ? bin_scratch_bytes(n) : 0), st);
   if (s) return s;
@@ -161,14 +168,11 @@ int run_moments(obs_context* ctx, bool comp, int n, const float* x, const float*
   ctx->launches += nl + 1;
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e);
 
-  MomArgs m;
-  std::memset(&m, 0, sizeof(m));
-  m.s.n = n; m.s.npad = npad; m.s.ngrp = ngrp; m.s.gpb = mom_gpb<OP>();
   m.s.counter = &h->counter;
   m.s.meta = h->meta;
   m.s.status = ctx->d_status;
   m.grp = grp;
-  m.colpart = ctx->work.as<float>(o_col);
+  m.colpart = ctx->work.as<char>(o_col);
   m.rowpart = ctx->work.as<float2>(o_row);
   m.run = ctx->work.as<float2>(o_run);
   out.p.nt = n;
@@ -176,18 +180,15 @@ int run_moments(obs_context* ctx, bool comp, int n, const float* x, const float*
   out.perm = perm;
 
   timing_main_begin(ctx);
-  for (int b = 0; b < nblk; b += pass_blk) {
-    m.s.blk0 = b;
-    m.s.nblk = std::min(pass_blk, nblk - b);
-    m.s.first = b == 0;
-    m.s.last = b + m.s.nblk == nblk;
-    sym_plan_pass(m.s, slots);
-    if (b > 0 && (e = cudaMemsetAsync(&h->counter, 0, sizeof(int), st)) != cudaSuccess) return cuda_status(e);
+  for (; m.s.blk0 < nblk; m.s.blk0 += m.s.nblk) {
+    sym_next_pass(m.s, nblk, slots, MOM_COL_BYTES / col);
+    if (!m.s.first && (e = cudaMemsetAsync(&h->counter, 0, sizeof(int), st)) != cudaSuccess) return cuda_status(e);
     const int grid = std::min(m.s.nrange, slots);
     if (comp) launch_early(sym_moments_kernel<OP, true>, grid, SYM_THREADS, st, m);
     else launch_early(sym_moments_kernel<OP, false>, grid, SYM_THREADS, st, m);
     if (m.s.last) timing_main_end(ctx);
-    launch_early(mom_reduce_kernel<OP, RES>, (n + MOM_RED_T - 1) / MOM_RED_T, MOM_RED_T * MOM_RED_SUB, st, m, out);
+    launch_early(comp ? mom_reduce_kernel<OP, RES, true> : mom_reduce_kernel<OP, RES, false>, (n + MOM_RED_T - 1) / MOM_RED_T,
+                 MOM_RED_T * MOM_RED_SUB, st, m, out);
     ctx->launches += 2;
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e);
   }

@@ -12,10 +12,10 @@
 //              the other sign, to the column, and a lv - b lu of the other particle to dL/dG
 // Beyond the core's far radius K = 1/d^2 and B = -2 K^2, so n = b^2 - K/2, h = a b, e = 0,
 // X / 2 = n wv + h wu, Y / 2 = n wu - h wv: far groups need no exponential and drop the sums of e.  A pair
-// of pairs takes 17 f32x2 operations for two gradient interactions (one-sided: 24) and 23 for two VJP
+// of pairs takes 17 f32x2 operations for two gradient interactions (one-sided: 24) and 28 for two VJP
 // interactions (one-sided: 34); bound by the registers' read ports like the velocity sum.
-// Measured, 131,072-particle patch, compensated (one-sided -> here): gradient 8.68 -> 6.85 ms, vorticity 5.7
-// -> 4.3, shear 6.2 -> 5.1, self VJP 12.1 -> 8.5 (11.3 in Hilbert order); 3 and 4 row pairs per thread take
+// Measured, 131,072-particle patch, compensated (one-sided -> here): gradient 8.66 -> 7.0 ms, vorticity 5.66
+// -> 4.5, shear 6.2 -> 5.3, self VJP 12.1 -> 8.8 (11.3 in Hilbert order); 3 and 4 row pairs per thread take
 // 2 to 20 % longer (fewer, larger row blocks; 128 registers either way), 5 and 6 CTAs per SM as long.
 #pragma once
 
@@ -35,6 +35,11 @@ struct MomShear { static constexpr int NP = 2, NF = 3, NN = 0; static constexpr 
 struct MomVjp { static constexpr int NP = 2, NF = 3, NN = 0; static constexpr bool VJP = true; static constexpr float FAR = 16.0f; };
 template <class OP> constexpr int mom_gpb() { return SYM_THREADS / 32 * 2 * OP::NP; }   // groups per row block
 template <class OP> constexpr int mom_rows() { return mom_gpb<OP>() * SYM_GRP; }
+// planes of a warp's column sums: the compensated gradient keeps the two halves of the rows apart and adds all
+// halves and warps in two-sums (131,072-particle patch: du/dx 8.3e-8 off FP64; 8.6e-8 with the halves added up
+// first, 9.4e-8 with one FP32 sum per row block, 8.5e-8 one-sided; 7.09, 6.93 and 6.80 ms).  The others' errors are
+// within 1 % of the one-sided ones or below with the halves added up
+template <class OP> constexpr int mom_planes(bool comp) { return comp && OP::NF == 4 ? 2 : 1; }
 
 // 32 columns as staged (SymGroup with the VJP's cotangents)
 template <bool VJP> struct MomGroup;
@@ -51,12 +56,12 @@ template <> struct __align__(128) MomGroup<true> {
 struct MomArgs {
   SymArgs s;               // grp, colpart, rowpart and run of SymArgs unused
   const void* grp;
-  float* colpart;          // [nblk][NF + NN][npad]
+  void* colpart;           // per row block, [NF + NN][its later columns]: float2 (hi, lo) when compensated, else float
   float2* rowpart;         // [nrange + nblk][NF + NN][rows] (hi, lo)
   float2* run;             // [NF + NN][npad] running sums over the passes
 };
 
-// a particle's weights: strength and, for the VJP, cotangents (the first one negated)
+// a particle's weights: strength (negated for the VJP) and, for the VJP, cotangents (the first one negated)
 struct MomW {
   float2 g, mlu, lv;
 };
@@ -69,11 +74,11 @@ __device__ __forceinline__ float2 nfma2(float2 a, float2 b, float2 c) {   // c -
 
 // one group against the warp's rows; FORM as sym_core's; csum: the warp's sums of the columns, as in sym_group
 // (velocity, X, Y and the dL/dG term as the row sees them: the reduction turns the signs)
-template <class OP, int FORM>
+template <class OP, int FORM, bool COMP>
 __device__ __forceinline__ void mom_group(const MomGroup<OP::VJP>& grp, int lane, float us2, float ucf,
                                           const float2 (&nx)[OP::NP], const float2 (&ny)[OP::NP], const MomW (&w)[OP::NP],
                                           const float* __restrict__ zrow, float2 (&acc)[OP::NP][OP::NF + OP::NN],
-                                          float (*csum)[MOM_TILE]) {
+                                          float (*csum)[mom_planes<OP>(COMP) * MOM_TILE], float2* nsum) {
   constexpr bool FAR = FORM == 0;
   constexpr int NC = OP::NF + (FAR ? 0 : OP::NN);
   const float2 half = f2(0.5f, 0.5f), mhalf = f2(-0.5f, -0.5f);
@@ -85,7 +90,7 @@ __device__ __forceinline__ void mom_group(const MomGroup<OP::VJP>& grp, int lane
     if (s0) {                                      // the first half's sums, at the lanes half a group away
 #pragma unroll
       for (int c = 0; c < OP::NF + OP::NN; ++c) {
-        csum[c][lane ^ s0] = cs[c];
+        csum[c][lane ^ (SYM_GRP / 2)] = cs[c];
         cs[c] = 0.0f;
       }
     }
@@ -127,26 +132,29 @@ __device__ __forceinline__ void mom_group(const MomGroup<OP::VJP>& grp, int lane
             B.y = (d2.y * ucf > 16.0f) ? -2.0f * k.y * k.y : B.y;
           }
         }
-        const float2 a = mul2(k, dx), b = mul2(k, dy);
         if constexpr (OP::VJP) {
-          const float2 wu = nfma2(cg, w[p].mlu, mul2(w[p].g, cmlu)), wv = nfma2(w[p].g, clv, mul2(cg, w[p].lv));
-          float2 X, Y;                               // halved
+          // -wu and wv from the row's negated strength (w.g here)
+          const float2 mwu = __ffma2_rn(w[p].g, cmlu, mul2(cg, w[p].mlu)), wv = __ffma2_rn(w[p].g, clv, mul2(cg, w[p].lv));
+          float2 X, Y;                               // halved and negated
           if constexpr (FAR) {
-            const float2 n = __ffma2_rn(b, b, mul2(k, mhalf)), h = mul2(a, b);
-            X = __ffma2_rn(n, wv, mul2(h, wu));
-            Y = nfma2(h, wv, mul2(n, wu));
+            const float2 b = mul2(k, dy), n = __ffma2_rn(b, b, mul2(k, mhalf)), h = mul2(mul2(k, dx), b);
+            X = nfma2(n, wv, mul2(h, mwu));
+            Y = __ffma2_rn(n, mwu, mul2(h, wv));
           } else {
-            const float2 q = nfma2(dy, wu, mul2(dx, wv)), bq = mul2(mul2(B, half), q), kh = mul2(k, half);
+            const float2 q = __ffma2_rn(dy, mwu, mul2(dx, wv)), bq = mul2(mul2(B, mhalf), q), kh = mul2(k, mhalf);
             X = __ffma2_rn(bq, dx, mul2(kh, wv));
-            Y = nfma2(kh, wu, mul2(bq, dy));
+            Y = __ffma2_rn(bq, dy, mul2(kh, mwu));
           }
           acc[p][0] = __fadd2_rn(acc[p][0], X);
           acc[p][1] = __fadd2_rn(acc[p][1], Y);
           t[0] = (p == 0) ? X : __fadd2_rn(t[0], X);
           t[1] = (p == 0) ? Y : __fadd2_rn(t[1], Y);
-          acc[p][2] = __ffma2_rn(b, cmlu, __ffma2_rn(a, clv, acc[p][2]));
-          t[2] = __ffma2_rn(b, w[p].mlu, (p == 0) ? mul2(a, w[p].lv) : __ffma2_rn(a, w[p].lv, t[2]));
+          // lv dx - lu dy first: it cancels, and K (lv dx) and K (lu dy) added one by one have 20 % more error
+          const float2 er = __ffma2_rn(dy, cmlu, mul2(dx, clv)), ec = __ffma2_rn(dy, w[p].mlu, mul2(dx, w[p].lv));
+          acc[p][2] = __ffma2_rn(k, er, acc[p][2]);
+          t[2] = (p == 0) ? mul2(k, ec) : __ffma2_rn(k, ec, t[2]);
         } else {
+          const float2 a = mul2(k, dx), b = mul2(k, dy);
           both(p, 0, b, cg, w[p].g);
           both(p, 1, a, cg, w[p].g);
           const float2 q = mul2(B, half);            // near: B / 2
@@ -173,10 +181,31 @@ __device__ __forceinline__ void mom_group(const MomGroup<OP::VJP>& grp, int lane
 #pragma unroll
       for (int c = 0; c < NC; ++c) cs[c] = __shfl_xor_sync(0xffffffffu, cs[c] + (t[c].x + t[c].y), m);
     }
-  }
-  __syncwarp();
+    if constexpr (!FAR && OP::NN > 0) {
+      // fold the near-only row sums, compensated in both modes and 16 columns at a time: in spatial order a
+      // particle's near ones come together (vorticity of 60,000: 1.4e-7 off FP64 with 32 at a time)
 #pragma unroll
-  for (int c = 0; c < OP::NF + OP::NN; ++c) csum[c][lane] += cs[c];
+      for (int c = 0; c < OP::NN; ++c)
+#pragma unroll
+        for (int p = 0; p < OP::NP; ++p)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            float2& n = nsum[(c * 2 * OP::NP + 2 * p + h) * SYM_THREADS];
+            float2 s = n;
+            two_sum_acc(s.x, s.y, h ? acc[p][OP::NF + c].y : acc[p][OP::NF + c].x);
+            n = s;
+            if (h) acc[p][OP::NF + c] = f2(0.0f, 0.0f);
+          }
+    }
+  }
+  if constexpr (mom_planes<OP>(COMP) == 2) {
+#pragma unroll
+    for (int c = 0; c < OP::NF + OP::NN; ++c) csum[c][MOM_TILE + lane] = cs[c];
+  } else {
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < OP::NF + OP::NN; ++c) csum[c][lane] += cs[c];
+  }
 }
 
 template <class OP, bool COMP>
@@ -187,7 +216,8 @@ __global__ void __launch_bounds__(SYM_THREADS, 4) sym_moments_kernel(const MomAr
   wait_for_previous();
   const SymArgs& a = m.s;
   __shared__ Group tile[NSTAGE][MOM_TG];
-  __shared__ float csum[SYM_THREADS / 32][NC][MOM_TILE];
+  constexpr int PLANES = mom_planes<OP>(COMP);
+  __shared__ float csum[SYM_THREADS / 32][NC][PLANES * MOM_TILE];
   __shared__ float2 nsum[NN > 0 ? NN : 1][2 * NP][SYM_THREADS];   // near-only row sums (hi, lo), each thread its own
   __shared__ float zrow[2 * NP * SYM_THREADS];
   __shared__ __align__(8) uint64_t bar[NSTAGE];
@@ -251,7 +281,7 @@ __global__ void __launch_bounds__(SYM_THREADS, 4) sym_moments_kernel(const MomAr
         }
         nx[p] = f2(-q0.x, -q1.x);
         ny[p] = f2(-q0.z, -q1.z);
-        w[p].g = f2(r0.g[lane].x, r1.g[lane].x);
+        w[p].g = OP::VJP ? f2(-r0.g[lane].x, -r1.g[lane].x) : f2(r0.g[lane].x, r1.g[lane].x);
         if (!unif) {                               // read by this thread alone
           zrow[(2 * p) * SYM_THREADS + tid] = r0.z[lane].x;
           zrow[(2 * p + 1) * SYM_THREADS + tid] = r1.z[lane].x;
@@ -271,7 +301,10 @@ __global__ void __launch_bounds__(SYM_THREADS, 4) sym_moments_kernel(const MomAr
         by0 = fminf(by0, __shfl_xor_sync(0xffffffffu, by0, o));
         by1 = fmaxf(by1, __shfl_xor_sync(0xffffffffu, by1, o));
       }
-      bool met_near = false;                       // warp-uniform: nsum holds sums of this piece
+#pragma unroll
+      for (int c = 0; c < NN; ++c)
+#pragma unroll
+        for (int r = 0; r < 2 * NP; ++r) nsum[c][r][tid] = f2(0.0f, 0.0f);
       for (int t = 0; t < ntile; ++t, ++kt) {
         const int st = kt % NSTAGE;
         const bool ok = mbar_wait_bounded(&bar[st], (kt / NSTAGE) & 1u, WAIT_TRIES);
@@ -285,7 +318,7 @@ __global__ void __launch_bounds__(SYM_THREADS, 4) sym_moments_kernel(const MomAr
         const int cnt = min(MOM_TG, ng - t * MOM_TG);
         for (int b = 0; b < cnt; ++b) {
           const Group& grp = tile[st][b];
-          float (*cw)[MOM_TILE] = reinterpret_cast<float (*)[MOM_TILE]>(&csum[warp][0][b * SYM_GRP]);
+          float (*cw)[PLANES * MOM_TILE] = reinterpret_cast<float (*)[PLANES * MOM_TILE]>(&csum[warp][0][b * SYM_GRP]);
           bool near = true;
           if (unif) {
             const float4 c = grp.xy[lane];
@@ -294,25 +327,10 @@ __global__ void __launch_bounds__(SYM_THREADS, 4) sym_moments_kernel(const MomAr
             near = __any_sync(0xffffffffu, !(fmaf(ex, ex, ey * ey) > lim));   // a NaN coordinate is near
           }
           if (!near) {
-            mom_group<OP, 0>(grp, lane, us2, ucf, nx, ny, w, zrow + tid, acc, cw);
+            mom_group<OP, 0, COMP>(grp, lane, us2, ucf, nx, ny, w, zrow + tid, acc, cw, &nsum[0][0][tid]);
           } else {
-            if (unif) mom_group<OP, 1>(grp, lane, us2, ucf, nx, ny, w, zrow + tid, acc, cw);
-            else mom_group<OP, 2>(grp, lane, us2, ucf, nx, ny, w, zrow + tid, acc, cw);
-            if constexpr (NN > 0) {
-              // fold this group's near-only row sums into shared memory, compensated in both modes
-#pragma unroll
-              for (int c = 0; c < NN; ++c)
-#pragma unroll
-                for (int p = 0; p < NP; ++p)
-#pragma unroll
-                  for (int h = 0; h < 2; ++h) {
-                    float2 s = met_near ? nsum[c][2 * p + h][tid] : f2(0.0f, 0.0f);
-                    two_sum_acc(s.x, s.y, h ? acc[p][NF + c].y : acc[p][NF + c].x);
-                    nsum[c][2 * p + h][tid] = s;
-                    if (h) acc[p][NF + c] = f2(0.0f, 0.0f);
-                  }
-              met_near = true;
-            }
+            if (unif) mom_group<OP, 1, COMP>(grp, lane, us2, ucf, nx, ny, w, zrow + tid, acc, cw, &nsum[0][0][tid]);
+            else mom_group<OP, 2, COMP>(grp, lane, us2, ucf, nx, ny, w, zrow + tid, acc, cw, &nsum[0][0][tid]);
           }
           if (COMP || b == cnt - 1) {              // plain sums fold once per tile
 #pragma unroll
@@ -333,10 +351,27 @@ __global__ void __launch_bounds__(SYM_THREADS, 4) sym_moments_kernel(const MomAr
         for (int c = tid; c < cnt * SYM_GRP; c += SYM_THREADS) {
           const int j = c0 + c;
           if (j < gdiag * SYM_GRP || j >= a.n) continue;
-          float* cp = m.colpart + (size_t)k * NC * a.npad + j;
+          const int wd = sym_width(a, k);
+          const size_t at = NC * sym_base(a, k) + (j - sym_first(a, k));
+          if constexpr (COMP) {
 #pragma unroll
-          for (int q = 0; q < NC; ++q)
-            cp[(size_t)q * a.npad] = (csum[0][q][c] + csum[1][q][c]) + (csum[2][q][c] + csum[3][q][c]);
+            for (int q = 0; q < NC; q += 2) {      // two components at a time
+              const int r = q + 1 < NC ? q + 1 : q;
+              float2 hi = f2(csum[0][q][c], csum[0][r][c]), lo = f2(0.0f, 0.0f);
+#pragma unroll
+              for (int w = 0; w < SYM_THREADS / 32; ++w)
+#pragma unroll
+                for (int g = w ? 0 : 1; g < PLANES; ++g)
+                  two_sum2(hi, lo, f2(csum[w][q][g * MOM_TILE + c], csum[w][r][g * MOM_TILE + c]));
+              float2* cp = static_cast<float2*>(m.colpart) + at;
+              cp[(size_t)q * wd] = f2(hi.x, lo.x);
+              if (r > q) cp[(size_t)r * wd] = f2(hi.y, lo.y);
+            }
+          } else {
+#pragma unroll
+            for (int q = 0; q < NC; ++q)
+              static_cast<float*>(m.colpart)[at + (size_t)q * wd] = (csum[0][q][c] + csum[1][q][c]) + (csum[2][q][c] + csum[3][q][c]);
+          }
         }
       }
       float2* rp = m.rowpart + (size_t)(range + k) * NC * ROWS;
@@ -349,7 +384,7 @@ __global__ void __launch_bounds__(SYM_THREADS, 4) sym_moments_kernel(const MomAr
           for (int c = 0; c < NF; ++c)
             rp[(size_t)c * ROWS + i] = h ? f2(hi[p][c].y, lo[p][c].y) : f2(hi[p][c].x, lo[p][c].x);
 #pragma unroll
-          for (int c = 0; c < NN; ++c) rp[(size_t)(NF + c) * ROWS + i] = met_near ? nsum[c][2 * p + h][tid] : f2(0.0f, 0.0f);
+          for (int c = 0; c < NN; ++c) rp[(size_t)(NF + c) * ROWS + i] = nsum[c][2 * p + h][tid];
         }
     }
     __syncthreads();
