@@ -128,6 +128,7 @@ cudaError_t sym_dispatch(int core, bool comp, const SymArgs& a, const P2PArgs& o
 // 31.2; the 1M patch 182 vs 194; 200,000 with varying Gaussian radii 13.2 vs 12.9)
 int sym_np(int n) { return n >= 30000 ? 8 : 4; }
 
+constexpr int SYM_LEAST = 32;                         // units of a range (4, 8 or 16: 0 to 8 % slower up to 80,000)
 constexpr size_t SYM_COL_BYTES = (size_t)1 << 30;     // column partials held at once
 
 }  // namespace
@@ -160,7 +161,7 @@ int run_p2p_sym(obs_context* ctx, const P2PRequest& rq) {
   const bool binned = (rq.core == CORE_GAUSS || rq.core == CORE_CEXP) && (double)n * n >= 4e9;
   SymArgs a;
   std::memset(&a, 0, sizeof(a));
-  a.n = n; a.npad = npad; a.ngrp = ngrp; a.gpb = sym_gpb(np);
+  a.n = n; a.npad = npad; a.ngrp = ngrp; a.gpb = sym_gpb(np); a.least = SYM_LEAST;
   const size_t col = comp ? sizeof(float4) : sizeof(float2);
   const SymScratch m = sym_scratch(a, nblk, slots, SYM_COL_BYTES / col);
 

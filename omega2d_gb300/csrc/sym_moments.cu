@@ -138,12 +138,15 @@ int run_moments(obs_context* ctx, bool comp, int n, const float* x, const float*
   const int npad = nblk * ROWS;
   const int ngrp = (n + SYM_GRP - 1) / SYM_GRP;
   const int slots = MOM_OCC * ctx->num_sms;
-  // binned vs not, us: 20,000 gradient 380 vs 369, VJP 399 vs 380; 30,000 gradient 691 vs 752, VJP 761 vs
-  // 794, shear at a wide core 717 vs 621; 40,000 918 vs 1298, 1103 vs 1487, 903 vs 1077
-  const bool binned = (double)n * n >= 7e8;
+  // Binned vs not, us (narrow to wide cores): 15,000 gradient 200-225 vs 232-240, vorticity 145-171 vs 175-183, shear
+  // 154-177 vs 174-181, VJP 201-222 vs 215-224; 11,500 gradient 155-176 vs 149-156, VJP 151-168 vs 137-144; 17,000 every
+  // one of them faster, VJP 237-261 vs 263-272.  Near units of a binned set cost three times the far ones and come
+  // together: in ranges of two or more units, not 32, 28,544 take 498-505 us, not 760 (gradient, wide core), 45,000
+  // 1029, not 1191
+  const bool binned = (double)n * n >= 2.8e8;
   MomArgs m;
   std::memset(&m, 0, sizeof(m));
-  m.s.n = n; m.s.npad = npad; m.s.ngrp = ngrp; m.s.gpb = mom_gpb<OP>();
+  m.s.n = n; m.s.npad = npad; m.s.ngrp = ngrp; m.s.gpb = mom_gpb<OP>(); m.s.least = binned ? 2 : 32;
   const size_t col = NC * (comp ? sizeof(float2) : sizeof(float));
   const SymScratch need = sym_scratch(m.s, nblk, slots, MOM_COL_BYTES / col);
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };

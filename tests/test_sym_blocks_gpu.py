@@ -32,3 +32,26 @@ def test_velocity_at_block_edges(ctx, restatement, core, spread, n):
         og.points_affect_points(p, p, og.VELONLY, og.ExecEnv(core, accum, ctx), finalize=True, fs=(1.0, -0.25))
         assert ctx.launches - before == 3          # packing, sums, reduction
         assert rel_err(1.0 + u / (2 * np.pi), p.u[k]) < tol and rel_err(-0.25 + v / (2 * np.pi), p.v[k]) < tol
+
+
+# sorted from 2.8e8 pairs (eight launches more), in ranges of two units or more
+@pytest.mark.parametrize("accum,tol", [(og.COMPENSATED, 2e-6), (og.PLAIN_F32, 2e-5)])    # as tests/test_sym_gpu.py
+@pytest.mark.parametrize("res", [og.VELANDGRAD, og.VELANDVORT, og.VELANDSHEAR])
+@pytest.mark.parametrize("n,launches", [(16_733, 3), (16_734, 11), (28_545, 11)])
+def test_results_about_the_spatial_order(ctx, accum, tol, res, n, launches):
+    rng = np.random.default_rng(n)
+    x, y = rng.uniform(-1, 1, (2, n)).astype(np.float32)
+    r, s = np.full(n, 0.02, np.float32), rng.normal(0, 1 / np.sqrt(n), n).astype(np.float32)
+    outs = []
+    try:
+        for variant in (og.VARIANT_GENERIC, og.VARIANT_AUTO):
+            ctx.set_kernel_variant(variant)
+            p = og.Points(x, y, r, s)
+            before = ctx.launches
+            og.points_affect_points(p, p, res, og.ExecEnv(og.CORE_GAUSSIAN, accum, ctx), finalize=True)
+            outs.append([p.u, p.v] + [a for a in (p.vort, p.shear) if a is not None] + list(p.grad or []))
+    finally:
+        ctx.set_kernel_variant(og.VARIANT_AUTO)
+    assert ctx.launches - before == launches
+    for a, b in zip(*outs):
+        assert rel_err(a, b) < tol
