@@ -1,0 +1,38 @@
+"""GPU tests of the lines between the one-launch kernels and the tiled ones (csrc/adjoint_small.cu, p2p_small.cu,
+p2p_small_res.cu) and of the tiled gathers' splits: which of them a call takes, by its launches, and its result against
+the FP64 oracle."""
+import numpy as np
+import pytest
+
+import omega2d_gb300 as og
+from conftest import rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+def points(n, seed):
+    rng = np.random.default_rng(seed)
+    x, y = rng.uniform(-1, 1, (2, n)).astype(np.float32)
+    return x, y, np.full(n, 0.02, np.float32), rng.normal(0, 1 / np.sqrt(n), n).astype(np.float32)
+
+
+def probe_vjp(ctx, core, accum, no, ne, seed):
+    """Gradients, their oracle's at the first, last and some other sources (a source's need no other), and launches."""
+    x, y, r, s = points(no, seed)
+    px, py, _, _ = points(ne, seed + 1)
+    lu, lv = np.random.default_rng(seed + 2).normal(0, 1, (2, ne)).astype(np.float32)
+    before = ctx.launches
+    got = og.points_affect_points_vjp(og.Points(x, y, r, s), og.Points(px, py), lu, lv, og.ExecEnv(core, accum, ctx))
+    k = np.unique(np.r_[:8, no - 8:no, np.linspace(0, no - 1, 24).astype(int)].clip(0, no - 1))
+    return [g[k] for g in got], (x[k], y[k], r[k], s[k], px, py, lu, lv), ctx.launches - before
+
+
+# the tolerances of tests/test_adjoint_packed_gpu.py
+@pytest.mark.parametrize("core", [og.CORE_GAUSSIAN, og.CORE_V2])
+@pytest.mark.parametrize("accum,tol", [(og.COMPENSATED, 1e-5), (og.PLAIN_F32, 1e-4)])
+@pytest.mark.parametrize("no,ne,small", [(8, 30_000, True), (8, 140_000, False), (100, 300_001, False)])
+def test_few_owners_many_elements(ctx, restatement, core, accum, tol, no, ne, small):
+    got, args, launches = probe_vjp(ctx, core, accum, no, ne, no + ne)
+    assert (launches == 1) == small
+    for a, b in zip(restatement.probe_vjp(core, *args), got):
+        assert rel_err(a, b) < tol
