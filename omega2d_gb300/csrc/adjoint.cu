@@ -252,6 +252,7 @@ __global__ void adj_reduce_kernel(const AdjArgs a) {
 #pragma unroll
   for (int q = 0; q < ADJ_NC; ++q) {
     double s = 0.0;
+#pragma unroll 8
     for (int k = 0; k < a.nsplit; ++k) s += p[((size_t)q * a.nsplit + k) * a.no + i];
     c[q] = s;
   }
@@ -286,6 +287,26 @@ cudaError_t adj_dispatch_any(int core, int mode, bool thick, bool comp, const Ad
   }
 }
 
+// Tiles per split of nob owner blocks over nst element tiles: splits of four tiles or more, but down to one tile
+// where the blocks would not fill the SMs (Vatistas-2, us: 33,000 sources x 3,200 probes 142 -> 117, 80,590 x 812
+// 112 -> 92, 70,000 x 4,500 321 -> 267).  Not where all blocks are resident at once and the busiest SM then takes
+// longer (33,000 x 7,000 208, not 224) or as long plus a reduction (100,000 x 400 64, not 70), a lone block needing
+// about the time of three for its tiles; and at most 80 splits, whose partials one thread adds up (64 x 300,000 204,
+// not 512).
+int split_tiles(int nob, int nst, int nsplit, int slots, int num_sms) {
+  auto up = [](int a, int b) { return (a + b - 1) / b; };
+  const int tps = up(nst, std::min(nsplit, std::max(1, nst / 4)));
+  const int fill = up(nst, std::min({nst, up(slots, nob), 80}));
+  if (fill >= tps) return tps;
+  // tile times of the first SM when blocks go to the SMs in turn, the shorter last split at the end
+  auto load = [&](int t) {
+    const int n = up(nst, t), whole = up((n - 1) * nob, num_sms);
+    return std::max(3 * t, whole * t + (up(n * nob, num_sms) - whole) * (nst - (n - 1) * t));
+  };
+  if ((long long)up(nst, fill) * nob <= slots && load(fill) >= load(tps) + (tps == nst ? 0 : 1)) return tps;
+  return fill;
+}
+
 }  // namespace
 
 // One VJP gather.  mode ADJ_SRC: owners = sources (ox.. = sx, sy, sr, sg), elements = targets
@@ -318,10 +339,7 @@ int run_adjoint(obs_context* ctx, int core, int accum, int mode,
   const int nob = (no + tb - 1) / tb;
   const int nst = (ne + ADJ_TILE - 1) / ADJ_TILE;
   int nsplit = std::max(1, (24 * slots + nob - 1) / nob);
-  // splits of four tiles or more, but down to one tile where the blocks would not fill the SMs: Vatistas-2,
-  // 33,000 sources x 3,200 probes 142 -> 117 us, 80,590 x 812 112 -> 92
-  nsplit = std::max(std::min(nsplit, std::max(1, nst / 4)), std::min(nst, (slots + nob - 1) / nob));
-  const int tps = (nst + nsplit - 1) / nsplit;
+  const int tps = split_tiles(nob, nst, nsplit, slots, ctx->num_sms);
   nsplit = (nst + tps - 1) / tps;
   const size_t hdr = 256;
   const size_t ebytes = (size_t)nst * ADJ_TILE * 2 * sizeof(float4);

@@ -477,6 +477,27 @@ cudaError_t pa_dispatch(int mode, bool thick, bool comp, const PAArgs* a, int gr
 
 size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 
+// Tiles per split of nob owner blocks over nst element tiles: splits of four tiles or more, but down to one tile
+// where the blocks would not fill the slots and the longest chain of tiles that a slot works off gets shorter (four
+// blocks an SM wait on latency: a tile takes as long with one of them).  80,590 sources x 812 probes 254 -> 117 us,
+// 40,000 x 600 165 -> 68, 33,000 x 3,200 217 -> 159; but 100,000 x 1,500 203 us with three splits and 249 with four,
+// some of whose blocks make a second wave, 26,000 x 4,500 204 and 237.
+int split_tiles(int nob, int nst, int nsplit, int slots) {
+  auto up = [](int a, int b) { return (a + b - 1) / b; };
+  const int tps = up(nst, std::min(nsplit, std::max(1, nst / 4)));
+  const int fill = up(nst, std::min(nst, up(slots, nob)));
+  // blocks in order of splits, the shorter last split's at the end
+  auto chain = [&](int t) {
+    const int n = up(nst, t), last = nst - (n - 1) * t;
+    const long long whole = (long long)(n - 1) * nob;
+    const int q = (int)(whole / slots), r = (int)(whole % slots);
+    const long long room = (long long)(slots - r) * (t / last);
+    if (nob > room) return (q + 1) * t + (int)((nob - room + slots - 1) / slots) * last;
+    return std::max(r ? (q + 1) * t : 0, q * t + up(nob, slots - r) * last);
+  };
+  return fill < tps && chain(fill) < chain(tps) ? fill : tps;
+}
+
 }  // namespace
 
 bool adjoint_packed_supported(int core) { return core == CORE_GAUSS; }
@@ -498,11 +519,7 @@ int run_adjoint_packed(obs_context* ctx, int accum, int mode, int no, const floa
   const int nob = (no + tb - 1) / tb;
   const int nst = (ne + PA_TILE - 1) / PA_TILE;
   int nsplit = std::max(1, (4 * slots + nob - 1) / nob);
-  // splits of four tiles or more, but down to one tile where the blocks would not fill the SMs: 80,590 sources x
-  // 812 probes 254 -> 117 us, 40,000 x 600 165 -> 68, 33,000 x 3,200 217 -> 159; two SM fills instead of one take
-  // 0 to 15 % longer in half of those
-  nsplit = std::max(std::min(nsplit, std::max(1, nst / 4)), std::min(nst, (slots + nob - 1) / nob));
-  const int tps = (nst + nsplit - 1) / nsplit;
+  const int tps = split_tiles(nob, nst, nsplit, slots);
   nsplit = (nst + tps - 1) / tps;
 
   // processing order: the owners are the gather's targets, the elements its sources

@@ -36,3 +36,14 @@ def test_few_owners_many_elements(ctx, restatement, core, accum, tol, no, ne, sm
     assert (launches == 1) == small
     for a, b in zip(restatement.probe_vjp(core, *args), got):
         assert rel_err(a, b) < tol
+
+
+# one split; splits of one tile; a shorter last split; a second wave of blocks; more splits than one thread unrolls
+@pytest.mark.parametrize("core", [og.CORE_GAUSSIAN, og.CORE_V2])
+@pytest.mark.parametrize("no,ne", [(40_000, 200), (33_001, 812), (80_590, 812), (100_000, 1500), (70_000, 4500), (26_000, 4500),
+                                   (17_000, 7001)])
+def test_gather_splits(ctx, restatement, core, no, ne):
+    got, args, launches = probe_vjp(ctx, core, og.COMPENSATED, no, ne, no + ne)
+    assert launches > 1
+    for a, b in zip(restatement.probe_vjp(core, *args), got):
+        assert rel_err(a, b) < 1e-5
