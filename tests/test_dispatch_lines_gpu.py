@@ -47,3 +47,20 @@ def test_gather_splits(ctx, restatement, core, no, ne):
     assert launches > 1
     for a, b in zip(restatement.probe_vjp(core, *args), got):
         assert rel_err(a, b) < 1e-5
+
+
+@pytest.mark.parametrize("core", [og.CORE_GAUSSIAN, og.CORE_V2])
+@pytest.mark.parametrize("res,ns,nt,small", [(og.VELONLY, 32_768, 2400, True), (og.VELONLY, 20_000, 2500, True),
+                                             (og.VELONLY, 20_001, 2500, False), (og.VELANDGRAD, 32_768, 1200, True),
+                                             (og.VELANDGRAD, 28_001, 1300, False), (og.VELANDGRAD, 1000, 17_000, False),
+                                             (og.VELANDVORT, 32_768, 1300, True)])
+def test_one_launch_sums_past_a_wave(ctx, restatement, core, res, ns, nt, small):
+    x, y, r, s = points(ns, ns + nt)
+    tx, ty, _, _ = points(nt, nt)
+    t = og.Points(tx, ty)
+    before = ctx.launches
+    og.points_affect_points(og.Points(x, y, r, s), t, res, og.ExecEnv(core, og.COMPENSATED, ctx))
+    assert (ctx.launches - before == 1) == small
+    k = np.r_[:16, nt - 16:nt]
+    u, v, _ = restatement.points_affect_points(core, 1, x, y, r, s, tx[k], ty[k], None, fp64=True)
+    assert rel_err(u, t.u[k]) < 2e-6 and rel_err(v, t.v[k]) < 2e-6
