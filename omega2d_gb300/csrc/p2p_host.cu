@@ -174,11 +174,11 @@ int run_p2p(obs_context* ctx, const P2PRequest& rq) {
   // exponential for far (warp, block) pairs
   const int order = ctx->target_order;
   const bool gauss_packed = packed && masked_core;
-  // Spatial order pays for the sort from ~7e8 pairs (field points, Gaussian, radius 0.01, binned vs
-  // not: 20,000 of 40,000 particles 368 vs 401 us, 4,000 of 500,000 788 vs 903, 2,000 of 500,000 515 vs
-  // 522, but 5,000 of 100,000 290 vs 274); for the compact exponential's costlier near form from ~3e8
+  // Spatial order pays for the sort from ~6e8 pairs (field points, Gaussian, radius 0.01, binned vs
+  // not: 20,000 of 40,000 particles 368 vs 401 us, 20,000 of 33,000 333 vs 345, 4,000 of 500,000 788 vs 903, 2,000 of
+  // 500,000 515 vs 522, but 5,000 of 100,000 290 vs 274); for the compact exponential's costlier near form from ~3e8
   const double pairs = (double)rq.ns * rq.nt;
-  const bool big = pairs >= (rq.core == CORE_CEXP ? 3e8 : 7e8) && rq.nt >= 2000 && rq.ns >= 4096;
+  const bool big = pairs >= (rq.core == CORE_CEXP ? 3e8 : 6e8) && rq.nt >= 2000 && rq.ns >= 4096;
   const bool bin_t = gauss_packed && (order == OBS_ORDER_BINNED || order == OBS_ORDER_BINNED_TARGETS ||
                                       (order == OBS_ORDER_AUTO && big));
   const bool bin_s = gauss_packed && (order == OBS_ORDER_BINNED || (order == OBS_ORDER_AUTO && big));

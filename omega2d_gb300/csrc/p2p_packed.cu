@@ -61,8 +61,8 @@ int packed_np(int core, int variant, int ns, int nt) {
   if (core == CORE_V3 || core == CORE_SING) return 2;
   // Many sources split over the grid fill it with fewer targets (field points, 4 vs 2 pairs): 10,000 of
   // 500,000 particles Gaussian 1569 vs 1609 us, Vatistas-2 1468 vs 1591; 20,000 of 1M 5530 vs 5765; but
-  // 20,000 of 40,000 371 vs 368
-  if (nt >= 4000 && (double)ns * nt >= 1e9) return 4;
+  // 20,000 of 40,000 371 vs 368, 4,500 of 1M Vatistas-2 1491 vs 1462
+  if (nt >= 5000 && (double)ns * nt >= 1e9) return 4;
   if (nt < (core == CORE_CEXP ? 98304 : 49152)) return 2;
   return 4;
 }
