@@ -81,6 +81,10 @@ int obs_last_failure(obs_context* ctx, int* bits, int* code, int* v1, int* v2);
  * Returns the status the next synchronizing call reads: OBS_ERR_TIMEOUT when the wait gave up
  * as designed; the context stays usable. */
 int obs_selftest_bounded_wait(obs_context* ctx, int which, int max_polls);
+/* Memory self-test: sums that evaluate each pair of one set once take no more than this many bytes of device
+ * work buffer (0: no limit), as if the device had no more: they run in more passes, and below what one pass
+ * of one row block needs the one-sided kernels serve. */
+int obs_selftest_pair_scratch(obs_context* ctx, unsigned long long bytes);
 /* Kernel variant for particle-on-particle sums.  AUTO uses the packed-FP32 kernels (two
  * targets per f32x2 register pair) where they exist -- velocity for every core, with 4 target
  * pairs per thread (2 for Vatistas n=3, the singular core and sums with fewer than 49,152

@@ -167,6 +167,10 @@ class Context:
         _check(lib().obs_last_failure(self._h, *[ctypes.byref(v) for v in w]), "obs_last_failure")
         return tuple(v.value for v in w)
 
+    def selftest_pair_scratch(self, max_bytes: int = 0) -> None:
+        """Most bytes of device work buffer for the sums that evaluate each pair once (0: no limit)."""
+        _check(lib().obs_selftest_pair_scratch(self._h, ctypes.c_ulonglong(max_bytes)), "obs_selftest_pair_scratch")
+
     def selftest_bounded_wait(self, which: int, max_polls: int = 64) -> int:
         """Run a bounded wait that nothing completes (0: mbarrier, 1: grid barrier) and return the
         status the host reads afterwards (OBS_ERR_TIMEOUT when it gave up as designed)."""

@@ -35,6 +35,24 @@ int DevBuf::ensure(size_t bytes, cudaStream_t st) {
   return OBS_OK;
 }
 
+int DevBuf::grow(size_t bytes, size_t most, cudaStream_t st) {
+  if (most && bytes > most) return OBS_ERR_ALLOC;
+  if (bytes <= cap) return OBS_OK;
+  const size_t want = most ? bytes : bytes + std::min(bytes / 4, (size_t)64 << 20);
+  void* q = nullptr;
+  if (cudaMalloc(&q, want) != cudaSuccess) {
+    cudaGetLastError();
+    return OBS_ERR_ALLOC;
+  }
+  if (p) {
+    cudaStreamSynchronize(st);
+    cudaFree(p);
+  }
+  p = q;
+  cap = want;
+  return OBS_OK;
+}
+
 void DevBuf::release() {
   if (p) cudaFree(p);
   p = nullptr;
@@ -227,6 +245,12 @@ int obs_last_failure(obs_context* ctx, int* bits, int* code, int* v1, int* v2) {
   if (code) *code = ctx->last_failure[1];
   if (v1) *v1 = ctx->last_failure[2];
   if (v2) *v2 = ctx->last_failure[3];
+  return OBS_OK;
+}
+
+int obs_selftest_pair_scratch(obs_context* ctx, unsigned long long bytes) {
+  if (!ctx) return OBS_ERR_ARG;
+  ctx->pair_scratch = (size_t)bytes;
   return OBS_OK;
 }
 

@@ -15,6 +15,9 @@ struct DevBuf {
   void* p = nullptr;
   size_t cap = 0;
   int ensure(size_t bytes, cudaStream_t st);
+  // The same, but a buffer in use is given up only once the larger one is there: OBS_ERR_ALLOC leaves it as it
+  // was.  No more than `most` bytes (0: no limit).
+  int grow(size_t bytes, size_t most, cudaStream_t st);
   void release();
   template <class T> T* as(size_t byte_offset = 0) const {
     return reinterpret_cast<T*>(static_cast<char*>(p) + byte_offset);
@@ -68,6 +71,7 @@ struct obs_context {
   long long launches = 0;
   int kernel_variant = 0;   // OBS_VARIANT_*
   int target_order = 0;     // OBS_ORDER_*
+  size_t pair_scratch = 0;  // most bytes the pair-once sums' work buffer grows to (0: no limit; a self-test sets it)
 };
 
 namespace obs {

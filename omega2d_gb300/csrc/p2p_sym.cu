@@ -163,19 +163,21 @@ int run_p2p_sym(obs_context* ctx, const P2PRequest& rq) {
   std::memset(&a, 0, sizeof(a));
   a.n = n; a.npad = npad; a.ngrp = ngrp; a.gpb = sym_gpb(np); a.least = SYM_LEAST;
   const size_t col = comp ? sizeof(float4) : sizeof(float2);
-  const SymScratch m = sym_scratch(a, nblk, slots, SYM_COL_BYTES / col);
-
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  const size_t hdr = 256;
-  const size_t o_pts = hdr;
-  const size_t o_run = o_pts + (size_t)(npad / SYM_GRP) * sizeof(SymGroup);
-  const size_t o_col = o_run + (m.passes > 1 ? al((size_t)npad * sizeof(float4)) : 0);
-  const size_t o_row = o_col + al(m.cols * col);
-  const size_t o_perm = o_row + m.rows * 2 * rows * sizeof(float2);
-  const size_t o_sort = o_perm + (binned ? al((size_t)n * sizeof(int)) : 0);
-  const size_t bytes = o_sort + (binned ? bin_scratch_bytes(n) : 0);
-  int s = ctx->work.ensure(bytes, st);
-  if (s) return s;
+  const size_t o_pts = 256, o_run = o_pts + (size_t)(npad / SYM_GRP) * sizeof(SymGroup);
+  size_t o_col, o_row, o_perm, o_sort, cap = SYM_COL_BYTES / col;
+  // column partials of at most a pass's share; of half as much, down to one row block at a time, where the device has
+  // no room
+  for (;; cap /= 2) {
+    const SymScratch m = sym_scratch(a, nblk, slots, cap);
+    o_col = o_run + (m.passes > 1 ? al((size_t)npad * sizeof(float4)) : 0);
+    o_row = o_col + al(m.cols * col);
+    o_perm = o_row + m.rows * 2 * rows * sizeof(float2);
+    o_sort = o_perm + (binned ? al((size_t)n * sizeof(int)) : 0);
+    const int s = ctx->work.grow(o_sort + (binned ? bin_scratch_bytes(n) : 0), ctx->pair_scratch, st);
+    if (s == OBS_OK) break;
+    if (m.passes == nblk) return s;
+  }
   WorkHeader* h = ctx->work.as<WorkHeader>(0);
   int* perm = binned ? ctx->work.as<int>(o_perm) : nullptr;
 
@@ -207,7 +209,7 @@ int run_p2p_sym(obs_context* ctx, const P2PRequest& rq) {
 
   timing_main_begin(ctx);
   for (; a.blk0 < nblk; a.blk0 += a.nblk) {
-    sym_next_pass(a, nblk, slots, SYM_COL_BYTES / col);
+    sym_next_pass(a, nblk, slots, cap);
     if (!a.first && (e = cudaMemsetAsync(&h->counter, 0, sizeof(int), st)) != cudaSuccess) return cuda_status(e);
     const int grid = std::min(a.nrange, slots);
     e = np == 8 ? sym_dispatch<8>(rq.core, comp, a, o, grid, st) : sym_dispatch<4>(rq.core, comp, a, o, grid, st);

@@ -148,16 +148,19 @@ int run_moments(obs_context* ctx, bool comp, int n, const float* x, const float*
   std::memset(&m, 0, sizeof(m));
   m.s.n = n; m.s.npad = npad; m.s.ngrp = ngrp; m.s.gpb = mom_gpb<OP>(); m.s.least = binned ? 2 : 32;
   const size_t col = NC * (comp ? sizeof(float2) : sizeof(float));
-  const SymScratch need = sym_scratch(m.s, nblk, slots, MOM_COL_BYTES / col);
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  const size_t o_grp = off + 256;
-  const size_t o_run = o_grp + (size_t)(npad / SYM_GRP) * sizeof(Group);
-  const size_t o_col = o_run + (need.passes > 1 ? al((size_t)npad * NC * sizeof(float2)) : 0);
-  const size_t o_row = o_col + al(need.cols * col);
-  const size_t o_perm = o_row + need.rows * NC * ROWS * sizeof(float2);
-  const size_t o_sort = o_perm + (binned ? al((size_t)n * sizeof(int)) : 0);
-  int s = ctx->work.ensure(o_sort + (binned ? bin_scratch_bytes(n) : 0), st);
-  if (s) return s;
+  const size_t o_grp = off + 256, o_run = o_grp + (size_t)(npad / SYM_GRP) * sizeof(Group);
+  size_t o_col, o_row, o_perm, o_sort, cap = MOM_COL_BYTES / col;
+  for (;; cap /= 2) {                              // as run_p2p_sym
+    const SymScratch need = sym_scratch(m.s, nblk, slots, cap);
+    o_col = o_run + (need.passes > 1 ? al((size_t)npad * NC * sizeof(float2)) : 0);
+    o_row = o_col + al(need.cols * col);
+    o_perm = o_row + need.rows * NC * ROWS * sizeof(float2);
+    o_sort = o_perm + (binned ? al((size_t)n * sizeof(int)) : 0);
+    const int s = ctx->work.grow(o_sort + (binned ? bin_scratch_bytes(n) : 0), ctx->pair_scratch, st);
+    if (s == OBS_OK) break;
+    if (need.passes == nblk) return s;
+  }
   WorkHeader* h = ctx->work.as<WorkHeader>(off);
   int* perm = binned ? ctx->work.as<int>(o_perm) : nullptr;
   Group* grp = ctx->work.as<Group>(o_grp);
@@ -184,7 +187,7 @@ int run_moments(obs_context* ctx, bool comp, int n, const float* x, const float*
 
   timing_main_begin(ctx);
   for (; m.s.blk0 < nblk; m.s.blk0 += m.s.nblk) {
-    sym_next_pass(m.s, nblk, slots, MOM_COL_BYTES / col);
+    sym_next_pass(m.s, nblk, slots, cap);
     if (!m.s.first && (e = cudaMemsetAsync(&h->counter, 0, sizeof(int), st)) != cudaSuccess) return cuda_status(e);
     const int grid = std::min(m.s.nrange, slots);
     if (comp) launch_early(sym_moments_kernel<OP, true>, grid, SYM_THREADS, st, m);
