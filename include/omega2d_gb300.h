@@ -443,12 +443,13 @@ int obs_points_affect_points_noalloc(void* cuda_stream, int core, int result, in
  * (results_t velonly), every core, thick (tr) or field-point (tr == NULL) targets; outputs
  * accumulated like obs_points_affect_points (OBS_FLAG_FINALIZE applies finalize_vels).
  * Sources in Hilbert order form a tree of 32-source leaves and 4-way nodes carrying `order`
- * multipole coefficients; a node acts on a warp of 32 targets through its expansion when its
+ * multipole coefficients; a node acts on a warp of 64 targets through its expansion when its
  * radius is at most theta times the distance from its centre to the targets' box and every
  * pair lies where the core equals 1/d^2 (exactly for the Gaussian and compact exponential cut-
  * offs and the singular core; within 2^-24 for the others), else it opens, down to direct
  * sums over leaves with the core.  Truncation per node is below theta^order/(1 - theta) of
- * its summed |strength|/distance.  theta in (0, 1) (0 selects the default), order 1..32 (0:
+ * its summed |strength|/distance; where |w| = radius/distance is smaller, fewer terms are
+ * taken, down to the first p with |w|^p below both theta^order/4 and 2^-26.  theta in (0, 1) (0 selects the default), order 1..32 (0:
  * default).  Compensated accumulation; flops (optional) receives the direct-sum count of the
  * same call.  _dev: device arrays, asynchronous on the context's stream.
  */

@@ -19,8 +19,9 @@
 //     when rho <= theta (|z - c| - r) for the warp's target box (r its half diagonal), so |w|
 //     <= theta and the truncation after P terms is below theta^P/(1 - theta) of the node's
 //     sum |G_j|/|z - z_j| (a node farther away stops at the first term count whose |w|^p is below
-//     theta^P / 4: about half of 24 terms on average); and only when every (target, source) pair of the node lies in the
-//     core's far regime, where the core is 1/d^2: for the Gaussian and the compact exponential
+//     both theta^P / 4 and 2^-26: about half of 24 terms on average; the second one keeps distant nodes at
+//     FP32's precision where a caller asks for few terms); and only when every (target, source) pair of the
+//     node lies in the core's far regime, where the core is 1/d^2: for the Gaussian and the compact exponential
 //     that is the reference's own cut-off (d^2/s^2 > 16, (d/s)^3 > 16: the far branch IS 1/d^2,
 //     src/CoreFunc.h:119-131), for the singular core always, and for Rosenhead-Moore,
 //     Winckelmans-Leonard and the Vatistas cores where the core differs from 1/d^2 by less
@@ -100,7 +101,7 @@ struct TreeArgs {
   int lev_cnt[TREE_MAXLEV];
   int P;
   float theta;
-  float lterm;       // log2(theta^P / 4): a node stops at the first p with p log2|w| below it
+  float lterm;       // log2 of the smaller of theta^P / 4 and 2^-26: a node stops at the first p with p log2|w| below it
   int one, two;      // blocks with a warp per target group, then blocks with two, then four
   int finalize;
   double fsx, fsy;
@@ -608,7 +609,7 @@ int run_tree(obs_context* ctx, int core, int flags, double fsx, double fsy, doub
   for (int l = 0; l < nlev; ++l) { a.lev_off[l] = lev_off[l]; a.lev_cnt[l] = lev_cnt[l]; }
   a.P = P;
   a.theta = (float)theta;
-  a.lterm = (float)((double)P * std::log2(theta) - 2.0);
+  a.lterm = (float)std::min((double)P * std::log2(theta) - 2.0, -26.0);
   a.finalize = (flags & OBS_FLAG_FINALIZE) ? 1 : 0;
   a.fsx = fsx; a.fsy = fsy;
   a.status = ctx->d_status;

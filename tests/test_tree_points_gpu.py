@@ -25,3 +25,19 @@ def test_nodes_of_radius_zero(ctx, n, unit, coincident):
     og.points_affect_points(b, b, og.VELONLY, env)
     assert np.isfinite(a.u).all() and np.isfinite(a.v).all()
     assert rel_err(b.u, a.u) < TOL and rel_err(b.v, a.v) < TOL
+
+
+@pytest.mark.parametrize("order", [2, 4, 6, 12])
+def test_distant_nodes_keep_their_terms(ctx, order):
+    """A leaf of radius 0.1 with its strength at one end, 0.35 from the targets: P terms leave at most |w|^P / (1 - |w|)
+    of sum |G| / |d|, |w| = 0.1 / 0.35, whatever theta is."""
+    sx = np.concatenate([[-0.1], np.full(31, 0.1)]).astype(np.float32)
+    sy, r = np.zeros(32, np.float32), np.full(32, 1e-3, np.float32)
+    s = np.concatenate([[1e-3], np.full(31, 1.0)]).astype(np.float32)
+    t = og.Points(np.linspace(0.35, 0.3501, 64).astype(np.float32), np.zeros(64, np.float32), np.full(64, 1e-3, np.float32))
+    og.points_affect_points_tree(og.Points(sx, sy, r, s), t, og.ExecEnv(og.CORE_GAUSSIAN, og.COMPENSATED, ctx), theta=0.7,
+                                 order=order)
+    d = t.x.astype(np.float64)[:, None] - sx.astype(np.float64)[None, :]
+    terms, w = s / np.abs(d), 0.1 / 0.35
+    err = np.abs(t.v - (s / d).sum(1))
+    assert np.all(err <= (w ** order / (1 - w) + 2e-6) * terms.sum(1))     # 2e-6: FP32, as TOL
