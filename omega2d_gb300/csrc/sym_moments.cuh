@@ -74,7 +74,9 @@ __device__ __forceinline__ float2 nfma2(float2 a, float2 b, float2 c) {   // c -
 
 // one group against the warp's rows; FORM as sym_core's; csum: the warp's sums of the columns, as in sym_group
 // (velocity, X, Y and the dL/dG term as the row sees them: the reduction turns the signs)
-template <class OP, int FORM, bool COMP>
+// OWN: columns of the rows' own block; the VJP's weights are then formed with both products rounded, so that a particle
+// with itself (and any with equal strength and cotangent) has none.
+template <class OP, int FORM, bool COMP, bool OWN>
 __device__ __forceinline__ void mom_group(const MomGroup<OP::VJP>& grp, int lane, float us2, float ucf,
                                           const float2 (&nx)[OP::NP], const float2 (&ny)[OP::NP], const MomW (&w)[OP::NP],
                                           const float* __restrict__ zrow, float2 (&acc)[OP::NP][OP::NF + OP::NN],
@@ -134,7 +136,16 @@ __device__ __forceinline__ void mom_group(const MomGroup<OP::VJP>& grp, int lane
         }
         if constexpr (OP::VJP) {
           // -wu and wv from the row's negated strength (w.g here)
-          const float2 mwu = __ffma2_rn(w[p].g, cmlu, mul2(cg, w[p].mlu)), wv = __ffma2_rn(w[p].g, clv, mul2(cg, w[p].lv));
+          const float2 gu = mul2(cg, w[p].mlu), gv = mul2(cg, w[p].lv);
+          float2 mwu, wv;
+          if constexpr (OWN) {
+            const float2 g = mul2(w[p].g, f2(-1.0f, -1.0f));
+            mwu = nfma2(g, cmlu, gu);
+            wv = nfma2(g, clv, gv);
+          } else {
+            mwu = __ffma2_rn(w[p].g, cmlu, gu);
+            wv = __ffma2_rn(w[p].g, clv, gv);
+          }
           float2 X, Y;                               // halved and negated
           if constexpr (FAR) {
             const float2 b = mul2(k, dy), n = __ffma2_rn(b, b, mul2(k, mhalf)), h = mul2(mul2(k, dx), b);
@@ -326,12 +337,14 @@ __global__ void __launch_bounds__(SYM_THREADS, 4) sym_moments_kernel(const MomAr
             const float ey = fmaxf(0.0f, fmaxf(by0 - c.z, c.z - by1));
             near = __any_sync(0xffffffffu, !(fmaf(ex, ex, ey * ey) > lim));   // a NaN coordinate is near
           }
-          if (!near) {
-            mom_group<OP, 0, COMP>(grp, lane, us2, ucf, nx, ny, w, zrow + tid, acc, cw, &nsum[0][0][tid]);
-          } else {
-            if (unif) mom_group<OP, 1, COMP>(grp, lane, us2, ucf, nx, ny, w, zrow + tid, acc, cw, &nsum[0][0][tid]);
-            else mom_group<OP, 2, COMP>(grp, lane, us2, ucf, nx, ny, w, zrow + tid, acc, cw, &nsum[0][0][tid]);
-          }
+          auto run = [&](auto own) {
+            constexpr bool OWN = OP::VJP && decltype(own)::value;
+            if (!near) mom_group<OP, 0, COMP, false>(grp, lane, us2, ucf, nx, ny, w, zrow + tid, acc, cw, &nsum[0][0][tid]);
+            else if (unif) mom_group<OP, 1, COMP, OWN>(grp, lane, us2, ucf, nx, ny, w, zrow + tid, acc, cw, &nsum[0][0][tid]);
+            else mom_group<OP, 2, COMP, OWN>(grp, lane, us2, ucf, nx, ny, w, zrow + tid, acc, cw, &nsum[0][0][tid]);
+          };
+          if (OP::VJP && g0 + t * MOM_TG + b < gdiag) run(std::true_type{});
+          else run(std::false_type{});
           if (COMP || b == cnt - 1) {              // plain sums fold once per tile
 #pragma unroll
             for (int p = 0; p < NP; ++p)

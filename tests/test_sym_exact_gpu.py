@@ -56,3 +56,17 @@ def test_vjp_columns_are_exact(ctx, seed):
     want = -2.0 * total / (2.0 * np.pi)
     for got in (gx, gy):
         assert np.all(np.abs(got[n - block:] - want) <= 2.0 ** -23 * abs(want))     # one FP32 rounding of the result
+
+
+@pytest.mark.parametrize("accum", [og.COMPENSATED, og.PLAIN_F32])
+def test_vjp_of_a_particle_with_itself_is_none(ctx, restatement, accum):
+    """Particles a million radii apart: the core at distance 0 is 1e14 times as large as between them, so anything left
+    of a particle's weight with itself would be all there is."""
+    n = 12_001
+    rng = np.random.default_rng(n)
+    x, y = (1e6 * rng.uniform(-1, 1, (2, n))).astype(np.float32)
+    r, s = np.full(n, 0.02, np.float32), rng.normal(0, 1, n).astype(np.float32)
+    lu, lv = rng.normal(0, 1, (2, n)).astype(np.float32)
+    got = og.points_affect_points_vjp_self(og.Points(x, y, r, s), lu, lv, og.ExecEnv(og.CORE_GAUSSIAN, accum, ctx))
+    for a, b in zip(restatement.self_vjp(og.CORE_GAUSSIAN, x, y, r, s, lu, lv), got):
+        assert np.max(np.abs(a - b)) < (2e-5 if accum == og.COMPENSATED else 1e-4) * np.max(np.abs(a))   # as test_sym_gpu.py
