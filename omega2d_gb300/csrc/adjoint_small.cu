@@ -1,5 +1,7 @@
 // adjoint_small.cu -- VJP gathers of small sets in one launch: the sums of adjoint.cu, organised like
 // p2p_small.cu with four owners per block, every pair with its own radii.
+#include <cfloat>
+
 #include "adjoint.h"
 #include "obs_context.h"
 #include "p2p_kernel.cuh"
@@ -34,6 +36,8 @@ __global__ void __launch_bounds__(SML_THREADS) adj_small_kernel(const SmallAdjAr
     ox[t] = a.ox[i];
     oy[t] = a.oy[i];
     oz[t] = a.orad ? radius_term(CORE, a.orad[i]) : 0.0f;
+    // a radius of 0 would make the Gaussian's derivative 1/s^2 times e^-x = inf times 0 at any distance
+    if (CORE == CORE_GAUSS && oz[t] == 0.0f) oz[t] = FLT_MIN;
     og[t] = SELF ? a.og[i] : 0.0f;
     olu[t] = SELF ? a.elu[i] : 0.0f;
     olv[t] = SELF ? a.elv[i] : 0.0f;
@@ -108,8 +112,9 @@ void adj_core(bool self, bool thick, bool comp, const SmallAdjArgs& a, int grid,
 // Where one launch beats the tiled gathers (compensated, this / those, us).  A block walks all the elements for its
 // four owners, so few owners with many elements leave most of the chip idle, where the tiled gathers split the
 // elements; and many owners with few elements end in one block sum for every four.
-//   Gaussian: 1 owner x 32,768 57 / 92, x 100,000 164 / 115; 8 owners x 20,000 37 / 103, x 100,000 161 / 221, x 300,000 475 / 341, x 1,000,000 1566 / 1001;
-//     26,000 owners x 1,000 66 / 67, 32,768 x 1,000 81 / 72, x 3,000 147 / 163; self 3,000 40 / 211, 9,000 175 / 246.
+//   Gaussian: 1 owner x 32,768 57 / 92, x 100,000 164 / 115; 8 owners x 20,000 37 / 103, x 100,000 161 / 221, x
+//     300,000 475 / 341, x 1,000,000 1566 / 1001; 26,000 owners x 1,000 66 / 67, 32,768 x 1,000 81 / 72, x 3,000
+//     147 / 163; self 3,000 40 / 211, 9,000 175 / 246.
 //   Vatistas-2 (cheaper pairs): 8 x 32,768 65 / 85, x 100,000 190 / 116, x 1,000,000 1850 / 523; 2,000 x 20,000
 //     82 / 90, x 32,768 134 / 127; 4,000 x 20,000 123 / 118; 14,000 x 1,800 43 / 45, 18,000 x 200 32 / 29, 26,000 x
 //     1,000 58 / 44, 32,768 x 200 56 / 31; self 9,000 128 / 153.

@@ -1,6 +1,7 @@
 // p2p_small_res.cu -- velocity with gradient, vorticity or shear of small sets in one launch: the
 // organisation of p2p_small.cu with four targets per block and the pair forms of p2p_kernel.cuh
 // (kernelug / kerneluw / kernelue, src/Kernels.h:112-231), every pair with its own radii.
+#include <cfloat>
 #include <cstring>
 
 #include "obs_context.h"
@@ -52,7 +53,9 @@ __global__ void __launch_bounds__(SML_THREADS) p2p_small_res_kernel(const SmallR
       k = 0;
     }
     const float x = a.sx[j], y = a.sy[j], g = a.ss[j];
-    const float z = a.sr ? radius_term(CORE, a.sr[j]) : 0.0f;
+    float z = a.sr ? radius_term(CORE, a.sr[j]) : 0.0f;
+    // a radius of 0 would make the Gaussian's derivative 1/s^2 times e^-x = inf times 0 at any distance
+    if (CORE == CORE_GAUSS && z == 0.0f) z = FLT_MIN;
 #pragma unroll
     for (int t = 0; t < SMR_T; ++t) {
       const float ndx = x - tx[t], ndy = y - ty[t];
