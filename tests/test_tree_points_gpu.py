@@ -41,3 +41,13 @@ def test_distant_nodes_keep_their_terms(ctx, order):
     terms, w = s / np.abs(d), 0.1 / 0.35
     err = np.abs(t.v - (s / d).sum(1))
     assert np.all(err <= (w ** order / (1 - w) + 2e-6) * terms.sum(1))     # 2e-6: FP32, as TOL
+
+
+def test_node_strengths_cancel(ctx):
+    """Four leaves at one point whose strengths add up to 2^24, 1, -2^24 and 0: their node has strength 1."""
+    s = np.concatenate([np.full(32, 2.0 ** 19), [1.0], np.zeros(31), np.full(32, -2.0 ** 19), np.zeros(32)]).astype(np.float32)
+    z, r = np.zeros(128, np.float32), np.full(128, 1e-3, np.float32)
+    d = np.linspace(1.0, 1.001, 64).astype(np.float32)
+    t = og.Points(d, np.zeros(64, np.float32), np.full(64, 1e-3, np.float32))
+    og.points_affect_points_tree(og.Points(z, z, r, s), t, og.ExecEnv(og.CORE_GAUSSIAN, og.COMPENSATED, ctx))
+    assert np.all(np.abs(t.v * d - 1.0) < 2e-6) and np.all(np.abs(t.u) < 2e-6)
