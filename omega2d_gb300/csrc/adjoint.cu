@@ -252,7 +252,6 @@ __global__ void adj_reduce_kernel(const AdjArgs a) {
 #pragma unroll
   for (int q = 0; q < ADJ_NC; ++q) {
     double s = 0.0;
-#pragma unroll 8
     for (int k = 0; k < a.nsplit; ++k) s += p[((size_t)q * a.nsplit + k) * a.no + i];
     c[q] = s;
   }

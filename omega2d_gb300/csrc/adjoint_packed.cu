@@ -478,8 +478,9 @@ cudaError_t pa_dispatch(int mode, bool thick, bool comp, const PAArgs* a, int gr
 size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 // Tiles per split of nob owner blocks over nst element tiles: splits of four tiles or more, but down to one tile
-// where the blocks would not fill the slots and the longest chain of tiles that a slot works off gets shorter (four
-// blocks an SM wait on latency: a tile takes as long with one of them).  80,590 sources x 812 probes 254 -> 117 us,
+// where the blocks would not fill the slots and the longest chain of tiles that a slot works off gets no longer (four
+// blocks an SM wait on latency: a tile takes as long with one of them; as long a chain of single tiles only adds
+// the reduction).  80,590 sources x 812 probes 254 -> 117 us,
 // 40,000 x 600 165 -> 68, 33,000 x 3,200 217 -> 159; but 100,000 x 1,500 203 us with three splits and 249 with four,
 // some of whose blocks make a second wave, 26,000 x 4,500 204 and 237.
 int split_tiles(int nob, int nst, int nsplit, int slots) {
@@ -495,7 +496,8 @@ int split_tiles(int nob, int nst, int nsplit, int slots) {
     if (nob > room) return (q + 1) * t + (int)((nob - room + slots - 1) / slots) * last;
     return std::max(r ? (q + 1) * t : 0, q * t + up(nob, slots - r) * last);
   };
-  return fill < tps && chain(fill) < chain(tps) ? fill : tps;
+  const int more = fill < tps ? chain(tps) - chain(fill) : -1;
+  return more > 0 || (more == 0 && fill > 1) ? fill : tps;
 }
 
 }  // namespace

@@ -113,16 +113,16 @@ void adj_core(bool self, bool thick, bool comp, const SmallAdjArgs& a, int grid,
 // four owners, so few owners with many elements leave most of the chip idle, where the tiled gathers split the
 // elements; and many owners with few elements end in one block sum for every four.
 //   Gaussian: 1 owner x 32,768 57 / 92, x 100,000 164 / 115; 8 owners x 20,000 37 / 103, x 100,000 161 / 221, x
-//     300,000 475 / 341, x 1,000,000 1566 / 1001; 26,000 owners x 1,000 66 / 67, 32,768 x 1,000 81 / 72, x 3,000
-//     147 / 163; self 3,000 40 / 211, 9,000 175 / 246.
+//     300,000 475 / 341, x 1,000,000 1566 / 1001; 26,000 owners x 1,000 66 / 67, 30,000 x 400 58 / 62, 32,768 x
+//     1,000 81 / 72, x 3,000 147 / 163; self 3,000 40 / 211, 9,000 175 / 246.
 //   Vatistas-2 (cheaper pairs): 8 x 32,768 65 / 85, x 100,000 190 / 116, x 1,000,000 1850 / 523; 2,000 x 20,000
-//     82 / 90, x 32,768 134 / 127; 4,000 x 20,000 123 / 118; 14,000 x 1,800 43 / 45, 18,000 x 200 32 / 29, 26,000 x
-//     1,000 58 / 44, 32,768 x 200 56 / 31; self 9,000 128 / 153.
+//     82 / 90, x 32,768 134 / 127; 4,000 x 20,000 123 / 118; 14,000 x 1,800 43 / 45, 18,000 x 200 32 / 29, 20,000 x
+//     1,500 51.7 / 53.6, 26,000 x 1,000 58 / 44, 32,768 x 200 56 / 31; self 9,000 128 / 153.
 bool adjoint_small_applies(const obs_context* ctx, int core, int no, int ne) {
   if (ctx->kernel_variant != OBS_VARIANT_AUTO || ctx->target_order != OBS_ORDER_AUTO) return false;
   const double pairs = (double)no * ne;
-  if (core == CORE_GAUSS) return pairs <= 1.0e8 && ne <= (no < 4 ? 65536 : 131072) && no <= (ne < 1200 ? 28000 : 32768);
-  return no <= 16384 && (ne <= 16384 ? pairs <= 1.0e8 : ne <= 40960 && pairs <= 6.0e7);
+  if (core == CORE_GAUSS) return pairs <= 1.0e8 && ne <= (no < 4 ? 65536 : 131072) && no <= (ne < 1200 ? 30720 : 32768);
+  return no <= (ne < 1200 ? 16384 : 20480) && (ne <= 16384 ? pairs <= 1.0e8 : ne <= 40960 && pairs <= 6.0e7);
 }
 
 int run_adjoint_small(obs_context* ctx, int core, int accum, int mode, int no, const float* ox, const float* oy,

@@ -13,7 +13,9 @@
 // that moved are searched again.  The listed exact evaluations are the only FP64 work (this GPU
 // issues about 2 FP64 lane-operations per SM-clock), and they run 32 points at a time.
 // 200,000 points against 2048 panels: 0.16 ms (the call 0.23 ms), with the panels in random order
-// 1.25 ms; one thread per point against every panel took 3.9 ms in either order.  It is bound by
+// 1.25 ms; one thread per point against every panel took 3.9 ms in either order, and more than this with few
+// panels too (the call, 3, 32 and 256 panels: 200,000 points 147, 157 and 165 us instead of 381, 612 and 959; 1,000
+// points 71, 82 and 80 instead of 96, 160 and 301).  It is bound by
 // instruction issue (0.6 per clock and scheduler, about 500 warp instructions a point) and, at
 // 38 %, FP64.  The removed circulation is summed in FP64 in a
 // fixed order: per warp, per block, and over the blocks by the last one to finish.  clear_inner.cuh

@@ -123,9 +123,9 @@ cudaError_t sym_dispatch(int core, bool comp, const SymArgs& a, const P2PArgs& o
 }
 
 // Row pairs per thread: eight pass a column's sums on half as often per pair as four, but their row
-// blocks are twice as large (8 vs 4: 20,000 Rosenhead-Moore, ten steps 1220 vs 1204 us; 33,001
-// Vatistas-2 with varying radii 284 vs 306 us; 131,072 plain 3.23 vs 3.49 ms; 400,000 Gaussian 29.8 vs
-// 31.2; the 1M patch 182 vs 194; 200,000 with varying Gaussian radii 13.2 vs 12.9)
+// blocks are twice as large (8 vs 4: 20,000 Rosenhead-Moore, ten steps 1220 vs 1204 us; 30,000 Gaussian 297 vs 300,
+// Vatistas-2 225 vs 231, with varying radii 237 vs 254; 33,001 of those 284 vs 306; 131,072 plain 3.23 vs 3.49 ms;
+// 400,000 Gaussian 29.8 vs 31.2; the 1M patch 182 vs 194; 200,000 with varying Gaussian radii 13.2 vs 12.9)
 int sym_np(int n) { return n >= 30000 ? 8 : 4; }
 
 constexpr int SYM_LEAST = 32;                         // units of a range (4, 8 or 16: 0 to 8 % slower up to 80,000)
@@ -133,12 +133,11 @@ constexpr size_t SYM_COL_BYTES = (size_t)1 << 30;     // column partials held at
 
 }  // namespace
 
-// One set as sources and targets (the same arrays) with two-radius cores: every size.  Measured
-// against the one-sided kernels (compensated, uniform clouds, calls back to back): 300 particles
-// 31 vs 48 us (both at the host's rate of issue), 1,200 31 vs 63, 7,000 52 vs 55 (its least
-// gain: hardly more units than CTA slots), 20,000 Rosenhead-Moore 114 vs 163, 65,536 Vatistas-2
-// 962 vs 1216, with varying radii 987 vs 1475; the 1M Gaussian patch 195 vs 249 ms.  An order or
-// kernel variant asked for by name keeps the one-sided kernels.
+// One set as sources and targets (the same arrays) with two-radius cores, from 6,709 particles (smaller sets take
+// p2p_small.cu).  Measured against the one-sided kernels (compensated, calls back to back): 8,000 Vatistas-2 43 vs 58
+// us, 10,000 Gaussian 61 vs 100, 20,000 Rosenhead-Moore 113 vs 164, 60,000 Vatistas-2 753 vs 1042, with varying radii
+// 795 vs 1220; the 1M Gaussian patch 185.4 vs 249 ms.  Its least gain is the Gaussian's at 60,000, 1017 vs 1002 us
+// plain, 1040 vs 1085 compensated.  An order or kernel variant asked for by name keeps the one-sided kernels.
 bool p2p_sym_applies(const obs_context* ctx, const P2PRequest& rq) {
   if (rq.result != RES_VEL || ctx->kernel_variant != OBS_VARIANT_AUTO || ctx->target_order != OBS_ORDER_AUTO) return false;
   if (rq.ns != rq.nt || rq.sx != rq.tx || rq.sy != rq.ty) return false;
