@@ -128,7 +128,10 @@ cudaError_t sym_dispatch(int core, bool comp, const SymArgs& a, const P2PArgs& o
 // 400,000 Gaussian 29.8 vs 31.2; the 1M patch 182 vs 194; 200,000 with varying Gaussian radii 13.2 vs 12.9)
 int sym_np(int n) { return n >= 30000 ? 8 : 4; }
 
-constexpr int SYM_LEAST = 32;                         // units of a range (4, 8 or 16: 0 to 8 % slower up to 80,000)
+// Units of a range (4, 8 or 16: 0 to 8 % slower up to 80,000 particles).  Sixteen ranges a CTA, not eight, balance the
+// cores whose units differ from 256 units a CTA on (131,072 Gaussian 3568 -> 3464 us, 178,513 6514 -> 6269), the others
+// from 1024 on (131,072 Vatistas-2 would take 3475, not 3411): their row partials are written and read twice as often.
+constexpr int SYM_LEAST = 32;
 constexpr size_t SYM_COL_BYTES = (size_t)1 << 30;     // column partials held at once
 
 }  // namespace
@@ -157,10 +160,12 @@ int run_p2p_sym(obs_context* ctx, const P2PRequest& rq) {
   // The near form costs little more here (MUFU under the register reads), so the sort (nine launches, 60 us)
   // pays late (Gaussian, binned vs not): 20,000 173-187 vs 155 us, 40,000 458-507 vs 469-483, 60,000
   // 982-1068 vs 995-1028
-  const bool binned = (rq.core == CORE_GAUSS || rq.core == CORE_CEXP) && (double)n * n >= 4e9;
+  const bool masked = rq.core == CORE_GAUSS || rq.core == CORE_CEXP;
+  const bool binned = masked && (double)n * n >= 4e9;
   SymArgs a;
   std::memset(&a, 0, sizeof(a));
   a.n = n; a.npad = npad; a.ngrp = ngrp; a.gpb = sym_gpb(np); a.least = SYM_LEAST;
+  a.many = masked ? 8 * SYM_LEAST : 32 * SYM_LEAST;
   const size_t col = comp ? sizeof(float4) : sizeof(float2);
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t o_pts = 256, o_run = o_pts + (size_t)(npad / SYM_GRP) * sizeof(SymGroup);

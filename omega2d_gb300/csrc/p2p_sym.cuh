@@ -67,6 +67,7 @@ struct SymArgs {
   int total;             // (block, group) units of this pass
   int nrange;
   int least;             // units of a range, where a CTA gets several
+  int many;              // units of a CTA from which it gets sixteen ranges
   int* counter;
   const unsigned* meta;  // radius extrema (~min, max bits)
   int* status;
@@ -120,7 +121,7 @@ inline void sym_plan_pass(SymArgs& a, int slots) {
   a.total = a.nblk * (a.ngrp - a.gpb * a.blk0) - (a.gpb / 2) * a.nblk * (a.nblk - 1);
   // one range per resident CTA for small sets; up to sixteen (a.least units or more each) for large
   // ones, whose units differ in cost (near and far column groups; eight: the 1M patch takes 186.8 instead of 185.5 ms)
-  const int per = a.total / slots, ranges = slots * (per < 2 * a.least ? 1 : per >= 1024 ? 16 : per >= 8 * a.least ? 8 : per / a.least);
+  const int per = a.total / slots, ranges = slots * (per < 2 * a.least ? 1 : per >= a.many ? 16 : per >= 8 * a.least ? 8 : per / a.least);
   a.nrange = a.total < ranges ? a.total : ranges;
 }
 

@@ -147,6 +147,7 @@ int run_moments(obs_context* ctx, bool comp, int n, const float* x, const float*
   MomArgs m;
   std::memset(&m, 0, sizeof(m));
   m.s.n = n; m.s.npad = npad; m.s.ngrp = ngrp; m.s.gpb = mom_gpb<OP>(); m.s.least = binned ? 2 : 32;
+  m.s.many = 1024;
   const size_t col = NC * (comp ? sizeof(float2) : sizeof(float));
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t o_grp = off + 256, o_run = o_grp + (size_t)(npad / SYM_GRP) * sizeof(Group);
