@@ -109,9 +109,9 @@ int obs_set_kernel_variant(obs_context* ctx, int variant);
  *   BINNED_TARGETS : binned targets; results are bit-identical to INPUT;
  *   BINNED         : binned targets and sources; sources are summed in the binned order, so
  *                    results differ from INPUT by rounding only (and are reproducible);
- *   AUTO           : BINNED where the sort pays (from about 6e8 pairs, 4e9 for the velocity of one set
- *                    on itself, 2.8e8 for its other results, 3e8 for the compact exponential at other
- *                    points), else INPUT. */
+ *   AUTO           : BINNED where the sort pays (the velocity from about 6e8 pairs, 3e8 for the compact
+ *                    exponential, 4e9 of one set on itself; the other results from 2e8, 2.8e8 of one
+ *                    set on itself), else INPUT. */
 #define OBS_ORDER_AUTO 0
 #define OBS_ORDER_INPUT 1
 #define OBS_ORDER_BINNED 2

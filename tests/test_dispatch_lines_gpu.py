@@ -64,3 +64,28 @@ def test_one_launch_sums_past_a_wave(ctx, restatement, core, res, ns, nt, small)
     k = np.r_[:16, nt - 16:nt]
     u, v, _ = restatement.points_affect_points(core, 1, x, y, r, s, tx[k], ty[k], None, fp64=True)
     assert rel_err(u, t.u[k]) < 2e-6 and rel_err(v, t.v[k]) < 2e-6
+
+
+# the spatial order's lines in pairs and in targets, from just below
+@pytest.mark.parametrize("core", [og.CORE_GAUSSIAN, og.CORE_COMPACT_EXP])
+@pytest.mark.parametrize("accum,tol", [(og.COMPENSATED, 2e-6), (og.PLAIN_F32, 2e-5)])
+@pytest.mark.parametrize("res", [og.VELANDGRAD, og.VELANDVORT, og.VELANDSHEAR])
+@pytest.mark.parametrize("ns,nt,order", [(14_142, 14_142, False), (14_143, 14_143, True), (60_000, 3999, False),
+                                         (60_000, 4000, True)])
+def test_results_of_two_sets_about_the_spatial_order(ctx, core, accum, tol, res, ns, nt, order):
+    x, y, r, s = points(ns, ns)
+    tx, ty, _, _ = points(nt, nt + 1)
+    outs, launches = [], []
+    try:
+        for by_name in (og.ORDER_INPUT, og.ORDER_AUTO):
+            ctx.set_target_order(by_name)
+            t = og.Points(tx, ty)
+            before = ctx.launches
+            og.points_affect_points(og.Points(x, y, r, s), t, res, og.ExecEnv(core, accum, ctx))
+            launches.append(ctx.launches - before)
+            outs.append([t.u, t.v] + [a for a in (t.vort, t.shear) if a is not None] + list(t.grad or []))
+    finally:
+        ctx.set_target_order(og.ORDER_AUTO)
+    assert (launches[1] > launches[0]) == order
+    for a, b in zip(*outs):
+        assert rel_err(a, b) < tol
