@@ -99,14 +99,16 @@ void small_launch(bool thick, bool comp, const SmallArgs& a, const P2PArgs& o, i
 // Field points, against the packed kernels: 1,000 x 1,000 26 -> 48-65, 16,000 x 4,000 49-62 ->
 // 73-99, 16,000 x 6,000 64-82 -> 71-97, 16,000 x 10,000 99-129 -> 87-120, 30,000 x 1,000 45-58 ->
 // 50-67, 65,536 x 200 80-107 -> 52-69 (too few blocks), 2,000 x 50,000 82-103 -> 80-107 and
-// 500 x 200,000 197 -> 74 (a block's reduction outweighs its sources).  Two blocks run per SM; past the first
-// wave of them a block's walk counts twice or more: 18,000 x 3,000 60 -> 76, 22,000 x 3,000 82 -> 76, 26,000 x 2,432
-// 47 -> 69 but x 2,433 81 -> 69, 32,768 x 3,000 106 -> 83 (Vatistas-2 78 -> 60).
+// 500 x 200,000 197 -> 74 (a block's reduction outweighs its sources).  Two compensated blocks run
+// per SM; past the first wave of them a block's walk counts twice or more: 18,000 x 3,000 60 -> 76, 22,000 x 3,000
+// 82 -> 76, 26,000 x 2,432 47 -> 69 but x 2,433 81 -> 69, 32,768 x 3,000 106 -> 83 (Vatistas-2 78 -> 60).  Plain sums
+// have three or four blocks per SM and stay ahead up to the limit of pairs (Vatistas-2 30,000 x 2,500 50 -> 57).
 bool p2p_small_applies(const obs_context* ctx, const P2PRequest& rq) {
   if (rq.result != RES_VEL || ctx->kernel_variant != OBS_VARIANT_AUTO || ctx->target_order != OBS_ORDER_AUTO) return false;
   const double pairs = (double)rq.ns * rq.nt;
   if (p2p_sym_applies(ctx, rq)) return pairs <= 4.5e7;
-  return pairs <= 9.0e7 && rq.ns <= (rq.nt <= 2 * SML_T * ctx->num_sms ? 32768 : 20000) && rq.nt <= 20480;
+  const bool one_wave = rq.accum != OBS_COMPENSATED || rq.nt <= 2 * SML_T * ctx->num_sms;
+  return pairs <= 9.0e7 && rq.ns <= (one_wave ? 32768 : 20000) && rq.nt <= 20480;
 }
 
 int run_p2p_small(obs_context* ctx, const P2PRequest& rq) {

@@ -112,8 +112,8 @@ void res_core(int res, bool thick, bool comp, const SmallResArgs& a, const P2PAr
 
 // Against the tiled kernels (compensated, this -> those, us): Gaussian gradient 1,000 52 -> 141, 5,000
 // 85 -> 134, 9,000 177 -> 228, shear 9,000 124 -> 202; Vatistas-2 gradient 5,000 68 -> 84, 7,000 99 -> 96,
-// 9,000 137 -> 127.  The gradient's 128 registers leave two blocks per SM, so past the first wave and the second its
-// sources count two and three times (sources x targets): Gaussian 26,000 x 1,800 107 -> 110, 32,768 x 1,217 131 ->
+// 9,000 137 -> 127.  The compensated gradient's 128 registers leave two blocks per SM, so past the first wave and the second
+// its sources count two and three times (sources x targets): Gaussian 26,000 x 1,800 107 -> 110, 32,768 x 1,217 131 ->
 // 119, 18,000 x 3,000 108 -> 120, 22,000 x 2,433 140 -> 119, and 2,000 x 20,000 113 -> 103; Vatistas-2 18,000 x 1,800
 // 62 -> 77, 22,000 x 1,217 78 -> 71, 14,000 x 3,000 63 -> 68, 18,000 x 2,433 92 -> 84, 500 x 9,000 42 -> 50,
 // 1,000 x 20,000 83 -> 60.
@@ -122,7 +122,7 @@ bool p2p_small_res_applies(const obs_context* ctx, const P2PRequest& rq) {
   if (ctx->kernel_variant != OBS_VARIANT_AUTO || ctx->target_order != OBS_ORDER_AUTO) return false;
   const double limit = rq.core == CORE_GAUSS ? 8.2e7 : 4.5e7;
   int most_s = 32768, most_t = 20480;
-  if (rq.result == RES_GRAD) {
+  if (rq.result == RES_GRAD && rq.accum == OBS_COMPENSATED) {
     const int wave = 2 * SMR_T * ctx->num_sms;
     const bool gauss = rq.core == CORE_GAUSS;
     if (rq.nt > wave) most_s = rq.nt <= 2 * wave ? (gauss ? 28000 : 20000) : (gauss ? 20000 : 16384);

@@ -89,3 +89,20 @@ def test_results_of_two_sets_about_the_spatial_order(ctx, core, accum, tol, res,
     assert (launches[1] > launches[0]) == order
     for a, b in zip(*outs):
         assert rel_err(a, b) < tol
+
+
+# plain sums: the one-launch kernels hold more blocks per SM and stay ahead further than the compensated ones
+@pytest.mark.parametrize("core", [og.CORE_GAUSSIAN, og.CORE_V2, og.CORE_RM])
+@pytest.mark.parametrize("res,ns,nt,small", [(og.VELONLY, 32_768, 2700, True), (og.VELONLY, 32_769, 2700, False),
+                                             (og.VELANDGRAD, 32_768, 1373, True), (og.VELANDGRAD, 2197, 20_480, True),
+                                             (og.VELANDGRAD, 2000, 20_481, False)])
+def test_one_launch_plain_sums(ctx, restatement, core, res, ns, nt, small):
+    x, y, r, s = points(ns, ns + nt)
+    tx, ty, _, _ = points(nt, nt)
+    t = og.Points(tx, ty)
+    before = ctx.launches
+    og.points_affect_points(og.Points(x, y, r, s), t, res, og.ExecEnv(core, og.PLAIN_F32, ctx))
+    assert (ctx.launches - before == 1) == small
+    k = np.r_[:16, nt - 16:nt]
+    u, v, _ = restatement.points_affect_points(core, 1, x, y, r, s, tx[k], ty[k], None, fp64=True)
+    assert rel_err(u, t.u[k]) < 2e-5 and rel_err(v, t.v[k]) < 2e-5
