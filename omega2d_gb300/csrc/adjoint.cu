@@ -317,7 +317,7 @@ int run_adjoint(obs_context* ctx, int core, int accum, int mode,
                 const float* elu, const float* elv,
                 float* gx, float* gy, float* gg, size_t off) {
   if (no == 0 || ne == 0) return OBS_OK;
-  if (adjoint_small_applies(ctx, core, no, ne))
+  if (adjoint_small_applies(ctx, core, accum, no, ne))
     return run_adjoint_small(ctx, core, accum, mode, no, ox, oy, orad, og, ne, ex, ey, er, eg, elu, elv, gx, gy, gg);
   if (mode == ADJ_SELF && core == CORE_GAUSS && ctx->kernel_variant == OBS_VARIANT_AUTO &&
       ctx->target_order == OBS_ORDER_AUTO) {

@@ -28,7 +28,7 @@ int run_adjoint_self_sym(obs_context* ctx, int accum, int n, const float* x, con
 
 // Small gathers in one launch (adjoint_small.cu), same arguments and results, every core; run_adjoint
 // asks first.
-bool adjoint_small_applies(const obs_context* ctx, int core, int no, int ne);
+bool adjoint_small_applies(const obs_context* ctx, int core, int accum, int no, int ne);
 int run_adjoint_small(obs_context* ctx, int core, int accum, int mode, int no, const float* ox, const float* oy,
                       const float* orad, const float* og, int ne, const float* ex, const float* ey, const float* er,
                       const float* eg, const float* elu, const float* elv, float* gx, float* gy, float* gg);

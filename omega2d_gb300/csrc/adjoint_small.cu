@@ -118,10 +118,13 @@ void adj_core(bool self, bool thick, bool comp, const SmallAdjArgs& a, int grid,
 //   Vatistas-2 (cheaper pairs): 8 x 32,768 65 / 85, x 100,000 190 / 116, x 1,000,000 1850 / 523; 2,000 x 20,000
 //     82 / 90, x 32,768 134 / 127; 4,000 x 20,000 123 / 118; 14,000 x 1,800 43 / 45, 18,000 x 200 32 / 29, 20,000 x
 //     1,500 51.7 / 53.6, 26,000 x 1,000 58 / 44, 32,768 x 200 56 / 31; self 9,000 128 / 153.
-bool adjoint_small_applies(const obs_context* ctx, int core, int no, int ne) {
+//   Vatistas-2, plain (half the registers): 8 x 50,000 54 / 94, 4,000 x 20,000 70 / 116, 22,000 x 200 31 / 33, x 1,500
+//     46 / 54, 26,000 x 200 35 / 34, 32,768 x 1,000 56 / 52.
+bool adjoint_small_applies(const obs_context* ctx, int core, int accum, int no, int ne) {
   if (ctx->kernel_variant != OBS_VARIANT_AUTO || ctx->target_order != OBS_ORDER_AUTO) return false;
   const double pairs = (double)no * ne;
   if (core == CORE_GAUSS) return pairs <= 1.0e8 && ne <= (no < 4 ? 65536 : 131072) && no <= (ne < 1200 ? 30720 : 32768);
+  if (accum != OBS_COMPENSATED) return pairs <= 1.0e8 && ne <= (no < 4 ? 65536 : 131072) && no <= 24576;
   return no <= (ne < 1200 ? 16384 : 20480) && (ne <= 16384 ? pairs <= 1.0e8 : ne <= 40960 && pairs <= 6.0e7);
 }
 

@@ -106,3 +106,13 @@ def test_one_launch_plain_sums(ctx, restatement, core, res, ns, nt, small):
     k = np.r_[:16, nt - 16:nt]
     u, v, _ = restatement.points_affect_points(core, 1, x, y, r, s, tx[k], ty[k], None, fp64=True)
     assert rel_err(u, t.u[k]) < 2e-5 and rel_err(v, t.v[k]) < 2e-5
+
+
+@pytest.mark.parametrize("core", [og.CORE_GAUSSIAN, og.CORE_V2])
+@pytest.mark.parametrize("no,ne,small", [(8, 131_072, True), (8, 131_073, False), (3, 65_536, True), (3, 65_537, False),
+                                         (24_576, 1500, True), (33_000, 1500, False)])
+def test_one_launch_plain_gathers(ctx, restatement, core, no, ne, small):
+    got, args, launches = probe_vjp(ctx, core, og.PLAIN_F32, no, ne, no + ne)
+    assert (launches == 1) == small
+    for a, b in zip(restatement.probe_vjp(core, *args), got):
+        assert rel_err(a, b) < 1e-4
