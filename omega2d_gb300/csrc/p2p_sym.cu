@@ -128,7 +128,9 @@ cudaError_t sym_dispatch(int core, bool comp, const SymArgs& a, const P2PArgs& o
 // 400,000 Gaussian 29.8 vs 31.2; the 1M patch 182 vs 194; 200,000 with varying Gaussian radii 13.2 vs 12.9)
 int sym_np(int n) { return n >= 30000 ? 8 : 4; }
 
-// Units of a range (4, 8 or 16: 0 to 8 % slower up to 80,000 particles).  Sixteen ranges a CTA, not eight, balance the
+// Units of a range, not sorted or a large Gaussian set (4, 8 or 16: 0 to 8 % slower up to 80,000 particles); four where
+// sorting put near and far units into runs (32 -> 4: Gaussian 36,000 352 -> 347 us, 50,000 682 -> 587, 60,000 954 ->
+// 805, but 64,000 883 -> 905; compact exponential 30,001 354 -> 287, 64,000 1072 -> 961, 100,000 2118 -> 2124).  Sixteen ranges a CTA, not eight, balance the
 // cores whose units differ from 256 units a CTA on (131,072 Gaussian 3568 -> 3464 us, 178,513 6514 -> 6269), the others
 // from 1024 on (131,072 Vatistas-2 would take 3475, not 3411): their row partials are written and read twice as often.
 constexpr int SYM_LEAST = 32;
@@ -139,8 +141,8 @@ constexpr size_t SYM_COL_BYTES = (size_t)1 << 30;     // column partials held at
 // One set as sources and targets (the same arrays) with two-radius cores, from 6,709 particles (smaller sets take
 // p2p_small.cu).  Measured against the one-sided kernels (compensated, calls back to back): 8,000 Vatistas-2 43 vs 58
 // us, 10,000 Gaussian 61 vs 100, 20,000 Rosenhead-Moore 113 vs 164, 60,000 Vatistas-2 753 vs 1042, with varying radii
-// 795 vs 1220; the 1M Gaussian patch 185.4 vs 249 ms.  Its least gain is the Gaussian's at 60,000, 1017 vs 1002 us
-// plain, 1040 vs 1085 compensated.  An order or kernel variant asked for by name keeps the one-sided kernels.
+// 795 vs 1220; the 1M Gaussian patch 185.4 vs 249 ms.  An order or kernel variant asked for by name
+// keeps the one-sided kernels.
 bool p2p_sym_applies(const obs_context* ctx, const P2PRequest& rq) {
   if (rq.result != RES_VEL || ctx->kernel_variant != OBS_VARIANT_AUTO || ctx->target_order != OBS_ORDER_AUTO) return false;
   if (rq.ns != rq.nt || rq.sx != rq.tx || rq.sy != rq.ty) return false;
@@ -157,14 +159,17 @@ int run_p2p_sym(obs_context* ctx, const P2PRequest& rq) {
   const int npad = nblk * rows;
   const int ngrp = (n + SYM_GRP - 1) / SYM_GRP;
   const int slots = sym_occ(np) * ctx->num_sms;
-  // The near form costs little more here (MUFU under the register reads), so the sort (nine launches, 60 us)
-  // pays late (Gaussian, binned vs not): 20,000 173-187 vs 155 us, 40,000 458-507 vs 469-483, 60,000
-  // 982-1068 vs 995-1028
-  const bool masked = rq.core == CORE_GAUSS || rq.core == CORE_CEXP;
-  const bool binned = masked && (double)n * n >= 4e9;
+  // The sort (eight launches, 60 us) pays once its ranges are fine enough to even out near and far units: at four units
+  // a range, compensated with one radius, sorted vs not in us: Gaussian 16,000 110 vs 95, 22,000 166 vs 164, 25,000 192
+  // vs 209, 36,000 347 vs 395, 50,000 587 vs 731, 60,000 805 vs 1033; compact exponential, whose near form costs twice
+  // the Gaussian's, 16,000 126 vs 127, 20,000 160 vs 190, 36,000 377 vs 565, 60,000 859 vs 1491
+  const bool gauss = rq.core == CORE_GAUSS, masked = gauss || rq.core == CORE_CEXP;
+  const double pairs = (double)n * n;
+  const bool binned = masked && pairs >= (gauss ? 6.25e8 : 3.24e8);
   SymArgs a;
   std::memset(&a, 0, sizeof(a));
-  a.n = n; a.npad = npad; a.ngrp = ngrp; a.gpb = sym_gpb(np); a.least = SYM_LEAST;
+  a.n = n; a.npad = npad; a.ngrp = ngrp; a.gpb = sym_gpb(np);
+  a.least = !binned || (gauss && pairs >= 4e9) ? SYM_LEAST : 4;
   a.many = masked ? 8 * SYM_LEAST : 32 * SYM_LEAST;
   const size_t col = comp ? sizeof(float4) : sizeof(float2);
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
