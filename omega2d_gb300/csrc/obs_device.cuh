@@ -68,6 +68,12 @@ __host__ __device__ __forceinline__ float radius_term(int core, float r) {
   return s2;
 }
 
+// The term that no radius of a set exceeds, from the largest of their bit patterns: infinite where a radius is negative
+// or NaN, as the pattern then isn't that of the largest one.
+__device__ __forceinline__ float max_radius_term(int core, unsigned bits) {
+  return bits <= 0x7f800000u ? radius_term(core, __uint_as_float(bits)) : __uint_as_float(0x7f800000u);
+}
+
 // ---------------------------------------------------------------- Gaussian-core series
 // g(x) = (1 - e^-x)/x = sum_{n>=0} (-x)^n/(n+1)!  and  g'(x) = sum_{m>=0} (m+1)(-1)^(m+1) x^m/(m+2)!
 // (Taylor series of the exponential).  Truncated after the x^12 term: for 0 <= x < 1 the

@@ -290,8 +290,11 @@ __global__ void __launch_bounds__(SYM_THREADS, sym_occ(NP)) p2p_sym_kernel(const
   q.us2 = unif ? 2.0f * radius_term(CORE, __uint_as_float(a.meta[1])) : 0.0f;
   q.ucf = __frcp_rn(q.us2);
   q.cfl = -q.ucf * kLog2e;
-  // far when every pair has d^2/s^2 > 16 (Gaussian) or (d/s)^3 > 16 (compact exponential), 1 % margin
-  q.lim = (CORE == CORE_CEXP ? 6.4131f : 16.16f) * q.us2;
+  // far when every pair has d^2/s^2 > 16 (Gaussian) or (d/s)^3 > 16 (compact exponential), 1 % margin, with the largest
+  // radius for both: every pair's own limit lies below, where its core gives the same bits.  Sets of varying radii then
+  // gain from their order too (Gaussian 30,001 in order, radii 0.6 to 1.4 times the mean: 405 us near only, 289 so, 352
+  // unsorted; 131,072 5841 -> 3555)
+  q.lim = (CORE == CORE_CEXP ? 6.4131f : 16.16f) * (unif ? q.us2 : 2.0f * max_radius_term(CORE, a.meta[1]));
 
   uint32_t kt = 0;                                 // tiles consumed: barrier phase
   for (;;) {
@@ -370,12 +373,12 @@ __global__ void __launch_bounds__(SYM_THREADS, sym_occ(NP)) p2p_sym_kernel(const
             const float ex = fmaxf(0.0f, fmaxf(bx0 - c.x, c.x - bx1));
             const float ey = fmaxf(0.0f, fmaxf(by0 - c.z, c.z - by1));
             // a NaN coordinate takes the near form
-            far = unif && __all_sync(0xffffffffu, fmaf(ex, ex, ey * ey) > q.lim);
+            far = __all_sync(0xffffffffu, fmaf(ex, ex, ey * ey) > q.lim);
           }
           auto run = [&](auto cols) {
             constexpr bool COLS = decltype(cols)::value;
-            if (!unif) sym_group<CORE, 2, COLS, COMP, NP>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, csum[warp] + b * SYM_GRP);
-            else if (MASKED && far) sym_group<CORE, MASKED ? 0 : 1, COLS, COMP, NP>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, csum[warp] + b * SYM_GRP);
+            if (MASKED && far) sym_group<CORE, MASKED ? 0 : 1, COLS, COMP, NP>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, csum[warp] + b * SYM_GRP);
+            else if (!unif) sym_group<CORE, 2, COLS, COMP, NP>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, csum[warp] + b * SYM_GRP);
             else sym_group<CORE, 1, COLS, COMP, NP>(grp, lane, q, nx, ny, g, zrow + tid, u, vn, csum[warp] + b * SYM_GRP);
           };
           if (g0 + t * SYM_TG + b < gdiag) run(std::false_type{});
