@@ -138,12 +138,13 @@ int run_moments(obs_context* ctx, bool comp, int n, const float* x, const float*
   const int npad = nblk * ROWS;
   const int ngrp = (n + SYM_GRP - 1) / SYM_GRP;
   const int slots = MOM_OCC * ctx->num_sms;
-  // Binned vs not, us (narrow to wide cores): 15,000 gradient 200-225 vs 232-240, vorticity 145-171 vs 175-183, shear
-  // 154-177 vs 174-181, VJP 201-222 vs 215-224; 11,500 gradient 155-176 vs 149-156, VJP 151-168 vs 137-144; 17,000 every
-  // one of them faster, VJP 237-261 vs 263-272.  Near units of a binned set cost three times the far ones and come
+  // Binned vs not, us (narrow to wide cores): 11,500 gradient 155-176 vs 149-156, VJP 151-168 vs 137-144; 17,000 every
+  // one of them faster, gradient 236 vs 272, vorticity 164 vs 205, shear 175 vs 203, VJP 241 vs 270.  The order brings a
+  // particle's near ones into the same FP32 sums (17,001 of a patch, du/dx 1.0e-7 off FP64 instead of 5.2e-8), so the
+  // line is no lower than the one-sided kernels' 3e8.  Near units of a binned set cost three times the far ones and come
   // together: in ranges of two or more units, not 32, 28,544 take 498-505 us, not 760 (gradient, wide core), 45,000
   // 1029, not 1191
-  const bool binned = (double)n * n >= 2.8e8;
+  const bool binned = (double)n * n >= 3e8;
   MomArgs m;
   std::memset(&m, 0, sizeof(m));
   m.s.n = n; m.s.npad = npad; m.s.ngrp = ngrp; m.s.gpb = mom_gpb<OP>(); m.s.least = binned ? 2 : 32;

@@ -243,7 +243,8 @@ __global__ void __launch_bounds__(SYM_THREADS, 4) sym_moments_kernel(const MomAr
   const bool unif = ~a.meta[0] == a.meta[1];
   const float us2 = unif ? 2.0f * radius_term(CORE_GAUSS, __uint_as_float(a.meta[1])) : 0.0f;
   const float ucf = __frcp_rn(us2);
-  const float lim = 1.01f * OP::FAR * us2;
+  // own radii: with the largest for both, from 25 on, where both forms agree to 4e-10; as in the velocity's kernel
+  const float lim = 1.01f * (unif ? OP::FAR * us2 : 50.0f * max_radius_term(CORE_GAUSS, a.meta[1]));
 
   uint32_t kt = 0;
   for (;;) {
@@ -330,13 +331,10 @@ __global__ void __launch_bounds__(SYM_THREADS, 4) sym_moments_kernel(const MomAr
         for (int b = 0; b < cnt; ++b) {
           const Group& grp = tile[st][b];
           float (*cw)[PLANES * MOM_TILE] = reinterpret_cast<float (*)[PLANES * MOM_TILE]>(&csum[warp][0][b * SYM_GRP]);
-          bool near = true;
-          if (unif) {
-            const float4 c = grp.xy[lane];
-            const float ex = fmaxf(0.0f, fmaxf(bx0 - c.x, c.x - bx1));
-            const float ey = fmaxf(0.0f, fmaxf(by0 - c.z, c.z - by1));
-            near = __any_sync(0xffffffffu, !(fmaf(ex, ex, ey * ey) > lim));   // a NaN coordinate is near
-          }
+          const float4 c = grp.xy[lane];
+          const float ex = fmaxf(0.0f, fmaxf(bx0 - c.x, c.x - bx1));
+          const float ey = fmaxf(0.0f, fmaxf(by0 - c.z, c.z - by1));
+          const bool near = __any_sync(0xffffffffu, !(fmaf(ex, ex, ey * ey) > lim));   // a NaN coordinate is near
           auto run = [&](auto own) {
             constexpr bool OWN = OP::VJP && decltype(own)::value;
             if (!near) mom_group<OP, 0, COMP, false>(grp, lane, us2, ucf, nx, ny, w, zrow + tid, acc, cw, &nsum[0][0][tid]);

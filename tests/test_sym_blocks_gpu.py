@@ -38,10 +38,10 @@ def test_velocity_at_block_edges(ctx, restatement, core, spread, n):
         assert rel_err(1.0 + u / (2 * np.pi), p.u[k]) < tol and rel_err(-0.25 + v / (2 * np.pi), p.v[k]) < tol
 
 
-# sorted from 2.8e8 pairs (eight launches more), in ranges of two units or more
+# sorted from 3e8 pairs (eight launches more), in ranges of two units or more
 @pytest.mark.parametrize("accum,tol", [(og.COMPENSATED, 2e-6), (og.PLAIN_F32, 2e-5)])    # as tests/test_sym_gpu.py
 @pytest.mark.parametrize("res", [og.VELANDGRAD, og.VELANDVORT, og.VELANDSHEAR])
-@pytest.mark.parametrize("n,launches", [(16_733, 3), (16_734, 11), (28_545, 11)])
+@pytest.mark.parametrize("n,launches", [(17_320, 3), (17_321, 11), (28_545, 11)])
 def test_results_about_the_spatial_order(ctx, accum, tol, res, n, launches):
     rng = np.random.default_rng(n)
     x, y = rng.uniform(-1, 1, (2, n)).astype(np.float32)

@@ -1,5 +1,5 @@
 """GPU tests of sets in spatial order whose radii vary: column groups beyond the largest radius' reach take the core's far
-form (csrc/p2p_sym.cuh); against the generic kernels."""
+form (csrc/p2p_sym.cuh, sym_moments.cuh); against the generic kernels."""
 import numpy as np
 import pytest
 
@@ -60,4 +60,26 @@ def test_velocity(ctx, core, n, accum, tol, kind):
         p = og.Points(*points(n, kind, n))
         og.points_affect_points(p, p, og.VELONLY, og.ExecEnv(core, accum, ctx))
         return outputs(p)
+    check(both(ctx, run), tol)
+
+
+@pytest.mark.parametrize("accum,tol", [(og.COMPENSATED, 2e-6), (og.PLAIN_F32, 2e-5)])
+@pytest.mark.parametrize("res", [og.VELANDGRAD, og.VELANDVORT, og.VELANDSHEAR])
+@pytest.mark.parametrize("kind", KINDS)
+def test_results(ctx, res, accum, tol, kind):
+    def run():
+        p = og.Points(*points(17_400, kind, 1))
+        og.points_affect_points(p, p, res, og.ExecEnv(og.CORE_GAUSSIAN, accum, ctx))
+        return outputs(p)
+    check(both(ctx, run), tol)
+
+
+@pytest.mark.parametrize("accum,tol", [(og.COMPENSATED, 1e-5), (og.PLAIN_F32, 1e-4)])
+@pytest.mark.parametrize("kind", KINDS)
+def test_vjp(ctx, accum, tol, kind):
+    lu, lv = np.random.default_rng(4).normal(0, 1, (2, 17_400)).astype(np.float32)
+
+    def run():
+        p = og.Points(*points(17_400, kind, 5))
+        return og.points_affect_points_vjp_self(p, lu, lv, og.ExecEnv(og.CORE_GAUSSIAN, accum, ctx))
     check(both(ctx, run), tol)
