@@ -177,12 +177,12 @@ int run_p2p(obs_context* ctx, const P2PRequest& rq) {
   // Spatial order pays for the sort from ~6e8 pairs (field points, Gaussian, radius 0.01, binned vs
   // not: 20,000 of 40,000 particles 368 vs 401 us, 20,000 of 33,000 333 vs 345, 4,000 of 500,000 788 vs 903, 2,000 of
   // 500,000 515 vs 522, but 5,000 of 100,000 290 vs 274); for the compact exponential's costlier near form from ~3e8.
-  // Gradients, vorticity and shear, whose near form costs three far ones, from ~2e8: 14,000 of 14,000 gradient 216 vs
-  // 282, vorticity 223 vs 251, plain 218-226 vs 241-252; 20,000 of 20,000 324 vs 529; 5,000 of 60,000 345 vs 432; but
-  // 10,000 of 10,000 vorticity 174 vs 160, 2,500 of 100,000 plain vorticity 324 vs 306, 1,000 of 150,000 247 vs 198
+  // Gradients, vorticity and shear, whose near form costs three far ones, from 3e8: 4,100 of 73,000 particles gradient
+  // 325 vs 432, vorticity 299 vs 421; 5,000 of 60,000 342 vs 418, 341 vs 417; 20,000 of 20,000 324 vs 529, 277 vs 459;
+  // 40,000 of 7,500 289 vs 427, 243 vs 351; but of 2e8 pairs 5,000 of 40,000 vorticity 294 vs 256
   const double pairs = (double)rq.ns * rq.nt;
   const bool big = res == RES_VEL ? pairs >= (rq.core == CORE_CEXP ? 3e8 : 6e8) && rq.nt >= 2000 && rq.ns >= 4096
-                                  : pairs >= 2e8 && rq.nt >= 4000 && rq.ns >= 4096;
+                                  : pairs >= (rq.nt >= 4096 ? 3e8 : 7e8) && rq.nt >= 2000 && rq.ns >= 4096;
   const bool bin_t = gauss_packed && (order == OBS_ORDER_BINNED || order == OBS_ORDER_BINNED_TARGETS ||
                                       (order == OBS_ORDER_AUTO && big));
   const bool bin_s = gauss_packed && (order == OBS_ORDER_BINNED || (order == OBS_ORDER_AUTO && big));

@@ -26,7 +26,7 @@ template <> struct PRes<RES_GRAD> { static constexpr int NC = 6, NP = 1; };
 template <> struct PRes<RES_VORT> { static constexpr int NC = 3, NP = 2; };
 template <> struct PRes<RES_SHEAR> { static constexpr int NC = 3, NP = 2; };
 
-// one 32-source block; FAR: every pair has d^2/s^2 > 25 (uniform radii)
+// one 32-source block; FAR: every pair has d^2/s^2 > 25
 template <int RES, bool FAR, bool THICK, bool UNIF, int NP, int NC>
 __device__ __forceinline__ void res_block(const float4* __restrict__ blk, float us2, float ucf,
                                           const float2 (&ntx)[NP], const float2 (&nty)[NP],
@@ -107,7 +107,9 @@ __global__ void __launch_bounds__(P2P_THREADS, 4) p2p_packed_res_kernel(const P2
           (THICK ? radius_term(CORE_GAUSS, __uint_as_float(a.meta[3])) : 0.0f);
     ucf = __frcp_rn(us2);
   }
-  const float lim = 25.25f * us2;                 // far test with a 1 % margin (d > 5.02 s)
+  // far test with a 1 % margin (d > 5.02 s); varying radii: with the largest ones, where both forms agree to 4e-10
+  const float lim = 25.25f * (unif ? us2 : max_radius_term(CORE_GAUSS, a.meta[1]) +
+                                           (THICK ? max_radius_term(CORE_GAUSS, a.meta[3]) : 0.0f));
 
   uint32_t kt = 0;
   for (;;) {
@@ -167,25 +169,20 @@ __global__ void __launch_bounds__(P2P_THREADS, 4) p2p_packed_res_kernel(const P2
         return;
       }
       const float4* tl = &tile[st][0];
-      if (unif) {
 #pragma unroll
-        for (int b = 0; b < PK_NB; ++b) {
-          const float4 A = tl[PK_ELEM * (b * PK_BLK + lane)];
-          const float dx = fmaxf(0.0f, fmaxf(bx0 - A.x, A.x - bx1));
-          const float dy = fmaxf(0.0f, fmaxf(by0 - A.z, A.z - by1));
-          const unsigned m = __ballot_sync(0xffffffffu, fmaf(dx, dx, dy * dy) <= lim);
-          if (lane == 0) smask[warp][b] = m;
-        }
-        __syncwarp();
+      for (int b = 0; b < PK_NB; ++b) {
+        const float4 A = tl[PK_ELEM * (b * PK_BLK + lane)];
+        const float dx = fmaxf(0.0f, fmaxf(bx0 - A.x, A.x - bx1));
+        const float dy = fmaxf(0.0f, fmaxf(by0 - A.z, A.z - by1));
+        const unsigned m = __ballot_sync(0xffffffffu, fmaf(dx, dx, dy * dy) <= lim);
+        if (lane == 0) smask[warp][b] = m;
       }
+      __syncwarp();
       for (int b = 0; b < PK_NB; ++b) {
         const float4* blk = tl + PK_ELEM * b * PK_BLK;
-        if (unif) {
-          if (smask[warp][b] == 0u) res_block<RES, true, THICK, true, NP, NC>(blk, us2, ucf, ntx, nty, tz, acc);
-          else res_block<RES, false, THICK, true, NP, NC>(blk, us2, ucf, ntx, nty, tz, acc);
-        } else {
-          res_block<RES, false, THICK, false, NP, NC>(blk, us2, ucf, ntx, nty, tz, acc);
-        }
+        if (smask[warp][b] == 0u) res_block<RES, true, THICK, true, NP, NC>(blk, us2, ucf, ntx, nty, tz, acc);
+        else if (unif) res_block<RES, false, THICK, true, NP, NC>(blk, us2, ucf, ntx, nty, tz, acc);
+        else res_block<RES, false, THICK, false, NP, NC>(blk, us2, ucf, ntx, nty, tz, acc);
         if constexpr (COMP) {
 #pragma unroll
           for (int c = 0; c < NC; ++c)

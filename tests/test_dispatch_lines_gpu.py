@@ -70,8 +70,8 @@ def test_one_launch_sums_past_a_wave(ctx, restatement, core, res, ns, nt, small)
 @pytest.mark.parametrize("core,sorts", [(og.CORE_GAUSSIAN, True), (og.CORE_COMPACT_EXP, False)])   # as the packed forms
 @pytest.mark.parametrize("accum,tol", [(og.COMPENSATED, 2e-6), (og.PLAIN_F32, 2e-5)])
 @pytest.mark.parametrize("res", [og.VELANDGRAD, og.VELANDVORT, og.VELANDSHEAR])
-@pytest.mark.parametrize("ns,nt,order", [(14_142, 14_142, False), (14_143, 14_143, True), (60_000, 3999, False),
-                                         (60_000, 4000, True)])
+@pytest.mark.parametrize("ns,nt,order", [(17_320, 17_320, False), (17_321, 17_321, True), (80_000, 4095, False),
+                                         (80_000, 4096, True), (200_000, 3499, False), (200_000, 3500, True)])
 def test_results_of_two_sets_about_the_spatial_order(ctx, core, sorts, accum, tol, res, ns, nt, order):
     x, y, r, s = points(ns, ns)
     tx, ty, _, _ = points(nt, nt + 1)

@@ -1,5 +1,5 @@
 """GPU tests of sets in spatial order whose radii vary: column groups beyond the largest radius' reach take the core's far
-form (csrc/p2p_sym.cuh, sym_moments.cuh); against the generic kernels."""
+form (csrc/p2p_sym.cuh, sym_moments.cuh, p2p_packed_res.cu); against the generic kernels."""
 import numpy as np
 import pytest
 
@@ -71,6 +71,20 @@ def test_results(ctx, res, accum, tol, kind):
         p = og.Points(*points(17_400, kind, 1))
         og.points_affect_points(p, p, res, og.ExecEnv(og.CORE_GAUSSIAN, accum, ctx))
         return outputs(p)
+    check(both(ctx, run), tol)
+
+
+@pytest.mark.parametrize("accum,tol", [(og.COMPENSATED, 2e-6), (og.PLAIN_F32, 2e-5)])
+@pytest.mark.parametrize("res", [og.VELANDGRAD, og.VELANDVORT, og.VELANDSHEAR])
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("thick", [False, True])
+def test_results_of_two_sets(ctx, res, accum, tol, kind, thick):
+    def run():
+        s = og.Points(*points(17_400, kind, 2))
+        x, y, r, g = points(17_301, "spread", 3)
+        t = og.Points(x, y, r, g) if thick else og.Points(x, y)
+        og.points_affect_points(s, t, res, og.ExecEnv(og.CORE_GAUSSIAN, accum, ctx))
+        return outputs(t)
     check(both(ctx, run), tol)
 
 
