@@ -110,7 +110,8 @@ int obs_set_kernel_variant(obs_context* ctx, int variant);
  *   BINNED         : binned targets and sources; sources are summed in the binned order, so
  *                    results differ from INPUT by rounding only (and are reproducible);
  *   AUTO           : BINNED where the sort pays (the velocity from about 6e8 pairs, 3e8 for the compact
- *                    exponential; the other results from 3e8), else INPUT. */
+ *                    exponential; the other results from 3e8, the VJPs from 2e8 at probes
+ *                    and 7e8 of one set on itself), else INPUT. */
 #define OBS_ORDER_AUTO 0
 #define OBS_ORDER_INPUT 1
 #define OBS_ORDER_BINNED 2

@@ -141,10 +141,11 @@ int run_moments(obs_context* ctx, bool comp, int n, const float* x, const float*
   // Binned vs not, us (narrow to wide cores): 11,500 gradient 155-176 vs 149-156, VJP 151-168 vs 137-144; 17,000 every
   // one of them faster, gradient 236 vs 272, vorticity 164 vs 205, shear 175 vs 203, VJP 241 vs 270.  The order brings a
   // particle's near ones into the same FP32 sums (17,001 of a patch, du/dx 1.0e-7 off FP64 instead of 5.2e-8), so the
-  // line is no lower than the one-sided kernels' 3e8.  Near units of a binned set cost three times the far ones and come
+  // line is no lower than the one-sided kernels' 3e8; the VJP's is 7e8 (25,000 of a patch, dL/dy 1.40e-7 instead of
+  // 1.29e-7; 437 vs 559 us).  Near units of a binned set cost three times the far ones and come
   // together: in ranges of two or more units, not 32, 28,544 take 498-505 us, not 760 (gradient, wide core), 45,000
   // 1029, not 1191
-  const bool binned = (double)n * n >= 3e8;
+  const bool binned = (double)n * n >= (OP::VJP ? 7e8 : 3e8);
   MomArgs m;
   std::memset(&m, 0, sizeof(m));
   m.s.n = n; m.s.npad = npad; m.s.ngrp = ngrp; m.s.gpb = mom_gpb<OP>(); m.s.least = binned ? 2 : 32;

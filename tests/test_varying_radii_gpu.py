@@ -91,9 +91,9 @@ def test_results_of_two_sets(ctx, res, accum, tol, kind, thick):
 @pytest.mark.parametrize("accum,tol", [(og.COMPENSATED, 1e-5), (og.PLAIN_F32, 1e-4)])
 @pytest.mark.parametrize("kind", KINDS)
 def test_vjp(ctx, accum, tol, kind):
-    lu, lv = np.random.default_rng(4).normal(0, 1, (2, 17_400)).astype(np.float32)
+    lu, lv = np.random.default_rng(4).normal(0, 1, (2, 26_500)).astype(np.float32)
 
     def run():
-        p = og.Points(*points(17_400, kind, 5))
+        p = og.Points(*points(26_500, kind, 5))
         return og.points_affect_points_vjp_self(p, lu, lv, og.ExecEnv(og.CORE_GAUSSIAN, accum, ctx))
     check(both(ctx, run), tol)
